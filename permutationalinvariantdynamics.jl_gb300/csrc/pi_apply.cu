@@ -523,9 +523,11 @@ cudaError_t launch_apply_rhs(const DevicePlan& dp, const void* coef, const void*
 template <typename T>
 cudaError_t launch_apply_fast(const DevicePlan& dp, const void* coef, const void* x, void* y, int ncols,
                               long long ld, const BorderArgs& border, cudaStream_t stream) {
-  if (dp.canon)
-    return dp.canon_plus ? launch_apply_canon<T, true>(dp, coef, x, y, ncols, ld, border, stream)
-                         : launch_apply_canon<T, false>(dp, coef, x, y, ncols, ld, border, stream);
+  if constexpr (sizeof(T) == sizeof(float)) {  // FP64: the strip apply (pi_apply64.cu)
+    if (dp.canon)
+      return dp.canon_plus ? launch_apply_canon<T, true>(dp, coef, x, y, ncols, ld, border, stream)
+                           : launch_apply_canon<T, false>(dp, coef, x, y, ncols, ld, border, stream);
+  }
   switch (dp.fast_sr) {
     case 5: return launch_apply_rhs<T, 2, 2, 5>(dp, coef, x, y, ncols, ld, border, stream);
     case 9: return launch_apply_rhs<T, 2, 2, 9>(dp, coef, x, y, ncols, ld, border, stream);

@@ -1,0 +1,213 @@
+// Coefficient planes of the FP64 strip apply (pi_apply64.cuh) and its launches.
+#include <algorithm>
+#include <vector>
+
+#include "../../include/picuda.h"
+#include "pi_apply64.cuh"
+#include "pi_handle.hpp"
+#include "pi_internal.hpp"
+
+namespace picuda {
+namespace {
+
+// Planes, line tables and strip items of sector blockIdx.y.
+__global__ void k_planes64(const DevSector* __restrict__ sectors, const int4* __restrict__ canon,
+                           const double2* __restrict__ coef, const int2* __restrict__ first, const Planes64 P, int nr,
+                           double* __restrict__ plane, double2* __restrict__ lrow, double2* __restrict__ rcol,
+                           StripItem* __restrict__ items) {
+  const int s = blockIdx.y;
+  const DevSector& sec = sectors[s];
+  const int n = sec.n;
+  const long long cnt = (long long)n * n;
+  const int4* ct = canon + (long long)s * kCanonEntries;
+  // sum of the real products at one sandwich position of the canonical table
+  auto sand = [&](int pos, int a, int b) {
+    double v = 0;
+    for (int t = 0; t < kCanonPerPos; ++t) {
+      const int4 e = ct[5 + pos * kCanonPerPos + t];
+      v = fma(coef[e.x + a].x, coef[e.y + b].x, v);
+    }
+    return v;
+  };
+  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < cnt; i += (long long)gridDim.x * blockDim.x) {
+    const int b = (int)(i / n), a = (int)(i - (long long)b * n);
+    const double2 al = coef[ct[0].x + a], be = coef[ct[0].y + b];
+    double* out = plane + sec.offset + i;
+    out[0] = (al.x + be.x) + sand(4, a, b);  // the own-sector centre gain joins the ADD term
+    out[P.dim] = al.y + be.y;
+    for (int k = 0; k < nr; ++k) {
+      const int src = P.gain[k].src;
+      const int slot = src == 0 ? 1 : src == 1 ? 0 : 2;
+      out[(2 + k) * P.dim] = sand(slot * 3 + P.gain[k].shift + 1, a, b);
+    }
+  }
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; 32LL * i < cnt; i += gridDim.x * blockDim.x) {
+    StripItem it{};
+    it.off = (int)sec.offset;
+    it.n = n;
+    if (sec.src[0] >= 0) it.off0 = (int)sectors[sec.src[0]].offset, it.m0 = sectors[sec.src[0]].n;
+    if (sec.src[2] >= 0) it.off2 = (int)sectors[sec.src[2]].offset, it.m2 = sectors[sec.src[2]].n;
+    it.local0 = 32 * i;
+    it.loff = first[s].x;
+    it.sector = s;
+    items[first[s].y + i] = it;
+  }
+  if (blockIdx.x == 0)
+    for (int i = threadIdx.x; i < n; i += blockDim.x) {
+      lrow[first[s].x + i] = make_double2(coef[ct[1].x + i].y, coef[ct[2].x + i].y);
+      rcol[first[s].x + i] = make_double2(coef[ct[3].y + i].y, coef[ct[4].y + i].y);
+    }
+}
+
+// 128 columns at N = 120 with emission, dephasing and collective decay (22 FP64 instructions
+// per entry, 97% of the FP64 pipe): 1.41 ms = 1.21 TFLOP/s, against 2.34 ms for 32 x 32 tiles
+// with staged windows; one vector at N = 200: 62 us against 125 us (products formed on the way).
+//
+// EPI: scale and trace border; without them their instructions are not in the kernel.
+template <int V, bool EPI>
+__global__ void __launch_bounds__(kStripThreads, 4)
+    k_apply_strip64(const Planes64 P, const DevSector* __restrict__ sectors, int ncols, int rc,
+                    const double2* __restrict__ x, double2* __restrict__ y, long long ld, const double2* alpha,
+                    int coords, double scale) {
+  const int item = blockIdx.x * kStripWarps + (threadIdx.x >> 5);
+  if (item >= P.nitems) return;
+  const StripItem it = P.items[item];
+  StripEntry<V> E;
+  if (!E.load(it, P, threadIdx.x & 31)) return;
+  const int c0 = blockIdx.y * rc, c1 = min(c0 + rc, ncols);
+  x += c0 * ld;
+  y += c0 * ld + E.e;
+#pragma unroll 1
+  for (int c = c0; c < c1; ++c) {
+    double2 out = E.apply(x);
+    if (EPI) {
+      out.x *= scale;
+      out.y *= scale;
+      if (alpha != nullptr && E.diag) {
+        const double v = coords ? sectors[it.sector].border_z : sectors[it.sector].border_x;
+        const double2 al = alpha[c];
+        out.x = fma(al.x, v, out.x);
+        out.y = fma(al.y, v, out.y);
+      }
+    }
+    *y = out;
+    x += ld;
+    y += ld;
+  }
+}
+
+// Lets this thread allocate and wait while another stream of the process is being captured.
+struct RelaxedCapture {
+  cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+  RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+  ~RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+};
+
+}  // namespace
+
+Planes64 planes64(pi_plan* plan, int coords) {
+  const DevicePlan& dp = plan->dev;
+  // 32-bit element indices within a vector
+  if (!dp.canon || dp.dim == 0 || dp.dim > 0x3fffffffLL) return Planes64{};
+  std::lock_guard<std::mutex> lk(plan->em_mu);
+  const int which = coords ? 1 : 0;
+  Planes64& P = plan->planes64[which];
+  if (P.items || plan->planes64_failed[which]) return P;
+  RelaxedCapture relaxed;
+  const int S = (int)plan->host.sectors.size();
+  std::vector<int2> first(S);  // per sector: first line, first strip item
+  int lines = 0, nitems = 0;
+  for (int s = 0; s < S; ++s) {
+    const int n = plan->host.sectors[s].n;
+    first[s] = make_int2(lines, nitems);
+    lines += n;
+    nitems += (n * n + 31) / 32;
+  }
+  // gain positions that some sector uses, in the order of the canonical kernels: own, smaller,
+  // larger sector
+  bool drive = false, used[3][3] = {};
+  for (const Sector& sec : plan->host.sectors)
+    for (const StencilTerm& t : sec.terms) {
+      drive = drive || t.kind == ST_LEFT || t.kind == ST_RIGHT;
+      if (t.kind == ST_SAND) used[t.e == 0 ? 0 : t.e < 0 ? 1 : 2][t.p + 1] = true;
+    }
+  used[0][1] = false;  // joins the centre
+  Planes64 Q;
+  Q.dim = dp.dim;
+  Q.nitems = nitems;
+  for (GainPos& g : Q.gain) g = GainPos{-1, 0};
+  int nr = 0;
+  for (int src = 0; src < 3; ++src)
+    for (int p = -1; p <= 1; ++p)
+      if (used[src][p + 1]) Q.gain[nr++] = GainPos{(signed char)src, (signed char)p};
+  Q.variant = drive ? (nr <= 1 ? 0 : nr <= 3 ? 1 : nr <= 5 ? 2 : nr <= 6 ? 3 : 4) : (nr <= 5 ? 5 : 6);
+  const int np = 2 + nr;
+  // one allocation: records, line tables, planes, per-sector starts
+  const size_t item_bytes = sizeof(StripItem) * (size_t)nitems, line_bytes = sizeof(double2) * (size_t)lines;
+  const size_t plane_bytes = (sizeof(double) * (size_t)dp.dim * np + 15) / 16 * 16;
+  const size_t bytes = item_bytes + 2 * line_bytes + plane_bytes + sizeof(int2) * (size_t)S;
+  char* d = nullptr;
+  cudaError_t e = cudaMalloc((void**)&d, bytes);
+  if (e == cudaSuccess) {
+    char* d_l = d + item_bytes;
+    char* d_plane = d_l + 2 * line_bytes;
+    char* d_first = d_plane + plane_bytes;
+    e = cudaMemcpyAsync(d_first, first.data(), sizeof(int2) * (size_t)S, cudaMemcpyHostToDevice, plan->stream);
+    if (e == cudaSuccess) {
+      const dim3 grid((unsigned)std::min<long long>(64, ((long long)plan->host.max_n * plan->host.max_n + 255) / 256),
+                      (unsigned)S);
+      k_planes64<<<grid, 256, 0, plan->stream>>>(dp.sectors, dp.canon, coords ? dp.coef64z : dp.coef64,
+                                                 (const int2*)d_first, Q, nr, (double*)d_plane, (double2*)d_l,
+                                                 (double2*)d_l + lines, (StripItem*)d);
+      e = cudaGetLastError();
+    }
+    if (e == cudaSuccess) e = cudaStreamSynchronize(plan->stream);
+    Q.items = (const StripItem*)d;
+    Q.lrow = (const double2*)d_l;
+    Q.rcol = (const double2*)d_l + lines;
+    Q.plane = (const double*)d_plane;
+  }
+  if (e != cudaSuccess) {  // no room: the plan keeps the general kernels
+    (void)cudaGetLastError();
+    if (d) cudaFree(d);
+    plan->planes64_failed[which] = true;
+    return Planes64{};
+  }
+  plan->allocations.push_back(d);
+  plan->device_bytes += bytes;
+  P = Q;
+  return P;
+}
+
+namespace {
+
+template <int V>
+void launch_strip(const dim3 grid, bool epi, cudaStream_t stream, const Planes64& P, const DevicePlan& dp, int ncols,
+                  int rc, const double* x, double* y, long long ld, const BorderArgs& border) {
+  auto k = epi ? k_apply_strip64<V, true> : k_apply_strip64<V, false>;
+  k<<<grid, kStripThreads, 0, stream>>>(P, dp.sectors, ncols, rc, (const double2*)x, (double2*)y, ld, border.alpha,
+                                        border.coords, border.scale);
+}
+
+}  // namespace
+
+cudaError_t launch_apply_strip64(const DevicePlan& dp, const Planes64& P, const double* x, double* y, int ncols,
+                                 long long ld, const BorderArgs& border, cudaStream_t stream) {
+  // Columns per block: the coefficients of an entry (11 loads) are shared by its columns.
+  const int rc = ncols >= 64 ? 8 : ncols >= 16 ? 4 : ncols >= 4 ? 2 : 1;
+  const dim3 grid((unsigned)((P.nitems + kStripWarps - 1) / kStripWarps), (unsigned)((ncols + rc - 1) / rc));
+  const bool epi = border.scale != 1.0 || border.alpha != nullptr;
+  static_assert(kVariants64 == 7, "one launch per variant");
+  switch (P.variant) {
+    case 0: launch_strip<0>(grid, epi, stream, P, dp, ncols, rc, x, y, ld, border); break;
+    case 1: launch_strip<1>(grid, epi, stream, P, dp, ncols, rc, x, y, ld, border); break;
+    case 2: launch_strip<2>(grid, epi, stream, P, dp, ncols, rc, x, y, ld, border); break;
+    case 3: launch_strip<3>(grid, epi, stream, P, dp, ncols, rc, x, y, ld, border); break;
+    case 4: launch_strip<4>(grid, epi, stream, P, dp, ncols, rc, x, y, ld, border); break;
+    case 5: launch_strip<5>(grid, epi, stream, P, dp, ncols, rc, x, y, ld, border); break;
+    default: launch_strip<6>(grid, epi, stream, P, dp, ncols, rc, x, y, ld, border);
+  }
+  return cudaGetLastError();
+}
+
+}  // namespace picuda

@@ -16,6 +16,7 @@
 #include <unordered_set>
 #include <utility>
 
+#include "pi_apply64.cuh"
 #include "pi_apply_impl.cuh"
 #include "pi_dense.hpp"
 
@@ -173,8 +174,51 @@ __global__ void __launch_bounds__(kRT) k_s1_trace(DevInst* __restrict__ st) {
   }
 }
 
-// Applies over the (instance, tile) list.  AUX: ay = aux_scale L ax (+ border), FP64;
-// otherwise the Arnoldi step w = scale L V_j (+ border) in the basis precision.
+constexpr int kBlockItems = kApplyThreads / 32;  // strip items of one block of an apply over the list
+
+// kBlockItems consecutive strip items of an instance with merged FP64 coefficients: y = scale
+// L x + alpha v on the diagonal (reference coordinates), or y = L x when `plain`.
+template <int V>
+__device__ __forceinline__ void strip_block(const DevInst& S, int block, const double2* __restrict__ x,
+                                            double2* __restrict__ y, bool plain, double scale, const double2* alpha) {
+  const int item = block * kBlockItems + (threadIdx.x >> 5);
+  if (item >= S.p64.nitems) return;
+  const StripItem it = S.p64.items[item];
+  StripEntry<V> E;
+  if (!E.load(it, S.p64, threadIdx.x & 31)) return;
+  double2 out = E.apply(x);
+  if (plain) {  // block-uniform, its own exit: the scaling below must not be if-converted into it
+    y[E.e] = out;
+    return;
+  }
+  out.x *= scale;
+  out.y *= scale;
+  if (alpha != nullptr && E.diag) {
+    const double v = S.sectors[it.sector].border_x;
+    out.x = fma(alpha->x, v, out.x);
+    out.y = fma(alpha->y, v, out.y);
+  }
+  y[E.e] = out;
+}
+
+__device__ __forceinline__ void strip_apply(const DevInst& S, int block, const double2* x, double2* y, double scale,
+                                            const double2* alpha) {
+  // an exact 1 is told by its bits: an FP64 comparison would go through the FP64 pipe
+  const bool plain = alpha == nullptr && __double_as_longlong(scale) == 0x3ff0000000000000LL;
+  switch (S.p64.variant) {
+    case 0: return strip_block<0>(S, block, x, y, plain, scale, alpha);
+    case 1: return strip_block<1>(S, block, x, y, plain, scale, alpha);
+    case 2: return strip_block<2>(S, block, x, y, plain, scale, alpha);
+    case 3: return strip_block<3>(S, block, x, y, plain, scale, alpha);
+    case 4: return strip_block<4>(S, block, x, y, plain, scale, alpha);
+    case 5: return strip_block<5>(S, block, x, y, plain, scale, alpha);
+    default: return strip_block<6>(S, block, x, y, plain, scale, alpha);
+  }
+}
+
+// Applies over the (instance, tile) list -- for an instance with merged FP64 coefficients an
+// (instance, strip block) list.  AUX: ay = aux_scale L ax (+ border), FP64; otherwise the
+// Arnoldi step w = scale L V_j (+ border) in the basis precision.
 template <typename T, bool AUX>
 __global__ void __launch_bounds__(kApplyThreads, sizeof(T) == 4 && !AUX ? 4 : 1)
     k_bapply(const DevInst* __restrict__ st, const int* __restrict__ tile_inst, const int* __restrict__ tile_local) {
@@ -186,15 +230,25 @@ __global__ void __launch_bounds__(kApplyThreads, sizeof(T) == 4 && !AUX ? 4 : 1)
   const DevInst& S = st[tile_inst[blockIdx.x]];
   if (AUX) {
     if (!S.ax) return;
+    if (S.p64.items != nullptr) {  // block-uniform
+      strip_apply(S, tile_local[blockIdx.x], S.ax, S.ay, S.aux_scale, S.aux_border ? &S.aux_alpha : nullptr);
+      return;
+    }
     const DevTile tile = S.tiles[tile_local[blockIdx.x]];
     BorderArgs b{S.aux_scale, nullptr, 0};
     apply_tile<T>(S.sectors, S.terms, (const T2*)S.coef64, tile, (const T2*)S.ax, (T2*)S.ay, b,
                   S.aux_border ? &S.aux_alpha : nullptr, win, sterms, ge);
   } else {
     if (S.done) return;
+    const T2* xin = (const T2*)S.V + (long long)S.j * S.ldv;
+    if constexpr (sizeof(T) == sizeof(double)) {
+      if (S.p64.items != nullptr) {  // block-uniform
+        strip_apply(S, tile_local[blockIdx.x], xin, (double2*)S.w, S.scale, S.border ? &S.alpha : nullptr);
+        return;
+      }
+    }
     const DevTile tile = S.tiles[tile_local[blockIdx.x]];
     BorderArgs b{S.scale, nullptr, S.coords};
-    const T2* xin = (const T2*)S.V + (long long)S.j * S.ldv;
     if constexpr (sizeof(T) == sizeof(float)) {
       if (S.planes.eplane != nullptr && S.coords == S.pwhich) {  // block-uniform
         const StoreSink<float2> sink{(float2*)S.w};
@@ -1760,8 +1814,11 @@ void Engine::rebuild() {
   any_border_ = false;
   for (int i = 0; i < n; ++i) any_border_ = any_border_ || jobs_[i]->bordered;
   std::vector<int> ti, tl, ci, nc(n);
+  std::vector<Planes64> p64(n);
   for (int i = 0; i < n; ++i) {
-    const int ntiles = jobs_[i]->plan->dev.ntiles;
+    // FP64 engines apply canonical plans from merged coefficients: strip blocks, not tiles
+    p64[i] = f32_ ? Planes64{} : planes64(jobs_[i]->plan, PI_COORDS_REFERENCE);
+    const int ntiles = p64[i].items ? (p64[i].nitems + kBlockItems - 1) / kBlockItems : jobs_[i]->plan->dev.ntiles;
     for (int t = 0; t < ntiles; ++t) {
       ti.push_back(i);
       tl.push_back(t);
@@ -1794,6 +1851,7 @@ void Engine::rebuild() {
     // population coordinates, steady-state cycles in reference coordinates
     d.planes = SplitPlanes{nullptr, nullptr, nullptr, nullptr, 0};
     d.pwhich = J->bordered ? 0 : 1;
+    d.p64 = p64[i];
     if (f32_ && dp.canon && em_split_planes(J->plan, d.pwhich, &d.planes) != PI_OK)
       d.planes = SplitPlanes{nullptr, nullptr, nullptr, nullptr, 0};
     for (int c = 0; c < nc[i]; ++c) ci.push_back(i);

@@ -87,6 +87,7 @@ struct DevInst {
   // system pwhich (eplane == nullptr: the generic stencil terms)
   SplitPlanes planes;
   int pwhich;
+  Planes64 p64;  // FP64 basis, canonical plan: merged FP64 coefficients (reference coordinates)
   double scale;  // multiplies L V_j
   double tol;    // GMRES: stop when |g[j+1]| <= tol
   double rem2;

@@ -745,7 +745,9 @@ int pi_apply_f64(pi_plan* plan, double* y_dev, const double* x_dev, int ncols, l
   if (rc) return rc;
   BorderArgs border{1.0, nullptr, 0};
   cudaStream_t s = (cudaStream_t)stream;  // NULL is the CUDA default stream
-  cudaError_t e = launch_apply_f64(plan->dev, x_dev, y_dev, ncols, ld, border, s);
+  const Planes64 P = planes64(plan, PI_COORDS_REFERENCE);
+  cudaError_t e = P.items ? launch_apply_strip64(plan->dev, P, x_dev, y_dev, ncols, ld, border, s)
+                          : launch_apply_f64(plan->dev, x_dev, y_dev, ncols, ld, border, s);
   if (e != cudaSuccess) return cuda_fail(e, "apply launch");
   return PI_OK;
 }
@@ -803,6 +805,7 @@ static int apply_host(pi_plan* plan, void* y_host, const void* x_host, int ncols
   const int nchunks = sizeof(T) == sizeof(double) ? 16 : 8;
   const int chunk = std::max(1, (ncols + nchunks - 1) / nchunks);
   BorderArgs border{1.0, nullptr, coords};
+  const Planes64 P = sizeof(T) == sizeof(double) ? planes64(plan, coords) : Planes64{};
   int k = 0;
   for (int c0 = 0; c0 < ncols && e == cudaSuccess; c0 += chunk, ++k) {
     const int nc = std::min(chunk, ncols - c0);
@@ -813,7 +816,8 @@ static int apply_host(pi_plan* plan, void* y_host, const void* x_host, int ncols
                         cudaMemcpyHostToDevice, s);
     if (e == cudaSuccess) {
       if (sizeof(T) == sizeof(double))
-        e = launch_apply_f64(plan->dev, (const double*)dx, (double*)dy, nc, plan->host.dim, border, s);
+        e = P.items ? launch_apply_strip64(plan->dev, P, (const double*)dx, (double*)dy, nc, plan->host.dim, border, s)
+                    : launch_apply_f64(plan->dev, (const double*)dx, (double*)dy, nc, plan->host.dim, border, s);
       else
         e = launch_apply_f32(plan->dev, (const float*)dx, (float*)dy, nc, plan->host.dim, border, s);
     }

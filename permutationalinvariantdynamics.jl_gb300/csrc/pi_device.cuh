@@ -96,4 +96,40 @@ struct SplitPlanes {
 constexpr int kSepF4 = 6;      // 24 floats: 6 + 3 x 6 positions
 constexpr int kSepF4Plus = 9;  // 36 floats: 6 + 3 x 9 positions, padded
 
+// ---- FP64 strip apply (pi_apply64.cuh) ----
+
+// 32 consecutive entries of one sector block (one warp's work).
+struct alignas(16) StripItem {
+  int off, n;        // own sector block: element offset, dimension
+  int off0, m0;      // smaller neighbour (m0 = 0: none)
+  int off2, m2;      // larger neighbour (m2 = 0: none)
+  int local0, loff;  // first entry within the block; start of the sector's line tables
+  int sector, pad[3];
+};
+static_assert(sizeof(StripItem) == 48, "strip record layout");
+
+// Real gain position of a canonical plan: source (0 own, 1 smaller, 2 larger sector) at the
+// diagonal shift `shift` from the entry with the same magnetic numbers there, in index terms
+// own (a + shift, b + shift), smaller (a - 1 + shift, ...), larger (a + 1 + shift, ...).
+struct GainPos {
+  signed char src, shift;
+};
+constexpr int kMaxGains = 8;
+
+// Merged FP64 coefficients of a canonical plan: the planes [2 + nr][dim] (centre re, centre im,
+// then one per gain position that some sector uses; the own-sector centre gain joins the
+// centre) and the imaginary coefficients of the row and column shifts per line.  `variant`
+// selects the kernel: the number of gain slots it has and whether it has the line shifts
+// (unused slots carry src = -1).
+struct Planes64 {
+  const StripItem* items = nullptr;  // nullptr: the plan has no planes
+  const double* plane = nullptr;
+  const double2* lrow = nullptr;  // per row: row shifts -1, +1
+  const double2* rcol = nullptr;  // per column: column shifts -1, +1
+  long long dim = 0;
+  int nitems = 0;
+  int variant = 0;
+  GainPos gain[kMaxGains] = {};
+};
+
 }  // namespace picuda

@@ -64,6 +64,7 @@ struct ExpvWork {
   double2* h2 = nullptr;
   double2* coef = nullptr;
   int applications = 0;
+  Planes64 planes;  // FP64 basis: merged coefficients
 
   void chk(cudaError_t e) {
     if (e != cudaSuccess && err == cudaSuccess) err = e;
@@ -97,7 +98,8 @@ struct ExpvWork {
       chk(launch_apply_f32(p->dev, (const float*)col(j), (float*)w, 1, n, b, s));
       chk(norm2_f32((const float2*)w, n, p->rs, 1, s));
     } else {
-      chk(launch_apply_f64(p->dev, (const double*)col(j), (double*)w, 1, n, b, s));
+      chk(planes.items ? launch_apply_strip64(p->dev, planes, (const double*)col(j), (double*)w, 1, n, b, s)
+                       : launch_apply_f64(p->dev, (const double*)col(j), (double*)w, 1, n, b, s));
       chk(norm2_f64((const double2*)w, n, p->rs, 1, s));
     }
     ++applications;
@@ -405,6 +407,7 @@ int pi_expv(pi_plan* plan, double* x_dev, double t, const pi_expv_opts_t* opts, 
   pi_expv_info_t loc;
   ExpvWork W{plan, plan->stream, plan->host.dim, (int)std::min<long long>(opts->krylovdim, plan->host.dim),
              opts->precision == PI_FP32};
+  if (!W.mixed) W.planes = planes64(plan, PI_COORDS_REFERENCE);
   {
     Bufs B;
     B.s = W.s;
@@ -449,6 +452,7 @@ int pi_solve_dynamics(pi_plan* plan, double* rho_dev, int nt, const double* time
   }
   ExpvWork W{plan, plan->stream, plan->host.dim, (int)std::min<long long>(opts->krylovdim, plan->host.dim),
              opts->precision == PI_FP32};
+  if (!W.mixed) W.planes = planes64(plan, PI_COORDS_REFERENCE);
   pi_expv_info_t total;
   std::memset(&total, 0, sizeof(total));
   total.converged = 1;

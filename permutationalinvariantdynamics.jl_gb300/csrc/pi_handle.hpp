@@ -71,6 +71,10 @@ struct pi_plan {
   };
   std::vector<EmChoice> em_choices;
   std::mutex em_tune_mu;
+  // Merged FP64 coefficient planes per coordinate system, built on first use (guarded by em_mu);
+  // a plan without room for them keeps the general kernels.
+  picuda::Planes64 planes64[2];
+  bool planes64_failed[2] = {false, false};
   // Single-instance solves run as one job of a batched engine kept with the plan (created on
   // first use for a Krylov dimension and basis precision, replaced when those change).
   picuda::Engine* engine = nullptr;
@@ -111,5 +115,10 @@ void* plan_alloc(pi_plan* plan, size_t bytes);
 // FP32 coordinates, built on first use (pi_apply_em.cu); PI_ERR_UNSUPPORTED for a plan whose
 // stencil does not sit at the canonical positions.
 int em_split_planes(pi_plan* plan, int which, SplitPlanes* out);
+
+// Merged FP64 coefficient planes of a canonical plan in reference (coords 0) or population
+// (1) coordinates, built on first use (pi_apply64.cu); items == nullptr when the plan is not
+// canonical or has no room for them.
+Planes64 planes64(pi_plan* plan, int coords);
 
 }  // namespace picuda

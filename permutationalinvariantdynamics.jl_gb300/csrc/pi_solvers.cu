@@ -52,6 +52,7 @@ struct Run {
   cudaError_t err = cudaSuccess;
   int applications = 0;
   int coords = 0;  // PI_COORDS_* of every vector of the solve
+  Planes64 planes;  // merged FP64 coefficients of an FP64 solve (mixed solves apply FP64 once per restart)
   explicit Run(pi_plan* plan, int c = 0) : p(plan), s(plan->stream), n(plan->host.dim), coords(c) {}
   bool ok() const { return err == cudaSuccess; }
   void chk(cudaError_t e) {
@@ -71,18 +72,17 @@ struct Run {
     return v;
   }
   double norm(const double2* w) { return std::sqrt(norm2(w)); }
-  // y = L x (unbordered)
-  void apply(const double2* x, double2* y) {
-    BorderArgs b{1.0, nullptr, coords};
-    chk(launch_apply_f64(p->dev, (const double*)x, (double*)y, 1, n, b, s));
+  void apply64(const double2* x, double2* y, const BorderArgs& b) {
+    chk(planes.items ? launch_apply_strip64(p->dev, planes, (const double*)x, (double*)y, 1, n, b, s)
+                     : launch_apply_f64(p->dev, (const double*)x, (double*)y, 1, n, b, s));
     ++applications;
   }
+  // y = L x (unbordered)
+  void apply(const double2* x, double2* y) { apply64(x, y, BorderArgs{1.0, nullptr, coords}); }
   // y = L x / scale + (t^H x) v  (krylov.jl:855-860)
   void apply_bordered(const double2* x, double2* y, double invscale, double2* alpha_dev) {
     chk(trace_dot(p->dev, x, 0, coords, alpha_dev, s));
-    BorderArgs b{invscale, alpha_dev, coords};
-    chk(launch_apply_f64(p->dev, (const double*)x, (double*)y, 1, n, b, s));
-    ++applications;
+    apply64(x, y, BorderArgs{invscale, alpha_dev, coords});
   }
   void apply_bordered_f32(const float2* x, float2* y, double invscale, double2* alpha_dev) {
     chk(trace_dot(p->dev, x, 1, coords, alpha_dev, s));
@@ -623,6 +623,7 @@ int pi_steady_state(pi_plan* plan, double* x_dev, const pi_gmres_opts_t* opts, p
   }
   const int coords = opts->coords;
   Run R(plan, coords);
+  if (opts->precision == PI_FP64) R.planes = planes64(plan, coords);
   const long long n = R.n;
   const int m = (int)std::min<long long>(opts->krylovdim, n);
   pi_gmres_info_t loc;
