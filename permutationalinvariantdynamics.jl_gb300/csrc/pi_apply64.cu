@@ -10,11 +10,29 @@
 namespace picuda {
 namespace {
 
-// Planes, line tables and strip items of sector blockIdx.y.
+// Strip items of sector blockIdx.y; first[s] = (first line, first item) of sector s.
+__global__ void k_strip_items(const DevSector* __restrict__ sectors, const int2* __restrict__ first,
+                              StripItem* __restrict__ items) {
+  const int s = blockIdx.y;
+  const DevSector& sec = sectors[s];
+  const int n = sec.n;
+  StripItem it{};
+  it.off = (int)sec.offset;
+  it.n = n;
+  if (sec.src[0] >= 0) it.off0 = (int)sectors[sec.src[0]].offset, it.m0 = sectors[sec.src[0]].n;
+  if (sec.src[2] >= 0) it.off2 = (int)sectors[sec.src[2]].offset, it.m2 = sectors[sec.src[2]].n;
+  it.loff = first[s].x;
+  it.sector = s;
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; 32LL * i < (long long)n * n; i += gridDim.x * blockDim.x) {
+    it.local0 = 32 * i;
+    items[first[s].y + i] = it;
+  }
+}
+
+// Planes and line tables of sector blockIdx.y.
 __global__ void k_planes64(const DevSector* __restrict__ sectors, const int4* __restrict__ canon,
                            const double2* __restrict__ coef, const int2* __restrict__ first, const Planes64 P, int nr,
-                           double* __restrict__ plane, double2* __restrict__ lrow, double2* __restrict__ rcol,
-                           StripItem* __restrict__ items) {
+                           double* __restrict__ plane, double2* __restrict__ lrow, double2* __restrict__ rcol) {
   const int s = blockIdx.y;
   const DevSector& sec = sectors[s];
   const int n = sec.n;
@@ -40,17 +58,6 @@ __global__ void k_planes64(const DevSector* __restrict__ sectors, const int4* __
       const int slot = src == 0 ? 1 : src == 1 ? 0 : 2;
       out[(2 + k) * P.dim] = sand(slot * 3 + P.gain[k].shift + 1, a, b);
     }
-  }
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; 32LL * i < cnt; i += gridDim.x * blockDim.x) {
-    StripItem it{};
-    it.off = (int)sec.offset;
-    it.n = n;
-    if (sec.src[0] >= 0) it.off0 = (int)sectors[sec.src[0]].offset, it.m0 = sectors[sec.src[0]].n;
-    if (sec.src[2] >= 0) it.off2 = (int)sectors[sec.src[2]].offset, it.m2 = sectors[sec.src[2]].n;
-    it.local0 = 32 * i;
-    it.loff = first[s].x;
-    it.sector = s;
-    items[first[s].y + i] = it;
   }
   if (blockIdx.x == 0)
     for (int i = threadIdx.x; i < n; i += blockDim.x) {
@@ -105,24 +112,74 @@ struct RelaxedCapture {
 
 }  // namespace
 
-Planes64 planes64(pi_plan* plan, int coords) {
+// Per sector (first line, first strip item); returns the totals.
+static int2 strip_starts(const pi_plan* plan, std::vector<int2>* first) {
+  int lines = 0, nitems = 0;
+  for (const Sector& sec : plan->host.sectors) {
+    first->push_back(make_int2(lines, nitems));
+    lines += sec.n;
+    nitems += (sec.n * sec.n + 31) / 32;
+  }
+  return make_int2(lines, nitems);
+}
+
+// Keeps `d` with the plan when e is success; otherwise releases it.
+static bool adopt(pi_plan* plan, void* d, size_t bytes, cudaError_t e) {
+  if (e != cudaSuccess) {
+    (void)cudaGetLastError();
+    if (d) cudaFree(d);
+    return false;
+  }
+  plan->allocations.push_back(d);
+  plan->device_bytes += bytes;
+  return true;
+}
+
+// Caller holds em_mu.
+static StripItems strip_items_locked(pi_plan* plan) {
   const DevicePlan& dp = plan->dev;
   // 32-bit element indices within a vector
-  if (!dp.canon || dp.dim == 0 || dp.dim > 0x3fffffffLL) return Planes64{};
+  if (dp.dim == 0 || dp.dim > 0x3fffffffLL) return StripItems{};
+  if (plan->strip_items) return StripItems{plan->strip_items, plan->nstrip_items};
+  RelaxedCapture relaxed;
+  std::vector<int2> first;
+  const int nitems = strip_starts(plan, &first).y;
+  const size_t bytes = sizeof(StripItem) * (size_t)nitems + sizeof(int2) * first.size();
+  char* d = nullptr;
+  cudaError_t e = cudaMalloc((void**)&d, bytes);
+  if (e == cudaSuccess) {
+    int2* d_first = (int2*)(d + sizeof(StripItem) * (size_t)nitems);
+    e = cudaMemcpyAsync(d_first, first.data(), sizeof(int2) * first.size(), cudaMemcpyHostToDevice, plan->stream);
+    if (e == cudaSuccess) {
+      k_strip_items<<<dim3(8, (unsigned)first.size()), 256, 0, plan->stream>>>(dp.sectors, d_first, (StripItem*)d);
+      e = cudaGetLastError();
+    }
+    if (e == cudaSuccess) e = cudaStreamSynchronize(plan->stream);
+  }
+  if (!adopt(plan, d, bytes, e)) return StripItems{};
+  plan->strip_items = (const StripItem*)d;
+  plan->nstrip_items = nitems;
+  return StripItems{plan->strip_items, nitems};
+}
+
+StripItems strip_items(pi_plan* plan) {
+  std::lock_guard<std::mutex> lk(plan->em_mu);
+  return strip_items_locked(plan);
+}
+
+Planes64 planes64(pi_plan* plan, int coords) {
+  const DevicePlan& dp = plan->dev;
+  if (!dp.canon) return Planes64{};
   std::lock_guard<std::mutex> lk(plan->em_mu);
   const int which = coords ? 1 : 0;
   Planes64& P = plan->planes64[which];
   if (P.items || plan->planes64_failed[which]) return P;
+  const StripItems strips = strip_items_locked(plan);
+  if (!strips.items) return Planes64{};
   RelaxedCapture relaxed;
   const int S = (int)plan->host.sectors.size();
-  std::vector<int2> first(S);  // per sector: first line, first strip item
-  int lines = 0, nitems = 0;
-  for (int s = 0; s < S; ++s) {
-    const int n = plan->host.sectors[s].n;
-    first[s] = make_int2(lines, nitems);
-    lines += n;
-    nitems += (n * n + 31) / 32;
-  }
+  std::vector<int2> first;
+  const int lines = strip_starts(plan, &first).x;
   // gain positions that some sector uses, in the order of the canonical kernels: own, smaller,
   // larger sector
   bool drive = false, used[3][3] = {};
@@ -134,7 +191,7 @@ Planes64 planes64(pi_plan* plan, int coords) {
   used[0][1] = false;  // joins the centre
   Planes64 Q;
   Q.dim = dp.dim;
-  Q.nitems = nitems;
+  Q.nitems = strips.n;
   for (GainPos& g : Q.gain) g = GainPos{-1, 0};
   int nr = 0;
   for (int src = 0; src < 3; ++src)
@@ -142,39 +199,34 @@ Planes64 planes64(pi_plan* plan, int coords) {
       if (used[src][p + 1]) Q.gain[nr++] = GainPos{(signed char)src, (signed char)p};
   Q.variant = drive ? (nr <= 1 ? 0 : nr <= 3 ? 1 : nr <= 5 ? 2 : nr <= 6 ? 3 : 4) : (nr <= 5 ? 5 : 6);
   const int np = 2 + nr;
-  // one allocation: records, line tables, planes, per-sector starts
-  const size_t item_bytes = sizeof(StripItem) * (size_t)nitems, line_bytes = sizeof(double2) * (size_t)lines;
+  // one allocation: line tables, planes, per-sector starts
+  const size_t line_bytes = sizeof(double2) * (size_t)lines;
   const size_t plane_bytes = (sizeof(double) * (size_t)dp.dim * np + 15) / 16 * 16;
-  const size_t bytes = item_bytes + 2 * line_bytes + plane_bytes + sizeof(int2) * (size_t)S;
+  const size_t bytes = 2 * line_bytes + plane_bytes + sizeof(int2) * (size_t)S;
   char* d = nullptr;
   cudaError_t e = cudaMalloc((void**)&d, bytes);
   if (e == cudaSuccess) {
-    char* d_l = d + item_bytes;
-    char* d_plane = d_l + 2 * line_bytes;
+    char* d_plane = d + 2 * line_bytes;
     char* d_first = d_plane + plane_bytes;
     e = cudaMemcpyAsync(d_first, first.data(), sizeof(int2) * (size_t)S, cudaMemcpyHostToDevice, plan->stream);
     if (e == cudaSuccess) {
       const dim3 grid((unsigned)std::min<long long>(64, ((long long)plan->host.max_n * plan->host.max_n + 255) / 256),
                       (unsigned)S);
       k_planes64<<<grid, 256, 0, plan->stream>>>(dp.sectors, dp.canon, coords ? dp.coef64z : dp.coef64,
-                                                 (const int2*)d_first, Q, nr, (double*)d_plane, (double2*)d_l,
-                                                 (double2*)d_l + lines, (StripItem*)d);
+                                                 (const int2*)d_first, Q, nr, (double*)d_plane, (double2*)d,
+                                                 (double2*)d + lines);
       e = cudaGetLastError();
     }
     if (e == cudaSuccess) e = cudaStreamSynchronize(plan->stream);
-    Q.items = (const StripItem*)d;
-    Q.lrow = (const double2*)d_l;
-    Q.rcol = (const double2*)d_l + lines;
+    Q.items = strips.items;
+    Q.lrow = (const double2*)d;
+    Q.rcol = (const double2*)d + lines;
     Q.plane = (const double*)d_plane;
   }
-  if (e != cudaSuccess) {  // no room: the plan keeps the general kernels
-    (void)cudaGetLastError();
-    if (d) cudaFree(d);
+  if (!adopt(plan, d, bytes, e)) {  // no room: the plan keeps the general kernels
     plan->planes64_failed[which] = true;
     return Planes64{};
   }
-  plan->allocations.push_back(d);
-  plan->device_bytes += bytes;
   P = Q;
   return P;
 }

@@ -367,50 +367,6 @@ __device__ __forceinline__ void sep_entries(const float* r, const float4* colp, 
   }
 }
 
-// The same tile from the separable line planes: each thread loads its row's factors once and
-// each column's factors as broadcast loads, so y is bitwise the same as apply_tile_planes_to's
-// while only 16 bytes per entry (x in, y out) come from memory.
-template <bool PLUS, typename Sink>
-__device__ __forceinline__ void apply_tile_sep_to(const DevSector* __restrict__ sectors, const DevTile tile,
-                                                  const float2* __restrict__ x, const Sink& sink,
-                                                  const BorderArgs& border, const double2* alpha,
-                                                  const SplitPlanes& pl, float2* win) {
-  constexpr int NF4 = PLUS ? kSepF4Plus : kSepF4;
-  __shared__ __align__(16) float4 colp[kTileCols * NF4];  // the tile's column planes
-  const DevSector& sec = sectors[tile.sector];
-  const int la = threadIdx.x & 31;
-  const int warp = threadIdx.x >> 5;
-  const int n = sec.n;
-  const int loff = __ldg(pl.line_off + tile.sector);
-  // column planes of the tile's 32 columns land with the source windows (one cp.async wait)
-  for (int i = threadIdx.x; i < kTileCols * NF4; i += blockDim.x) {
-    const int b = tile.b0 + i / NF4;
-    const bool ok = b < n;
-    cp_async_zfill<16>(colp + i, ok ? pl.scol + (long long)(loff + b) * NF4 + i % NF4 : pl.scol, ok);
-  }
-  // this thread's row factors, in flight during the staging
-  const int a = tile.a0 + la;
-  const int ar = a < n ? a : 0;
-  float4 rv[NF4];
-#pragma unroll
-  for (int k = 0; k < NF4; ++k) rv[k] = __ldg(pl.srow + (long long)(loff + ar) * NF4 + k);
-  stage_windows<float>(sectors, sec, tile, x, win);
-  const int lb = warp * kColsPerThread;
-  const int b0 = tile.b0 + lb;
-  if (a >= n || b0 >= n) return;
-  float r[4 * NF4];
-#pragma unroll
-  for (int k = 0; k < NF4; ++k) {
-    r[4 * k] = rv[k].x;
-    r[4 * k + 1] = rv[k].y;
-    r[4 * k + 2] = rv[k].z;
-    r[4 * k + 3] = rv[k].w;
-  }
-  const float2* wb = win + (la + kHalo) + (lb + kHalo) * kWinRows;
-  sep_entries<PLUS, kWinRows, kWinElems>(r, colp, wb, lb, min(kColsPerThread, n - b0), a, b0, sec, border, alpha,
-                                         sink);
-}
-
 // ---------------------------------------------------------------------------------------
 // Two-stage separable-plane tiles for persistent launches.  The canonical positions read
 // only the shifts -1..+1 around (a + e, b + e), so each source window needs a halo of one

@@ -13,6 +13,7 @@
 #include <mutex>
 #include <random>
 #include <tuple>
+#include <type_traits>
 #include <unordered_set>
 #include <utility>
 
@@ -178,13 +179,12 @@ constexpr int kBlockItems = kApplyThreads / 32;  // strip items of one block of 
 
 // kBlockItems consecutive strip items of an instance with merged FP64 coefficients: y = scale
 // L x + alpha v on the diagonal (reference coordinates), or y = L x when `plain`.
-template <int V>
-__device__ __forceinline__ void strip_block(const DevInst& S, int block, const double2* __restrict__ x,
-                                            double2* __restrict__ y, bool plain, double scale, const double2* alpha) {
+template <int V, bool NC>
+__device__ __forceinline__ void strip_block(const DevInst& S, int block, const double2* x, double2* y, bool plain, double scale, const double2* alpha) {
   const int item = block * kBlockItems + (threadIdx.x >> 5);
   if (item >= S.p64.nitems) return;
   const StripItem it = S.p64.items[item];
-  StripEntry<V> E;
+  StripEntry<V, NC> E;
   if (!E.load(it, S.p64, threadIdx.x & 31)) return;
   double2 out = E.apply(x);
   if (plain) {  // block-uniform, its own exit: the scaling below must not be if-converted into it
@@ -201,23 +201,98 @@ __device__ __forceinline__ void strip_block(const DevInst& S, int block, const d
   y[E.e] = out;
 }
 
+template <bool NC>
 __device__ __forceinline__ void strip_apply(const DevInst& S, int block, const double2* x, double2* y, double scale,
                                             const double2* alpha) {
   // an exact 1 is told by its bits: an FP64 comparison would go through the FP64 pipe
   const bool plain = alpha == nullptr && __double_as_longlong(scale) == 0x3ff0000000000000LL;
   switch (S.p64.variant) {
-    case 0: return strip_block<0>(S, block, x, y, plain, scale, alpha);
-    case 1: return strip_block<1>(S, block, x, y, plain, scale, alpha);
-    case 2: return strip_block<2>(S, block, x, y, plain, scale, alpha);
-    case 3: return strip_block<3>(S, block, x, y, plain, scale, alpha);
-    case 4: return strip_block<4>(S, block, x, y, plain, scale, alpha);
-    case 5: return strip_block<5>(S, block, x, y, plain, scale, alpha);
-    default: return strip_block<6>(S, block, x, y, plain, scale, alpha);
+    case 0: return strip_block<0, NC>(S, block, x, y, plain, scale, alpha);
+    case 1: return strip_block<1, NC>(S, block, x, y, plain, scale, alpha);
+    case 2: return strip_block<2, NC>(S, block, x, y, plain, scale, alpha);
+    case 3: return strip_block<3, NC>(S, block, x, y, plain, scale, alpha);
+    case 4: return strip_block<4, NC>(S, block, x, y, plain, scale, alpha);
+    case 5: return strip_block<5, NC>(S, block, x, y, plain, scale, alpha);
+    default: return strip_block<6, NC>(S, block, x, y, plain, scale, alpha);
   }
 }
 
-// Applies over the (instance, tile) list -- for an instance with merged FP64 coefficients an
-// (instance, strip block) list.  AUX: ay = aux_scale L ax (+ border), FP64; otherwise the
+// kBlockItems strip items of an FP32 instance of a canonical plan: w = scale L x (+ alpha v on
+// the diagonal) from the merged entry, row and column planes, one thread per entry.  The
+// arithmetic of an entry is apply_tile_planes_to's (and sep_entries'), operation for operation,
+// so every schedule gives the same bits.  Per entry: 32-48 bytes of planes and ten sources
+// through L1, no window staging and no idle lanes; the 32 x 32 tiles it replaces spent 1,113
+// instructions per warp and tile, most of them on staging.
+template <bool PLUS, bool NC>
+__device__ __forceinline__ void strip_block32(const DevInst& S, int block, const float2* x, float2* y,
+                                              const double2* alpha) {
+  constexpr int NE = PLUS ? 3 : 2;
+  const int item = block * kBlockItems + (threadIdx.x >> 5);
+  if (item >= S.nitems32) return;
+  const StripItem it = S.items32[item];
+  const int n = it.n;
+  const int i = it.local0 + (threadIdx.x & 31);
+  if (i >= n * n) return;
+  const int b = (int)((unsigned)i / (unsigned)n), a = i - b * n;
+  const int e = it.off + i;
+  const float4* ep = S.planes.eplane + (long long)e * NE;
+  const float4 c0 = __ldg(ep), c1 = __ldg(ep + 1);
+  const float4 lv = __ldg(S.planes.lrow + it.loff + a), rc = __ldg(S.planes.rcol + it.loff + b);
+  const float2 zero = make_float2(0.f, 0.f);
+  auto ld = [&](long long k, bool in) { return in ? (NC ? __ldg(x + k) : x[k]) : zero; };
+  const int m0 = it.m0, m2 = it.m2;
+  auto box = [](int u, int v, int m) { return (unsigned)u < (unsigned)m && (unsigned)v < (unsigned)m; };
+  const int s0 = it.off0 + (a - 2) + (b - 2) * m0, g0 = it.off2 + a + b * m2;
+  const float2 xc = ld(e, true), xu = ld(e - 1, a > 0), xd = ld(e + 1, a < n - 1);
+  const float2 xl = ld(e - n, b > 0), xr = ld(e + n, b < n - 1), xo = ld(e - n - 1, a > 0 && b > 0);
+  const float2 v0 = ld(s0, box(a - 2, b - 2, m0)), v1 = ld(s0 + m0 + 1, box(a - 1, b - 1, m0));
+  const float2 w0 = ld(g0, box(a, b, m2)), w1 = ld(g0 + m2 + 1, box(a + 1, b + 1, m2));
+  float2 acc = zero;
+  pmac(acc, c0.x, c0.y, xc);  // centre
+  pmac(acc, lv.x, lv.y, xu);  // LEFT -1
+  pmac(acc, lv.z, lv.w, xd);  // LEFT +1
+  pmac(acc, rc.x, rc.y, xl);  // RIGHT -1
+  pmac(acc, rc.z, rc.w, xr);  // RIGHT +1
+  prmac(acc, c0.z, xo);       // own (-1,-1)
+  if (m0 > 0) {
+    prmac(acc, c0.w, v0);     // smaller (-2,-2)
+    prmac(acc, c1.x, v1);     // smaller (-1,-1)
+  }
+  if (m2 > 0) {
+    prmac(acc, c1.y, w0);     // larger (0,0)
+    prmac(acc, c1.z, w1);     // larger (1,1)
+  }
+  if (PLUS) {
+    const float4 c2 = __ldg(ep + 2);
+    prmac(acc, c1.w, ld(e + n + 1, a < n - 1 && b < n - 1));              // own (1,1)
+    if (m0 > 0) prmac(acc, c2.x, ld(s0 + 2 * (m0 + 1), box(a, b, m0)));   // smaller (0,0)
+    if (m2 > 0) prmac(acc, c2.y, ld(g0 + 2 * (m2 + 1), box(a + 2, b + 2, m2)));  // larger (2,2)
+  }
+  if (__double_as_longlong(S.scale) != 0x3ff0000000000000LL) {
+    const float scale = (float)S.scale;
+    acc.x *= scale;
+    acc.y *= scale;
+  }
+  if (alpha != nullptr && a == b) {
+    const double2 al = *alpha;
+    const double v = S.coords ? S.sectors[it.sector].border_z : S.sectors[it.sector].border_x;
+    acc.x += (float)(al.x * v);
+    acc.y += (float)(al.y * v);
+  }
+  y[e] = acc;
+}
+
+template <bool NC>
+__device__ __forceinline__ void strip_apply32(const DevInst& S, int block, const float2* x, float2* y,
+                                              const double2* alpha) {
+  if (S.planes.plus)
+    strip_block32<true, NC>(S, block, x, y, alpha);
+  else
+    strip_block32<false, NC>(S, block, x, y, alpha);
+}
+
+// Applies over the (instance, tile) list -- for an instance of a canonical plan an (instance,
+// strip block) list.  AUX: ay = aux_scale L ax (+ border), FP64; otherwise the
 // Arnoldi step w = scale L V_j (+ border) in the basis precision.
 template <typename T, bool AUX>
 __global__ void __launch_bounds__(kApplyThreads, sizeof(T) == 4 && !AUX ? 4 : 1)
@@ -231,7 +306,7 @@ __global__ void __launch_bounds__(kApplyThreads, sizeof(T) == 4 && !AUX ? 4 : 1)
   if (AUX) {
     if (!S.ax) return;
     if (S.p64.items != nullptr) {  // block-uniform
-      strip_apply(S, tile_local[blockIdx.x], S.ax, S.ay, S.aux_scale, S.aux_border ? &S.aux_alpha : nullptr);
+      strip_apply<true>(S, tile_local[blockIdx.x], S.ax, S.ay, S.aux_scale, S.aux_border ? &S.aux_alpha : nullptr);
       return;
     }
     const DevTile tile = S.tiles[tile_local[blockIdx.x]];
@@ -243,28 +318,18 @@ __global__ void __launch_bounds__(kApplyThreads, sizeof(T) == 4 && !AUX ? 4 : 1)
     const T2* xin = (const T2*)S.V + (long long)S.j * S.ldv;
     if constexpr (sizeof(T) == sizeof(double)) {
       if (S.p64.items != nullptr) {  // block-uniform
-        strip_apply(S, tile_local[blockIdx.x], xin, (double2*)S.w, S.scale, S.border ? &S.alpha : nullptr);
+        strip_apply<true>(S, tile_local[blockIdx.x], xin, (double2*)S.w, S.scale, S.border ? &S.alpha : nullptr);
+        return;
+      }
+    }
+    if constexpr (sizeof(T) == sizeof(float)) {
+      if (S.items32 != nullptr) {  // block-uniform
+        strip_apply32<true>(S, tile_local[blockIdx.x], xin, (float2*)S.w, S.border ? &S.alpha : nullptr);
         return;
       }
     }
     const DevTile tile = S.tiles[tile_local[blockIdx.x]];
     BorderArgs b{S.scale, nullptr, S.coords};
-    if constexpr (sizeof(T) == sizeof(float)) {
-      if (S.planes.eplane != nullptr && S.coords == S.pwhich) {  // block-uniform
-        const StoreSink<float2> sink{(float2*)S.w};
-        if (S.planes.srow != nullptr) {  // separable line planes: x in, y out per entry
-          if (S.planes.plus)
-            apply_tile_sep_to<true>(S.sectors, tile, xin, sink, b, S.border ? &S.alpha : nullptr, S.planes, win);
-          else
-            apply_tile_sep_to<false>(S.sectors, tile, xin, sink, b, S.border ? &S.alpha : nullptr, S.planes, win);
-        } else if (S.planes.plus) {
-          apply_tile_planes_to<true>(S.sectors, tile, xin, sink, b, S.border ? &S.alpha : nullptr, S.planes, win);
-        } else {
-          apply_tile_planes_to<false>(S.sectors, tile, xin, sink, b, S.border ? &S.alpha : nullptr, S.planes, win);
-        }
-        return;
-      }
-    }
     apply_tile<T>(S.sectors, S.terms, (const T2*)S.coefb, tile, xin, (T2*)S.w, b, S.border ? &S.alpha : nullptr, win,
                   sterms, ge);
   }
@@ -455,16 +520,16 @@ __global__ void __launch_bounds__(kRT)
       sx += red[o][wdx].x;
       sy += red[o][wdx].y;
     }
-    partv[(long long)blockIdx.x * kMaxDots + o] = make_double2(sx, sy);
+    partv[(long long)blockIdx.x * S.pstride + o] = make_double2(sx, sy);
   }
 }
 
 // Per-instance sums of chunk partials: one warp per value, fixed order.
-__device__ __forceinline__ double2 warp_chunk_sum(const double2* partv, int begin, int nc, int i) {
+__device__ __forceinline__ double2 warp_chunk_sum(const double2* partv, int begin, int nc, int stride, int i) {
   const int lane = threadIdx.x & 31;
   double sx = 0, sy = 0;
   for (int c = lane; c < nc; c += 32) {
-    const double2 p = partv[(long long)(begin + c) * kMaxDots + i];
+    const double2 p = partv[(long long)(begin + c) * stride + i];
     sx += p.x;
     sy += p.y;
   }
@@ -483,7 +548,7 @@ __global__ void __launch_bounds__(kRT)
   if (nob == 0) return;
   const int warp = threadIdx.x >> 5;
   for (int o = warp; o < nob; o += blockDim.x >> 5) {
-    const double2 v = warp_chunk_sum(partv, S.chunk_begin, nchunks[blockIdx.x], o);
+    const double2 v = warp_chunk_sum(partv, S.chunk_begin, nchunks[blockIdx.x], S.pstride, o);
     if ((threadIdx.x & 31) == 0) {
       S.out[4 + 2 * o] = v.x;
       S.out[5 + 2 * o] = v.y;
@@ -513,13 +578,16 @@ __global__ void __launch_bounds__(kRT) k_load_v0(const DevInst* __restrict__ st,
     for (int r = threadIdx.x; r < S.ldh; r += blockDim.x) S.g[r] = make_double2(r == 0 ? S.v0norm : 0.0, 0.0);
 }
 
-// alpha = t^H V_j for bordered cycles.
+// The phases of one Arnoldi step are device functions of (job, input column j, chunk): the
+// step kernels below launch one phase each, and k_cycle runs all phases of all steps of a
+// small job set in one launch.  Pointers to data that the step writes carry no __restrict__
+// and no read-only loads, as one kernel writes and reads them.
+
+// alpha = t^H V_j for bordered cycles (whole block).
 template <typename T2>
-__global__ void __launch_bounds__(kRT) k_step_trace(DevInst* __restrict__ st) {
+__device__ void step_trace(DevInst& S, int j) {
   __shared__ double smem[32 * 2];
-  DevInst& S = st[blockIdx.x];
-  if (S.done || !S.border) return;
-  const T2* x = (const T2*)S.V + (long long)S.j * S.ldv;
+  const T2* x = (const T2*)S.V + (long long)j * S.ldv;
   double acc[2] = {0, 0};
   for (int i = threadIdx.x; i < S.ndiag; i += blockDim.x) {
     const double w = S.coords ? 1.0 : S.sectors[S.diag_sector[i]].sqrt_f;
@@ -529,220 +597,287 @@ __global__ void __launch_bounds__(kRT) k_step_trace(DevInst* __restrict__ st) {
   }
   block_sum<2>(acc, smem);
   if (threadIdx.x == 0) S.alpha = make_double2(acc[0], acc[1]);
+  __syncthreads();  // smem is free for the block's next job
 }
 
-// |w|^2 partials (image norm, skipped by GMRES cycles which do not use it).
 template <typename T2>
-__global__ void __launch_bounds__(kRT)
-    k_step_image_partial(const DevInst* __restrict__ st, const int* __restrict__ chunk_inst, double* __restrict__ part) {
-  __shared__ double smem[32];
-  const DevInst& S = st[chunk_inst[blockIdx.x]];
-  if (S.done || S.givens) return;
-  long long beg, end;
-  chunk_range(S, blockIdx.x, beg, end);
-  const T2* w = (const T2*)S.w;
-  double acc[1] = {0};
-  for (long long e = beg + threadIdx.x; e < end; e += blockDim.x) {
-    const double2 v = ld2(w + e);
-    acc[0] = fma(v.x, v.x, acc[0]);
-    acc[0] = fma(v.y, v.y, acc[0]);
-  }
-  block_sum<1>(acc, smem);
-  if (threadIdx.x == 0) part[blockIdx.x] = acc[0];
-}
-
-// CGS2 projections: partv[c][i] = sum over chunk c of conj(V_i) w, i in [8 y, 8 y + 8).
-template <typename T2, bool DFACC>
-__global__ void __launch_bounds__(kRT)
-    k_step_mdot_partial(const DevInst* __restrict__ st, const int* __restrict__ chunk_inst, double2* __restrict__ partv) {
-  __shared__ double smem[32 * 16];
-  const DevInst& S = st[chunk_inst[blockIdx.x]];
-  if (S.done) return;
-  const int nv = S.j + 1;
-  const int g0 = blockIdx.y * 8;
-  if (g0 >= nv) return;
-  const int cnt = min(8, nv - g0);
-  long long beg, end;
-  chunk_range(S, blockIdx.x, beg, end);
-  const long long dim = S.ldv;
-  const T2* V = (const T2*)S.V + (long long)g0 * dim;
-  const T2* w = (const T2*)S.w;
-  double acc[16];
-  if (DFACC) {
-    DF re[8], im[8];
-#pragma unroll
-    for (int k = 0; k < 8; ++k) re[k] = im[k] = DF{0.f, 0.f};
-    for (long long e = beg + threadIdx.x; e < end; e += blockDim.x) {
-      const float2 wv = reinterpret_cast<const float2*>(w)[e];
-#pragma unroll
-      for (int k = 0; k < 8; ++k) {
-        if (k < cnt) {
-          const float2 v = reinterpret_cast<const float2*>(V)[(long long)k * dim + e];
-          df_add_prod(re[k], v.x, wv.x);
-          df_add_prod(re[k], v.y, wv.y);
-          df_add_prod(im[k], v.x, wv.y);
-          df_add_prod(im[k], -v.y, wv.x);
-        }
-      }
-    }
-#pragma unroll
-    for (int k = 0; k < 8; ++k) {
-      acc[2 * k] = (double)re[k].hi + (double)re[k].lo;
-      acc[2 * k + 1] = (double)im[k].hi + (double)im[k].lo;
-    }
-  } else {
-#pragma unroll
-    for (int k = 0; k < 16; ++k) acc[k] = 0;
-    for (long long e = beg + threadIdx.x; e < end; e += blockDim.x) {
-      const double2 wv = ld2(w + e);
-#pragma unroll
-      for (int k = 0; k < 8; ++k) {
-        if (k < cnt) {
-          const double2 v = ld2(V + (long long)k * dim + e);
-          acc[2 * k] = fma(v.x, wv.x, acc[2 * k]);
-          acc[2 * k] = fma(v.y, wv.y, acc[2 * k]);
-          acc[2 * k + 1] = fma(v.x, wv.y, acc[2 * k + 1]);
-          acc[2 * k + 1] = fma(-v.y, wv.x, acc[2 * k + 1]);
-        }
-      }
-    }
-  }
-  block_sum<16>(acc, smem);
-  if (threadIdx.x == 0)
-    for (int k = 0; k < cnt; ++k)
-      partv[(long long)blockIdx.x * kMaxDots + g0 + k] = make_double2(acc[2 * k], acc[2 * k + 1]);
-}
-
-// which 0: hA, 1: hB.  Grid (instances, column groups): warp w of block (x, y) reduces
-// column i = y * warps + w, so every column of every instance has its own warp (one warp
-// walking several columns left a single SM reducing a long chunk list per column).
-__global__ void __launch_bounds__(kRT)
-    k_step_mdot_final(const DevInst* __restrict__ st, const int* __restrict__ nchunks, const double2* __restrict__ partv,
-                      int which) {
-  const DevInst& S = st[blockIdx.x];
-  if (S.done) return;
-  const int nv = S.j + 1;
-  double2* h = which == 0 ? S.hA : S.hB;
-  const int i = blockIdx.y * (blockDim.x >> 5) + (threadIdx.x >> 5);
-  if (i >= nv) return;  // warp-uniform
-  const double2 v = warp_chunk_sum(partv, S.chunk_begin, nchunks[blockIdx.x], i);
-  if ((threadIdx.x & 31) == 0) h[i] = v;
-}
-
-// The first-pass reductions of a step in one launch: blocks (x, y < gridDim.y - 1) reduce the
-// projections into hA as k_step_mdot_final(which 0) does, blocks (x, gridDim.y - 1) the
-// image norm |w|^2 into image2 (expv cycles): thread t sums the chunk partials t, t + 256,
-// ... and a deterministic block sum combines the threads.
-__global__ void __launch_bounds__(kRT)
-    k_step_first_final(DevInst* __restrict__ st, const int* __restrict__ nchunks, const double2* __restrict__ partv,
-                       const double* __restrict__ part, int all_images) {
-  __shared__ double smem[32];
+__global__ void __launch_bounds__(kRT) k_step_trace(DevInst* st) {
   DevInst& S = st[blockIdx.x];
-  if (S.done) return;
-  if (blockIdx.y == gridDim.y - 1) {  // image norm (block-uniform)
-    if (S.givens && !all_images) return;
-    double acc[1] = {0};
-    for (int c = threadIdx.x; c < nchunks[blockIdx.x]; c += blockDim.x) acc[0] += part[S.chunk_begin + c];
-    block_sum<1>(acc, smem);
-    if (threadIdx.x == 0) S.image2 = acc[0];
-    return;
+  if (S.done || !S.border) return;
+  step_trace<T2>(S, S.j);
+}
+
+// ---- FP64-basis projections and updates ------------------------------------------------
+// GB300's FP64 pipe bounds both (4 FMAs per element and basis vector against 16 bytes), so the
+// reductions are kept off it as far as they go: a warp sums 2K values over its lanes by
+// exchanging halves (2K - 1 additions, against 10K for K columns summed one by one), each lane
+// holding 4 elements of w in registers across all columns.  N = 120, 31 columns: 43 us against 129 us
+// (60 of them reductions) when every block summed eight columns one by one; 52 -> 4 us at one column.
+
+// Sums v[k] over the warp's lanes; afterwards v[0] of lane l is the total of value
+// l / (32 / NV).
+template <int NV>
+__device__ __forceinline__ void warp_transpose_sum(double (&v)[NV]) {
+  const int lane = threadIdx.x & 31;
+  int off = 16;
+#pragma unroll
+  for (int s = NV / 2; s >= 1; s >>= 1, off >>= 1) {
+    const bool up = lane & off;
+#pragma unroll
+    for (int i = 0; i < s; ++i) {
+      const double send = up ? v[i] : v[i + s];
+      const double keep = up ? v[i + s] : v[i];
+      v[i] = keep + __shfl_xor_sync(0xffffffffu, send, off);
+    }
   }
-  const int nv = S.j + 1;
+  for (; off >= 1; off >>= 1) v[0] += __shfl_xor_sync(0xffffffffu, v[0], off);
+}
+
+// Projections of the lane's 4 elements onto K columns, summed over the warp into row[2 k ..].
+template <int K>
+__device__ __forceinline__ void dot_cols64(const double2* V, long long ld, const double2 (&w)[4], int left,
+                                           double* row) {
+  double acc[2 * K];
+#pragma unroll
+  for (int k = 0; k < 2 * K; ++k) acc[k] = 0;
+#pragma unroll
+  for (int k = 0; k < K; ++k) {
+    double2 v[4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) v[q] = 32 * q < left ? V[k * ld + 32 * q] : make_double2(0.0, 0.0);
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      acc[2 * k] = fma(v[q].x, w[q].x, acc[2 * k]);
+      acc[2 * k] = fma(v[q].y, w[q].y, acc[2 * k]);
+      acc[2 * k + 1] = fma(v[q].x, w[q].y, acc[2 * k + 1]);
+      acc[2 * k + 1] = fma(-v[q].y, w[q].x, acc[2 * k + 1]);
+    }
+  }
+  warp_transpose_sum<2 * K>(acc);
+  constexpr int span = 32 / (2 * K);
+  const int lane = threadIdx.x & 31;
+  if (lane % span == 0) row[lane / span] = acc[0];
+}
+
+struct Dot64Smem {
+  double row[8][2 * (kBatchMaxKrylov + 2)];  // per element group: (re, im) per column
+  double norm[8];
+};
+
+// partv[c][i] = sum over chunk c of conj(V_i) w for i < nv, and ipart[c] = |w|^2 over the chunk
+// (ipart != nullptr).  The chunk is cut into groups of 128 elements (4 per lane); the warps
+// that a chunk of fewer than 8 groups leaves free take the groups' columns in parts.
+__device__ __forceinline__ void step_dot64(const DevInst& S, int nv, int c, double2* partv, double* ipart,
+                                           Dot64Smem& sm) {
+  long long beg, end;
+  chunk_range(S, c, beg, end);
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int groups = S.chunk / 128, parts = 8 / groups;
+  const int g = warp % groups, part = warp / groups;
+  const long long e0 = beg + g * 128 + lane;
+  const int left = (int)min(end - e0, 1024LL);  // element 32 q of the lane exists when 32 q < left
+  double2 w[4];
+#pragma unroll
+  for (int q = 0; q < 4; ++q) w[q] = 32 * q < left ? ((const double2*)S.w)[e0 + 32 * q] : make_double2(0.0, 0.0);
+  if (ipart != nullptr && part == 0) {
+    double a = 0;
+#pragma unroll
+    for (int q = 0; q < 4; ++q) a = fma(w[q].y, w[q].y, fma(w[q].x, w[q].x, a));
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) a += __shfl_xor_sync(0xffffffffu, a, off);
+    if (lane == 0) sm.norm[g] = a;
+  }
+  const int per = (nv + parts - 1) / parts;
+  int k = part * per;
+  const int k1 = min(k + per, nv);
+  const double2* V = (const double2*)S.V + e0;
+  const long long ld = S.ldv;
+  double* row = sm.row[g];
+  for (; k + 16 <= k1; k += 16) dot_cols64<16>(V + k * ld, ld, w, left, row + 2 * k);
+  if (k + 8 <= k1) dot_cols64<8>(V + k * ld, ld, w, left, row + 2 * k), k += 8;
+  if (k + 4 <= k1) dot_cols64<4>(V + k * ld, ld, w, left, row + 2 * k), k += 4;
+  if (k + 2 <= k1) dot_cols64<2>(V + k * ld, ld, w, left, row + 2 * k), k += 2;
+  if (k < k1) dot_cols64<1>(V + k * ld, ld, w, left, row + 2 * k);
+  __syncthreads();
+  for (int i = threadIdx.x; i < 2 * nv; i += blockDim.x) {
+    double t = 0;
+    for (int q = 0; q < groups; ++q) t += sm.row[q][i];
+    reinterpret_cast<double*>(partv + (long long)c * S.pstride)[i] = t;
+  }
+  if (ipart != nullptr && threadIdx.x == 0) {
+    double t = 0;
+    for (int q = 0; q < groups; ++q) t += sm.norm[q];
+    ipart[c] = t;
+  }
+  __syncthreads();  // sm is free for the block's next chunk
+}
+
+// pass 1: hA and |w|^2; pass 2 only for jobs that reorthogonalise.
+__global__ void __launch_bounds__(kRT, 2)
+    k_step_dot64(const DevInst* st, const int* chunk_inst, double2* partv, double* ipart, int second) {
+  __shared__ Dot64Smem sm;
+  const DevInst& S = st[chunk_inst[blockIdx.x]];
+  if (S.done || (second && !S.reorth)) return;
+  step_dot64(S, S.j + 1, blockIdx.x, partv, ipart, sm);
+}
+
+// which 0: hA, 1: hB (jobs that reorthogonalise).  Grid (instances, column groups): warp w of
+// block (x, y) reduces column i = y * warps + w, so every column of every instance has its own
+// warp (one warp walking several columns left a single SM reducing a long chunk list per
+// column).
+__global__ void __launch_bounds__(kRT)
+    k_step_mdot_final(const DevInst* st, const int* __restrict__ nchunks, const double2* partv) {
+  const DevInst& S = st[blockIdx.x];
+  if (S.done || !S.reorth) return;
   const int i = blockIdx.y * (blockDim.x >> 5) + (threadIdx.x >> 5);
-  if (i >= nv) return;  // warp-uniform
-  const double2 v = warp_chunk_sum(partv, S.chunk_begin, nchunks[blockIdx.x], i);
-  if ((threadIdx.x & 31) == 0) S.hA[i] = v;
+  if (i > S.j) return;  // warp-uniform
+  const double2 v = warp_chunk_sum(partv, S.chunk_begin, nchunks[blockIdx.x], S.pstride, i);
+  if ((threadIdx.x & 31) == 0) S.hB[i] = v;
 }
 
 // |w|^2 of job S from its chunk partials (thread t sums partials t, t + 256, ..., then a
-// deterministic block sum), broadcast to the whole block: every block of the job obtains
-// the same value.
-__device__ __forceinline__ double job_norm2(const DevInst& S, int nchunks, const double* __restrict__ part) {
+// deterministic block sum); the result is valid in thread 0.
+__device__ __forceinline__ double job_norm2(const DevInst& S, int nchunks, const double* part) {
   __shared__ double smem[32];
-  __shared__ double total;
   double acc[1] = {0};
   for (int c = threadIdx.x; c < nchunks; c += blockDim.x) acc[0] += part[S.chunk_begin + c];
   block_sum<1>(acc, smem);
-  if (threadIdx.x == 0) total = acc[0];
-  __syncthreads();
-  return total;
+  __syncthreads();  // smem is free for the block's next job
+  return acc[0];
 }
 
-// w -= sum_i V_i h_i (which 0: hA, 1: hB); with part != nullptr also |w|^2 partials.
-template <typename T2>
+// The first-pass reductions of a step in one launch: blocks (x, y < gridDim.y - 1) reduce the
+// projections into hA, blocks (x, gridDim.y - 1) the image norm |L V_j|^2.
 __global__ void __launch_bounds__(kRT)
-    k_step_maxpy(const DevInst* __restrict__ st, const int* __restrict__ chunk_inst, int which, double* __restrict__ part) {
-  __shared__ double2 hs[kMaxDots];
-  __shared__ double smem[32];
-  const DevInst& S = st[chunk_inst[blockIdx.x]];
+    k_step_first_final(DevInst* st, const int* __restrict__ nchunks, const double2* partv, const double* part) {
+  DevInst& S = st[blockIdx.x];
   if (S.done) return;
-  const int nv = S.j + 1;
-  const double2* h = which == 0 ? S.hA : S.hB;
-  for (int i = threadIdx.x; i < nv; i += blockDim.x) hs[i] = h[i];
+  if (blockIdx.y == gridDim.y - 1) {  // image norm (block-uniform)
+    const double v = job_norm2(S, nchunks[blockIdx.x], part);
+    if (threadIdx.x == 0) S.image2 = v;
+    return;
+  }
+  const int i = blockIdx.y * (blockDim.x >> 5) + (threadIdx.x >> 5);
+  if (i > S.j) return;  // warp-uniform
+  const double2 v = warp_chunk_sum(partv, S.chunk_begin, nchunks[blockIdx.x], S.pstride, i);
+  if ((threadIdx.x & 31) == 0) S.hA[i] = v;
+}
+
+// After the first update (whole block): |w1|^2 and whether the job reorthogonalises.  Selective
+// reorthogonalisation (Daniel, Gragg, Kaufman, Stewart, Math. Comp. 30, 772 (1976)): when
+// |w1|^2 >= |w0|^2 / 2 (w0 = L V_j before any projection) the first pass has left w orthogonal
+// to the basis to working precision, and the second pass is skipped (zero hB).
+__device__ __forceinline__ void step_norm1(DevInst& S, int nv, int nchunks, const double* part) {
+  const double v = job_norm2(S, nchunks, part);
+  if (threadIdx.x == 0) {
+    S.rem2 = v;
+    S.reorth = v < 0.5 * S.image2 ? 1 : 0;
+  }
+  for (int i = threadIdx.x; i < nv; i += blockDim.x) S.hB[i] = make_double2(0.0, 0.0);
+}
+
+// One block per job.  second 0: step_norm1; 1: |w|^2 after the second update of a job that
+// reorthogonalised.
+__global__ void __launch_bounds__(kRT)
+    k_step_norm(DevInst* st, const int* __restrict__ nchunks, const double* part, int second) {
+  DevInst& S = st[blockIdx.x];
+  if (S.done) return;
+  if (!second) {
+    step_norm1(S, S.j + 1, nchunks[blockIdx.x], part);
+  } else if (S.reorth) {
+    const double v = job_norm2(S, nchunks[blockIdx.x], part);
+    if (threadIdx.x == 0) S.rem2 = v;
+  }
+}
+
+// w -= sum_i V_i h_i over chunk c and part[c] = |w|^2 of the result.  A thread holds up to 4
+// elements; chunks of 128 elements split the columns between the block's two halves.
+struct Axpy64Smem {
+  double2 h[kBatchMaxKrylov + 2];
+  double2 half[128];
+  double red[32];
+};
+
+__device__ __forceinline__ void axpy_cols64(const double2* V, long long ld, const double2* h, int k0, int k1,
+                                            double2& w) {
+#pragma unroll 8
+  for (int i = k0; i < k1; ++i) {
+    const double2 v = V[i * ld];
+    const double2 c = h[i];
+    w.x = fma(-v.x, c.x, w.x);
+    w.x = fma(v.y, c.y, w.x);
+    w.y = fma(-v.x, c.y, w.y);
+    w.y = fma(-v.y, c.x, w.y);
+  }
+}
+
+__device__ __forceinline__ void step_axpy64(const DevInst& S, int nv, int c, const double2* h, double* part,
+                                            Axpy64Smem& sm) {
+  for (int i = threadIdx.x; i < nv; i += blockDim.x) sm.h[i] = h[i];
   __syncthreads();
   long long beg, end;
-  chunk_range(S, blockIdx.x, beg, end);
-  const long long dim = S.ldv;
-  const T2* V = (const T2*)S.V;
-  T2* w = (T2*)S.w;
-  constexpr bool F32 = sizeof(T2) == sizeof(float2);
+  chunk_range(S, c, beg, end);
+  const double2* V = (const double2*)S.V;
+  double2* w = (double2*)S.w;
+  const long long ld = S.ldv;
   double acc[1] = {0};
-  for (long long e = beg + threadIdx.x; e < end; e += blockDim.x) {
-    double2 out;
-    if (F32) {  // FP32 basis: FP32 update
-      float2 wv = reinterpret_cast<const float2*>(w)[e];
-      for (int i = 0; i < nv; ++i) {
-        const float2 v = reinterpret_cast<const float2*>(V)[(long long)i * dim + e];
-        const float cx = (float)hs[i].x, cy = (float)hs[i].y;
-        wv.x = fmaf(-v.x, cx, wv.x);
-        wv.x = fmaf(v.y, cy, wv.x);
-        wv.y = fmaf(-v.x, cy, wv.y);
-        wv.y = fmaf(-v.y, cx, wv.y);
-      }
-      reinterpret_cast<float2*>(w)[e] = wv;
-      out = make_double2(wv.x, wv.y);
-    } else {
-      double2 wv = ld2(w + e);
-      for (int i = 0; i < nv; ++i) {
-        const double2 v = ld2(V + (long long)i * dim + e);
-        wv.x = fma(-v.x, hs[i].x, wv.x);
-        wv.x = fma(v.y, hs[i].y, wv.x);
-        wv.y = fma(-v.x, hs[i].y, wv.y);
-        wv.y = fma(-v.y, hs[i].x, wv.y);
-      }
-      st2(w + e, wv.x, wv.y);
-      out = wv;
+  if (S.chunk == 128) {  // block-uniform
+    const int lo = threadIdx.x & 127, upper = threadIdx.x >> 7;
+    const long long e = beg + lo;
+    const int mid = (nv + 1) / 2;
+    double2 v = make_double2(0.0, 0.0);
+    if (e < end) {
+      if (!upper) v = w[e];
+      axpy_cols64(V + e, ld, sm.h, upper ? mid : 0, upper ? nv : mid, v);
     }
-    acc[0] = fma(out.x, out.x, acc[0]);
-    acc[0] = fma(out.y, out.y, acc[0]);
+    if (upper) sm.half[lo] = v;
+    __syncthreads();
+    if (!upper && e < end) {
+      v.x += sm.half[lo].x;
+      v.y += sm.half[lo].y;
+      w[e] = v;
+      acc[0] = fma(v.y, v.y, v.x * v.x);
+    }
+  } else {
+    for (long long e = beg + threadIdx.x; e < end; e += blockDim.x) {
+      double2 v = w[e];
+      axpy_cols64(V + e, ld, sm.h, 0, nv, v);
+      w[e] = v;
+      acc[0] = fma(v.x, v.x, acc[0]);
+      acc[0] = fma(v.y, v.y, acc[0]);
+    }
   }
-  if (part) {
-    block_sum<1>(acc, smem);
-    if (threadIdx.x == 0) part[blockIdx.x] = acc[0];
-  }
+  block_sum<1>(acc, sm.red);
+  if (threadIdx.x == 0) part[c] = acc[0];
+  __syncthreads();  // sm is free for the block's next chunk
 }
 
-// V_{j+1} = w / |w| (zero on an exact breakdown).  Every block reduces the job's |w|^2
-// partials itself (the job's first block stores rem2 for the step finish), so no separate
-// reduction launch sits between the second-pass update and the normalisation.
-template <typename T2>
-__global__ void __launch_bounds__(kRT) k_step_normalize(DevInst* __restrict__ st, const int* __restrict__ chunk_inst,
-                                                        const int* __restrict__ nchunks, const double* __restrict__ part) {
-  const int inst = chunk_inst[blockIdx.x];
-  DevInst& S = st[inst];
-  if (S.done) return;
-  const double rem2 = job_norm2(S, nchunks[inst], part);
-  if (blockIdx.x == S.chunk_begin && threadIdx.x == 0) S.rem2 = rem2;
-  const double r = sqrt(rem2);
+__global__ void __launch_bounds__(kRT, 2)
+    k_step_axpy64(const DevInst* st, const int* chunk_inst, double* part, int second) {
+  __shared__ Axpy64Smem sm;
+  const DevInst& S = st[chunk_inst[blockIdx.x]];
+  if (S.done || (second && !S.reorth)) return;
+  step_axpy64(S, S.j + 1, blockIdx.x, second ? S.hB : S.hA, part, sm);
+}
+
+// V_{j+1} = w / |w| over chunk c (zero on an exact breakdown).
+__device__ __forceinline__ void step_normalize64(const DevInst& S, int j, int c) {
+  const double r = sqrt(S.rem2);
   const double f = r > 0 ? 1.0 / r : 0.0;
   long long beg, end;
-  chunk_range(S, blockIdx.x, beg, end);
-  const T2* w = (const T2*)S.w;
-  T2* out = (T2*)S.V + (long long)(S.j + 1) * S.ldv;
+  chunk_range(S, c, beg, end);
+  const double2* w = (const double2*)S.w;
+  double2* out = (double2*)S.V + (long long)(j + 1) * S.ldv;
   for (long long e = beg + threadIdx.x; e < end; e += blockDim.x) {
-    const double2 v = ld2(w + e);
-    st2(out + e, f * v.x, f * v.y);
+    const double2 v = w[e];
+    out[e] = make_double2(f * v.x, f * v.y);
   }
+}
+
+__global__ void __launch_bounds__(kRT) k_step_normalize64(const DevInst* st, const int* chunk_inst) {
+  const DevInst& S = st[chunk_inst[blockIdx.x]];
+  if (S.done) return;
+  step_normalize64(S, S.j, blockIdx.x);
 }
 
 // ---- FP32-basis CGS2 kernels: pairs of complex elements per 16-byte load ---------------
@@ -812,51 +947,35 @@ __device__ __forceinline__ void pair_terms(const float4 a, const float4 b, DF& r
 // its chunk for the image norm |L V_j| (the expv error estimate and the reorthogonalisation
 // test) -- the same pairs in the same order as a separate sweep over w would take -- while w
 // is staged anyway.
-//
-// Second pass with npart1 (selective reorthogonalisation, Daniel-Gragg-Kaufman-Stewart): the
-// block first sums its job's |w1|^2 partials of the first-pass update; when |w1|^2 >= |w0|^2
-// / 2 (w0 = L V_j before any projection, image2) the first pass left w orthogonal to the
-// basis to working precision, so the block writes zero projections instead of sweeping the
-// basis again, and the job's first block records the choice in reorth for the update.
 template <int CH>
-__global__ void __launch_bounds__(kRT, 3)
-    k_step_mdot_f32(DevInst* __restrict__ st, const int* __restrict__ chunk_inst, double2* __restrict__ partv,
-                    double* __restrict__ ipart, const int* __restrict__ nchunks, const double* __restrict__ npart1) {
-  constexpr int kPairs = CH / 2 / kRT;  // element pairs per thread and chunk
-  __shared__ float4 wsm[CH / 2];
+struct Dot32Smem {
+  float4 w[CH / 2];
   // per warp: (re.hi, re.lo, im.hi, im.lo) of each basis column (at most kBatchMaxKrylov + 1);
   // sized to the engine's Krylov limit so the block stays inside 48 KB of static shared memory
-  __shared__ float4 red[kBatchMaxKrylov + 2][kRT / 32];
-  const int inst = chunk_inst[blockIdx.x];
-  DevInst& S = st[inst];
-  if (S.done) return;
-  const int nv = S.j + 1;
-  if (npart1 != nullptr) {
-    const bool reorth = job_norm2(S, nchunks[inst], npart1) < 0.5 * S.image2;  // block-uniform
-    if (blockIdx.x == S.chunk_begin && threadIdx.x == 0) S.reorth = reorth ? 1 : 0;
-    if (!reorth) {
-      for (int kk = threadIdx.x; kk < nv; kk += blockDim.x)
-        partv[(long long)blockIdx.x * kMaxDots + kk] = make_double2(0.0, 0.0);
-      return;
-    }
-  }
+  float4 red[kBatchMaxKrylov + 2][kRT / 32];
+};
+
+template <int CH>
+__device__ __forceinline__ void step_dot32(const DevInst& S, int nv, int c, double2* partv, double* ipart,
+                                           Dot32Smem<CH>& sm) {
+  constexpr int kPairs = CH / 2 / kRT;  // element pairs per thread and chunk
   long long beg, end;
-  pair_range(S, blockIdx.x, beg, end);
+  pair_range(S, c, beg, end);
   const int npair = (int)(end - beg);
-  const float4* __restrict__ w4 = reinterpret_cast<const float4*>(S.w) + beg;
-  const float4* __restrict__ V4 = reinterpret_cast<const float4*>(S.V) + beg;
+  const float4* w4 = reinterpret_cast<const float4*>(S.w) + beg;
+  const float4* V4 = reinterpret_cast<const float4*>(S.V) + beg;
   const long long ld4 = S.ldv / 2;
   DF nrm{0.f, 0.f};
 #pragma unroll
   for (int q = 0; q < kPairs; ++q) {
     const int p = threadIdx.x + q * kRT;
     const float4 wv = p < npair ? w4[p] : make_float4(0.f, 0.f, 0.f, 0.f);
-    wsm[p] = wv;
+    sm.w[p] = wv;
     if (p < npair) df_add(nrm, fmaf(wv.x, wv.x, fmaf(wv.y, wv.y, fmaf(wv.z, wv.z, wv.w * wv.w))));
   }
   if (ipart != nullptr) {  // block-uniform
-    const double r = block_df_sum(nrm, reinterpret_cast<float2*>(&red[0][0]));
-    if (threadIdx.x == 0) ipart[blockIdx.x] = r;
+    const double r = block_df_sum(nrm, reinterpret_cast<float2*>(&sm.red[0][0]));
+    if (threadIdx.x == 0) ipart[c] = r;
   }
   __syncthreads();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -864,8 +983,8 @@ __global__ void __launch_bounds__(kRT, 3)
   int k = 0;
   // two columns per iteration: 2 * kPairs independent 16-byte loads in flight per thread
   for (; k + 1 < nv; k += 2) {
-    const float4* __restrict__ c0 = V4 + (long long)k * ld4;
-    const float4* __restrict__ c1 = c0 + ld4;
+    const float4* c0 = V4 + (long long)k * ld4;
+    const float4* c1 = c0 + ld4;
     float4 a[kPairs], b[kPairs];
 #pragma unroll
     for (int q = 0; q < kPairs; ++q) {
@@ -876,7 +995,7 @@ __global__ void __launch_bounds__(kRT, 3)
     DF r0{0.f, 0.f}, i0{0.f, 0.f}, r1{0.f, 0.f}, i1{0.f, 0.f};
 #pragma unroll
     for (int q = 0; q < kPairs; ++q) {
-      const float4 wv = wsm[threadIdx.x + q * kRT];
+      const float4 wv = sm.w[threadIdx.x + q * kRT];
       pair_terms(a[q], wv, r0, i0);
       pair_terms(b[q], wv, r1, i1);
     }
@@ -885,34 +1004,44 @@ __global__ void __launch_bounds__(kRT, 3)
     r1 = warp_df_sum(r1);
     i1 = warp_df_sum(i1);
     if (lane == 0) {
-      red[k][warp] = make_float4(r0.hi, r0.lo, i0.hi, i0.lo);
-      red[k + 1][warp] = make_float4(r1.hi, r1.lo, i1.hi, i1.lo);
+      sm.red[k][warp] = make_float4(r0.hi, r0.lo, i0.hi, i0.lo);
+      sm.red[k + 1][warp] = make_float4(r1.hi, r1.lo, i1.hi, i1.lo);
     }
   }
   if (k < nv) {
-    const float4* __restrict__ c0 = V4 + (long long)k * ld4;
+    const float4* c0 = V4 + (long long)k * ld4;
     DF r0{0.f, 0.f}, i0{0.f, 0.f};
 #pragma unroll
     for (int q = 0; q < kPairs; ++q) {
       const int p = threadIdx.x + q * kRT;
-      pair_terms(p < npair ? c0[p] : zero, wsm[p], r0, i0);
+      pair_terms(p < npair ? c0[p] : zero, sm.w[p], r0, i0);
     }
     r0 = warp_df_sum(r0);
     i0 = warp_df_sum(i0);
-    if (lane == 0) red[k][warp] = make_float4(r0.hi, r0.lo, i0.hi, i0.lo);
+    if (lane == 0) sm.red[k][warp] = make_float4(r0.hi, r0.lo, i0.hi, i0.lo);
   }
   __syncthreads();
   for (int kk = threadIdx.x; kk < nv; kk += blockDim.x) {
     DF sr{0.f, 0.f}, si{0.f, 0.f};
 #pragma unroll
     for (int wdx = 0; wdx < kRT / 32; ++wdx) {
-      const float4 r = red[kk][wdx];
+      const float4 r = sm.red[kk][wdx];
       sr = df_sum(sr, DF{r.x, r.y});
       si = df_sum(si, DF{r.z, r.w});
     }
-    partv[(long long)blockIdx.x * kMaxDots + kk] =
+    partv[(long long)c * S.pstride + kk] =
         make_double2((double)sr.hi + (double)sr.lo, (double)si.hi + (double)si.lo);
   }
+  __syncthreads();  // sm is free for the block's next chunk
+}
+
+template <int CH>
+__global__ void __launch_bounds__(kRT, 3)
+    k_step_mdot_f32(const DevInst* st, const int* chunk_inst, double2* partv, double* ipart, int second) {
+  __shared__ Dot32Smem<CH> sm;
+  const DevInst& S = st[chunk_inst[blockIdx.x]];
+  if (S.done || (second && !S.reorth)) return;
+  step_dot32<CH>(S, S.j + 1, blockIdx.x, partv, ipart, sm);
 }
 
 // cout (+)= sum_k ccoef[k] V_k for an FP32 basis in double-float arithmetic: each FP64
@@ -968,74 +1097,72 @@ __global__ void __launch_bounds__(kRT)
   }
 }
 
-// w -= sum_i V_i h_i for an FP32 basis (which 0: hA, 1: hB), FP32 update; with part also
-// the double-float |w|^2 partial of the result.
-// With npart1 (second pass under selective reorthogonalisation) a job that skipped the second
-// projection keeps w and forwards its first-pass |w1|^2 partials as this pass's partials.
-__global__ void __launch_bounds__(kRT)
-    k_step_maxpy_f32(const DevInst* __restrict__ st, const int* __restrict__ chunk_inst, int which,
-                     double* __restrict__ part, const double* __restrict__ npart1) {
-  __shared__ float2 hs[kMaxDots];
-  __shared__ float2 smem[32];
-  const DevInst& S = st[chunk_inst[blockIdx.x]];
-  if (S.done) return;
-  if (npart1 != nullptr && !S.reorth) {
-    if (threadIdx.x == 0) part[blockIdx.x] = npart1[blockIdx.x];
-    return;
-  }
-  const int nv = S.j + 1;
-  const double2* h = which == 0 ? S.hA : S.hB;
-  for (int i = threadIdx.x; i < nv; i += blockDim.x) hs[i] = make_float2((float)h[i].x, (float)h[i].y);
+// w -= sum_i V_i h_i over chunk c of an FP32 basis, FP32 update, and the double-float |w|^2
+// partial of the result.
+struct Axpy32Smem {
+  float2 h[kBatchMaxKrylov + 2];
+  float2 red[32];
+};
+
+__device__ __forceinline__ void step_axpy32(const DevInst& S, int nv, int c, const double2* h, double* part,
+                                            Axpy32Smem& sm) {
+  for (int i = threadIdx.x; i < nv; i += blockDim.x) sm.h[i] = make_float2((float)h[i].x, (float)h[i].y);
   __syncthreads();
   long long beg, end;
-  pair_range(S, blockIdx.x, beg, end);
-  float4* __restrict__ w4 = reinterpret_cast<float4*>(S.w);
-  const float4* __restrict__ V4 = reinterpret_cast<const float4*>(S.V);
+  pair_range(S, c, beg, end);
+  float4* w4 = reinterpret_cast<float4*>(S.w);
+  const float4* V4 = reinterpret_cast<const float4*>(S.V);
   const long long ld4 = S.ldv / 2;
   DF nrm{0.f, 0.f};
   for (long long p = beg + threadIdx.x; p < end; p += blockDim.x) {
     float4 wv = w4[p];
-#pragma unroll 4
+#pragma unroll 8
     for (int i = 0; i < nv; ++i) {
       const float4 v = V4[(long long)i * ld4 + p];
-      const float2 c = hs[i];
-      wv.x = fmaf(-v.x, c.x, wv.x);
-      wv.x = fmaf(v.y, c.y, wv.x);
-      wv.y = fmaf(-v.x, c.y, wv.y);
-      wv.y = fmaf(-v.y, c.x, wv.y);
-      wv.z = fmaf(-v.z, c.x, wv.z);
-      wv.z = fmaf(v.w, c.y, wv.z);
-      wv.w = fmaf(-v.z, c.y, wv.w);
-      wv.w = fmaf(-v.w, c.x, wv.w);
+      const float2 cf = sm.h[i];
+      wv.x = fmaf(-v.x, cf.x, wv.x);
+      wv.x = fmaf(v.y, cf.y, wv.x);
+      wv.y = fmaf(-v.x, cf.y, wv.y);
+      wv.y = fmaf(-v.y, cf.x, wv.y);
+      wv.z = fmaf(-v.z, cf.x, wv.z);
+      wv.z = fmaf(v.w, cf.y, wv.z);
+      wv.w = fmaf(-v.z, cf.y, wv.w);
+      wv.w = fmaf(-v.w, cf.x, wv.w);
     }
     w4[p] = wv;
     df_add(nrm, fmaf(wv.x, wv.x, fmaf(wv.y, wv.y, fmaf(wv.z, wv.z, wv.w * wv.w))));
   }
-  if (part) {
-    const double r = block_df_sum(nrm, smem);
-    if (threadIdx.x == 0) part[blockIdx.x] = r;
-  }
+  const double r = block_df_sum(nrm, sm.red);
+  if (threadIdx.x == 0) part[c] = r;
+  __syncthreads();  // sm is free for the block's next chunk
 }
 
-// V_{j+1} = w / |w| (zero on an exact breakdown), FP32 basis; |w|^2 as in k_step_normalize.
 __global__ void __launch_bounds__(kRT)
-    k_step_normalize_f32(DevInst* __restrict__ st, const int* __restrict__ chunk_inst, const int* __restrict__ nchunks,
-                         const double* __restrict__ part) {
-  const int inst = chunk_inst[blockIdx.x];
-  DevInst& S = st[inst];
-  if (S.done) return;
-  const double rem2 = job_norm2(S, nchunks[inst], part);
-  if (blockIdx.x == S.chunk_begin && threadIdx.x == 0) S.rem2 = rem2;
-  const double r = sqrt(rem2);
+    k_step_maxpy_f32(const DevInst* st, const int* chunk_inst, double* part, int second) {
+  __shared__ Axpy32Smem sm;
+  const DevInst& S = st[chunk_inst[blockIdx.x]];
+  if (S.done || (second && !S.reorth)) return;
+  step_axpy32(S, S.j + 1, blockIdx.x, second ? S.hB : S.hA, part, sm);
+}
+
+// V_{j+1} = w / |w| over chunk c (zero on an exact breakdown), FP32 basis.
+__device__ __forceinline__ void step_normalize32(const DevInst& S, int j, int c) {
+  const double r = sqrt(S.rem2);
   const float f = r > 0 ? (float)(1.0 / r) : 0.f;
   long long beg, end;
-  pair_range(S, blockIdx.x, beg, end);
-  const float4* __restrict__ w4 = reinterpret_cast<const float4*>(S.w);
-  float4* __restrict__ out = reinterpret_cast<float4*>(S.V) + (long long)(S.j + 1) * (S.ldv / 2);
+  pair_range(S, c, beg, end);
+  const float4* w4 = reinterpret_cast<const float4*>(S.w);
+  float4* out = reinterpret_cast<float4*>(S.V) + (long long)(j + 1) * (S.ldv / 2);
   for (long long p = beg + threadIdx.x; p < end; p += blockDim.x) {
     const float4 v = w4[p];
     out[p] = make_float4(f * v.x, f * v.y, f * v.z, f * v.w);
   }
+}
+
+__global__ void __launch_bounds__(kRT) k_step_normalize_f32(const DevInst* st, const int* chunk_inst) {
+  const DevInst& S = st[chunk_inst[blockIdx.x]];
+  if (S.done) return;
+  step_normalize32(S, S.j, blockIdx.x);
 }
 
 // Per instance (one warp): records Hessenberg column j, applies the GMRES rotations and stop
@@ -1043,17 +1170,20 @@ __global__ void __launch_bounds__(kRT)
 // fill and the stored rotations into shared memory in parallel; lane 0 then runs the
 // sequential rotation arithmetic on shared memory (the same operations in the same order
 // as a single-thread pass over global memory, whose dependent loads dominated the step) and
-// the warp writes the column back.
-__global__ void __launch_bounds__(32) k_step_finish(DevInst* __restrict__ st, int n) {
-  __shared__ double2 colv[kBatchMaxKrylov + 2];
-  __shared__ double csv[kBatchMaxKrylov + 2];
-  __shared__ double2 snv[kBatchMaxKrylov + 2];
-  const int i = blockIdx.x;
-  if (i >= n) return;
-  DevInst& S = st[i];
-  if (S.done) return;
-  const int lane = threadIdx.x;
-  const int j = S.j;
+// the warp writes the column back.  True (in lane 0) when the job takes no further step.  Not
+// inlined: the step kernel and k_cycle share one body, so both round alike.
+struct FinishSmem {
+  double2 col[kBatchMaxKrylov + 2];
+  double cs[kBatchMaxKrylov + 2];
+  double2 sn[kBatchMaxKrylov + 2];
+};
+
+__device__ __noinline__ bool step_finish(DevInst& S, int j, FinishSmem& sm) {
+  const int lane = threadIdx.x & 31;
+  double2* colv = sm.col;
+  double* csv = sm.cs;
+  double2* snv = sm.sn;
+  bool stop = false;
   const int ld = S.ldh;
   double2* col = S.H + (long long)j * ld;
   double2* cs = S.csn;
@@ -1071,7 +1201,7 @@ __global__ void __launch_bounds__(32) k_step_finish(DevInst* __restrict__ st, in
     colv[j + 1] = make_double2(rem, 0.0);
     S.image[j] = sqrt(S.image2);
     S.kdone = j + 1;
-    bool stop = (j + 1 >= S.m) || rem == 0.0 || (long long)(j + 1) == S.dim;
+    stop = (j + 1 >= S.m) || rem == 0.0 || (long long)(j + 1) == S.dim;
     if (S.givens) {
       for (int r = 0; r < j; ++r) {
         const double2 h1 = colv[r], h2 = colv[r + 1];
@@ -1114,13 +1244,186 @@ __global__ void __launch_bounds__(32) k_step_finish(DevInst* __restrict__ st, in
       S.g[j + 1] = make_double2(-csg1.x + c * g2.x, -csg1.y + c * g2.y);
       if (hypot(S.g[j + 1].x, S.g[j + 1].y) <= S.tol) stop = true;
     }
+  }
+  __syncwarp();
+  for (int r = lane; r < ld; r += 32) col[r] = colv[r];
+  __syncwarp();
+  return stop;
+}
+
+__global__ void __launch_bounds__(32) k_step_finish(DevInst* st) {
+  __shared__ FinishSmem sm;
+  DevInst& S = st[blockIdx.x];
+  if (S.done) return;
+  const int j = S.j;
+  const bool stop = step_finish(S, j, sm);
+  if (threadIdx.x == 0) {
     if (stop)
       S.done = 1;
     else
       S.j = j + 1;
   }
-  __syncwarp();
-  for (int r = lane; r < ld; r += 32) col[r] = colv[r];
+}
+
+// ---- one launch per Krylov cycle -------------------------------------------------------
+// The m steps of a small job set in one cooperative launch: its blocks walk each phase's work
+// list and meet at a grid barrier between phases.  As separate launches (one graph of 11 nodes
+// per step) the phases of such sets last about as long as a launch takes to start and drain.
+// Per entry, chunk and job the arithmetic is that of the step kernels.  Measured per Arnoldi
+// step, graph -> one launch: N = 8 FP64 68 -> 35 us, N = 120 FP32 63 -> 37 us (m = 30).
+
+// Grid barrier: arrivals are counted up over the whole launch.  A block that waits in vain
+// raises err, which ends every wait of the launch; the host reads it after the cycle.
+struct GridBar {
+  unsigned count;
+  int err;
+};
+constexpr int kGridWaitLimit = 1 << 24;  // polls, several seconds
+
+__device__ __forceinline__ bool grid_sync(GridBar* bar, unsigned& target) {
+  if (gridDim.x == 1) {
+    __syncthreads();
+    return true;
+  }
+  __shared__ int ok;
+  __syncthreads();
+  target += gridDim.x;
+  if (threadIdx.x == 0) {
+    __threadfence();  // the block's writes before its arrival
+    atomicAdd(&bar->count, 1u);
+    ok = 1;
+    for (int it = 0;; ++it) {
+      unsigned seen;
+      asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(&bar->count) : "memory");
+      if ((int)(seen - target) >= 0) break;
+      if (it >= kGridWaitLimit || ((it & 1023) == 1023 && atomicAdd(&bar->err, 0) != 0)) {
+        atomicExch(&bar->err, 1);
+        ok = 0;
+        break;
+      }
+    }
+    __threadfence();  // the other blocks' writes after it
+  }
+  __syncthreads();
+  return ok != 0;
+}
+
+template <bool F32>
+__global__ void __launch_bounds__(kRT, 2)
+    k_cycle(DevInst* st, int n, const int* chunk_inst, int nchunk, const int* item_inst, const int* item_local,
+            int nitem, const int* nchunks, double2* partv, double* part, int steps, int border, GridBar* bar) {
+  __shared__ __align__(16) union {
+    Dot64Smem dot64;
+    Axpy64Smem axpy64;
+    Dot32Smem<kBatchChunkSmall> dot32;
+    Axpy32Smem axpy32;
+    FinishSmem finish;
+  } sm;
+  using T2 = typename Vec2<typename std::conditional<F32, float, double>::type>::type;
+  const int nblk = gridDim.x, blk = blockIdx.x;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  unsigned target = 0;
+  double* part1 = part + nchunk;
+  for (int j = 0; j < steps; ++j) {
+    // stop[j & 1] holds a job's state for step j; the finish of step j writes the other one
+    const int ph = j & 1;
+    auto live = [&](const DevInst& S) { return !S.stop[ph]; };
+    bool any = false;
+    for (int i = threadIdx.x; i < n; i += kRT) any = any || live(st[i]);
+    if (!__syncthreads_or(any)) return;  // uniform over the grid
+    if (border) {
+      for (int i = blk; i < n; i += nblk)
+        if (live(st[i]) && st[i].border) step_trace<T2>(st[i], j);
+      if (!grid_sync(bar, target)) return;
+    }
+    for (int t = blk; t < nitem; t += nblk) {
+      DevInst& S = st[item_inst[t]];
+      if (!live(S)) continue;
+      const T2* x = (const T2*)S.V + (long long)j * S.ldv;
+      const double2* alpha = S.border ? &S.alpha : nullptr;
+      if constexpr (F32)
+        strip_apply32<false>(S, item_local[t], x, (float2*)S.w, alpha);
+      else
+        strip_apply<false>(S, item_local[t], x, (double2*)S.w, S.scale, alpha);
+    }
+    if (!grid_sync(bar, target)) return;
+    auto dots = [&](bool second) {
+      for (int c = blk; c < nchunk; c += nblk) {
+        const DevInst& S = st[chunk_inst[c]];
+        if (!live(S) || (second && !S.reorth)) continue;
+        if constexpr (F32)
+          step_dot32<kBatchChunkSmall>(S, j + 1, c, partv, second ? nullptr : part, sm.dot32);
+        else
+          step_dot64(S, j + 1, c, partv, second ? nullptr : part, sm.dot64);
+      }
+    };
+    auto finals = [&](bool second) {  // one warp per (job, column), spread over the blocks
+      for (int t = blk + nblk * warp; t < n * (j + 1); t += nblk * (kRT / 32)) {
+        const int i = t / (j + 1), k = t - i * (j + 1);
+        const DevInst& S = st[i];
+        if (!live(S) || (second && !S.reorth)) continue;
+        const double2 v = warp_chunk_sum(partv, S.chunk_begin, nchunks[i], S.pstride, k);
+        if (lane == 0) (second ? S.hB : S.hA)[k] = v;
+      }
+    };
+    auto update = [&](bool second) {
+      for (int c = blk; c < nchunk; c += nblk) {
+        const DevInst& S = st[chunk_inst[c]];
+        if (!live(S) || (second && !S.reorth)) continue;
+        if constexpr (F32)
+          step_axpy32(S, j + 1, c, second ? S.hB : S.hA, second ? part : part1, sm.axpy32);
+        else
+          step_axpy64(S, j + 1, c, second ? S.hB : S.hA, second ? part : part1, sm.axpy64);
+      }
+    };
+    dots(false);
+    if (!grid_sync(bar, target)) return;
+    for (int i = nblk - 1 - blk; i < n; i += nblk) {
+      if (!live(st[i])) continue;
+      const double v = job_norm2(st[i], nchunks[i], part);
+      if (threadIdx.x == 0) st[i].image2 = v;
+    }
+    finals(false);
+    if (!grid_sync(bar, target)) return;
+    update(false);
+    if (!grid_sync(bar, target)) return;
+    for (int i = blk; i < n; i += nblk)
+      if (live(st[i])) step_norm1(st[i], j + 1, nchunks[i], part1);
+    if (!grid_sync(bar, target)) return;
+    any = false;
+    for (int i = threadIdx.x; i < n; i += kRT) any = any || (live(st[i]) && st[i].reorth);
+    if (__syncthreads_or(any)) {  // uniform over the grid
+      dots(true);
+      if (!grid_sync(bar, target)) return;
+      finals(true);
+      if (!grid_sync(bar, target)) return;
+      update(true);
+      if (!grid_sync(bar, target)) return;
+      for (int i = blk; i < n; i += nblk) {
+        if (!live(st[i]) || !st[i].reorth) continue;
+        const double v = job_norm2(st[i], nchunks[i], part);
+        if (threadIdx.x == 0) st[i].rem2 = v;
+      }
+      if (!grid_sync(bar, target)) return;
+    }
+    // the last block's first warp finishes the first job beside the normalisation, and so on
+    for (int c = blk; c < nchunk; c += nblk) {
+      const DevInst& S = st[chunk_inst[c]];
+      if (!live(S)) continue;
+      if constexpr (F32)
+        step_normalize32(S, j, c);
+      else
+        step_normalize64(S, j, c);
+    }
+    __syncthreads();
+    if (warp == 0)
+      for (int i = nblk - 1 - blk; i < n; i += nblk) {
+        DevInst& S = st[i];
+        const bool stop = live(S) ? step_finish(S, j, sm.finish) : true;
+        if (lane == 0) S.stop[ph ^ 1] = stop;
+      }
+    if (!grid_sync(bar, target)) return;
+  }
 }
 
 // Dense normalized trace vector v = t / (t^H t) in reference coordinates.
@@ -1753,6 +2056,11 @@ Engine::Engine(int device, int krylovdim, bool f32, bool use_graphs)
   set_smem(k_bapply<double, false>, smem64, err);
   set_smem(k_bapply<float, false>, smem32, err);
   set_smem(k_bapply_persist, kSepSmemBytes, err);
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&cycle_max_, f32 ? k_cycle<true> : k_cycle<false>, kRT, 0) !=
+      cudaSuccess) {
+    cycle_max_ = 0;
+    (void)cudaGetLastError();  // no one-launch cycles; the error is not the engine's
+  }
   chk(cudaDeviceGetAttribute(&sm_count_, cudaDevAttrMultiProcessorCount, device));
   if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&persist_max_, k_bapply_persist, kApplyThreads,
                                                     kSepSmemBytes) != cudaSuccess) {
@@ -1765,7 +2073,7 @@ Engine::Engine(int device, int krylovdim, bool f32, bool use_graphs)
 Engine::~Engine() {
   if (graph_) cudaGraphExecDestroy(graph_);
   if (s_) cudaStreamSynchronize(s_);
-  for (void* p : {st_, tile_inst_, tile_local_, chunk_inst_, nchunks_, part1_, partv_, hab_, rec_, out_, coefs_})
+  for (void* p : {st_, tile_inst_, tile_local_, strip_inst_, strip_local_, bar_, chunk_inst_, nchunks_, part1_, partv_, hab_, rec_, out_, coefs_})
     if (p) cudaFree(p);
   for (void* p : {st_h_, st_dl_, rec_h_, out_h_, coefs_h_})
     if (p) cudaFreeHost(p);
@@ -1805,6 +2113,7 @@ std::vector<Job*> Engine::retire() {
 void Engine::rebuild() {
   const int n = (int)jobs_.size();
   const size_t nn = std::max(n, 1);
+  const int pstride = std::max(m_ + 2, kBatchMaxObs);  // chunk partials: basis columns or observables
   // Chunk size: large chunks amortise the per-block reductions; when the active jobs hold
   // fewer elements than about eight large chunks per SM, small chunks keep the GPU full.
   long long total_elems = 0;
@@ -1813,17 +2122,39 @@ void Engine::rebuild() {
   // the trace of each step's input column is only needed by bordered (steady-state) cycles
   any_border_ = false;
   for (int i = 0; i < n; ++i) any_border_ = any_border_ || jobs_[i]->bordered;
-  std::vector<int> ti, tl, ci, nc(n);
+  std::vector<int> ti, tl, si, sl, ci, nc(n);
   std::vector<Planes64> p64(n);
+  std::vector<SplitPlanes> p32(n, SplitPlanes{nullptr, nullptr, nullptr, nullptr, 0});
+  std::vector<StripItems> it32(n);
+  bool canonical = true;  // every job steps by strips
   for (int i = 0; i < n; ++i) {
-    // FP64 engines apply canonical plans from merged coefficients: strip blocks, not tiles
-    p64[i] = f32_ ? Planes64{} : planes64(jobs_[i]->plan, PI_COORDS_REFERENCE);
-    const int ntiles = p64[i].items ? (p64[i].nitems + kBlockItems - 1) / kBlockItems : jobs_[i]->plan->dev.ntiles;
+    pi_plan* plan = jobs_[i]->plan;
+    // Step applies of canonical plans run over strip blocks, of other plans over tiles.  FP32
+    // dynamics cycles run in population coordinates, steady-state cycles in reference ones.
+    int strips = 0;
+    if (f32_) {
+      if (plan->dev.canon && em_split_planes(plan, jobs_[i]->bordered ? 0 : 1, &p32[i]) == PI_OK)
+        it32[i] = strip_items(plan);
+      else
+        p32[i] = SplitPlanes{nullptr, nullptr, nullptr, nullptr, 0};
+      strips = it32[i].n;
+    } else {
+      p64[i] = planes64(plan, PI_COORDS_REFERENCE);
+      strips = p64[i].nitems;
+    }
+    const int ntiles = plan->dev.ntiles;
+    const int nstrip = strips ? (strips + kBlockItems - 1) / kBlockItems : ntiles;
+    canonical = canonical && strips > 0;
     for (int t = 0; t < ntiles; ++t) {
       ti.push_back(i);
       tl.push_back(t);
     }
-    nc[i] = (int)((jobs_[i]->dim + chunk_ - 1) / chunk_);
+    for (int t = 0; t < nstrip; ++t) {
+      si.push_back(i);
+      sl.push_back(t);
+    }
+    const int chunk = f32_ ? chunk_ : chunk64(jobs_[i]->dim);
+    nc[i] = (int)((jobs_[i]->dim + chunk - 1) / chunk);
   }
   reserve(&hab_, &hab_cap_, sizeof(double2) * 2 * kMaxDots * nn, false);
   reserve(&rec_, &rec_cap_, sizeof(double2) * rec_stride_ * nn, false);
@@ -1846,11 +2177,12 @@ void Engine::rebuild() {
     d.ldv = J->ldv;
     d.ndiag = dp.ndiag;
     d.chunk_begin = (int)ci.size();
-    d.chunk = chunk_;
-    // FP32 Arnoldi applies of canonical plans read merged coefficients: dynamics cycles run in
-    // population coordinates, steady-state cycles in reference coordinates
-    d.planes = SplitPlanes{nullptr, nullptr, nullptr, nullptr, 0};
+    d.chunk = f32_ ? chunk_ : chunk64(J->dim);
+    d.pstride = pstride;
+    d.planes = p32[i];
     d.pwhich = J->bordered ? 0 : 1;
+    d.items32 = it32[i].items;
+    d.nitems32 = it32[i].n;
     d.p64 = p64[i];
     if (f32_ && dp.canon && em_split_planes(J->plan, d.pwhich, &d.planes) != PI_OK)
       d.planes = SplitPlanes{nullptr, nullptr, nullptr, nullptr, 0};
@@ -1872,14 +2204,19 @@ void Engine::rebuild() {
     d.done = 1;
   }
   total_tiles_ = (int)ti.size();
+  total_strips_ = (int)si.size();
+  cycle_kernel_ = canonical && n > 0 && total_elems <= kCycleElems && cycle_max_ > 0 && sm_count_ > 0;
   total_chunks_ = (int)ci.size();
   reserve(&st_, &st_cap_, sizeof(DevInst) * nn, false);
   reserve(&tile_inst_, &tile_inst_cap_, sizeof(int) * std::max<size_t>(ti.size(), 1), false);
   reserve(&tile_local_, &tile_local_cap_, sizeof(int) * std::max<size_t>(tl.size(), 1), false);
+  reserve(&strip_inst_, &strip_inst_cap_, sizeof(int) * std::max<size_t>(si.size(), 1), false);
+  reserve(&strip_local_, &strip_local_cap_, sizeof(int) * std::max<size_t>(sl.size(), 1), false);
+  reserve(&bar_, &bar_cap_, sizeof(GridBar), false);
   reserve(&chunk_inst_, &chunk_inst_cap_, sizeof(int) * std::max<size_t>(ci.size(), 1), false);
   reserve(&nchunks_, &nchunks_cap_, sizeof(int) * nn, false);
   reserve(&part1_, &part1_cap_, sizeof(double) * 2 * std::max(total_chunks_, 1), false);
-  reserve(&partv_, &partv_cap_, sizeof(double2) * kMaxDots * std::max(total_chunks_, 1), false);
+  reserve(&partv_, &partv_cap_, sizeof(double2) * (size_t)pstride * std::max(total_chunks_, 1), false);
   reserve(&st_h_, &st_h_cap_, sizeof(DevInst) * nn, true);
   reserve(&st_dl_, &st_dl_cap_, sizeof(DevInst) * nn, true);
   reserve(&rec_h_, &rec_h_cap_, sizeof(double2) * rec_stride_ * nn, true);
@@ -1887,6 +2224,8 @@ void Engine::rebuild() {
   reserve(&coefs_h_, &coefs_h_cap_, sizeof(double2) * (m_ + 2) * nn, true);
   if (!ti.empty()) chk(cudaMemcpyAsync(tile_inst_, ti.data(), sizeof(int) * ti.size(), cudaMemcpyHostToDevice, s_));
   if (!tl.empty()) chk(cudaMemcpyAsync(tile_local_, tl.data(), sizeof(int) * tl.size(), cudaMemcpyHostToDevice, s_));
+  if (!si.empty()) chk(cudaMemcpyAsync(strip_inst_, si.data(), sizeof(int) * si.size(), cudaMemcpyHostToDevice, s_));
+  if (!sl.empty()) chk(cudaMemcpyAsync(strip_local_, sl.data(), sizeof(int) * sl.size(), cudaMemcpyHostToDevice, s_));
   if (!ci.empty()) chk(cudaMemcpyAsync(chunk_inst_, ci.data(), sizeof(int) * ci.size(), cudaMemcpyHostToDevice, s_));
   if (n) chk(cudaMemcpyAsync(nchunks_, nc.data(), sizeof(int) * n, cudaMemcpyHostToDevice, s_));
   chk(cudaStreamSynchronize(s_));  // the host vectors above go out of scope
@@ -1916,8 +2255,8 @@ void Engine::launch_step_apply(int schedule) {
     const int grid = std::max(1, std::min(total_tiles_, schedule * sm_count_));
     launch(k_bapply_persist, grid, kApplyThreads, kSepSmemBytes, (const DevInst*)st, ti, tl, total_tiles_);
   } else {
-    launch(k_bapply<float, false>, total_tiles_, kApplyThreads, 3 * kWinElems * sizeof(float2), (const DevInst*)st,
-           ti, tl);
+    launch(k_bapply<float, false>, total_strips_, kApplyThreads, 3 * kWinElems * sizeof(float2), (const DevInst*)st,
+           (const int*)strip_inst_, (const int*)strip_local_);
   }
 }
 
@@ -2022,59 +2361,85 @@ void Engine::launch(void (*k)(KArgs...), dim3 grid, dim3 block, size_t smem, Arg
 
 void Engine::arnoldi_step() {
   DevInst* st = (DevInst*)st_;
+  const DevInst* cst = st;
   const int* ci = (const int*)chunk_inst_;
   const int* nc = (const int*)nchunks_;
-  const int* ti = (const int*)tile_inst_;
-  const int* tl = (const int*)tile_local_;
   double* part = (double*)part1_;
   double2* partv = (double2*)partv_;
-  double* none = nullptr;
+  const double2* cpartv = partv;
   const int n = (int)jobs_.size();
-  const dim3 gmd(total_chunks_, (m_ + 1 + 7) / 8);
   const dim3 gfin(n, (m_ + 1 + kRT / 32 - 1) / (kRT / 32));
   const dim3 gfirst(n, gfin.y + 1);  // projections into hA plus one row of image-norm blocks
   const int C = total_chunks_;
+  double* npart1 = part + C;  // |w1|^2 partials of the first update (second half of part)
+  // Classical Gram-Schmidt with selective reorthogonalisation: the first pass also takes the
+  // image norm |w0|^2 and the first update the |w1|^2 partials; the blocks of the second pass
+  // return at once for jobs that need none (step_norm1).
+  auto dots = [&](int second) {
+    double* ipart = second ? nullptr : part;
+    if (!f32_)
+      launch(k_step_dot64, C, kRT, 0, cst, ci, partv, ipart, second);
+    else if (chunk_ == kBatchChunk)
+      launch(k_step_mdot_f32<kBatchChunk>, C, kRT, 0, cst, ci, partv, ipart, second);
+    else
+      launch(k_step_mdot_f32<kBatchChunkSmall>, C, kRT, 0, cst, ci, partv, ipart, second);
+  };
+  auto update = [&](int second) {
+    double* out = second ? part : npart1;
+    if (f32_)
+      launch(k_step_maxpy_f32, C, kRT, 0, cst, ci, out, second);
+    else
+      launch(k_step_axpy64, C, kRT, 0, cst, ci, out, second);
+  };
   if (f32_) {
     if (any_border_) launch(k_step_trace<float2>, n, kRT, 0, st);
     launch_step_apply(apply_schedule_);
-    // CGS with selective reorthogonalisation: the first pass also takes the image norm
-    // |w0|^2 (every job) and the first update the |w1|^2 partials (second half of part);
-    // the second pass runs only for jobs whose first projection removed more than half of
-    // |w0|^2 (k_step_mdot_f32)
-    double* npart1 = part + C;
-    const int* ncn = nullptr;
-    const double* npn = nullptr;
-    if (chunk_ == kBatchChunk)
-      launch(k_step_mdot_f32<kBatchChunk>, C, kRT, 0, st, ci, partv, part, ncn, npn);
-    else
-      launch(k_step_mdot_f32<kBatchChunkSmall>, C, kRT, 0, st, ci, partv, part, ncn, npn);
-    launch(k_step_first_final, gfirst, kRT, 0, st, nc, (const double2*)partv, (const double*)part, 1);
-    launch(k_step_maxpy_f32, C, kRT, 0, (const DevInst*)st, ci, 0, npart1, npn);
-    double* noi = nullptr;
-    if (chunk_ == kBatchChunk)
-      launch(k_step_mdot_f32<kBatchChunk>, C, kRT, 0, st, ci, partv, noi, nc, (const double*)npart1);
-    else
-      launch(k_step_mdot_f32<kBatchChunkSmall>, C, kRT, 0, st, ci, partv, noi, nc, (const double*)npart1);
-    launch(k_step_mdot_final, gfin, kRT, 0, (const DevInst*)st, nc, (const double2*)partv, 1);
-    launch(k_step_maxpy_f32, C, kRT, 0, (const DevInst*)st, ci, 1, part, (const double*)npart1);
-    launch(k_step_normalize_f32, C, kRT, 0, st, ci, nc, (const double*)part);
   } else {
     if (any_border_) launch(k_step_trace<double2>, n, kRT, 0, st);
-    launch(k_bapply<double, false>, total_tiles_, kApplyThreads, 3 * kWinElems * sizeof(double2), (const DevInst*)st, ti, tl);
-    launch(k_step_image_partial<double2>, C, kRT, 0, (const DevInst*)st, ci, part);
-    launch(k_step_mdot_partial<double2, false>, gmd, kRT, 0, (const DevInst*)st, ci, partv);
-    launch(k_step_first_final, gfirst, kRT, 0, st, nc, (const double2*)partv, (const double*)part, 0);
-    launch(k_step_maxpy<double2>, C, kRT, 0, (const DevInst*)st, ci, 0, none);
-    launch(k_step_mdot_partial<double2, false>, gmd, kRT, 0, (const DevInst*)st, ci, partv);
-    launch(k_step_mdot_final, gfin, kRT, 0, (const DevInst*)st, nc, (const double2*)partv, 1);
-    launch(k_step_maxpy<double2>, C, kRT, 0, (const DevInst*)st, ci, 1, part);
-    launch(k_step_normalize<double2>, C, kRT, 0, st, ci, nc, (const double*)part);
+    launch(k_bapply<double, false>, total_strips_, kApplyThreads, 3 * kWinElems * sizeof(double2), cst,
+           (const int*)strip_inst_, (const int*)strip_local_);
   }
-  launch(k_step_finish, n, 32, 0, st, n);
+  dots(0);
+  launch(k_step_first_final, gfirst, kRT, 0, st, nc, cpartv, (const double*)part);
+  update(0);
+  launch(k_step_norm, n, kRT, 0, st, nc, (const double*)npart1, 0);
+  dots(1);
+  launch(k_step_mdot_final, gfin, kRT, 0, cst, nc, cpartv);
+  update(1);
+  launch(k_step_norm, n, kRT, 0, st, nc, (const double*)part, 1);
+  if (f32_)
+    launch(k_step_normalize_f32, C, kRT, 0, cst, ci);
+  else
+    launch(k_step_normalize64, C, kRT, 0, cst, ci);
+  launch(k_step_finish, n, 32, 0, st);
   if (!build_) chk(cudaGetLastError());
 }
 
+// The cycle of a small job set in one cooperative launch: as many blocks as its longest work
+// list has entries, at most what is resident at once.
+void Engine::launch_cycle() {
+  const int n = (int)jobs_.size();
+  const int grid = std::max(1, std::min(std::max(total_chunks_, total_strips_), cycle_max_ * sm_count_));
+  DevInst* st = (DevInst*)st_;
+  const int *ci = (const int*)chunk_inst_, *si = (const int*)strip_inst_, *sl = (const int*)strip_local_;
+  const int* nc = (const int*)nchunks_;
+  double2* partv = (double2*)partv_;
+  double* part = (double*)part1_;
+  GridBar* bar = (GridBar*)bar_;
+  int nn = n, C = total_chunks_, T = total_strips_, steps = m_, border = any_border_ ? 1 : 0;
+  chk(cudaMemsetAsync(bar, 0, sizeof(GridBar), s_));
+  void* args[] = {&st, &nn, &ci, &C, &si, &sl, &T, &nc, &partv, &part, &steps, &border, &bar};
+  chk(cudaLaunchCooperativeKernel(f32_ ? (const void*)k_cycle<true> : (const void*)k_cycle<false>, dim3(grid),
+                                  dim3(kRT), args, 0, s_));
+}
+
 void Engine::run_cycle_steps() {
+  // an explicit step-apply schedule asks for the step kernels
+  ran_cycle_ = cycle_kernel_ && (!f32_ || g_apply_schedule.load() == PI_SCHEDULE_AUTO);
+  if (ran_cycle_) {
+    launch_cycle();
+    return;
+  }
   if (!schedule_chosen_) choose_apply_schedule();
   if (err != cudaSuccess) return;
   if (!graphs_) {
@@ -2129,7 +2494,9 @@ bool Engine::tick() {
     if (flags & S1_PROBE) k_s1_probe<<<C, kRT, 0, s_>>>(st, ci);
     if (flags & (S1_AUX | S1_TRACE)) k_s1_trace<<<n, kRT, 0, s_>>>(st);
     if (flags & S1_AUX)
-      k_bapply<double, true><<<total_tiles_, kApplyThreads, 3 * kWinElems * sizeof(double2), s_>>>(st, ti, tl);
+      // an FP64 engine's canonical plans by strips, an FP32 engine's by tiles
+      k_bapply<double, true><<<f32_ ? total_tiles_ : total_strips_, kApplyThreads, 3 * kWinElems * sizeof(double2),
+                               s_>>>(st, f32_ ? ti : (const int*)strip_inst_, f32_ ? tl : (const int*)strip_local_);
     if (flags & S1_RESID) k_s1_resid<<<C, kRT, 0, s_>>>(st, ci);
     if (flags & S1_NORM) {
       k_s1_norm_partial<<<C, kRT, 0, s_>>>(st, ci, (double*)part1_);
@@ -2155,6 +2522,7 @@ bool Engine::tick() {
       in_cycle[i] = 1;
       any = true;
     }
+    sth[i].stop[0] = sth[i].stop[1] = sth[i].done;
   }
   if (!any) return err == cudaSuccess;
   ++cycles;
@@ -2170,7 +2538,11 @@ bool Engine::tick() {
   const double2* rech = (const double2*)rec_h_;
   chk(cudaMemcpyAsync(st_dl_, st_, sizeof(DevInst) * n, cudaMemcpyDeviceToHost, s_));
   chk(cudaMemcpyAsync(rec_h_, rec_, sizeof(double2) * rec_stride_ * n, cudaMemcpyDeviceToHost, s_));
+  GridBar bar{0, 0};
+  if (ran_cycle_) chk(cudaMemcpyAsync(out_h_, bar_, sizeof(GridBar), cudaMemcpyDeviceToHost, s_));
   chk(cudaStreamSynchronize(s_));
+  if (ran_cycle_) std::memcpy(&bar, out_h_, sizeof(bar));
+  if (bar.err) chk(cudaErrorLaunchTimeout);  // a grid barrier gave up waiting
   if (err != cudaSuccess) return false;
   bool enl = false;
   std::vector<char> in_enl(n, 0);

@@ -39,6 +39,20 @@ constexpr int kBatchMaxKrylov = 120;
 // element pairs; the padding is zero).
 inline long long basis_stride(long long dim) { return (dim + 63) / 64 * 64; }
 
+// Elements per reduction chunk of an FP64 job, by its own size (so that its sums do not depend
+// on the other jobs of the set): about two chunks per SM, 128 to 1024 elements.
+inline int chunk64(long long dim) {
+  int c = 128;
+  while (c < kBatchChunkSmall && dim > 304LL * c) c *= 2;
+  return c;
+}
+
+// Job sets of at most this many elements, all of canonical plans, run a Krylov cycle as one
+// cooperative launch (k_cycle): their step phases last about as long as a launch takes to start
+// and drain.  Larger sets keep one graph of step kernels, which leave SMs to other streams
+// between phases.
+constexpr long long kCycleElems = 1LL << 19;
+
 // Stage-1 operation flags.
 enum : unsigned {
   S1_COMBINE = 1u,
@@ -64,7 +78,8 @@ struct DevInst {
   long long ldv;    // basis column stride: dim rounded up to a multiple of 64, zero padded
   int ndiag;
   int chunk_begin;  // first chunk of this job in the engine's chunk list
-  int chunk;        // elements per chunk (the engine's choice, kBatchChunkSmall or kBatchChunk)
+  int chunk;        // elements per chunk (FP32: kBatchChunkSmall or kBatchChunk; FP64: chunk64(dim))
+  int pstride;      // chunk partials: columns per chunk
   // Krylov cycle
   void* V;  // m + 2 basis columns (FP64 or FP32)
   void* w;
@@ -82,11 +97,14 @@ struct DevInst {
   int j;         // input column of the next step
   int done;      // no further steps this cycle
   int kdone;     // completed steps
-  int reorth;    // FP32 basis: this step's second CGS projection ran (selective reorthogonalisation)
+  int reorth;    // this step's second CGS pass runs (selective reorthogonalisation)
+  int stop[2];   // k_cycle: done, by step parity
   // FP32 basis, canonical plan: merged coefficients of the Arnoldi applies in the coordinate
   // system pwhich (eplane == nullptr: the generic stencil terms)
   SplitPlanes planes;
   int pwhich;
+  const StripItem* items32;  // the strip items of those applies (nullptr: tiles)
+  int nitems32;
   Planes64 p64;  // FP64 basis, canonical plan: merged FP64 coefficients (reference coordinates)
   double scale;  // multiplies L V_j
   double tol;    // GMRES: stop when |g[j+1]| <= tol
@@ -293,6 +311,9 @@ class Engine {
   std::vector<Job*> jobs_;
   bool dirty_ = true;
   int total_tiles_ = 0, total_chunks_ = 0;
+  int total_strips_ = 0;   // step-apply list: strip blocks, or tiles of general plans
+  bool cycle_kernel_ = false;  // the current set may run k_cycle
+  bool ran_cycle_ = false;     // its last cycle did
   int chunk_ = kBatchChunk;
   bool any_border_ = true;  // some job of the current set runs bordered cycles
   size_t rec_stride_ = 0;  // double2 per job record
@@ -300,6 +321,9 @@ class Engine {
   void* st_ = nullptr; size_t st_cap_ = 0;
   void* tile_inst_ = nullptr; size_t tile_inst_cap_ = 0;
   void* tile_local_ = nullptr; size_t tile_local_cap_ = 0;
+  void* strip_inst_ = nullptr; size_t strip_inst_cap_ = 0;
+  void* strip_local_ = nullptr; size_t strip_local_cap_ = 0;
+  void* bar_ = nullptr; size_t bar_cap_ = 0;
   void* chunk_inst_ = nullptr; size_t chunk_inst_cap_ = 0;
   void* nchunks_ = nullptr; size_t nchunks_cap_ = 0;
   void* part1_ = nullptr; size_t part1_cap_ = 0;
@@ -324,9 +348,11 @@ class Engine {
   // job-set shape)
   void choose_apply_schedule();
   void launch_step_apply(int schedule);
+  void launch_cycle();
   int apply_schedule_ = PI_SCHEDULE_PER_TILE;
   bool schedule_chosen_ = false;
   int sm_count_ = 0;
+  int cycle_max_ = 0;    // resident blocks per SM of k_cycle
   int persist_max_ = 0;  // resident blocks per SM of the persistent apply (0: unavailable)
 };
 

@@ -75,6 +75,8 @@ struct pi_plan {
   // a plan without room for them keeps the general kernels.
   picuda::Planes64 planes64[2];
   bool planes64_failed[2] = {false, false};
+  const picuda::StripItem* strip_items = nullptr;
+  int nstrip_items = 0;
   // Single-instance solves run as one job of a batched engine kept with the plan (created on
   // first use for a Krylov dimension and basis precision, replaced when those change).
   picuda::Engine* engine = nullptr;
@@ -115,6 +117,14 @@ void* plan_alloc(pi_plan* plan, size_t bytes);
 // FP32 coordinates, built on first use (pi_apply_em.cu); PI_ERR_UNSUPPORTED for a plan whose
 // stencil does not sit at the canonical positions.
 int em_split_planes(pi_plan* plan, int which, SplitPlanes* out);
+
+// Strip items of a plan (32 consecutive entries of one sector block each), built on first use;
+// items == nullptr without room for them.
+struct StripItems {
+  const StripItem* items = nullptr;
+  int n = 0;
+};
+StripItems strip_items(pi_plan* plan);
 
 // Merged FP64 coefficient planes of a canonical plan in reference (coords 0) or population
 // (1) coordinates, built on first use (pi_apply64.cu); items == nullptr when the plan is not
