@@ -39,20 +39,28 @@ __device__ __forceinline__ double2 ld2(const float2* p) {
 __device__ __forceinline__ void st2(double2* p, double x, double y) { *p = make_double2(x, y); }
 __device__ __forceinline__ void st2(float2* p, double x, double y) { *p = make_float2((float)x, (float)y); }
 
-// Deterministic block sum of NV values (blockDim.x a multiple of 32); result in thread 0.
+constexpr int kRT = kReduceThreads;  // threads of the chunk kernels
+
+// Deterministic block sum of NV values (blockDim.x a multiple of 32); result in thread 0.  Warps
+// from `nw` on hold zeros and stay off the FP64 pipe; the sum is the same.
 template <int NV>
-__device__ __forceinline__ void block_sum(double (&v)[NV], double* smem) {
+__device__ __forceinline__ void block_sum(double (&v)[NV], double* smem, int nw = kRT / 32) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  if (warp < nw) {
 #pragma unroll
-  for (int k = 0; k < NV; ++k)
+    for (int k = 0; k < NV; ++k)
 #pragma unroll
-    for (int off = 16; off > 0; off >>= 1) v[k] += __shfl_down_sync(0xffffffffu, v[k], off);
+      for (int off = 16; off > 0; off >>= 1) v[k] += __shfl_down_sync(0xffffffffu, v[k], off);
+  }
+  if (nw == 1) {  // uniform
+    __syncthreads();
+    return;
+  }
   if (lane == 0)
 #pragma unroll
     for (int k = 0; k < NV; ++k) smem[warp * NV + k] = v[k];
   __syncthreads();
   if (warp == 0) {
-    const int nw = blockDim.x >> 5;
 #pragma unroll
     for (int k = 0; k < NV; ++k) v[k] = lane < nw ? smem[lane * NV + k] : 0.0;
 #pragma unroll
@@ -81,15 +89,27 @@ __device__ __forceinline__ void chunk_range(const DevInst& S, int c, long long& 
   end = min(beg + (long long)S.chunk, S.dim);
 }
 
-constexpr int kRT = kReduceThreads;  // threads of the chunk kernels
 
 // ---------------------------------------------------------------------------------------
 // Stage-1 kernels
 // ---------------------------------------------------------------------------------------
 
+// Norm partial of a combination whose result is the vector to be normed (dynamics trials): the
+// chunk's |cout|^2 into part, as k_s1_norm_partial would leave it.
+__device__ __forceinline__ void combined_norm(const DevInst& S, double v, double* part) {
+  __shared__ double smem[kRT / 32];
+  if (S.nrm0 != S.cout) return;  // block-uniform
+  double acc[1] = {v};
+  block_sum<1>(acc, smem);
+  if (threadIdx.x == 0) {
+    part[2 * blockIdx.x] = acc[0];
+    part[2 * blockIdx.x + 1] = 0.0;
+  }
+}
+
 // cout (+)= sum_k ccoef[k] V_k, FP64 accumulation.
-template <typename T2>
-__global__ void __launch_bounds__(kRT) k_s1_combine(const DevInst* __restrict__ st, const int* __restrict__ chunk_inst) {
+__global__ void __launch_bounds__(kRT)
+    k_s1_combine(const DevInst* __restrict__ st, const int* __restrict__ chunk_inst, double* __restrict__ part) {
   __shared__ double2 cs[kBatchMaxKrylov + 2];
   const DevInst& S = st[chunk_inst[blockIdx.x]];
   double2* out = S.cout;
@@ -99,13 +119,15 @@ __global__ void __launch_bounds__(kRT) k_s1_combine(const DevInst* __restrict__ 
   __syncthreads();
   long long beg, end;
   chunk_range(S, blockIdx.x, beg, end);
-  const T2* V = (const T2*)S.V;
-  const long long dim = S.ldv;
+  const double2* V = (const double2*)S.V;
+  const long long ld = S.ldv;
   const int acc = S.cacc;
+  double nrm = 0;
   for (long long e = beg + threadIdx.x; e < end; e += blockDim.x) {
     double yx = 0, yy = 0;
+#pragma unroll 8
     for (int k = 0; k < nc; ++k) {
-      const double2 v = ld2(V + (long long)k * dim + e);
+      const double2 v = V[(long long)k * ld + e];
       yx = fma(v.x, cs[k].x, yx);
       yx = fma(-v.y, cs[k].y, yx);
       yy = fma(v.x, cs[k].y, yy);
@@ -117,7 +139,9 @@ __global__ void __launch_bounds__(kRT) k_s1_combine(const DevInst* __restrict__ 
       yy += o.y;
     }
     out[e] = make_double2(yx, yy);
+    nrm = fma(yy, yy, fma(yx, yx, nrm));
   }
+  combined_norm(S, nrm, part);
 }
 
 __device__ __forceinline__ unsigned long long mix64(unsigned long long z) {
@@ -177,13 +201,14 @@ __global__ void __launch_bounds__(kRT) k_s1_trace(DevInst* __restrict__ st) {
   }
 }
 
-constexpr int kBlockItems = kApplyThreads / 32;  // strip items of one block of an apply over the list
+constexpr int kBlockItems = kApplyThreads / 32;  // strip items that a block takes at once
+constexpr int kRounds32 = 4;                     // times per entry of an FP32 apply list
 
-// kBlockItems consecutive strip items of an instance with merged FP64 coefficients: y = scale
+// A warp's strip item of an instance with merged FP64 coefficients: y = scale
 // L x + alpha v on the diagonal (reference coordinates), or y = L x when `plain`.
 template <int V, bool NC>
-__device__ __forceinline__ void strip_block(const DevInst& S, int block, const double2* x, double2* y, bool plain, double scale, const double2* alpha) {
-  const int item = block * kBlockItems + (threadIdx.x >> 5);
+__device__ __forceinline__ void strip_item(const DevInst& S, int item, const double2* x, double2* y, bool plain,
+                                           double scale, const double2* alpha) {
   if (item >= S.p64.nitems) return;
   const StripItem it = S.p64.items[item];
   StripEntry<V, NC> E;
@@ -204,93 +229,136 @@ __device__ __forceinline__ void strip_block(const DevInst& S, int block, const d
 }
 
 template <bool NC>
-__device__ __forceinline__ void strip_apply(const DevInst& S, int block, const double2* x, double2* y, double scale,
+__device__ __forceinline__ void strip_apply(const DevInst& S, int item, const double2* x, double2* y, double scale,
                                             const double2* alpha) {
   // an exact 1 is told by its bits: an FP64 comparison would go through the FP64 pipe
   const bool plain = alpha == nullptr && __double_as_longlong(scale) == 0x3ff0000000000000LL;
   switch (S.p64.variant) {
-    case 0: return strip_block<0, NC>(S, block, x, y, plain, scale, alpha);
-    case 1: return strip_block<1, NC>(S, block, x, y, plain, scale, alpha);
-    case 2: return strip_block<2, NC>(S, block, x, y, plain, scale, alpha);
-    case 3: return strip_block<3, NC>(S, block, x, y, plain, scale, alpha);
-    case 4: return strip_block<4, NC>(S, block, x, y, plain, scale, alpha);
-    case 5: return strip_block<5, NC>(S, block, x, y, plain, scale, alpha);
-    default: return strip_block<6, NC>(S, block, x, y, plain, scale, alpha);
+    case 0: return strip_item<0, NC>(S, item, x, y, plain, scale, alpha);
+    case 1: return strip_item<1, NC>(S, item, x, y, plain, scale, alpha);
+    case 2: return strip_item<2, NC>(S, item, x, y, plain, scale, alpha);
+    case 3: return strip_item<3, NC>(S, item, x, y, plain, scale, alpha);
+    case 4: return strip_item<4, NC>(S, item, x, y, plain, scale, alpha);
+    case 5: return strip_item<5, NC>(S, item, x, y, plain, scale, alpha);
+    default: return strip_item<6, NC>(S, item, x, y, plain, scale, alpha);
   }
 }
 
-// kBlockItems strip items of an FP32 instance of a canonical plan: w = scale L x (+ alpha v on
-// the diagonal) from the merged entry, row and column planes, one thread per entry.  The
-// arithmetic of an entry is apply_tile_planes_to's (and sep_entries'), operation for operation,
-// so every schedule gives the same bits.  Per entry: 32-48 bytes of planes and ten sources
-// through L1, no window staging and no idle lanes; the 32 x 32 tiles it replaces spent 1,113
-// instructions per warp and tile, most of them on staging.
+// Strip items of an FP32 instance of a canonical plan: w = scale L x (+ alpha v on the diagonal)
+// from the merged entry, row and column planes, one thread per entry.  The arithmetic of an
+// entry is apply_tile_planes_to's (and sep_entries'), operation for operation, so every schedule
+// gives the same bits.  Per entry: 32-48 bytes of planes and ten sources through L1, no window
+// staging and no idle lanes.  What bounds it is the chain of loads behind an entry (work list,
+// control block, record, then planes and sources), so a block takes four rounds of items per
+// list entry.
 template <bool PLUS, bool NC>
-__device__ __forceinline__ void strip_block32(const DevInst& S, int block, const float2* x, float2* y,
-                                              const double2* alpha) {
-  constexpr int NE = PLUS ? 3 : 2;
-  const int item = block * kBlockItems + (threadIdx.x >> 5);
-  if (item >= S.nitems32) return;
-  const StripItem it = S.items32[item];
-  const int n = it.n;
-  const int i = it.local0 + (threadIdx.x & 31);
-  if (i >= n * n) return;
-  const int b = (int)((unsigned)i / (unsigned)n), a = i - b * n;
-  const int e = it.off + i;
-  const float4* ep = S.planes.eplane + (long long)e * NE;
-  const float4 c0 = __ldg(ep), c1 = __ldg(ep + 1);
-  const float4 lv = __ldg(S.planes.lrow + it.loff + a), rc = __ldg(S.planes.rcol + it.loff + b);
-  const float2 zero = make_float2(0.f, 0.f);
-  auto ld = [&](long long k, bool in) { return in ? (NC ? __ldg(x + k) : x[k]) : zero; };
-  const int m0 = it.m0, m2 = it.m2;
-  auto box = [](int u, int v, int m) { return (unsigned)u < (unsigned)m && (unsigned)v < (unsigned)m; };
-  const int s0 = it.off0 + (a - 2) + (b - 2) * m0, g0 = it.off2 + a + b * m2;
-  const float2 xc = ld(e, true), xu = ld(e - 1, a > 0), xd = ld(e + 1, a < n - 1);
-  const float2 xl = ld(e - n, b > 0), xr = ld(e + n, b < n - 1), xo = ld(e - n - 1, a > 0 && b > 0);
-  const float2 v0 = ld(s0, box(a - 2, b - 2, m0)), v1 = ld(s0 + m0 + 1, box(a - 1, b - 1, m0));
-  const float2 w0 = ld(g0, box(a, b, m2)), w1 = ld(g0 + m2 + 1, box(a + 1, b + 1, m2));
-  float2 acc = zero;
-  pmac(acc, c0.x, c0.y, xc);  // centre
-  pmac(acc, lv.x, lv.y, xu);  // LEFT -1
-  pmac(acc, lv.z, lv.w, xd);  // LEFT +1
-  pmac(acc, rc.x, rc.y, xl);  // RIGHT -1
-  pmac(acc, rc.z, rc.w, xr);  // RIGHT +1
-  prmac(acc, c0.z, xo);       // own (-1,-1)
-  if (m0 > 0) {
-    prmac(acc, c0.w, v0);     // smaller (-2,-2)
-    prmac(acc, c1.x, v1);     // smaller (-1,-1)
+struct StripEntry32 {
+  float4 c0, c1, c2, lv, rc;
+  float2 xc, xu, xd, xl, xr, xo, v0, v1, w0, w1, xp, v2, w2;
+  int e, m0, m2, sector;
+  bool in, diag;
+
+  __device__ __forceinline__ void load(const DevInst& S, const StripItem& it, const float2* x) {
+    const int n = it.n;
+    const int i = it.local0 + (threadIdx.x & 31);
+    in = i < n * n;
+    if (!in) return;
+    constexpr int NE = PLUS ? 3 : 2;
+    const int b = (int)((unsigned)i / (unsigned)n), a = i - b * n;
+    e = it.off + i;
+    sector = it.sector;
+    diag = a == b;
+    m0 = it.m0;
+    m2 = it.m2;
+    const float4* ep = S.planes.eplane + (long long)e * NE;
+    c0 = __ldg(ep);
+    c1 = __ldg(ep + 1);
+    if (PLUS) c2 = __ldg(ep + 2);
+    lv = __ldg(S.planes.lrow + it.loff + a);
+    rc = __ldg(S.planes.rcol + it.loff + b);
+    auto ld = [&](int k, bool ok) { return ok ? (NC ? __ldg(x + k) : x[k]) : make_float2(0.f, 0.f); };
+    auto box = [](int u, int v, int m) { return (unsigned)u < (unsigned)m && (unsigned)v < (unsigned)m; };
+    const int s0 = it.off0 + (a - 2) + (b - 2) * m0, g0 = it.off2 + a + b * m2;
+    xc = ld(e, true);
+    xu = ld(e - 1, a > 0);
+    xd = ld(e + 1, a < n - 1);
+    xl = ld(e - n, b > 0);
+    xr = ld(e + n, b < n - 1);
+    xo = ld(e - n - 1, a > 0 && b > 0);
+    v0 = ld(s0, box(a - 2, b - 2, m0));
+    v1 = ld(s0 + m0 + 1, box(a - 1, b - 1, m0));
+    w0 = ld(g0, box(a, b, m2));
+    w1 = ld(g0 + m2 + 1, box(a + 1, b + 1, m2));
+    if (PLUS) {
+      xp = ld(e + n + 1, a < n - 1 && b < n - 1);
+      v2 = ld(s0 + 2 * (m0 + 1), box(a, b, m0));
+      w2 = ld(g0 + 2 * (m2 + 1), box(a + 2, b + 2, m2));
+    }
   }
-  if (m2 > 0) {
-    prmac(acc, c1.y, w0);     // larger (0,0)
-    prmac(acc, c1.z, w1);     // larger (1,1)
+
+  __device__ __forceinline__ void store(const DevInst& S, float2* y, const double2* alpha) const {
+    if (!in) return;
+    float2 acc = make_float2(0.f, 0.f);
+    pmac(acc, c0.x, c0.y, xc);  // centre
+    pmac(acc, lv.x, lv.y, xu);  // LEFT -1
+    pmac(acc, lv.z, lv.w, xd);  // LEFT +1
+    pmac(acc, rc.x, rc.y, xl);  // RIGHT -1
+    pmac(acc, rc.z, rc.w, xr);  // RIGHT +1
+    prmac(acc, c0.z, xo);       // own (-1,-1)
+    if (m0 > 0) {
+      prmac(acc, c0.w, v0);     // smaller (-2,-2)
+      prmac(acc, c1.x, v1);     // smaller (-1,-1)
+    }
+    if (m2 > 0) {
+      prmac(acc, c1.y, w0);     // larger (0,0)
+      prmac(acc, c1.z, w1);     // larger (1,1)
+    }
+    if (PLUS) {
+      prmac(acc, c1.w, xp);               // own (1,1)
+      if (m0 > 0) prmac(acc, c2.x, v2);   // smaller (0,0)
+      if (m2 > 0) prmac(acc, c2.y, w2);   // larger (2,2)
+    }
+    if (__double_as_longlong(S.scale) != 0x3ff0000000000000LL) {
+      const float scale = (float)S.scale;
+      acc.x *= scale;
+      acc.y *= scale;
+    }
+    if (alpha != nullptr && diag) {
+      const double2 al = *alpha;
+      const double v = S.coords ? S.sectors[sector].border_z : S.sectors[sector].border_x;
+      acc.x += (float)(al.x * v);
+      acc.y += (float)(al.y * v);
+    }
+    y[e] = acc;
   }
-  if (PLUS) {
-    const float4 c2 = __ldg(ep + 2);
-    prmac(acc, c1.w, ld(e + n + 1, a < n - 1 && b < n - 1));              // own (1,1)
-    if (m0 > 0) prmac(acc, c2.x, ld(s0 + 2 * (m0 + 1), box(a, b, m0)));   // smaller (0,0)
-    if (m2 > 0) prmac(acc, c2.y, ld(g0 + 2 * (m2 + 1), box(a + 2, b + 2, m2)));  // larger (2,2)
+};
+
+// Items first, first + step, ... (at most `count`) by one warp; the record of the next item is
+// in flight while an item is computed.
+template <bool PLUS, bool NC>
+__device__ __forceinline__ void strip_items32(const DevInst& S, int first, int step, int count, const float2* x,
+                                              float2* y, const double2* alpha) {
+  const int nitems = S.nitems32;
+  if (first >= nitems) return;
+  const StripItem* items = S.items32;
+  StripItem next = items[first];
+#pragma unroll 1
+  for (int k = 0, item = first; k < count && item < nitems; ++k, item += step) {
+    const StripItem it = next;
+    if (k + 1 < count && item + step < nitems) next = items[item + step];
+    StripEntry32<PLUS, NC> E;
+    E.load(S, it, x);
+    E.store(S, y, alpha);
   }
-  if (__double_as_longlong(S.scale) != 0x3ff0000000000000LL) {
-    const float scale = (float)S.scale;
-    acc.x *= scale;
-    acc.y *= scale;
-  }
-  if (alpha != nullptr && a == b) {
-    const double2 al = *alpha;
-    const double v = S.coords ? S.sectors[it.sector].border_z : S.sectors[it.sector].border_x;
-    acc.x += (float)(al.x * v);
-    acc.y += (float)(al.y * v);
-  }
-  y[e] = acc;
 }
 
 template <bool NC>
-__device__ __forceinline__ void strip_apply32(const DevInst& S, int block, const float2* x, float2* y,
-                                              const double2* alpha) {
+__device__ __forceinline__ void strip_apply32(const DevInst& S, int first, int step, int count, const float2* x,
+                                              float2* y, const double2* alpha) {
   if (S.planes.plus)
-    strip_block32<true, NC>(S, block, x, y, alpha);
+    strip_items32<true, NC>(S, first, step, count, x, y, alpha);
   else
-    strip_block32<false, NC>(S, block, x, y, alpha);
+    strip_items32<false, NC>(S, first, step, count, x, y, alpha);
 }
 
 // Applies over the (instance, tile) list -- for an instance of a canonical plan an (instance,
@@ -308,7 +376,8 @@ __global__ void __launch_bounds__(kApplyThreads, sizeof(T) == 4 && !AUX ? 4 : 1)
   if (AUX) {
     if (!S.ax) return;
     if (S.p64.items != nullptr) {  // block-uniform
-      strip_apply<true>(S, tile_local[blockIdx.x], S.ax, S.ay, S.aux_scale, S.aux_border ? &S.aux_alpha : nullptr);
+      strip_apply<true>(S, tile_local[blockIdx.x] * kBlockItems + (threadIdx.x >> 5), S.ax, S.ay, S.aux_scale,
+                        S.aux_border ? &S.aux_alpha : nullptr);
       return;
     }
     const DevTile tile = S.tiles[tile_local[blockIdx.x]];
@@ -320,13 +389,14 @@ __global__ void __launch_bounds__(kApplyThreads, sizeof(T) == 4 && !AUX ? 4 : 1)
     const T2* xin = (const T2*)S.V + (long long)S.j * S.ldv;
     if constexpr (sizeof(T) == sizeof(double)) {
       if (S.p64.items != nullptr) {  // block-uniform
-        strip_apply<true>(S, tile_local[blockIdx.x], xin, (double2*)S.w, S.scale, S.border ? &S.alpha : nullptr);
+        strip_apply<true>(S, tile_local[blockIdx.x] * kBlockItems + (threadIdx.x >> 5), xin, (double2*)S.w, S.scale, S.border ? &S.alpha : nullptr);
         return;
       }
     }
     if constexpr (sizeof(T) == sizeof(float)) {
       if (S.items32 != nullptr) {  // block-uniform
-        strip_apply32<true>(S, tile_local[blockIdx.x], xin, (float2*)S.w, S.border ? &S.alpha : nullptr);
+        strip_apply32<true>(S, tile_local[blockIdx.x] * kBlockItems * kRounds32 + (threadIdx.x >> 5), kBlockItems,
+                            kRounds32, xin, (float2*)S.w, S.border ? &S.alpha : nullptr);
         return;
       }
     }
@@ -428,101 +498,100 @@ __global__ void __launch_bounds__(kRT) k_s1_resid(const DevInst* __restrict__ st
   }
 }
 
+// Sums v[k] over the warp's lanes by exchanging halves of the values (NV - 1 additions and a few
+// more instead of 5 NV); afterwards v[0] of lane l is the total of value l / (32 / NV).
+template <int NV>
+__device__ __forceinline__ void warp_transpose_sum(double (&v)[NV]) {
+  const int lane = threadIdx.x & 31;
+  int off = 16;
+#pragma unroll
+  for (int s = NV / 2; s >= 1; s >>= 1, off >>= 1) {
+    const bool up = lane & off;
+#pragma unroll
+    for (int i = 0; i < s; ++i) {
+      const double send = up ? v[i] : v[i + s];
+      const double keep = up ? v[i + s] : v[i];
+      v[i] = keep + __shfl_xor_sync(0xffffffffu, send, off);
+    }
+  }
+  for (; off >= 1; off >>= 1) v[0] += __shfl_xor_sync(0xffffffffu, v[0], off);
+}
+
+// |nrm0|^2 and |nrm1|^2 over one chunk; a combination's own norm is already there.
 __global__ void __launch_bounds__(kRT)
     k_s1_norm_partial(const DevInst* __restrict__ st, const int* __restrict__ chunk_inst, double* __restrict__ part) {
-  __shared__ double smem[32 * 2];
+  __shared__ double2 red[kRT / 32];
   const DevInst& S = st[chunk_inst[blockIdx.x]];
-  const double2* a = S.nrm0;
+  const double2* a = S.nrm0 != S.cout ? S.nrm0 : nullptr;
   const double2* b = S.nrm1;
   if (!a && !b) return;
   long long beg, end;
   chunk_range(S, blockIdx.x, beg, end);
   double acc[2] = {0, 0};
-  for (long long e = beg + threadIdx.x; e < end; e += blockDim.x) {
-    if (a) {
+  if (a)
+    for (long long e = beg + threadIdx.x; e < end; e += blockDim.x) {
       const double2 v = a[e];
-      acc[0] = fma(v.x, v.x, acc[0]);
-      acc[0] = fma(v.y, v.y, acc[0]);
+      acc[0] = fma(v.y, v.y, fma(v.x, v.x, acc[0]));
     }
-    if (b) {
+  if (b)
+    for (long long e = beg + threadIdx.x; e < end; e += blockDim.x) {
       const double2 v = b[e];
-      acc[1] = fma(v.x, v.x, acc[1]);
-      acc[1] = fma(v.y, v.y, acc[1]);
+      acc[1] = fma(v.y, v.y, fma(v.x, v.x, acc[1]));
+    }
+  warp_transpose_sum<2>(acc);
+  const int lane = threadIdx.x & 31;
+  if (lane % 16 == 0) reinterpret_cast<double*>(&red[threadIdx.x >> 5])[lane / 16] = acc[0];
+  __syncthreads();
+  if (threadIdx.x < 2) {
+    double t = 0;
+    for (int w = 0; w < kRT / 32; ++w) t += reinterpret_cast<const double*>(&red[w])[threadIdx.x];
+    part[2 * blockIdx.x + threadIdx.x] = t;
+  }
+}
+
+// Dots conj(ob_o) . obx of K observables over the thread's elements, summed over the warp.
+template <int K>
+__device__ __forceinline__ void obs_cols(const DevInst& S, long long beg, long long end, int o0, double* row) {
+  double acc[2 * K];
+#pragma unroll
+  for (int k = 0; k < 2 * K; ++k) acc[k] = 0;
+  for (long long e = beg + threadIdx.x; e < end; e += blockDim.x) {
+    const double2 x = S.obx[e];
+#pragma unroll
+    for (int k = 0; k < K; ++k) {
+      const double2 v = S.ob[(long long)(o0 + k) * S.dim + e];
+      acc[2 * k] = fma(v.x, x.x, acc[2 * k]);
+      acc[2 * k] = fma(v.y, x.y, acc[2 * k]);
+      acc[2 * k + 1] = fma(v.x, x.y, acc[2 * k + 1]);
+      acc[2 * k + 1] = fma(-v.y, x.x, acc[2 * k + 1]);
     }
   }
-  block_sum<2>(acc, smem);
-  if (threadIdx.x == 0) {
-    part[2 * blockIdx.x] = acc[0];
-    part[2 * blockIdx.x + 1] = acc[1];
-  }
+  warp_transpose_sum<2 * K>(acc);
+  constexpr int span = 32 / (2 * K);
+  const int lane = threadIdx.x & 31;
+  if (lane % span == 0) row[2 * o0 + lane / span] = acc[0];
 }
 
-__global__ void __launch_bounds__(kRT)
-    k_s1_norm_final(const DevInst* __restrict__ st, const int* __restrict__ nchunks, const double* __restrict__ part) {
-  __shared__ double smem[32 * 2];
-  const DevInst& S = st[blockIdx.x];
-  if (!S.nrm0 && !S.nrm1) return;
-  double acc[2] = {0, 0};
-  for (int c = threadIdx.x; c < nchunks[blockIdx.x]; c += blockDim.x) {
-    acc[0] += part[2 * (S.chunk_begin + c)];
-    acc[1] += part[2 * (S.chunk_begin + c) + 1];
-  }
-  block_sum<2>(acc, smem);
-  if (threadIdx.x == 0) {
-    S.out[0] = acc[0];
-    S.out[1] = acc[1];
-  }
-}
-
-// Observable dots conj(ob_o) . obx over one chunk (FP64 data).  Only the live observables
-// are reduced: warp shuffles per observable, then one shared-memory pass.
+// Observable dots conj(ob_o) . obx over one chunk (FP64 data).
 __global__ void __launch_bounds__(kRT)
     k_s1_obs_partial(const DevInst* __restrict__ st, const int* __restrict__ chunk_inst, double2* __restrict__ partv) {
-  __shared__ double2 red[kBatchMaxObs][kRT / 32];
+  __shared__ double red[kRT / 32][2 * kBatchMaxObs];
   const DevInst& S = st[chunk_inst[blockIdx.x]];
   const int nob = S.nob;
   if (nob == 0) return;
   long long beg, end;
   chunk_range(S, blockIdx.x, beg, end);
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  for (int o0 = 0; o0 < nob; o0 += 4) {
-    double acc[8];
-#pragma unroll
-    for (int k = 0; k < 8; ++k) acc[k] = 0;
-    for (long long e = beg + threadIdx.x; e < end; e += blockDim.x) {
-      const double2 x = S.obx[e];
-#pragma unroll
-      for (int k = 0; k < 4; ++k) {
-        if (o0 + k < nob) {
-          const double2 v = S.ob[(long long)(o0 + k) * S.dim + e];
-          acc[2 * k] = fma(v.x, x.x, acc[2 * k]);
-          acc[2 * k] = fma(v.y, x.y, acc[2 * k]);
-          acc[2 * k + 1] = fma(v.x, x.y, acc[2 * k + 1]);
-          acc[2 * k + 1] = fma(-v.y, x.x, acc[2 * k + 1]);
-        }
-      }
-    }
-#pragma unroll
-    for (int k = 0; k < 4; ++k) {
-      if (o0 + k < nob) {
-#pragma unroll
-        for (int off = 16; off > 0; off >>= 1) {
-          acc[2 * k] += __shfl_down_sync(0xffffffffu, acc[2 * k], off);
-          acc[2 * k + 1] += __shfl_down_sync(0xffffffffu, acc[2 * k + 1], off);
-        }
-        if (lane == 0) red[o0 + k][warp] = make_double2(acc[2 * k], acc[2 * k + 1]);
-      }
-    }
-  }
+  double* row = red[threadIdx.x >> 5];
+  int o = 0;
+  for (; o + 4 <= nob; o += 4) obs_cols<4>(S, beg, end, o, row);
+  if (o + 2 <= nob) obs_cols<2>(S, beg, end, o, row), o += 2;
+  if (o < nob) obs_cols<1>(S, beg, end, o, row);
   __syncthreads();
-  for (int o = threadIdx.x; o < nob; o += blockDim.x) {
-    double sx = 0, sy = 0;
+  for (int i = threadIdx.x; i < 2 * nob; i += blockDim.x) {
+    double t = 0;
 #pragma unroll
-    for (int wdx = 0; wdx < kRT / 32; ++wdx) {
-      sx += red[o][wdx].x;
-      sy += red[o][wdx].y;
-    }
-    partv[(long long)blockIdx.x * S.pstride + o] = make_double2(sx, sy);
+    for (int w = 0; w < kRT / 32; ++w) t += red[w][i];
+    reinterpret_cast<double*>(partv + (long long)blockIdx.x * S.pstride)[i] = t;
   }
 }
 
@@ -543,18 +612,30 @@ __device__ __forceinline__ double2 warp_chunk_sum(const double2* partv, int begi
   return make_double2(sx, sy);
 }
 
+// A job's norms and observables from its chunk partials.
 __global__ void __launch_bounds__(kRT)
-    k_s1_obs_final(const DevInst* __restrict__ st, const int* __restrict__ nchunks, const double2* __restrict__ partv) {
+    k_s1_final(const DevInst* __restrict__ st, const int* __restrict__ nchunks, const double* __restrict__ part,
+               const double2* __restrict__ partv) {
+  __shared__ double smem[32 * 2];
   const DevInst& S = st[blockIdx.x];
-  const int nob = S.nob;
-  if (nob == 0) return;
-  const int warp = threadIdx.x >> 5;
-  for (int o = warp; o < nob; o += blockDim.x >> 5) {
-    const double2 v = warp_chunk_sum(partv, S.chunk_begin, nchunks[blockIdx.x], S.pstride, o);
+  const int warp = threadIdx.x >> 5, nc = nchunks[blockIdx.x];
+  for (int o = warp; o < S.nob; o += blockDim.x >> 5) {
+    const double2 v = warp_chunk_sum(partv, S.chunk_begin, nc, S.pstride, o);
     if ((threadIdx.x & 31) == 0) {
       S.out[4 + 2 * o] = v.x;
       S.out[5 + 2 * o] = v.y;
     }
+  }
+  if (!S.nrm0 && !S.nrm1) return;
+  double acc[2] = {0, 0};
+  for (int c = threadIdx.x; c < nc; c += blockDim.x) {
+    acc[0] += part[2 * (S.chunk_begin + c)];
+    acc[1] += part[2 * (S.chunk_begin + c) + 1];
+  }
+  block_sum<2>(acc, smem, min((nc + 31) / 32, kRT / 32));
+  if (threadIdx.x == 0) {
+    S.out[0] = acc[0];
+    S.out[1] = acc[1];
   }
 }
 
@@ -585,10 +666,11 @@ __global__ void __launch_bounds__(kRT) k_load_v0(const DevInst* __restrict__ st,
 // small job set in one launch.  Pointers to data that the step writes carry no __restrict__
 // and no read-only loads, as one kernel writes and reads them.
 
-// alpha = t^H V_j for bordered cycles (whole block).
+// t^H V_j for bordered cycles (whole block; every thread gets the value).
 template <typename T2>
-__device__ void step_trace(DevInst& S, int j) {
+__device__ double2 step_trace(const DevInst& S, int j) {
   __shared__ double smem[32 * 2];
+  __shared__ double2 total;
   const T2* x = (const T2*)S.V + (long long)j * S.ldv;
   double acc[2] = {0, 0};
   for (int i = threadIdx.x; i < S.ndiag; i += blockDim.x) {
@@ -597,16 +679,18 @@ __device__ void step_trace(DevInst& S, int j) {
     acc[0] = fma(w, v.x, acc[0]);
     acc[1] = fma(w, v.y, acc[1]);
   }
-  block_sum<2>(acc, smem);
-  if (threadIdx.x == 0) S.alpha = make_double2(acc[0], acc[1]);
-  __syncthreads();  // smem is free for the block's next job
+  block_sum<2>(acc, smem, min((S.ndiag + 31) / 32, kRT / 32));
+  if (threadIdx.x == 0) total = make_double2(acc[0], acc[1]);
+  __syncthreads();
+  return total;
 }
 
 template <typename T2>
 __global__ void __launch_bounds__(kRT) k_step_trace(DevInst* st) {
   DevInst& S = st[blockIdx.x];
   if (S.done || !S.border) return;
-  step_trace<T2>(S, S.j);
+  const double2 a = step_trace<T2>(S, S.j);
+  if (threadIdx.x == 0) S.alpha = a;
 }
 
 // ---- FP64-basis projections and updates ------------------------------------------------
@@ -616,27 +700,8 @@ __global__ void __launch_bounds__(kRT) k_step_trace(DevInst* st) {
 // holding 4 elements of w in registers across all columns.  N = 120, 31 columns: 43 us against 129 us
 // (60 of them reductions) when every block summed eight columns one by one; 52 -> 4 us at one column.
 
-// Sums v[k] over the warp's lanes; afterwards v[0] of lane l is the total of value
-// l / (32 / NV).
-template <int NV>
-__device__ __forceinline__ void warp_transpose_sum(double (&v)[NV]) {
-  const int lane = threadIdx.x & 31;
-  int off = 16;
-#pragma unroll
-  for (int s = NV / 2; s >= 1; s >>= 1, off >>= 1) {
-    const bool up = lane & off;
-#pragma unroll
-    for (int i = 0; i < s; ++i) {
-      const double send = up ? v[i] : v[i + s];
-      const double keep = up ? v[i + s] : v[i];
-      v[i] = keep + __shfl_xor_sync(0xffffffffu, send, off);
-    }
-  }
-  for (; off >= 1; off >>= 1) v[0] += __shfl_xor_sync(0xffffffffu, v[0], off);
-}
-
-// Projections of the lane's 4 elements onto K columns, summed over the warp into row[2 k ..].
-template <int K>
+// Projections of the lane's E elements onto K columns, summed over the warp into row[2 k ..].
+template <int K, int E>
 __device__ __forceinline__ void dot_cols64(const double2* V, long long ld, const double2 (&w)[4], int left,
                                            double* row) {
   double acc[2 * K];
@@ -644,11 +709,11 @@ __device__ __forceinline__ void dot_cols64(const double2* V, long long ld, const
   for (int k = 0; k < 2 * K; ++k) acc[k] = 0;
 #pragma unroll
   for (int k = 0; k < K; ++k) {
-    double2 v[4];
+    double2 v[E];
 #pragma unroll
-    for (int q = 0; q < 4; ++q) v[q] = 32 * q < left ? V[k * ld + 32 * q] : make_double2(0.0, 0.0);
+    for (int q = 0; q < E; ++q) v[q] = 32 * q < left ? V[k * ld + 32 * q] : make_double2(0.0, 0.0);
 #pragma unroll
-    for (int q = 0; q < 4; ++q) {
+    for (int q = 0; q < E; ++q) {
       acc[2 * k] = fma(v[q].x, w[q].x, acc[2 * k]);
       acc[2 * k] = fma(v[q].y, w[q].y, acc[2 * k]);
       acc[2 * k + 1] = fma(v[q].x, w[q].y, acc[2 * k + 1]);
@@ -661,66 +726,92 @@ __device__ __forceinline__ void dot_cols64(const double2* V, long long ld, const
   if (lane % span == 0) row[lane / span] = acc[0];
 }
 
+template <int E>
+__device__ __forceinline__ void dot_range64(const double2* V, long long ld, const double2 (&w)[4], int left, int k,
+                                            int k1, double* row) {
+  for (; k + 16 <= k1; k += 16) dot_cols64<16, E>(V + k * ld, ld, w, left, row + 2 * k);
+  if (k + 8 <= k1) dot_cols64<8, E>(V + k * ld, ld, w, left, row + 2 * k), k += 8;
+  if (k + 4 <= k1) dot_cols64<4, E>(V + k * ld, ld, w, left, row + 2 * k), k += 4;
+  if (k + 2 <= k1) dot_cols64<2, E>(V + k * ld, ld, w, left, row + 2 * k), k += 2;
+  if (k < k1) dot_cols64<1, E>(V + k * ld, ld, w, left, row + 2 * k);
+}
+
 struct Dot64Smem {
   double row[8][2 * (kBatchMaxKrylov + 2)];  // per element group: (re, im) per column
   double norm[8];
 };
 
 // partv[c][i] = sum over chunk c of conj(V_i) w for i < nv, and ipart[c] = |w|^2 over the chunk
-// (ipart != nullptr).  The chunk is cut into groups of 128 elements (4 per lane); the warps
-// that a chunk of fewer than 8 groups leaves free take the groups' columns in parts.
+// (ipart != nullptr).  The chunk is cut into groups of 128 elements (4 per lane; chunks of 32
+// and 64 elements: 1 and 2 per lane); the warps that a chunk of fewer than 8 groups leaves
+// free take the groups' columns in parts.
 __device__ __forceinline__ void step_dot64(const DevInst& S, int nv, int c, double2* partv, double* ipart,
                                            Dot64Smem& sm) {
   long long beg, end;
   chunk_range(S, c, beg, end);
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int groups = S.chunk / 128, parts = 8 / groups;
+  const int groups = max(S.chunk / 128, 1), parts = 8 / groups;
   const int g = warp % groups, part = warp / groups;
   const long long e0 = beg + g * 128 + lane;
   const int left = (int)min(end - e0, 1024LL);  // element 32 q of the lane exists when 32 q < left
   double2 w[4];
 #pragma unroll
-  for (int q = 0; q < 4; ++q) w[q] = 32 * q < left ? ((const double2*)S.w)[e0 + 32 * q] : make_double2(0.0, 0.0);
+  for (int q = 0; q < 4; ++q)
+    w[q] = 32 * q < left ? ((const double2*)S.w)[e0 + 32 * q] : make_double2(0.0, 0.0);
   if (ipart != nullptr && part == 0) {
     double a = 0;
 #pragma unroll
-    for (int q = 0; q < 4; ++q) a = fma(w[q].y, w[q].y, fma(w[q].x, w[q].x, a));
+    for (int q = 0; q < 4; ++q)
+      if (32 * q < S.chunk) a = fma(w[q].y, w[q].y, fma(w[q].x, w[q].x, a));
 #pragma unroll
     for (int off = 16; off > 0; off >>= 1) a += __shfl_xor_sync(0xffffffffu, a, off);
     if (lane == 0) sm.norm[g] = a;
   }
   const int per = (nv + parts - 1) / parts;
-  int k = part * per;
-  const int k1 = min(k + per, nv);
+  const int k = part * per, k1 = min(k + per, nv);
   const double2* V = (const double2*)S.V + e0;
   const long long ld = S.ldv;
   double* row = sm.row[g];
-  for (; k + 16 <= k1; k += 16) dot_cols64<16>(V + k * ld, ld, w, left, row + 2 * k);
-  if (k + 8 <= k1) dot_cols64<8>(V + k * ld, ld, w, left, row + 2 * k), k += 8;
-  if (k + 4 <= k1) dot_cols64<4>(V + k * ld, ld, w, left, row + 2 * k), k += 4;
-  if (k + 2 <= k1) dot_cols64<2>(V + k * ld, ld, w, left, row + 2 * k), k += 2;
-  if (k < k1) dot_cols64<1>(V + k * ld, ld, w, left, row + 2 * k);
+  if (S.chunk == 32)  // block-uniform
+    dot_range64<1>(V, ld, w, left, k, k1, row);
+  else if (S.chunk == 64)
+    dot_range64<2>(V, ld, w, left, k, k1, row);
+  else
+    dot_range64<4>(V, ld, w, left, k, k1, row);
   __syncthreads();
   for (int i = threadIdx.x; i < 2 * nv; i += blockDim.x) {
-    double t = 0;
-    for (int q = 0; q < groups; ++q) t += sm.row[q][i];
+    double t = sm.row[0][i];
+    for (int q = 1; q < groups; ++q) t += sm.row[q][i];
     reinterpret_cast<double*>(partv + (long long)c * S.pstride)[i] = t;
   }
   if (ipart != nullptr && threadIdx.x == 0) {
-    double t = 0;
-    for (int q = 0; q < groups; ++q) t += sm.norm[q];
+    double t = sm.norm[0];
+    for (int q = 1; q < groups; ++q) t += sm.norm[q];
     ipart[c] = t;
   }
   __syncthreads();  // sm is free for the block's next chunk
 }
 
-// pass 1: hA and |w|^2; pass 2 only for jobs that reorthogonalise.
+// The chunk kernels take an `again` word: null in the first pass (one block per chunk); in the
+// second pass, which few jobs need, it says whether any does (k_step_norm), and a grid of a few
+// blocks per SM returns at once or walks the chunks of the jobs that do.
+template <typename F>
+__device__ __forceinline__ void for_chunks(const DevInst* st, const int* chunk_inst, int nchunk, const int* again,
+                                           const F& f) {
+  if (again != nullptr && *again == 0) return;
+  for (int c = blockIdx.x; c < nchunk; c += gridDim.x) {  // first pass: gridDim.x == nchunk
+    const DevInst& S = st[chunk_inst[c]];
+    if (!S.done && (again == nullptr || S.reorth)) f(S, c);
+  }
+}
+constexpr int kSecondPassBlocks = 4 * 152;
+
 __global__ void __launch_bounds__(kRT, 2)
-    k_step_dot64(const DevInst* st, const int* chunk_inst, double2* partv, double* ipart, int second) {
+    k_step_dot64(const DevInst* st, const int* chunk_inst, int nchunk, double2* partv, double* ipart,
+                 const int* again) {
   __shared__ Dot64Smem sm;
-  const DevInst& S = st[chunk_inst[blockIdx.x]];
-  if (S.done || (second && !S.reorth)) return;
-  step_dot64(S, S.j + 1, blockIdx.x, partv, ipart, sm);
+  for_chunks(st, chunk_inst, nchunk, again,
+             [&](const DevInst& S, int c) { step_dot64(S, S.j + 1, c, partv, ipart, sm); });
 }
 
 // which 0: hA, 1: hB (jobs that reorthogonalise).  Grid (instances, column groups): warp w of
@@ -737,66 +828,103 @@ __global__ void __launch_bounds__(kRT)
   if ((threadIdx.x & 31) == 0) S.hB[i] = v;
 }
 
-// |w|^2 of job S from its chunk partials (thread t sums partials t, t + 256, ..., then a
-// deterministic block sum); the result is valid in thread 0.
-__device__ __forceinline__ double job_norm2(const DevInst& S, int nchunks, const double* part) {
-  __shared__ double smem[32];
-  double acc[1] = {0};
-  for (int c = threadIdx.x; c < nchunks; c += blockDim.x) acc[0] += part[S.chunk_begin + c];
-  block_sum<1>(acc, smem);
-  __syncthreads();  // smem is free for the block's next job
-  return acc[0];
+// Sums of a job's chunk partials (thread t sums partials t, t + 256, ..., then a deterministic
+// block sum), to the whole block: x from a, y from b (b != nullptr).
+__device__ __forceinline__ double2 job_norms(const DevInst& S, int nchunks, const double* a, const double* b) {
+  __shared__ double smem[32 * 2];
+  __shared__ double2 total;
+  double acc[2] = {0, 0};
+  for (int c = threadIdx.x; c < nchunks; c += blockDim.x) {
+    acc[0] += a[S.chunk_begin + c];
+    if (b != nullptr) acc[1] += b[S.chunk_begin + c];
+  }
+  block_sum<2>(acc, smem, min((nchunks + 31) / 32, kRT / 32));
+  if (threadIdx.x == 0) total = make_double2(acc[0], acc[1]);
+  __syncthreads();
+  const double2 t = total;
+  __syncthreads();  // total is free for the block's next job
+  return t;
 }
 
-// The first-pass reductions of a step in one launch: blocks (x, y < gridDim.y - 1) reduce the
-// projections into hA, blocks (x, gridDim.y - 1) the image norm |L V_j|^2.
+// The first-pass projections of a step into hA (grid as k_step_mdot_final's).
 __global__ void __launch_bounds__(kRT)
-    k_step_first_final(DevInst* st, const int* __restrict__ nchunks, const double2* partv, const double* part) {
+    k_step_first_final(DevInst* st, const int* __restrict__ nchunks, const double2* partv) {
   DevInst& S = st[blockIdx.x];
   if (S.done) return;
-  if (blockIdx.y == gridDim.y - 1) {  // image norm (block-uniform)
-    const double v = job_norm2(S, nchunks[blockIdx.x], part);
-    if (threadIdx.x == 0) S.image2 = v;
-    return;
-  }
   const int i = blockIdx.y * (blockDim.x >> 5) + (threadIdx.x >> 5);
   if (i > S.j) return;  // warp-uniform
   const double2 v = warp_chunk_sum(partv, S.chunk_begin, nchunks[blockIdx.x], S.pstride, i);
   if ((threadIdx.x & 31) == 0) S.hA[i] = v;
 }
 
-// After the first update (whole block): |w1|^2 and whether the job reorthogonalises.  Selective
-// reorthogonalisation (Daniel, Gragg, Kaufman, Stewart, Math. Comp. 30, 772 (1976)): when
-// |w1|^2 >= |w0|^2 / 2 (w0 = L V_j before any projection) the first pass has left w orthogonal
-// to the basis to working precision, and the second pass is skipped (zero hB).
-__device__ __forceinline__ void step_norm1(DevInst& S, int nv, int nchunks, const double* part) {
-  const double v = job_norm2(S, nchunks, part);
-  if (threadIdx.x == 0) {
-    S.rem2 = v;
-    S.reorth = v < 0.5 * S.image2 ? 1 : 0;
+// 1 / |w| (zero on an exact breakdown).
+__device__ __forceinline__ double inverse_norm(double rem2) {
+  const double r = sqrt(rem2);
+  return r > 0 ? 1.0 / r : 0.0;
+}
+
+// The same for the whole block: one warp computes it, as the FP64 root and quotient of eight
+// warps would queue on the pipe.
+__device__ __forceinline__ double block_inverse_norm(double rem2) {
+  __shared__ double inv;
+  __syncthreads();  // an earlier value has been read
+  if (threadIdx.x < 32) {
+    const double f = inverse_norm(rem2);
+    if (threadIdx.x == 0) inv = f;
   }
-  for (int i = threadIdx.x; i < nv; i += blockDim.x) S.hB[i] = make_double2(0.0, 0.0);
+  __syncthreads();
+  return inv;
+}
+
+// After the first update (whole block): |L V_j|^2, |w1|^2 and whether the job reorthogonalises.
+// Selective reorthogonalisation (Daniel, Gragg, Kaufman, Stewart, Math. Comp. 30, 772 (1976)):
+// when |w1|^2 >= |w0|^2 / 2 (w0 = L V_j before any projection) the first pass has left w
+// orthogonal to the basis to working precision, and the second pass is skipped (zero hB).
+// `store`: this block writes the job's record.
+struct StepNorms {
+  double rem2;
+  bool reorth;
+};
+__device__ __forceinline__ StepNorms step_norm1(DevInst& S, int nv, int nchunks, const double* part,
+                                                const double* part1, bool store) {
+  const double2 v = job_norms(S, nchunks, part, part1);
+  const bool reorth = v.y < 0.5 * v.x;
+  if (store) {
+    if (threadIdx.x == 0) {
+      S.image2 = v.x;
+      S.rem2 = v.y;
+      S.reorth = reorth ? 1 : 0;
+      if (!reorth) S.inv = inverse_norm(v.y);
+    }
+    for (int i = threadIdx.x; i < nv; i += blockDim.x) S.hB[i] = make_double2(0.0, 0.0);
+  }
+  return StepNorms{v.y, reorth};
 }
 
 // One block per job.  second 0: step_norm1; 1: |w|^2 after the second update of a job that
 // reorthogonalised.
 __global__ void __launch_bounds__(kRT)
-    k_step_norm(DevInst* st, const int* __restrict__ nchunks, const double* part, int second) {
+    k_step_norm(DevInst* st, const int* __restrict__ nchunks, const double* part, const double* part1, int second,
+                int* again) {
   DevInst& S = st[blockIdx.x];
   if (S.done) return;
   if (!second) {
-    step_norm1(S, S.j + 1, nchunks[blockIdx.x], part);
+    const StepNorms r = step_norm1(S, S.j + 1, nchunks[blockIdx.x], part, part1, true);
+    if (r.reorth && threadIdx.x == 0) atomicExch(again, 1);
   } else if (S.reorth) {
-    const double v = job_norm2(S, nchunks[blockIdx.x], part);
-    if (threadIdx.x == 0) S.rem2 = v;
+    const double2 v = job_norms(S, nchunks[blockIdx.x], part, nullptr);
+    if (threadIdx.x == 0) {
+      S.rem2 = v.x;
+      S.inv = inverse_norm(v.x);
+    }
   }
 }
 
 // w -= sum_i V_i h_i over chunk c and part[c] = |w|^2 of the result.  A thread holds up to 4
-// elements; chunks of 128 elements split the columns between the block's two halves.
+// elements; chunks of fewer than 256 elements split the columns between parts of the block.
 struct Axpy64Smem {
   double2 h[kBatchMaxKrylov + 2];
-  double2 half[128];
+  double2 share[kRT];
   double red[32];
 };
 
@@ -813,30 +941,30 @@ __device__ __forceinline__ void axpy_cols64(const double2* V, long long ld, cons
   }
 }
 
-__device__ __forceinline__ void step_axpy64(const DevInst& S, int nv, int c, const double2* h, double* part,
-                                            Axpy64Smem& sm) {
-  for (int i = threadIdx.x; i < nv; i += blockDim.x) sm.h[i] = h[i];
-  __syncthreads();
+// sm.h holds the projections (the caller has synchronised).
+__device__ __forceinline__ void step_axpy64(const DevInst& S, int nv, int c, double* part, Axpy64Smem& sm) {
   long long beg, end;
   chunk_range(S, c, beg, end);
   const double2* V = (const double2*)S.V;
   double2* w = (double2*)S.w;
   const long long ld = S.ldv;
   double acc[1] = {0};
-  if (S.chunk == 128) {  // block-uniform
-    const int lo = threadIdx.x & 127, upper = threadIdx.x >> 7;
-    const long long e = beg + lo;
-    const int mid = (nv + 1) / 2;
+  if (S.chunk < kRT) {  // block-uniform
+    const int at = threadIdx.x % S.chunk, p = threadIdx.x / S.chunk, parts = kRT / S.chunk;
+    const long long e = beg + at;
+    const int per = (nv + parts - 1) / parts;
     double2 v = make_double2(0.0, 0.0);
     if (e < end) {
-      if (!upper) v = w[e];
-      axpy_cols64(V + e, ld, sm.h, upper ? mid : 0, upper ? nv : mid, v);
+      if (p == 0) v = w[e];
+      axpy_cols64(V + e, ld, sm.h, p * per, min(p * per + per, nv), v);
     }
-    if (upper) sm.half[lo] = v;
+    sm.share[threadIdx.x] = v;
     __syncthreads();
-    if (!upper && e < end) {
-      v.x += sm.half[lo].x;
-      v.y += sm.half[lo].y;
+    if (p == 0 && e < end) {
+      for (int q = 1; q < parts; ++q) {
+        v.x += sm.share[q * S.chunk + at].x;
+        v.y += sm.share[q * S.chunk + at].y;
+      }
       w[e] = v;
       acc[0] = fma(v.y, v.y, v.x * v.x);
     }
@@ -849,23 +977,24 @@ __device__ __forceinline__ void step_axpy64(const DevInst& S, int nv, int c, con
       acc[0] = fma(v.y, v.y, acc[0]);
     }
   }
-  block_sum<1>(acc, sm.red);
+  block_sum<1>(acc, sm.red, min(S.chunk, kRT) / 32);
   if (threadIdx.x == 0) part[c] = acc[0];
   __syncthreads();  // sm is free for the block's next chunk
 }
 
 __global__ void __launch_bounds__(kRT, 2)
-    k_step_axpy64(const DevInst* st, const int* chunk_inst, double* part, int second) {
+    k_step_axpy64(const DevInst* st, const int* chunk_inst, int nchunk, double* part, const int* again) {
   __shared__ Axpy64Smem sm;
-  const DevInst& S = st[chunk_inst[blockIdx.x]];
-  if (S.done || (second && !S.reorth)) return;
-  step_axpy64(S, S.j + 1, blockIdx.x, second ? S.hB : S.hA, part, sm);
+  for_chunks(st, chunk_inst, nchunk, again, [&](const DevInst& S, int c) {
+    const double2* h = again ? S.hB : S.hA;
+    for (int i = threadIdx.x; i <= S.j; i += blockDim.x) sm.h[i] = h[i];
+    __syncthreads();
+    step_axpy64(S, S.j + 1, c, part, sm);
+  });
 }
 
-// V_{j+1} = w / |w| over chunk c (zero on an exact breakdown).
-__device__ __forceinline__ void step_normalize64(const DevInst& S, int j, int c) {
-  const double r = sqrt(S.rem2);
-  const double f = r > 0 ? 1.0 / r : 0.0;
+// V_{j+1} = f w over chunk c, f = 1 / |w|.
+__device__ __forceinline__ void step_normalize64(const DevInst& S, int j, int c, double f) {
   long long beg, end;
   chunk_range(S, c, beg, end);
   const double2* w = (const double2*)S.w;
@@ -879,7 +1008,7 @@ __device__ __forceinline__ void step_normalize64(const DevInst& S, int j, int c)
 __global__ void __launch_bounds__(kRT) k_step_normalize64(const DevInst* st, const int* chunk_inst) {
   const DevInst& S = st[chunk_inst[blockIdx.x]];
   if (S.done) return;
-  step_normalize64(S, S.j, blockIdx.x);
+  step_normalize64(S, S.j, blockIdx.x, S.inv);
 }
 
 // ---- FP32-basis CGS2 kernels: pairs of complex elements per 16-byte load ---------------
@@ -949,18 +1078,72 @@ __device__ __forceinline__ void pair_terms(const float4 a, const float4 b, DF& r
 // its chunk for the image norm |L V_j| (the expv error estimate and the reorthogonalisation
 // test) -- the same pairs in the same order as a separate sweep over w would take -- while w
 // is staged anyway.
+//
+// The lane sums of K columns exchange halves of the accumulators (2K - 1 double-float additions
+// and as many shuffles, against 10K one value at a time, which at 1024 elements per chunk were
+// two thirds of the instructions); each value is still summed over the same tree of lanes.
+template <int NV>
+__device__ __forceinline__ void warp_transpose_sum(DF (&v)[NV]) {
+  const int lane = threadIdx.x & 31;
+  int off = 16;
+#pragma unroll
+  for (int s = NV / 2; s >= 1; s >>= 1, off >>= 1) {
+    const bool up = lane & off;
+#pragma unroll
+    for (int i = 0; i < s; ++i) {
+      const DF send = up ? v[i] : v[i + s], keep = up ? v[i + s] : v[i];
+      v[i] = df_sum(keep, DF{__shfl_xor_sync(0xffffffffu, send.hi, off), __shfl_xor_sync(0xffffffffu, send.lo, off)});
+    }
+  }
+  for (; off >= 1; off >>= 1)
+    v[0] = df_sum(v[0], DF{__shfl_xor_sync(0xffffffffu, v[0].hi, off), __shfl_xor_sync(0xffffffffu, v[0].lo, off)});
+}
+
 template <int CH>
 struct Dot32Smem {
   float4 w[CH / 2];
-  // per warp: (re.hi, re.lo, im.hi, im.lo) of each basis column (at most kBatchMaxKrylov + 1);
-  // sized to the engine's Krylov limit so the block stays inside 48 KB of static shared memory
-  float4 red[kBatchMaxKrylov + 2][kRT / 32];
+  // per warp: double-float (hi, lo) of re and im of each basis column (at most kBatchMaxKrylov
+  // + 1); sized to the engine's Krylov limit so the block stays inside 48 KB of shared memory
+  float2 red[kRT / 32][2 * (kBatchMaxKrylov + 2)];
 };
 
-template <int CH>
+// K columns from V4 on: row[2 k], row[2 k + 1] = the warp's sums.
+template <int K, int CH>
+__device__ __forceinline__ void dot_cols32(const float4* V4, long long ld4, const float4* w, int npair, float2* row) {
+  constexpr int kPairs = CH / 2 / kRT;  // element pairs per thread and chunk
+  constexpr int kStep = K * kPairs <= 16 ? kPairs : 2;  // pairs whose K loads are in flight together
+  const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+  DF acc[2 * K];
+#pragma unroll
+  for (int k = 0; k < 2 * K; ++k) acc[k] = DF{0.f, 0.f};
+#pragma unroll 1
+  for (int q0 = 0; q0 < kPairs; q0 += kStep) {
+    float4 v[K][kStep];
+#pragma unroll
+    for (int k = 0; k < K; ++k)
+#pragma unroll
+      for (int q = 0; q < kStep; ++q) {
+        const int p = threadIdx.x + (q0 + q) * kRT;
+        v[k][q] = p < npair ? V4[k * ld4 + p] : zero;
+      }
+#pragma unroll
+    for (int q = 0; q < kStep; ++q) {
+      const float4 wv = w[threadIdx.x + (q0 + q) * kRT];
+#pragma unroll
+      for (int k = 0; k < K; ++k) pair_terms(v[k][q], wv, acc[2 * k], acc[2 * k + 1]);
+    }
+  }
+  warp_transpose_sum<2 * K>(acc);
+  constexpr int span = 32 / (2 * K);
+  const int lane = threadIdx.x & 31;
+  if (lane % span == 0) row[lane / span] = make_float2(acc[0].hi, acc[0].lo);
+}
+
+// KMAX: columns per group, by the registers that the kernel has (every split sums alike).
+template <int CH, int KMAX>
 __device__ __forceinline__ void step_dot32(const DevInst& S, int nv, int c, double2* partv, double* ipart,
                                            Dot32Smem<CH>& sm) {
-  constexpr int kPairs = CH / 2 / kRT;  // element pairs per thread and chunk
+  constexpr int kPairs = CH / 2 / kRT;
   long long beg, end;
   pair_range(S, c, beg, end);
   const int npair = (int)(end - beg);
@@ -976,74 +1159,34 @@ __device__ __forceinline__ void step_dot32(const DevInst& S, int nv, int c, doub
     if (p < npair) df_add(nrm, fmaf(wv.x, wv.x, fmaf(wv.y, wv.y, fmaf(wv.z, wv.z, wv.w * wv.w))));
   }
   if (ipart != nullptr) {  // block-uniform
-    const double r = block_df_sum(nrm, reinterpret_cast<float2*>(&sm.red[0][0]));
+    const double r = block_df_sum(nrm, &sm.red[0][0]);
     if (threadIdx.x == 0) ipart[c] = r;
+    __syncthreads();  // red is free
   }
-  __syncthreads();
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+  // a thread reads back its own entries of sm.w only
+  float2* row = sm.red[threadIdx.x >> 5];
   int k = 0;
-  // two columns per iteration: 2 * kPairs independent 16-byte loads in flight per thread
-  for (; k + 1 < nv; k += 2) {
-    const float4* c0 = V4 + (long long)k * ld4;
-    const float4* c1 = c0 + ld4;
-    float4 a[kPairs], b[kPairs];
-#pragma unroll
-    for (int q = 0; q < kPairs; ++q) {
-      const int p = threadIdx.x + q * kRT;
-      a[q] = p < npair ? c0[p] : zero;
-      b[q] = p < npair ? c1[p] : zero;
-    }
-    DF r0{0.f, 0.f}, i0{0.f, 0.f}, r1{0.f, 0.f}, i1{0.f, 0.f};
-#pragma unroll
-    for (int q = 0; q < kPairs; ++q) {
-      const float4 wv = sm.w[threadIdx.x + q * kRT];
-      pair_terms(a[q], wv, r0, i0);
-      pair_terms(b[q], wv, r1, i1);
-    }
-    r0 = warp_df_sum(r0);
-    i0 = warp_df_sum(i0);
-    r1 = warp_df_sum(r1);
-    i1 = warp_df_sum(i1);
-    if (lane == 0) {
-      sm.red[k][warp] = make_float4(r0.hi, r0.lo, i0.hi, i0.lo);
-      sm.red[k + 1][warp] = make_float4(r1.hi, r1.lo, i1.hi, i1.lo);
-    }
-  }
-  if (k < nv) {
-    const float4* c0 = V4 + (long long)k * ld4;
-    DF r0{0.f, 0.f}, i0{0.f, 0.f};
-#pragma unroll
-    for (int q = 0; q < kPairs; ++q) {
-      const int p = threadIdx.x + q * kRT;
-      pair_terms(p < npair ? c0[p] : zero, sm.w[p], r0, i0);
-    }
-    r0 = warp_df_sum(r0);
-    i0 = warp_df_sum(i0);
-    if (lane == 0) sm.red[k][warp] = make_float4(r0.hi, r0.lo, i0.hi, i0.lo);
-  }
+  for (; k + KMAX <= nv; k += KMAX) dot_cols32<KMAX, CH>(V4 + k * ld4, ld4, sm.w, npair, row + 2 * k);
+  if (KMAX > 4 && k + 4 <= nv) dot_cols32<4, CH>(V4 + k * ld4, ld4, sm.w, npair, row + 2 * k), k += 4;
+  if (k + 2 <= nv) dot_cols32<2, CH>(V4 + k * ld4, ld4, sm.w, npair, row + 2 * k), k += 2;
+  if (k < nv) dot_cols32<1, CH>(V4 + k * ld4, ld4, sm.w, npair, row + 2 * k);
   __syncthreads();
-  for (int kk = threadIdx.x; kk < nv; kk += blockDim.x) {
-    DF sr{0.f, 0.f}, si{0.f, 0.f};
+  for (int i = threadIdx.x; i < 2 * nv; i += blockDim.x) {
+    DF t{0.f, 0.f};
 #pragma unroll
-    for (int wdx = 0; wdx < kRT / 32; ++wdx) {
-      const float4 r = sm.red[kk][wdx];
-      sr = df_sum(sr, DF{r.x, r.y});
-      si = df_sum(si, DF{r.z, r.w});
-    }
-    partv[(long long)c * S.pstride + kk] =
-        make_double2((double)sr.hi + (double)sr.lo, (double)si.hi + (double)si.lo);
+    for (int wdx = 0; wdx < kRT / 32; ++wdx) t = df_sum(t, DF{sm.red[wdx][i].x, sm.red[wdx][i].y});
+    reinterpret_cast<double*>(partv + (long long)c * S.pstride)[i] = (double)t.hi + (double)t.lo;
   }
   __syncthreads();  // sm is free for the block's next chunk
 }
 
 template <int CH>
 __global__ void __launch_bounds__(kRT, 3)
-    k_step_mdot_f32(const DevInst* st, const int* chunk_inst, double2* partv, double* ipart, int second) {
+    k_step_mdot_f32(const DevInst* st, const int* chunk_inst, int nchunk, double2* partv, double* ipart,
+                    const int* again) {
   __shared__ Dot32Smem<CH> sm;
-  const DevInst& S = st[chunk_inst[blockIdx.x]];
-  if (S.done || (second && !S.reorth)) return;
-  step_dot32<CH>(S, S.j + 1, blockIdx.x, partv, ipart, sm);
+  for_chunks(st, chunk_inst, nchunk, again,
+             [&](const DevInst& S, int c) { step_dot32<CH, 4>(S, S.j + 1, c, partv, ipart, sm); });
 }
 
 // cout (+)= sum_k ccoef[k] V_k for an FP32 basis in double-float arithmetic: each FP64
@@ -1061,7 +1204,7 @@ __device__ __forceinline__ void df_axpy(DF& acc, float ch, float cl, float v) {
 }
 
 __global__ void __launch_bounds__(kRT)
-    k_s1_combine_f32(const DevInst* __restrict__ st, const int* __restrict__ chunk_inst) {
+    k_s1_combine_f32(const DevInst* __restrict__ st, const int* __restrict__ chunk_inst, double* __restrict__ part) {
   __shared__ float4 cs[kBatchMaxKrylov + 2];  // (re.hi, re.lo, im.hi, im.lo)
   const DevInst& S = st[chunk_inst[blockIdx.x]];
   double2* out = S.cout;
@@ -1074,29 +1217,40 @@ __global__ void __launch_bounds__(kRT)
   }
   __syncthreads();
   long long beg, end;
-  chunk_range(S, blockIdx.x, beg, end);
-  const float2* __restrict__ V = reinterpret_cast<const float2*>(S.V);
-  const long long ld = S.ldv;
+  pair_range(S, blockIdx.x, beg, end);
+  const float4* __restrict__ V4 = reinterpret_cast<const float4*>(S.V);
+  const long long ld4 = S.ldv / 2;
   const int acc = S.cacc;
-  for (long long e = beg + threadIdx.x; e < end; e += blockDim.x) {
-    DF yr{0.f, 0.f}, yi{0.f, 0.f};
-#pragma unroll 4
+  double nrm = 0;
+  for (long long p = beg + threadIdx.x; p < end; p += blockDim.x) {
+    DF y0r{0.f, 0.f}, y0i{0.f, 0.f}, y1r{0.f, 0.f}, y1i{0.f, 0.f};
+#pragma unroll 8
     for (int k = 0; k < nc; ++k) {
-      const float2 v = V[(long long)k * ld + e];
+      const float4 v = V4[(long long)k * ld4 + p];
       const float4 c = cs[k];
-      df_axpy(yr, c.x, c.y, v.x);
-      df_axpy(yr, -c.z, -c.w, v.y);
-      df_axpy(yi, c.x, c.y, v.y);
-      df_axpy(yi, c.z, c.w, v.x);
+      df_axpy(y0r, c.x, c.y, v.x);
+      df_axpy(y0r, -c.z, -c.w, v.y);
+      df_axpy(y0i, c.x, c.y, v.y);
+      df_axpy(y0i, c.z, c.w, v.x);
+      df_axpy(y1r, c.x, c.y, v.z);
+      df_axpy(y1r, -c.z, -c.w, v.w);
+      df_axpy(y1i, c.x, c.y, v.w);
+      df_axpy(y1i, c.z, c.w, v.z);
     }
-    double ox = (double)yr.hi + (double)yr.lo, oy = (double)yi.hi + (double)yi.lo;
-    if (acc) {
-      const double2 o = out[e];
-      ox += o.x;
-      oy += o.y;
-    }
-    out[e] = make_double2(ox, oy);
+    auto put = [&](long long e, DF r, DF i) {
+      double ox = (double)r.hi + (double)r.lo, oy = (double)i.hi + (double)i.lo;
+      if (acc) {
+        const double2 o = out[e];
+        ox += o.x;
+        oy += o.y;
+      }
+      out[e] = make_double2(ox, oy);
+      nrm = fma(oy, oy, fma(ox, ox, nrm));
+    };
+    put(2 * p, y0r, y0i);
+    if (2 * p + 1 < S.dim) put(2 * p + 1, y1r, y1i);
   }
+  combined_norm(S, nrm, part);
 }
 
 // w -= sum_i V_i h_i over chunk c of an FP32 basis, FP32 update, and the double-float |w|^2
@@ -1106,10 +1260,8 @@ struct Axpy32Smem {
   float2 red[32];
 };
 
-__device__ __forceinline__ void step_axpy32(const DevInst& S, int nv, int c, const double2* h, double* part,
-                                            Axpy32Smem& sm) {
-  for (int i = threadIdx.x; i < nv; i += blockDim.x) sm.h[i] = make_float2((float)h[i].x, (float)h[i].y);
-  __syncthreads();
+// sm.h holds the projections (the caller has synchronised).
+__device__ __forceinline__ void step_axpy32(const DevInst& S, int nv, int c, double* part, Axpy32Smem& sm) {
   long long beg, end;
   pair_range(S, c, beg, end);
   float4* w4 = reinterpret_cast<float4*>(S.w);
@@ -1140,17 +1292,18 @@ __device__ __forceinline__ void step_axpy32(const DevInst& S, int nv, int c, con
 }
 
 __global__ void __launch_bounds__(kRT)
-    k_step_maxpy_f32(const DevInst* st, const int* chunk_inst, double* part, int second) {
+    k_step_maxpy_f32(const DevInst* st, const int* chunk_inst, int nchunk, double* part, const int* again) {
   __shared__ Axpy32Smem sm;
-  const DevInst& S = st[chunk_inst[blockIdx.x]];
-  if (S.done || (second && !S.reorth)) return;
-  step_axpy32(S, S.j + 1, blockIdx.x, second ? S.hB : S.hA, part, sm);
+  for_chunks(st, chunk_inst, nchunk, again, [&](const DevInst& S, int c) {
+    const double2* h = again ? S.hB : S.hA;
+    for (int i = threadIdx.x; i <= S.j; i += blockDim.x) sm.h[i] = make_float2((float)h[i].x, (float)h[i].y);
+    __syncthreads();
+    step_axpy32(S, S.j + 1, c, part, sm);
+  });
 }
 
-// V_{j+1} = w / |w| over chunk c (zero on an exact breakdown), FP32 basis.
-__device__ __forceinline__ void step_normalize32(const DevInst& S, int j, int c) {
-  const double r = sqrt(S.rem2);
-  const float f = r > 0 ? (float)(1.0 / r) : 0.f;
+// V_{j+1} = f w over chunk c, f = 1 / |w|, FP32 basis.
+__device__ __forceinline__ void step_normalize32(const DevInst& S, int j, int c, float f) {
   long long beg, end;
   pair_range(S, c, beg, end);
   const float4* w4 = reinterpret_cast<const float4*>(S.w);
@@ -1164,98 +1317,130 @@ __device__ __forceinline__ void step_normalize32(const DevInst& S, int j, int c)
 __global__ void __launch_bounds__(kRT) k_step_normalize_f32(const DevInst* st, const int* chunk_inst) {
   const DevInst& S = st[chunk_inst[blockIdx.x]];
   if (S.done) return;
-  step_normalize32(S, S.j, blockIdx.x);
+  step_normalize32(S, S.j, blockIdx.x, (float)S.inv);
 }
 
 // Per instance (one warp): records Hessenberg column j, applies the GMRES rotations and stop
-// test (krylov.jl:759-777), advances j.  The warp gathers the column (hA + hB), the zero
-// fill and the stored rotations into shared memory in parallel; lane 0 then runs the
-// sequential rotation arithmetic on shared memory (the same operations in the same order
-// as a single-thread pass over global memory, whose dependent loads dominated the step) and
-// the warp writes the column back.  True (in lane 0) when the job takes no further step.  Not
-// inlined: the step kernel and k_cycle share one body, so both round alike.
+// test (krylov.jl:759-777).  True (in every lane) when the job takes no further step.  An FP64
+// instruction of one lane holds the pipe as long as one of 32, so the work is spread over the
+// lanes: the rotations of the column are a linear recurrence in the running entry t (t' = c h -
+// conj(s) t) whose products with c h are formed for all rows at once and whose real and
+// imaginary part advance in two lanes together; the rotated entries c t + s h follow for all
+// rows at once.  25 rotations: 25 -> 10 us against one lane doing the whole column.  Not inlined:
+// the step kernel and k_cycle share one body, so both round alike.
 struct FinishSmem {
-  double2 col[kBatchMaxKrylov + 2];
-  double cs[kBatchMaxKrylov + 2];
+  double2 h[kBatchMaxKrylov + 2];   // the new column
+  double2 t[kBatchMaxKrylov + 2];   // running entry before rotation r
+  double2 ch[kBatchMaxKrylov + 2];  // c_r h_{r+1}
   double2 sn[kBatchMaxKrylov + 2];
+  double cs[kBatchMaxKrylov + 2];
 };
 
 __device__ __noinline__ bool step_finish(DevInst& S, int j, FinishSmem& sm) {
   const int lane = threadIdx.x & 31;
-  double2* colv = sm.col;
-  double* csv = sm.cs;
-  double2* snv = sm.sn;
-  bool stop = false;
   const int ld = S.ldh;
   double2* col = S.H + (long long)j * ld;
   double2* cs = S.csn;
   double2* sn = S.csn + ld;
+  const double root = sqrt(lane & 1 ? S.image2 : S.rem2);
+  const double rem = __shfl_sync(0xffffffffu, root, 0);
+  if (lane == 1) S.image[j] = root;
+  if (lane == 0) S.kdone = j + 1;
   for (int r = lane; r < ld; r += 32)
-    colv[r] = r <= j ? make_double2(S.hA[r].x + S.hB[r].x, S.hA[r].y + S.hB[r].y) : make_double2(0.0, 0.0);
-  if (S.givens)
-    for (int r = lane; r < j; r += 32) {
-      csv[r] = cs[r].x;
-      snv[r] = sn[r];
-    }
+    sm.h[r] = r <= j       ? make_double2(S.hA[r].x + S.hB[r].x, S.hA[r].y + S.hB[r].y)
+              : r == j + 1 ? make_double2(rem, 0.0)
+                           : make_double2(0.0, 0.0);
+  bool stop = (j + 1 >= S.m) || rem == 0.0 || (long long)(j + 1) == S.dim;
   __syncwarp();
-  if (lane == 0) {
-    const double rem = sqrt(S.rem2);
-    colv[j + 1] = make_double2(rem, 0.0);
-    S.image[j] = sqrt(S.image2);
-    S.kdone = j + 1;
-    stop = (j + 1 >= S.m) || rem == 0.0 || (long long)(j + 1) == S.dim;
-    if (S.givens) {
-      for (int r = 0; r < j; ++r) {
-        const double2 h1 = colv[r], h2 = colv[r + 1];
-        const double c = csv[r];
-        const double2 s = snv[r];
-        const double2 sh2 = cmul(s, h2);
-        const double2 csh1 = cmul(conjd(s), h1);
-        colv[r] = make_double2(c * h1.x + sh2.x, c * h1.y + sh2.y);
-        colv[r + 1] = make_double2(-csh1.x + c * h2.x, -csh1.y + c * h2.y);
+  if (S.givens) {
+    for (int r = lane; r < j; r += 32) {
+      const double c = cs[r].x;
+      sm.cs[r] = c;
+      sm.sn[r] = sn[r];
+      sm.ch[r] = make_double2(c * sm.h[r + 1].x, c * sm.h[r + 1].y);
+    }
+    __syncwarp();
+    // even lanes carry Re t, odd lanes Im t
+    const int im = lane & 1;
+    double mine = im ? sm.h[0].y : sm.h[0].x;
+#pragma unroll 4
+    for (int r = 0; r < j; ++r) {
+      const double other = __shfl_xor_sync(0xffffffffu, mine, 1);
+      if (lane < 2) reinterpret_cast<double*>(sm.t)[2 * r + im] = mine;
+      const double2 s = sm.sn[r], ch = sm.ch[r];
+      // -conj(s) t: Re = -(s.x t.x + s.y t.y), Im = -(s.x t.y - s.y t.x)
+      mine = fma(-s.x, mine, fma(im ? s.y : -s.y, other, im ? ch.y : ch.x));
+    }
+    const double other = __shfl_xor_sync(0xffffffffu, mine, 1);
+    const double2 a = im ? make_double2(other, mine) : make_double2(mine, other);  // entry j, rotated
+    __syncwarp();
+    for (int base = 0; base < j; base += 32) {
+      const int r = base + lane;
+      double2 v = make_double2(0.0, 0.0);
+      if (r < j) {
+        const double2 t = sm.t[r], h = sm.h[r + 1], s = sm.sn[r];
+        const double c = sm.cs[r];
+        v = make_double2(fma(c, t.x, fma(s.x, h.x, -s.y * h.y)), fma(c, t.y, fma(s.x, h.y, s.y * h.x)));
       }
-      // complex Givens rotation (krylov.jl:710-716)
-      const double2 a = colv[j], b = colv[j + 1];
-      double c;
-      double2 s;
-      if (b.x == 0.0 && b.y == 0.0) {
-        c = 1.0;
-        s = make_double2(0.0, 0.0);
-      } else if (a.x == 0.0 && a.y == 0.0) {
-        c = 0.0;
-        s = make_double2(1.0, 0.0);
+      __syncwarp();  // h[r] is the next lane's h_{r+1}
+      if (r < j) sm.h[r] = v;
+      __syncwarp();
+    }
+    // complex Givens rotation of (a, rem) (krylov.jl:710-716; rem is real and not negative):
+    // c = |a| / |(a, rem)|, s = (a / |a|) rem / |(a, rem)|, the four quotients in four lanes
+    double c;
+    double2 s;
+    if (rem == 0.0) {
+      c = 1.0;
+      s = make_double2(0.0, 0.0);
+    } else if (a.x == 0.0 && a.y == 0.0) {
+      c = 0.0;
+      s = make_double2(1.0, 0.0);
+    } else {
+      // |a| and |(a, rem)|; their squares are formed unless they could leave the FP64 range
+      const double big = fmax(fabs(a.x), fabs(a.y));
+      double aa, nn;
+      if (big > 1e-140 && fmax(big, rem) < 1e140) {
+        const double a2 = fma(a.x, a.x, a.y * a.y);
+        const double two = sqrt(lane & 1 ? fma(rem, rem, a2) : a2);
+        aa = __shfl_sync(0xffffffffu, two, 0);
+        nn = __shfl_sync(0xffffffffu, two, 1);
       } else {
-        const double aa = hypot(a.x, a.y), bb = hypot(b.x, b.y);
-        const double sc = aa + bb;
-        const double ax = a.x / sc, ay = a.y / sc, bx = b.x / sc, by = b.y / sc;
-        const double normab = sc * sqrt((ax * ax + ay * ay) + (bx * bx + by * by));
-        const double2 al = make_double2(a.x / aa, a.y / aa);
-        c = aa / normab;
-        const double2 t = cmul(al, conjd(b));
-        s = make_double2(t.x / normab, t.y / normab);
+        aa = hypot(a.x, a.y);
+        nn = hypot(aa, rem);
       }
+      const int q = lane & 3;
+      const double quot = (q == 0 ? aa : q == 1 ? rem : q == 2 ? a.x : a.y) / (q < 2 ? nn : aa);
+      c = __shfl_sync(0xffffffffu, quot, 0);
+      const double f = __shfl_sync(0xffffffffu, quot, 1);
+      s = make_double2(f * __shfl_sync(0xffffffffu, quot, 2), f * __shfl_sync(0xffffffffu, quot, 3));
+    }
+    const double2 g1 = S.g[j], g2 = S.g[j + 1];
+    const double2 sg2 = cmul(s, g2), csg1 = cmul(conjd(s), g1);
+    const double2 n1 = make_double2(fma(c, g1.x, sg2.x), fma(c, g1.y, sg2.y));
+    const double2 n2 = make_double2(fma(c, g2.x, -csg1.x), fma(c, g2.y, -csg1.y));
+    __syncwarp();
+    if (lane == 0) {
       cs[j] = make_double2(c, 0.0);
       sn[j] = s;
-      const double2 sb = cmul(s, b);
-      colv[j] = make_double2(c * a.x + sb.x, c * a.y + sb.y);
-      colv[j + 1] = make_double2(0.0, 0.0);
-      const double2 g1 = S.g[j], g2 = S.g[j + 1];
-      const double2 sg2 = cmul(s, g2);
-      const double2 csg1 = cmul(conjd(s), g1);
-      S.g[j] = make_double2(c * g1.x + sg2.x, c * g1.y + sg2.y);
-      S.g[j + 1] = make_double2(-csg1.x + c * g2.x, -csg1.y + c * g2.y);
-      if (hypot(S.g[j + 1].x, S.g[j + 1].y) <= S.tol) stop = true;
+      sm.h[j] = make_double2(fma(c, a.x, s.x * rem), fma(c, a.y, s.y * rem));
+      sm.h[j + 1] = make_double2(0.0, 0.0);
+      S.g[j] = n1;
+      S.g[j + 1] = n2;
     }
+    const double tol = S.tol;
+    if (tol > 1e-140 ? fma(n2.x, n2.x, n2.y * n2.y) <= tol * tol : hypot(n2.x, n2.y) <= tol) stop = true;
   }
   __syncwarp();
-  for (int r = lane; r < ld; r += 32) col[r] = colv[r];
+  for (int r = lane; r < ld; r += 32) col[r] = sm.h[r];
   __syncwarp();
   return stop;
 }
 
-__global__ void __launch_bounds__(32) k_step_finish(DevInst* st) {
+__global__ void __launch_bounds__(32) k_step_finish(DevInst* st, int* again) {
   __shared__ FinishSmem sm;
   DevInst& S = st[blockIdx.x];
+  if (blockIdx.x == 0 && threadIdx.x == 0) *again = 0;  // for the next step
   if (S.done) return;
   const int j = S.j;
   const bool stop = step_finish(S, j, sm);
@@ -1272,7 +1457,10 @@ __global__ void __launch_bounds__(32) k_step_finish(DevInst* st) {
 // list and meet at a grid barrier between phases.  As separate launches (one graph of 11 nodes
 // per step) the phases of such sets last about as long as a launch takes to start and drain.
 // Per entry, chunk and job the arithmetic is that of the step kernels.  Measured per Arnoldi
-// step, graph -> one launch: N = 8 FP64 68 -> 35 us, N = 120 FP32 63 -> 37 us (m = 30).
+// step, graph -> one launch: N = 8 FP64 68 -> 24 us, N = 16 GMRES(50) about 120 -> 30 us, N = 120
+// FP32 63 -> 27 us (m = 30).  A barrier takes about 1 us and a phase of a small set 3-7 us, most
+// of it the latency of loads that miss L1 (the barrier's fence empties it) and of FP64
+// instructions (64 cycles each per quarter of an SM).
 
 // Grid barrier: arrivals are counted up over the whole launch.  A block that waits in vain
 // raises err, which ends every wait of the launch; the host reads it after the cycle.
@@ -1282,17 +1470,21 @@ struct GridBar {
 };
 constexpr int kGridWaitLimit = 1 << 24;  // polls, several seconds
 
-__device__ __forceinline__ bool grid_sync(GridBar* bar, unsigned& target) {
-  if (gridDim.x == 1) {
-    __syncthreads();
-    return true;
-  }
-  __shared__ int ok;
+// Arrival of this block; its writes so far are visible to blocks that wait for it.
+__device__ __forceinline__ void grid_arrive(GridBar* bar, unsigned& target) {
   __syncthreads();
   target += gridDim.x;
-  if (threadIdx.x == 0) {
-    __threadfence();  // the block's writes before its arrival
+  if (gridDim.x > 1 && threadIdx.x == 0) {
+    __threadfence();
     atomicAdd(&bar->count, 1u);
+  }
+}
+
+// Waits for the arrival of every block; false when the launch has given up.
+__device__ __forceinline__ bool grid_wait(GridBar* bar, unsigned target) {
+  if (gridDim.x == 1) return true;
+  __shared__ int ok;
+  if (threadIdx.x == 0) {
     ok = 1;
     for (int it = 0;; ++it) {
       unsigned seen;
@@ -1310,6 +1502,27 @@ __device__ __forceinline__ bool grid_sync(GridBar* bar, unsigned& target) {
   return ok != 0;
 }
 
+__device__ __forceinline__ bool grid_sync(GridBar* bar, unsigned& target) {
+  grid_arrive(bar, target);
+  return grid_wait(bar, target);
+}
+
+// Sum of a job's nc <= 32 chunk partials of projection i in the order of warp_chunk_sum (lane c
+// holds partial c, halves added pairwise), by one thread.
+__device__ __noinline__ double few_chunk_sum(const double2* partv, int begin, int nc, int stride, int value) {
+  const double* p = reinterpret_cast<const double*>(partv) + (long long)begin * stride * 2 + value;
+  double v[32];
+#pragma unroll
+  for (int c = 0; c < 32; ++c) v[c] = c < nc ? p[(long long)c * stride * 2] : 0.0;
+#pragma unroll
+  for (int off = 16; off > 0; off >>= 1)
+#pragma unroll
+    for (int c = 0; c < off; ++c)
+      if (c + off < nc) v[c] += v[c + off];  // uniform; adding the zero of a missing chunk changes nothing
+  return v[0];
+}
+constexpr int kFewChunks = 32;
+
 template <bool F32>
 __global__ void __launch_bounds__(kRT, 2)
     k_cycle(DevInst* st, int n, const int* chunk_inst, int nchunk, const int* item_inst, const int* item_local,
@@ -1321,40 +1534,98 @@ __global__ void __launch_bounds__(kRT, 2)
     Axpy32Smem axpy32;
     FinishSmem finish;
   } sm;
+  __shared__ double2 tr;
+  __shared__ DevInst fixed;  // a single job's control block, for the fields that stay as they are
   using T2 = typename Vec2<typename std::conditional<F32, float, double>::type>::type;
   const int nblk = gridDim.x, blk = blockIdx.x;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  unsigned target = 0;
+  unsigned target = 0;  // arrivals at the barrier that comes next
   double* part1 = part + nchunk;
-  for (int j = 0; j < steps; ++j) {
-    // stop[j & 1] holds a job's state for step j; the finish of step j writes the other one
+  // A single job: its norms and its trace are reduced by every block for itself, which costs
+  // less than a designated block and a barrier.
+  const bool one = n == 1;
+  // Its last block takes no share of the applies and, the grid having a block more than there
+  // are chunks, of the chunk phases of smaller jobs: it arrives at the apply's barrier before it
+  // starts the finish, so that only the end of the projections waits for it.
+  const int workers = one && nblk > 1 ? nblk - 1 : nblk;
+  for (int i = threadIdx.x; one && i < (int)(sizeof(DevInst) / 4); i += kRT)
+    reinterpret_cast<int*>(&fixed)[i] = reinterpret_cast<const int*>(st)[i];
+  __syncthreads();
+  auto job = [&](int i) -> const DevInst& { return one ? fixed : st[i]; };
+  const bool own_trace = one && border && st[0].border && st[0].ndiag <= 4 * kRT;
+  const int nc0 = nchunks[0];
+  bool many = false;  // some job's projections are reduced in a phase of their own
+  for (int i = threadIdx.x; i < n; i += kRT) many = many || nchunks[i] > kFewChunks;
+  many = __syncthreads_or(many);
+  for (int j = 0;; ++j) {
+    // The finish of step j - 1 runs beside the first phases of step j, which for a job that
+    // has just stopped are in vain.  stop[j & 1]: jobs that take no step j.
     const int ph = j & 1;
+    auto finish = [&]() {  // the last block's first warp takes the first job, and so on
+      __syncthreads();     // sm is free
+      if (warp == 0)
+        for (int i = nblk - 1 - blk; i < n; i += nblk) {
+          DevInst& S = st[i];
+          const bool stop = S.stop[ph ^ 1] ? true : step_finish(S, j - 1, sm.finish);
+          if (lane == 0) S.stop[ph] = stop;
+        }
+      __syncthreads();
+    };
+    auto was_live = [&](const DevInst& S) { return !S.stop[j > 0 ? ph ^ 1 : ph]; };
     auto live = [&](const DevInst& S) { return !S.stop[ph]; };
-    bool any = false;
-    for (int i = threadIdx.x; i < n; i += kRT) any = any || live(st[i]);
-    if (!__syncthreads_or(any)) return;  // uniform over the grid
-    if (border) {
+    const bool traces = border && !own_trace;
+    const bool beside = workers < nblk && !traces;  // the last block finishes beside apply and dots
+    if (j > 0 && !beside) finish();
+    if (j == steps) {
+      if (beside) finish();
+      return;
+    }
+    if (traces) {
       for (int i = blk; i < n; i += nblk)
-        if (live(st[i]) && st[i].border) step_trace<T2>(st[i], j);
+        if (was_live(st[i]) && st[i].border) {
+          const double2 a = step_trace<T2>(st[i], j);
+          if (threadIdx.x == 0) st[i].alpha = a;
+          __syncthreads();
+        }
       if (!grid_sync(bar, target)) return;
     }
-    for (int t = blk; t < nitem; t += nblk) {
-      DevInst& S = st[item_inst[t]];
-      if (!live(S)) continue;
-      const T2* x = (const T2*)S.V + (long long)j * S.ldv;
-      const double2* alpha = S.border ? &S.alpha : nullptr;
-      if constexpr (F32)
-        strip_apply32<false>(S, item_local[t], x, (float2*)S.w, alpha);
-      else
-        strip_apply<false>(S, item_local[t], x, (double2*)S.w, S.scale, alpha);
+    if (own_trace && blk < workers) {
+      const double2 a = step_trace<T2>(fixed, j);
+      if (threadIdx.x == 0) tr = a;
+      __syncthreads();
     }
-    if (!grid_sync(bar, target)) return;
+    // items first, first + step, ... of S by this warp
+    auto apply = [&](const DevInst& S, int first, int step, int count) {
+      const T2* x = (const T2*)S.V + (long long)j * S.ldv;
+      const double2* alpha = !S.border ? nullptr : own_trace ? &tr : one ? &st[0].alpha : &S.alpha;
+      if constexpr (F32)
+        strip_apply32<false>(S, first, step, count, x, (float2*)S.w, alpha);
+      else
+        for (int k = 0; k < count && first + k * step < S.p64.nitems; ++k)
+          strip_apply<false>(S, first + k * step, x, (double2*)S.w, S.scale, alpha);
+    };
+    if (one) {  // one item per warp, spread over the blocks first
+      if (blk < workers) apply(fixed, blk + workers * warp, workers * (kRT / 32), 1 << 30);
+    } else {
+      for (int t = blk; t < nitem; t += nblk) {
+        DevInst& S = st[item_inst[t]];
+        if (was_live(S))
+          apply(S, item_local[t] * kBlockItems * (F32 ? kRounds32 : 1) + warp, kBlockItems, F32 ? kRounds32 : 1);
+      }
+    }
+    grid_arrive(bar, target);
+    if (beside && blk == workers && j > 0) finish();
+    if (!grid_wait(bar, target)) return;
+    bool any = one;
+    for (int i = threadIdx.x; !one && i < n; i += kRT) any = any || live(st[i]);
+    if (!__syncthreads_or(any)) return;  // uniform over the grid
     auto dots = [&](bool second) {
       for (int c = blk; c < nchunk; c += nblk) {
-        const DevInst& S = st[chunk_inst[c]];
-        if (!live(S) || (second && !S.reorth)) continue;
+        const int inst = one ? 0 : chunk_inst[c];
+        if (!one && (!live(st[inst]) || (second && !st[inst].reorth))) continue;
+        const DevInst& S = job(inst);
         if constexpr (F32)
-          step_dot32<kBatchChunkSmall>(S, j + 1, c, partv, second ? nullptr : part, sm.dot32);
+          step_dot32<kBatchChunkSmall, 8>(S, j + 1, c, partv, second ? nullptr : part, sm.dot32);
         else
           step_dot64(S, j + 1, c, partv, second ? nullptr : part, sm.dot64);
       }
@@ -1362,68 +1633,109 @@ __global__ void __launch_bounds__(kRT, 2)
     auto finals = [&](bool second) {  // one warp per (job, column), spread over the blocks
       for (int t = blk + nblk * warp; t < n * (j + 1); t += nblk * (kRT / 32)) {
         const int i = t / (j + 1), k = t - i * (j + 1);
-        const DevInst& S = st[i];
-        if (!live(S) || (second && !S.reorth)) continue;
-        const double2 v = warp_chunk_sum(partv, S.chunk_begin, nchunks[i], S.pstride, k);
+        if (!one && (!live(st[i]) || (second && !st[i].reorth) || nchunks[i] <= kFewChunks)) continue;
+        const DevInst& S = job(i);
+        const double2 v = warp_chunk_sum(partv, S.chunk_begin, one ? nc0 : nchunks[i], S.pstride, k);
         if (lane == 0) (second ? S.hB : S.hA)[k] = v;
       }
     };
+    // projections of the chunk's job into sm: of a job of few chunks summed here (its first
+    // chunk's block keeps them for the finish), otherwise read
+    auto projections = [&](const DevInst& S, int inst, int c, bool second, auto* h) {
+      double2* keep = second ? S.hB : S.hA;
+      auto put = [&](int k, double2 v) {
+        if constexpr (F32)
+          h[k] = make_float2((float)v.x, (float)v.y);
+        else
+          h[k] = v;
+      };
+      const int nc = one ? nc0 : nchunks[inst];
+      if (nc <= kFewChunks) {
+        for (int k = threadIdx.x; k < 2 * (j + 1); k += kRT) {
+          const double v = few_chunk_sum(partv, S.chunk_begin, nc, S.pstride, k);
+          if (c == S.chunk_begin) reinterpret_cast<double*>(keep)[k] = v;
+          if constexpr (F32)
+            reinterpret_cast<float*>(h)[k] = (float)v;
+          else
+            reinterpret_cast<double*>(h)[k] = v;
+        }
+      } else {
+        for (int k = threadIdx.x; k <= j; k += kRT) put(k, keep[k]);
+      }
+      __syncthreads();
+    };
     auto update = [&](bool second) {
       for (int c = blk; c < nchunk; c += nblk) {
-        const DevInst& S = st[chunk_inst[c]];
-        if (!live(S) || (second && !S.reorth)) continue;
-        if constexpr (F32)
-          step_axpy32(S, j + 1, c, second ? S.hB : S.hA, second ? part : part1, sm.axpy32);
-        else
-          step_axpy64(S, j + 1, c, second ? S.hB : S.hA, second ? part : part1, sm.axpy64);
+        const int inst = one ? 0 : chunk_inst[c];
+        if (!one && (!live(st[inst]) || (second && !st[inst].reorth))) continue;
+        const DevInst& S = job(inst);
+        if constexpr (F32) {
+          projections(S, inst, c, second, sm.axpy32.h);
+          step_axpy32(S, j + 1, c, second ? part : part1, sm.axpy32);
+        } else {
+          projections(S, inst, c, second, sm.axpy64.h);
+          step_axpy64(S, j + 1, c, second ? part : part1, sm.axpy64);
+        }
       }
     };
     dots(false);
     if (!grid_sync(bar, target)) return;
-    for (int i = nblk - 1 - blk; i < n; i += nblk) {
-      if (!live(st[i])) continue;
-      const double v = job_norm2(st[i], nchunks[i], part);
-      if (threadIdx.x == 0) st[i].image2 = v;
+    if (one && !live(st[0])) return;  // uniform over the grid
+    if (many) {
+      finals(false);
+      if (!grid_sync(bar, target)) return;
     }
-    finals(false);
-    if (!grid_sync(bar, target)) return;
     update(false);
     if (!grid_sync(bar, target)) return;
-    for (int i = blk; i < n; i += nblk)
-      if (live(st[i])) step_norm1(st[i], j + 1, nchunks[i], part1);
-    if (!grid_sync(bar, target)) return;
-    any = false;
-    for (int i = threadIdx.x; i < n; i += kRT) any = any || (live(st[i]) && st[i].reorth);
-    if (__syncthreads_or(any)) {  // uniform over the grid
+    bool again;
+    double rem2 = 0;
+    if (one) {
+      const StepNorms r = step_norm1(st[0], j + 1, nc0, part, part1, blk == 0);
+      again = r.reorth;  // uniform over the grid
+      rem2 = r.rem2;
+    } else {
+      for (int i = blk; i < n; i += nblk)
+        if (live(st[i])) step_norm1(st[i], j + 1, nchunks[i], part, part1, true);
+      if (!grid_sync(bar, target)) return;
+      any = false;
+      for (int i = threadIdx.x; i < n; i += kRT) any = any || (live(st[i]) && st[i].reorth);
+      again = __syncthreads_or(any);  // uniform over the grid
+    }
+    if (again) {
       dots(true);
       if (!grid_sync(bar, target)) return;
-      finals(true);
-      if (!grid_sync(bar, target)) return;
+      if (many) {
+        finals(true);
+        if (!grid_sync(bar, target)) return;
+      }
       update(true);
       if (!grid_sync(bar, target)) return;
-      for (int i = blk; i < n; i += nblk) {
-        if (!live(st[i]) || !st[i].reorth) continue;
-        const double v = job_norm2(st[i], nchunks[i], part);
-        if (threadIdx.x == 0) st[i].rem2 = v;
+      if (one) {
+        rem2 = job_norms(fixed, nc0, part, nullptr).x;
+        if (blk == 0 && threadIdx.x == 0) st[0].rem2 = rem2;
+      } else {
+        for (int i = blk; i < n; i += nblk) {
+          if (!live(st[i]) || !st[i].reorth) continue;
+          const double2 v = job_norms(st[i], nchunks[i], part, nullptr);
+          if (threadIdx.x == 0) {
+            st[i].rem2 = v.x;
+            st[i].inv = inverse_norm(v.x);
+          }
+        }
+        if (!grid_sync(bar, target)) return;
       }
-      if (!grid_sync(bar, target)) return;
     }
-    // the last block's first warp finishes the first job beside the normalisation, and so on
+    double f = one ? block_inverse_norm(rem2) : 0.0;
     for (int c = blk; c < nchunk; c += nblk) {
-      const DevInst& S = st[chunk_inst[c]];
-      if (!live(S)) continue;
+      const int inst = one ? 0 : chunk_inst[c];
+      if (!one && !live(st[inst])) continue;
+      const DevInst& S = job(inst);
+      if (!one) f = st[inst].inv;
       if constexpr (F32)
-        step_normalize32(S, j, c);
+        step_normalize32(S, j, c, (float)f);
       else
-        step_normalize64(S, j, c);
+        step_normalize64(S, j, c, f);
     }
-    __syncthreads();
-    if (warp == 0)
-      for (int i = nblk - 1 - blk; i < n; i += nblk) {
-        DevInst& S = st[i];
-        const bool stop = live(S) ? step_finish(S, j, sm.finish) : true;
-        if (lane == 0) S.stop[ph ^ 1] = stop;
-      }
     if (!grid_sync(bar, target)) return;
   }
 }
@@ -2080,7 +2392,7 @@ Engine::Engine(int device, int krylovdim, bool f32, bool use_graphs)
 Engine::~Engine() {
   if (graph_) cudaGraphExecDestroy(graph_);
   if (s_) cudaStreamSynchronize(s_);
-  for (void* p : {st_, tile_inst_, tile_local_, strip_inst_, strip_local_, bar_, chunk_inst_, nchunks_, part1_, partv_, hab_, rec_, out_, coefs_})
+  for (void* p : {st_, tile_inst_, tile_local_, strip_inst_, strip_local_, bar_, again_, chunk_inst_, nchunks_, part1_, partv_, hab_, rec_, out_, coefs_})
     if (p) cudaFree(p);
   for (void* p : {st_h_, st_dl_, rec_h_, out_h_, coefs_h_})
     if (p) cudaFreeHost(p);
@@ -2150,7 +2462,8 @@ void Engine::rebuild() {
       strips = p64[i].nitems;
     }
     const int ntiles = plan->dev.ntiles;
-    const int nstrip = strips ? (strips + kBlockItems - 1) / kBlockItems : ntiles;
+    const int per = f32_ ? kBlockItems * kRounds32 : kBlockItems;
+    const int nstrip = strips ? (strips + per - 1) / per : ntiles;
     canonical = canonical && strips > 0;
     for (int t = 0; t < ntiles; ++t) {
       ti.push_back(i);
@@ -2220,6 +2533,8 @@ void Engine::rebuild() {
   reserve(&strip_inst_, &strip_inst_cap_, sizeof(int) * std::max<size_t>(si.size(), 1), false);
   reserve(&strip_local_, &strip_local_cap_, sizeof(int) * std::max<size_t>(sl.size(), 1), false);
   reserve(&bar_, &bar_cap_, sizeof(GridBar), false);
+  reserve(&again_, &again_cap_, sizeof(int), false);
+  chk(cudaMemsetAsync(again_, 0, sizeof(int), s_));
   reserve(&chunk_inst_, &chunk_inst_cap_, sizeof(int) * std::max<size_t>(ci.size(), 1), false);
   reserve(&nchunks_, &nchunks_cap_, sizeof(int) * nn, false);
   reserve(&part1_, &part1_cap_, sizeof(double) * 2 * std::max(total_chunks_, 1), false);
@@ -2376,27 +2691,29 @@ void Engine::arnoldi_step() {
   const double2* cpartv = partv;
   const int n = (int)jobs_.size();
   const dim3 gfin(n, (m_ + 1 + kRT / 32 - 1) / (kRT / 32));
-  const dim3 gfirst(n, gfin.y + 1);  // projections into hA plus one row of image-norm blocks
   const int C = total_chunks_;
   double* npart1 = part + C;  // |w1|^2 partials of the first update (second half of part)
   // Classical Gram-Schmidt with selective reorthogonalisation: the first pass also takes the
   // image norm |w0|^2 and the first update the |w1|^2 partials; the blocks of the second pass
   // return at once for jobs that need none (step_norm1).
+  const int* again = (const int*)again_;
+  auto grid = [&](int second) { return second ? std::min(C, kSecondPassBlocks) : C; };
   auto dots = [&](int second) {
     double* ipart = second ? nullptr : part;
     if (!f32_)
-      launch(k_step_dot64, C, kRT, 0, cst, ci, partv, ipart, second);
+      launch(k_step_dot64, grid(second), kRT, 0, cst, ci, C, partv, ipart, second ? again : nullptr);
     else if (chunk_ == kBatchChunk)
-      launch(k_step_mdot_f32<kBatchChunk>, C, kRT, 0, cst, ci, partv, ipart, second);
+      launch(k_step_mdot_f32<kBatchChunk>, grid(second), kRT, 0, cst, ci, C, partv, ipart, second ? again : nullptr);
     else
-      launch(k_step_mdot_f32<kBatchChunkSmall>, C, kRT, 0, cst, ci, partv, ipart, second);
+      launch(k_step_mdot_f32<kBatchChunkSmall>, grid(second), kRT, 0, cst, ci, C, partv, ipart,
+             second ? again : nullptr);
   };
   auto update = [&](int second) {
     double* out = second ? part : npart1;
     if (f32_)
-      launch(k_step_maxpy_f32, C, kRT, 0, cst, ci, out, second);
+      launch(k_step_maxpy_f32, grid(second), kRT, 0, cst, ci, C, out, second ? again : nullptr);
     else
-      launch(k_step_axpy64, C, kRT, 0, cst, ci, out, second);
+      launch(k_step_axpy64, grid(second), kRT, 0, cst, ci, C, out, second ? again : nullptr);
   };
   if (f32_) {
     if (any_border_) launch(k_step_trace<float2>, n, kRT, 0, st);
@@ -2407,26 +2724,26 @@ void Engine::arnoldi_step() {
            (const int*)strip_inst_, (const int*)strip_local_);
   }
   dots(0);
-  launch(k_step_first_final, gfirst, kRT, 0, st, nc, cpartv, (const double*)part);
+  launch(k_step_first_final, gfin, kRT, 0, st, nc, cpartv);
   update(0);
-  launch(k_step_norm, n, kRT, 0, st, nc, (const double*)npart1, 0);
+  launch(k_step_norm, n, kRT, 0, st, nc, (const double*)part, (const double*)npart1, 0, (int*)again_);
   dots(1);
   launch(k_step_mdot_final, gfin, kRT, 0, cst, nc, cpartv);
   update(1);
-  launch(k_step_norm, n, kRT, 0, st, nc, (const double*)part, 1);
+  launch(k_step_norm, n, kRT, 0, st, nc, (const double*)part, (const double*)npart1, 1, (int*)again_);
   if (f32_)
     launch(k_step_normalize_f32, C, kRT, 0, cst, ci);
   else
     launch(k_step_normalize64, C, kRT, 0, cst, ci);
-  launch(k_step_finish, n, 32, 0, st);
+  launch(k_step_finish, n, 32, 0, st, (int*)again_);
   if (!build_) chk(cudaGetLastError());
 }
 
-// The cycle of a small job set in one cooperative launch: as many blocks as its longest work
-// list has entries, at most what is resident at once.
+// The cycle of a small job set in one cooperative launch: a block more than its longest work
+// list has entries (the finish of a single job), at most what is resident at once.
 void Engine::launch_cycle() {
   const int n = (int)jobs_.size();
-  const int grid = std::max(1, std::min(std::max(total_chunks_, total_strips_), cycle_max_ * sm_count_));
+  const int grid = std::max(1, std::min(std::max(total_chunks_, total_strips_) + 1, cycle_max_ * sm_count_));
   DevInst* st = (DevInst*)st_;
   const int *ci = (const int*)chunk_inst_, *si = (const int*)strip_inst_, *sl = (const int*)strip_local_;
   const int* nc = (const int*)nchunks_;
@@ -2514,9 +2831,9 @@ bool Engine::tick() {
     if (flags & S1_COMBINE) {
       chk(cudaMemcpyAsync(coefs_, coefs_h_, sizeof(double2) * (m_ + 2) * n, cudaMemcpyHostToDevice, s_));
       if (f32_)
-        k_s1_combine_f32<<<C, kRT, 0, s_>>>(st, ci);
+        k_s1_combine_f32<<<C, kRT, 0, s_>>>(st, ci, (double*)part1_);
       else
-        k_s1_combine<double2><<<C, kRT, 0, s_>>>(st, ci);
+        k_s1_combine<<<C, kRT, 0, s_>>>(st, ci, (double*)part1_);
     }
     if (flags & S1_PROBE) k_s1_probe<<<C, kRT, 0, s_>>>(st, ci);
     if (flags & (S1_AUX | S1_TRACE)) k_s1_trace<<<n, kRT, 0, s_>>>(st);
@@ -2525,14 +2842,12 @@ bool Engine::tick() {
       k_bapply<double, true><<<f32_ ? total_tiles_ : total_strips_, kApplyThreads, 3 * kWinElems * sizeof(double2),
                                s_>>>(st, f32_ ? ti : (const int*)strip_inst_, f32_ ? tl : (const int*)strip_local_);
     if (flags & S1_RESID) k_s1_resid<<<C, kRT, 0, s_>>>(st, ci);
-    if (flags & S1_NORM) {
-      k_s1_norm_partial<<<C, kRT, 0, s_>>>(st, ci, (double*)part1_);
-      k_s1_norm_final<<<n, kRT, 0, s_>>>(st, (const int*)nchunks_, (const double*)part1_);
-    }
-    if (flags & S1_OBS) {
-      k_s1_obs_partial<<<C, kRT, 0, s_>>>(st, ci, (double2*)partv_);
-      k_s1_obs_final<<<n, kRT, 0, s_>>>(st, (const int*)nchunks_, (const double2*)partv_);
-    }
+    bool norms = false;  // beyond those of combinations
+    for (int i = 0; i < n; ++i) norms = norms || (sth[i].nrm0 && sth[i].nrm0 != sth[i].cout) || sth[i].nrm1;
+    if (norms) k_s1_norm_partial<<<C, kRT, 0, s_>>>(st, ci, (double*)part1_);
+    if (flags & S1_OBS) k_s1_obs_partial<<<C, kRT, 0, s_>>>(st, ci, (double2*)partv_);
+    if (flags & (S1_NORM | S1_OBS))
+      k_s1_final<<<n, kRT, 0, s_>>>(st, (const int*)nchunks_, (const double*)part1_, (const double2*)partv_);
     chk(cudaGetLastError());
     chk(cudaMemcpyAsync(out_h_, out_, sizeof(double) * kOutSlots * n, cudaMemcpyDeviceToHost, s_));
     chk(cudaStreamSynchronize(s_));

@@ -40,9 +40,12 @@ constexpr int kBatchMaxKrylov = 120;
 inline long long basis_stride(long long dim) { return (dim + 63) / 64 * 64; }
 
 // Elements per reduction chunk of an FP64 job, by its own size (so that its sums do not depend
-// on the other jobs of the set): about two chunks per SM, 128 to 1024 elements.
+// on the other jobs of the set): 32 to 128 elements in at most 32 chunks for the smallest jobs
+// (an SM's FP64 pipe takes 64 cycles for a warp's FMA, so their work is spread over SMs), then
+// about two chunks per SM of up to 1024 elements.
 inline int chunk64(long long dim) {
-  int c = 128;
+  int c = 32;
+  while (c < 128 && dim > 32LL * c) c *= 2;
   while (c < kBatchChunkSmall && dim > 304LL * c) c *= 2;
   return c;
 }
@@ -109,6 +112,7 @@ struct DevInst {
   double scale;  // multiplies L V_j
   double tol;    // GMRES: stop when |g[j+1]| <= tol
   double rem2;
+  double inv;    // 1 / |w| of the step's new vector
   double image2;
   double2 alpha;
   const double2* v0;  // V_0 = v0 / v0norm (FP64 source)
@@ -324,6 +328,7 @@ class Engine {
   void* strip_inst_ = nullptr; size_t strip_inst_cap_ = 0;
   void* strip_local_ = nullptr; size_t strip_local_cap_ = 0;
   void* bar_ = nullptr; size_t bar_cap_ = 0;
+  void* again_ = nullptr; size_t again_cap_ = 0;  // whether some job reorthogonalises this step
   void* chunk_inst_ = nullptr; size_t chunk_inst_cap_ = 0;
   void* nchunks_ = nullptr; size_t nchunks_cap_ = 0;
   void* part1_ = nullptr; size_t part1_cap_ = 0;
