@@ -75,7 +75,7 @@ int pi_arnoldi(pi_plan* plan, const double* v0_dev, int m, double* V_dev, long l
   for (int j = 0; j < m && rc == PI_OK && z.err == cudaSuccess; ++j) {
     double2* w = col(j + 1);
     const double* vj = reinterpret_cast<const double*>(col(j));
-    z.chk(P.items ? launch_apply_strip64(plan->dev, P, vj, reinterpret_cast<double*>(w), 1, n, none, s)
+    z.chk(P.items ? launch_apply_strip<double>(plan->dev, P, vj, reinterpret_cast<double*>(w), 1, n, none, s)
                   : launch_apply_f64(plan->dev, vj, reinterpret_cast<double*>(w), 1, n, none, s));
     ++out.operator_applications;
     z.chk(norm2_f64(w, n, rs, 0, s));  // image norm

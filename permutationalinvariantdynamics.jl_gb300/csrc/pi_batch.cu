@@ -19,7 +19,7 @@
 #include <unordered_set>
 #include <utility>
 
-#include "pi_apply64.cuh"
+#include "pi_strip.cuh"
 #include "pi_apply_impl.cuh"
 #include "pi_dense.hpp"
 
@@ -211,7 +211,7 @@ __device__ __forceinline__ void strip_item(const DevInst& S, int item, const dou
                                            double scale, const double2* alpha) {
   if (item >= S.p64.nitems) return;
   const StripItem it = S.p64.items[item];
-  StripEntry<V, NC> E;
+  StripEntry<double, V, NC> E;
   if (!E.load(it, S.p64, threadIdx.x & 31)) return;
   double2 out = E.apply(x);
   if (plain) {  // block-uniform, its own exit: the scaling below must not be if-converted into it

@@ -746,7 +746,7 @@ int pi_apply_f64(pi_plan* plan, double* y_dev, const double* x_dev, int ncols, l
   BorderArgs border{1.0, nullptr, 0};
   cudaStream_t s = (cudaStream_t)stream;  // NULL is the CUDA default stream
   const Planes64 P = planes64(plan, PI_COORDS_REFERENCE);
-  cudaError_t e = P.items ? launch_apply_strip64(plan->dev, P, x_dev, y_dev, ncols, ld, border, s)
+  cudaError_t e = P.items ? launch_apply_strip<double>(plan->dev, P, x_dev, y_dev, ncols, ld, border, s)
                           : launch_apply_f64(plan->dev, x_dev, y_dev, ncols, ld, border, s);
   if (e != cudaSuccess) return cuda_fail(e, "apply launch");
   return PI_OK;
@@ -760,7 +760,9 @@ int pi_apply_f32(pi_plan* plan, float* y_dev, const float* x_dev, int ncols, lon
     return fail(PI_ERR_INVALID_ARGUMENT, "coords must be PI_COORDS_REFERENCE or PI_COORDS_POPULATION");
   BorderArgs border{1.0, nullptr, coords};
   cudaStream_t s = (cudaStream_t)stream;  // NULL is the CUDA default stream
-  cudaError_t e = launch_apply_f32(plan->dev, x_dev, y_dev, ncols, ld, border, s);
+  const Planes32 P = planes32(plan, coords);
+  cudaError_t e = P.items ? launch_apply_strip<float>(plan->dev, P, x_dev, y_dev, ncols, ld, border, s)
+                          : launch_apply_f32(plan->dev, x_dev, y_dev, ncols, ld, border, s);
   if (e != cudaSuccess) return cuda_fail(e, "apply launch");
   return PI_OK;
 }
@@ -805,7 +807,11 @@ static int apply_host(pi_plan* plan, void* y_host, const void* x_host, int ncols
   const int nchunks = sizeof(T) == sizeof(double) ? 16 : 8;
   const int chunk = std::max(1, (ncols + nchunks - 1) / nchunks);
   BorderArgs border{1.0, nullptr, coords};
-  const Planes64 P = sizeof(T) == sizeof(double) ? planes64(plan, coords) : Planes64{};
+  StripPlanes<T> P;
+  if constexpr (sizeof(T) == sizeof(double))
+    P = planes64(plan, coords);
+  else
+    P = planes32(plan, coords);
   int k = 0;
   for (int c0 = 0; c0 < ncols && e == cudaSuccess; c0 += chunk, ++k) {
     const int nc = std::min(chunk, ncols - c0);
@@ -815,9 +821,10 @@ static int apply_host(pi_plan* plan, void* y_host, const void* x_host, int ncols
     e = cudaMemcpyAsync(dx, (const char*)x_host + (size_t)c0 * col_bytes, (size_t)nc * col_bytes,
                         cudaMemcpyHostToDevice, s);
     if (e == cudaSuccess) {
-      if (sizeof(T) == sizeof(double))
-        e = P.items ? launch_apply_strip64(plan->dev, P, (const double*)dx, (double*)dy, nc, plan->host.dim, border, s)
-                    : launch_apply_f64(plan->dev, (const double*)dx, (double*)dy, nc, plan->host.dim, border, s);
+      if (P.items)
+        e = launch_apply_strip<T>(plan->dev, P, (const T*)dx, (T*)dy, nc, plan->host.dim, border, s);
+      else if (sizeof(T) == sizeof(double))
+        e = launch_apply_f64(plan->dev, (const double*)dx, (double*)dy, nc, plan->host.dim, border, s);
       else
         e = launch_apply_f32(plan->dev, (const float*)dx, (float*)dy, nc, plan->host.dim, border, s);
     }

@@ -96,7 +96,7 @@ struct SplitPlanes {
 constexpr int kSepF4 = 6;      // 24 floats: 6 + 3 x 6 positions
 constexpr int kSepF4Plus = 9;  // 36 floats: 6 + 3 x 9 positions, padded
 
-// ---- FP64 strip apply (pi_apply64.cuh) ----
+// ---- strip apply (pi_strip.cuh) ----
 
 // 32 consecutive entries of one sector block (one warp's work).
 struct alignas(16) StripItem {
@@ -116,20 +116,34 @@ struct GainPos {
 };
 constexpr int kMaxGains = 8;
 
-// Merged FP64 coefficients of a canonical plan: the planes [2 + nr][dim] (centre re, centre im,
+// Merged coefficients of a canonical plan: the planes [2 + nr][dim] (centre re, centre im,
 // then one per gain position that some sector uses; the own-sector centre gain joins the
 // centre) and the imaginary coefficients of the row and column shifts per line.  `variant`
 // selects the kernel: the number of gain slots it has and whether it has the line shifts
 // (unused slots carry src = -1).
-struct Planes64 {
+template <typename T>
+struct StripPair;
+template <>
+struct StripPair<double> {
+  using type = double2;
+};
+template <>
+struct StripPair<float> {
+  using type = float2;
+};
+template <typename T>
+struct StripPlanes {
+  using T2 = typename StripPair<T>::type;
   const StripItem* items = nullptr;  // nullptr: the plan has no planes
-  const double* plane = nullptr;
-  const double2* lrow = nullptr;  // per row: row shifts -1, +1
-  const double2* rcol = nullptr;  // per column: column shifts -1, +1
+  const T* plane = nullptr;
+  const T2* lrow = nullptr;  // per row: row shifts -1, +1
+  const T2* rcol = nullptr;  // per column: column shifts -1, +1
   long long dim = 0;
   int nitems = 0;
   int variant = 0;
   GainPos gain[kMaxGains] = {};
 };
+using Planes64 = StripPlanes<double>;
+using Planes32 = StripPlanes<float>;
 
 }  // namespace picuda

@@ -98,7 +98,7 @@ struct ExpvWork {
       chk(launch_apply_f32(p->dev, (const float*)col(j), (float*)w, 1, n, b, s));
       chk(norm2_f32((const float2*)w, n, p->rs, 1, s));
     } else {
-      chk(planes.items ? launch_apply_strip64(p->dev, planes, (const double*)col(j), (double*)w, 1, n, b, s)
+      chk(planes.items ? launch_apply_strip<double>(p->dev, planes, (const double*)col(j), (double*)w, 1, n, b, s)
                        : launch_apply_f64(p->dev, (const double*)col(j), (double*)w, 1, n, b, s));
       chk(norm2_f64((const double2*)w, n, p->rs, 1, s));
     }

@@ -71,10 +71,12 @@ struct pi_plan {
   };
   std::vector<EmChoice> em_choices;
   std::mutex em_tune_mu;
-  // Merged FP64 coefficient planes per coordinate system, built on first use (guarded by em_mu);
-  // a plan without room for them keeps the general kernels.
+  // Merged coefficient planes per coordinate system, built on first use (guarded by em_mu); a
+  // plan without room for them keeps the general kernels.
   picuda::Planes64 planes64[2];
+  picuda::Planes32 planes32[2];
   bool planes64_failed[2] = {false, false};
+  bool planes32_failed[2] = {false, false};
   const picuda::StripItem* strip_items = nullptr;
   int nstrip_items = 0;
   // Single-instance solves run as one job of a batched engine kept with the plan (created on
@@ -126,9 +128,10 @@ struct StripItems {
 };
 StripItems strip_items(pi_plan* plan);
 
-// Merged FP64 coefficient planes of a canonical plan in reference (coords 0) or population
-// (1) coordinates, built on first use (pi_apply64.cu); items == nullptr when the plan is not
-// canonical or has no room for them.
+// Merged coefficient planes of a canonical plan in reference (coords 0) or population (1)
+// coordinates, built on first use (pi_strip.cu); items == nullptr when the plan is not canonical
+// or has no room for them.
 Planes64 planes64(pi_plan* plan, int coords);
+Planes32 planes32(pi_plan* plan, int coords);
 
 }  // namespace picuda

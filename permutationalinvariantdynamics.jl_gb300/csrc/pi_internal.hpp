@@ -44,9 +44,10 @@ constexpr int kCanonEntries = 5 + 9 * kCanonPerPos;  // 32
 // coordinates.
 cudaError_t launch_apply_f64(const DevicePlan& dp, const double* x, double* y, int ncols, long long ld,
                              const BorderArgs& border, cudaStream_t stream);
-// The FP64 apply from merged coefficient planes (pi_apply64.cu), P built for border.coords.
-cudaError_t launch_apply_strip64(const DevicePlan& dp, const Planes64& P, const double* x, double* y, int ncols,
-                                 long long ld, const BorderArgs& border, cudaStream_t stream);
+// The apply from merged coefficient planes (pi_strip.cu), P built for border.coords.
+template <typename T>
+cudaError_t launch_apply_strip(const DevicePlan& dp, const StripPlanes<T>& P, const T* x, T* y, int ncols,
+                               long long ld, const BorderArgs& border, cudaStream_t stream);
 // FP32 action; border.coords selects reference (0) or population (1) coordinates.
 cudaError_t launch_apply_f32(const DevicePlan& dp, const float* x, float* y, int ncols, long long ld,
                              const BorderArgs& border, cudaStream_t stream);

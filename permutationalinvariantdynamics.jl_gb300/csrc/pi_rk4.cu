@@ -32,7 +32,7 @@
 #include <vector>
 
 #include "../../include/picuda.h"
-#include "pi_apply64.cuh"
+#include "pi_strip.cuh"
 #include "pi_apply_impl.cuh"
 #include "pi_handle.hpp"
 
@@ -140,7 +140,7 @@ __global__ void __launch_bounds__(kApplyThreads) k_rk4_stage64(Rk4Params p) {
                         win, st, ge);
 }
 
-// The FP64 stage of a canonical plan: strip apply (pi_apply64.cuh) with the stage update, 25.5
+// The FP64 stage of a canonical plan: strip apply (pi_strip.cuh) with the stage update, 25.5
 // FP64 instructions per entry on average.  18.7 us a stage at N = 120, against 44 us for the tile
 // kernel (41 instructions per entry, 20% idle lanes, 432 tiles on 152 SMs).
 template <int STAGE, int V>
@@ -148,7 +148,7 @@ __global__ void __launch_bounds__(kStripThreads, 4) k_rk4_strip64(Rk4Params p) {
   const int item = blockIdx.x * kStripWarps + (threadIdx.x >> 5);
   if (item >= p.p64.nitems) return;
   const StripItem it = p.p64.items[item];
-  StripEntry<V> E;
+  StripEntry<double, V> E;
   if (!E.load(it, p.p64, threadIdx.x & 31)) return;
   const double2* x = STAGE == 0 ? (const double2*)p.dest : (const double2*)(STAGE == 2 ? p.ta : p.tb);
   double2* next = (double2*)(STAGE == 1 ? p.ta : p.tb);

@@ -73,7 +73,7 @@ struct Run {
   }
   double norm(const double2* w) { return std::sqrt(norm2(w)); }
   void apply64(const double2* x, double2* y, const BorderArgs& b) {
-    chk(planes.items ? launch_apply_strip64(p->dev, planes, (const double*)x, (double*)y, 1, n, b, s)
+    chk(planes.items ? launch_apply_strip<double>(p->dev, planes, (const double*)x, (double*)y, 1, n, b, s)
                      : launch_apply_f64(p->dev, (const double*)x, (double*)y, 1, n, b, s));
     ++applications;
   }

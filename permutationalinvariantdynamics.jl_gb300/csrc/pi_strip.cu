@@ -1,9 +1,9 @@
-// Coefficient planes of the FP64 strip apply (pi_apply64.cuh) and its launches.
+// Coefficient planes of the strip apply (pi_strip.cuh) and its launches.
 #include <algorithm>
 #include <vector>
 
 #include "../../include/picuda.h"
-#include "pi_apply64.cuh"
+#include "pi_strip.cuh"
 #include "pi_handle.hpp"
 #include "pi_internal.hpp"
 
@@ -29,10 +29,13 @@ __global__ void k_strip_items(const DevSector* __restrict__ sectors, const int2*
   }
 }
 
-// Planes and line tables of sector blockIdx.y.
-__global__ void k_planes64(const DevSector* __restrict__ sectors, const int4* __restrict__ canon,
-                           const double2* __restrict__ coef, const int2* __restrict__ first, const Planes64 P, int nr,
-                           double* __restrict__ plane, double2* __restrict__ lrow, double2* __restrict__ rcol) {
+// Planes and line tables of sector blockIdx.y, merged in FP64 for either precision.
+template <typename T>
+__global__ void k_planes(const DevSector* __restrict__ sectors, const int4* __restrict__ canon,
+                         const double2* __restrict__ coef, const int2* __restrict__ first, const StripPlanes<T> P,
+                         int nr, T* __restrict__ plane, typename Vec2<T>::type* __restrict__ lrow,
+                         typename Vec2<T>::type* __restrict__ rcol) {
+  using T2 = typename Vec2<T>::type;
   const int s = blockIdx.y;
   const DevSector& sec = sectors[s];
   const int n = sec.n;
@@ -50,51 +53,57 @@ __global__ void k_planes64(const DevSector* __restrict__ sectors, const int4* __
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < cnt; i += (long long)gridDim.x * blockDim.x) {
     const int b = (int)(i / n), a = (int)(i - (long long)b * n);
     const double2 al = coef[ct[0].x + a], be = coef[ct[0].y + b];
-    double* out = plane + sec.offset + i;
-    out[0] = (al.x + be.x) + sand(4, a, b);  // the own-sector centre gain joins the ADD term
-    out[P.dim] = al.y + be.y;
+    T* out = plane + sec.offset + i;
+    out[0] = (T)((al.x + be.x) + sand(4, a, b));  // the own-sector centre gain joins the ADD term
+    out[P.dim] = (T)(al.y + be.y);
     for (int k = 0; k < nr; ++k) {
       const int src = P.gain[k].src;
       const int slot = src == 0 ? 1 : src == 1 ? 0 : 2;
-      out[(2 + k) * P.dim] = sand(slot * 3 + P.gain[k].shift + 1, a, b);
+      out[(2 + k) * P.dim] = (T)sand(slot * 3 + P.gain[k].shift + 1, a, b);
     }
   }
   if (blockIdx.x == 0)
     for (int i = threadIdx.x; i < n; i += blockDim.x) {
-      lrow[first[s].x + i] = make_double2(coef[ct[1].x + i].y, coef[ct[2].x + i].y);
-      rcol[first[s].x + i] = make_double2(coef[ct[3].y + i].y, coef[ct[4].y + i].y);
+      lrow[first[s].x + i] = T2{(T)coef[ct[1].x + i].y, (T)coef[ct[2].x + i].y};
+      rcol[first[s].x + i] = T2{(T)coef[ct[3].y + i].y, (T)coef[ct[4].y + i].y};
     }
 }
 
-// 128 columns at N = 120 with emission, dephasing and collective decay (22 FP64 instructions
-// per entry, 97% of the FP64 pipe): 1.41 ms = 1.21 TFLOP/s, against 2.34 ms for 32 x 32 tiles
-// with staged windows; one vector at N = 200: 62 us against 125 us (products formed on the way).
-//
+// 128 columns at N = 120 with emission, dephasing and collective decay: FP64 1.41 ms = 1.21 TFLOP/s,
+// 97% of the FP64 pipe (2.34 ms for 32 x 32 tiles with staged windows); FP32 200 us = 3.1 TB/s,
+// bound by L1 (350 us).  37 columns at N = 97 with pumping: FP32 40 us against 75 us.  One vector
+// at N = 200: FP64 62 us against 125 us, FP32 19 us against 26 us (products formed on the way).
 // EPI: scale and trace border; without them their instructions are not in the kernel.
-template <int V, bool EPI>
-__global__ void __launch_bounds__(kStripThreads, 4)
-    k_apply_strip64(const Planes64 P, const DevSector* __restrict__ sectors, int ncols, int rc,
-                    const double2* __restrict__ x, double2* __restrict__ y, long long ld, const double2* alpha,
-                    int coords, double scale) {
+template <typename T, int V, bool EPI>
+__global__ void __launch_bounds__(kStripThreads, sizeof(T) == 4 ? 8 : 4)
+    k_apply_strip(const StripPlanes<T> P, const DevSector* __restrict__ sectors, int ncols, int rc,
+                  const typename Vec2<T>::type* __restrict__ x, typename Vec2<T>::type* __restrict__ y, long long ld,
+                  const double2* alpha, int coords, double scale) {
+  using T2 = typename Vec2<T>::type;
   const int item = blockIdx.x * kStripWarps + (threadIdx.x >> 5);
   if (item >= P.nitems) return;
   const StripItem it = P.items[item];
-  StripEntry<V> E;
+  StripEntry<T, V> E;
   if (!E.load(it, P, threadIdx.x & 31)) return;
   const int c0 = blockIdx.y * rc, c1 = min(c0 + rc, ncols);
   x += c0 * ld;
   y += c0 * ld + E.e;
 #pragma unroll 1
   for (int c = c0; c < c1; ++c) {
-    double2 out = E.apply(x);
+    T2 out = E.apply(x);
     if (EPI) {
-      out.x *= scale;
-      out.y *= scale;
+      out.x *= (T)scale;
+      out.y *= (T)scale;
       if (alpha != nullptr && E.diag) {
         const double v = coords ? sectors[it.sector].border_z : sectors[it.sector].border_x;
         const double2 al = alpha[c];
-        out.x = fma(al.x, v, out.x);
-        out.y = fma(al.y, v, out.y);
+        if constexpr (sizeof(T) == 4) {
+          out.x += (float)(al.x * v);
+          out.y += (float)(al.y * v);
+        } else {
+          out.x = fma(al.x, v, out.x);
+          out.y = fma(al.y, v, out.y);
+        }
       }
     }
     *y = out;
@@ -167,15 +176,17 @@ StripItems strip_items(pi_plan* plan) {
   return strip_items_locked(plan);
 }
 
-Planes64 planes64(pi_plan* plan, int coords) {
+template <typename T>
+static StripPlanes<T> build_planes(pi_plan* plan, int coords, StripPlanes<T> (&kept)[2], bool (&failed)[2]) {
+  using T2 = typename Vec2<T>::type;
   const DevicePlan& dp = plan->dev;
-  if (!dp.canon) return Planes64{};
+  if (!dp.canon) return StripPlanes<T>{};
   std::lock_guard<std::mutex> lk(plan->em_mu);
   const int which = coords ? 1 : 0;
-  Planes64& P = plan->planes64[which];
-  if (P.items || plan->planes64_failed[which]) return P;
+  StripPlanes<T>& P = kept[which];
+  if (P.items || failed[which]) return P;
   const StripItems strips = strip_items_locked(plan);
-  if (!strips.items) return Planes64{};
+  if (!strips.items) return StripPlanes<T>{};
   RelaxedCapture relaxed;
   const int S = (int)plan->host.sectors.size();
   std::vector<int2> first;
@@ -189,7 +200,7 @@ Planes64 planes64(pi_plan* plan, int coords) {
       if (t.kind == ST_SAND) used[t.e == 0 ? 0 : t.e < 0 ? 1 : 2][t.p + 1] = true;
     }
   used[0][1] = false;  // joins the centre
-  Planes64 Q;
+  StripPlanes<T> Q;
   Q.dim = dp.dim;
   Q.nitems = strips.n;
   for (GainPos& g : Q.gain) g = GainPos{-1, 0};
@@ -200,8 +211,8 @@ Planes64 planes64(pi_plan* plan, int coords) {
   Q.variant = drive ? (nr <= 1 ? 0 : nr <= 3 ? 1 : nr <= 5 ? 2 : nr <= 6 ? 3 : 4) : (nr <= 5 ? 5 : 6);
   const int np = 2 + nr;
   // one allocation: line tables, planes, per-sector starts
-  const size_t line_bytes = sizeof(double2) * (size_t)lines;
-  const size_t plane_bytes = (sizeof(double) * (size_t)dp.dim * np + 15) / 16 * 16;
+  const size_t line_bytes = (sizeof(T2) * (size_t)lines + 15) / 16 * 16;
+  const size_t plane_bytes = (sizeof(T) * (size_t)dp.dim * np + 15) / 16 * 16;
   const size_t bytes = 2 * line_bytes + plane_bytes + sizeof(int2) * (size_t)S;
   char* d = nullptr;
   cudaError_t e = cudaMalloc((void**)&d, bytes);
@@ -212,54 +223,72 @@ Planes64 planes64(pi_plan* plan, int coords) {
     if (e == cudaSuccess) {
       const dim3 grid((unsigned)std::min<long long>(64, ((long long)plan->host.max_n * plan->host.max_n + 255) / 256),
                       (unsigned)S);
-      k_planes64<<<grid, 256, 0, plan->stream>>>(dp.sectors, dp.canon, coords ? dp.coef64z : dp.coef64,
-                                                 (const int2*)d_first, Q, nr, (double*)d_plane, (double2*)d,
-                                                 (double2*)d + lines);
+      k_planes<T><<<grid, 256, 0, plan->stream>>>(dp.sectors, dp.canon, coords ? dp.coef64z : dp.coef64,
+                                                  (const int2*)d_first, Q, nr, (T*)d_plane, (T2*)d,
+                                                  (T2*)(d + line_bytes));
       e = cudaGetLastError();
     }
     if (e == cudaSuccess) e = cudaStreamSynchronize(plan->stream);
     Q.items = strips.items;
-    Q.lrow = (const double2*)d;
-    Q.rcol = (const double2*)d + lines;
-    Q.plane = (const double*)d_plane;
+    Q.lrow = (const T2*)d;
+    Q.rcol = (const T2*)(d + line_bytes);
+    Q.plane = (const T*)d_plane;
   }
   if (!adopt(plan, d, bytes, e)) {  // no room: the plan keeps the general kernels
-    plan->planes64_failed[which] = true;
-    return Planes64{};
+    failed[which] = true;
+    return StripPlanes<T>{};
   }
   P = Q;
   return P;
 }
 
+Planes64 planes64(pi_plan* plan, int coords) {
+  return build_planes<double>(plan, coords, plan->planes64, plan->planes64_failed);
+}
+
+Planes32 planes32(pi_plan* plan, int coords) {
+  return build_planes<float>(plan, coords, plan->planes32, plan->planes32_failed);
+}
+
 namespace {
 
-template <int V>
-void launch_strip(const dim3 grid, bool epi, cudaStream_t stream, const Planes64& P, const DevicePlan& dp, int ncols,
-                  int rc, const double* x, double* y, long long ld, const BorderArgs& border) {
-  auto k = epi ? k_apply_strip64<V, true> : k_apply_strip64<V, false>;
-  k<<<grid, kStripThreads, 0, stream>>>(P, dp.sectors, ncols, rc, (const double2*)x, (double2*)y, ld, border.alpha,
+template <typename T, int V>
+void launch_variant(const dim3 grid, cudaStream_t stream, const StripPlanes<T>& P, const DevicePlan& dp, int ncols,
+                    int rc, const T* x, T* y, long long ld, const BorderArgs& border) {
+  using T2 = typename Vec2<T>::type;
+  const bool epi = border.scale != 1.0 || border.alpha != nullptr;
+  auto k = epi ? k_apply_strip<T, V, true> : k_apply_strip<T, V, false>;
+  k<<<grid, kStripThreads, 0, stream>>>(P, dp.sectors, ncols, rc, (const T2*)x, (T2*)y, ld, border.alpha,
                                         border.coords, border.scale);
 }
 
 }  // namespace
 
-cudaError_t launch_apply_strip64(const DevicePlan& dp, const Planes64& P, const double* x, double* y, int ncols,
-                                 long long ld, const BorderArgs& border, cudaStream_t stream) {
-  // Columns per block: the coefficients of an entry (11 loads) are shared by its columns.
-  const int rc = ncols >= 64 ? 8 : ncols >= 16 ? 4 : ncols >= 4 ? 2 : 1;
+template <typename T>
+cudaError_t launch_apply_strip(const DevicePlan& dp, const StripPlanes<T>& P, const T* x, T* y, int ncols,
+                               long long ld, const BorderArgs& border, cudaStream_t s) {
+  // Columns per block: an entry's coefficients are about as many loads as a column's sources, so
+  // up to 16 columns share them while two waves of warps remain.  FP32, 37 columns at N = 97 (two
+  // to 32 per block): 55, 44, 41, 40, 48 us; 128 at N = 120: 302, 240, 212, 203, 199 us.
+  int rc = 16;
+  while (rc > 1 && (long long)P.nitems * ((ncols + rc - 1) / rc) < 2LL * 152 * 32) rc /= 2;
   const dim3 grid((unsigned)((P.nitems + kStripWarps - 1) / kStripWarps), (unsigned)((ncols + rc - 1) / rc));
-  const bool epi = border.scale != 1.0 || border.alpha != nullptr;
-  static_assert(kVariants64 == 7, "one launch per variant");
+  static_assert(kStripVariants == 7, "one launch per variant");
   switch (P.variant) {
-    case 0: launch_strip<0>(grid, epi, stream, P, dp, ncols, rc, x, y, ld, border); break;
-    case 1: launch_strip<1>(grid, epi, stream, P, dp, ncols, rc, x, y, ld, border); break;
-    case 2: launch_strip<2>(grid, epi, stream, P, dp, ncols, rc, x, y, ld, border); break;
-    case 3: launch_strip<3>(grid, epi, stream, P, dp, ncols, rc, x, y, ld, border); break;
-    case 4: launch_strip<4>(grid, epi, stream, P, dp, ncols, rc, x, y, ld, border); break;
-    case 5: launch_strip<5>(grid, epi, stream, P, dp, ncols, rc, x, y, ld, border); break;
-    default: launch_strip<6>(grid, epi, stream, P, dp, ncols, rc, x, y, ld, border);
+    case 0: launch_variant<T, 0>(grid, s, P, dp, ncols, rc, x, y, ld, border); break;
+    case 1: launch_variant<T, 1>(grid, s, P, dp, ncols, rc, x, y, ld, border); break;
+    case 2: launch_variant<T, 2>(grid, s, P, dp, ncols, rc, x, y, ld, border); break;
+    case 3: launch_variant<T, 3>(grid, s, P, dp, ncols, rc, x, y, ld, border); break;
+    case 4: launch_variant<T, 4>(grid, s, P, dp, ncols, rc, x, y, ld, border); break;
+    case 5: launch_variant<T, 5>(grid, s, P, dp, ncols, rc, x, y, ld, border); break;
+    default: launch_variant<T, 6>(grid, s, P, dp, ncols, rc, x, y, ld, border);
   }
   return cudaGetLastError();
 }
+
+template cudaError_t launch_apply_strip<double>(const DevicePlan&, const Planes64&, const double*, double*, int,
+                                                long long, const BorderArgs&, cudaStream_t);
+template cudaError_t launch_apply_strip<float>(const DevicePlan&, const Planes32&, const float*, float*, int,
+                                               long long, const BorderArgs&, cudaStream_t);
 
 }  // namespace picuda

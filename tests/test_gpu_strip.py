@@ -1,4 +1,4 @@
-"""FP64 strip apply (merged coefficient planes) against the host-lowered stencil tables.
+"""Strip apply (merged coefficient planes) against the host-lowered stencil tables.
 
 Per output entry at most 11 products are summed, each of rounded factors, so the result lies
 within 32 rounding units of the sum of the products' magnitudes."""
@@ -58,6 +58,28 @@ def test_strip_apply_matches_tables(torch_cuda, family, N):
                     ref = evaluate(model.basis, table, coef, X[c])
                     tol = 32 * np.finfo(float).eps * _bound(model.basis, table, coef, X[c])
                     assert (np.abs(y[c] - ref) <= tol).all(), (sectors, adjoint, ncols, c)
+
+
+@pytest.mark.parametrize("N", [1, 2, 7, 15, 34])
+@pytest.mark.parametrize("family", sorted(FAMILIES))
+def test_strip_apply_f32_matches_tables(torch_cuda, family, N):
+    torch = torch_cuda
+    model = picuda.qubit_ensemble_model(N, **FAMILIES[family])
+    compiled = picuda.compile(model)
+    n = len(model.basis)
+    root = np.repeat(model.basis.multiplicity_scales(), np.array(model.basis.dims) ** 2)  # z = root x
+    table, coef = picuda.stencil_tables(model)
+    for ncols in (1, 3, 17, 65):
+        X = np.stack([M.random_state_vector(n, 5 * c + N) for c in range(ncols)]).astype(np.complex64)
+        xd = torch.from_numpy(X if ncols > 1 else X[0]).cuda()
+        for coords, scale in (("reference", np.ones(n)), ("population", root)):
+            y = picuda.apply_(torch.full_like(xd, float("nan")), compiled, xd, precision="fp32", coords=coords)
+            y = y.cpu().numpy().reshape(ncols, n)
+            for c in {0, ncols // 2, ncols - 1}:
+                x = X[c].astype(np.complex128) / scale
+                ref = scale * evaluate(model.basis, table, coef, x)
+                tol = 32 * np.finfo(np.float32).eps * scale * _bound(model.basis, table, coef, x)
+                assert (np.abs(y[c] - ref) <= tol).all(), (coords, ncols, c)
 
 
 @pytest.mark.parametrize("family", ["undriven", "all", "btc"])
