@@ -22,6 +22,7 @@
 #include "pi_strip.cuh"
 #include "pi_apply_impl.cuh"
 #include "pi_dense.hpp"
+#include "pi_reduce.cuh"
 
 namespace picuda {
 namespace {
@@ -68,20 +69,6 @@ __device__ __forceinline__ void block_sum(double (&v)[NV], double* smem, int nw 
 #pragma unroll
       for (int off = 16; off > 0; off >>= 1) v[k] += __shfl_down_sync(0xffffffffu, v[k], off);
   }
-}
-
-// Double-float accumulator (FP32 pair): exact products by FMA, TwoSum accumulation.
-struct DF {
-  float hi, lo;
-};
-__device__ __forceinline__ void df_add_prod(DF& acc, float a, float b) {
-  const float p = a * b;
-  const float e = fmaf(a, b, -p);
-  const float s = acc.hi + p;
-  const float bb = s - acc.hi;
-  const float err = (acc.hi - (s - bb)) + (p - bb);
-  acc.hi = s;
-  acc.lo += err + e;
 }
 
 __device__ __forceinline__ void chunk_range(const DevInst& S, int c, long long& beg, long long& end) {
@@ -496,25 +483,6 @@ __global__ void __launch_bounds__(kRT) k_s1_resid(const DevInst* __restrict__ st
     const double2 b = S.rb[e], a = S.ay[e];
     r[e] = make_double2(b.x - a.x, b.y - a.y);
   }
-}
-
-// Sums v[k] over the warp's lanes by exchanging halves of the values (NV - 1 additions and a few
-// more instead of 5 NV); afterwards v[0] of lane l is the total of value l / (32 / NV).
-template <int NV>
-__device__ __forceinline__ void warp_transpose_sum(double (&v)[NV]) {
-  const int lane = threadIdx.x & 31;
-  int off = 16;
-#pragma unroll
-  for (int s = NV / 2; s >= 1; s >>= 1, off >>= 1) {
-    const bool up = lane & off;
-#pragma unroll
-    for (int i = 0; i < s; ++i) {
-      const double send = up ? v[i] : v[i + s];
-      const double keep = up ? v[i + s] : v[i];
-      v[i] = keep + __shfl_xor_sync(0xffffffffu, send, off);
-    }
-  }
-  for (; off >= 1; off >>= 1) v[0] += __shfl_xor_sync(0xffffffffu, v[0], off);
 }
 
 // |nrm0|^2 and |nrm1|^2 over one chunk; a combination's own norm is already there.
@@ -1020,23 +988,6 @@ __device__ __forceinline__ void pair_range(const DevInst& S, int c, long long& b
   end = min(beg + (long long)(S.chunk / 2), (S.dim + 1) / 2);
 }
 
-// a += t, the rounding error of the addition carried in a.lo (TwoSum).
-__device__ __forceinline__ void df_add(DF& a, float t) {
-  const float s = a.hi + t;
-  const float bb = s - a.hi;
-  const float err = (a.hi - (s - bb)) + (t - bb);
-  a.hi = s;
-  a.lo += err;
-}
-
-// a + b for double-float values (TwoSum of the leading parts).
-__device__ __forceinline__ DF df_sum(DF a, DF b) {
-  const float s = a.hi + b.hi;
-  const float bb = s - a.hi;
-  const float err = (a.hi - (s - bb)) + (b.hi - bb);
-  return DF{s, (a.lo + b.lo) + err};
-}
-
 // Warp sum of double-float values in FP32 arithmetic (GB300's FP64 pipe is narrow: the
 // per-column reductions stay off it); the result is valid in lane 0.
 __device__ __forceinline__ DF warp_df_sum(DF v) {
@@ -1082,23 +1033,6 @@ __device__ __forceinline__ void pair_terms(const float4 a, const float4 b, DF& r
 // The lane sums of K columns exchange halves of the accumulators (2K - 1 double-float additions
 // and as many shuffles, against 10K one value at a time, which at 1024 elements per chunk were
 // two thirds of the instructions); each value is still summed over the same tree of lanes.
-template <int NV>
-__device__ __forceinline__ void warp_transpose_sum(DF (&v)[NV]) {
-  const int lane = threadIdx.x & 31;
-  int off = 16;
-#pragma unroll
-  for (int s = NV / 2; s >= 1; s >>= 1, off >>= 1) {
-    const bool up = lane & off;
-#pragma unroll
-    for (int i = 0; i < s; ++i) {
-      const DF send = up ? v[i] : v[i + s], keep = up ? v[i + s] : v[i];
-      v[i] = df_sum(keep, DF{__shfl_xor_sync(0xffffffffu, send.hi, off), __shfl_xor_sync(0xffffffffu, send.lo, off)});
-    }
-  }
-  for (; off >= 1; off >>= 1)
-    v[0] = df_sum(v[0], DF{__shfl_xor_sync(0xffffffffu, v[0].hi, off), __shfl_xor_sync(0xffffffffu, v[0].lo, off)});
-}
-
 template <int CH>
 struct Dot32Smem {
   float4 w[CH / 2];
@@ -1193,16 +1127,6 @@ __global__ void __launch_bounds__(kRT, 3)
 // coefficient is split into hi + lo floats, hi * v is formed exactly (FMA residual), lo * v
 // in FP32, and the sum is carried as a double-float per component, so the FP64 output
 // matches an FP64 accumulation to ~1e-14 while the FP64 pipe stays idle.
-__device__ __forceinline__ void df_axpy(DF& acc, float ch, float cl, float v) {
-  const float p = ch * v;
-  const float e = fmaf(ch, v, -p);
-  const float s = acc.hi + p;
-  const float bb = s - acc.hi;
-  const float err = (acc.hi - (s - bb)) + (p - bb);
-  acc.hi = s;
-  acc.lo += err + fmaf(cl, v, e);
-}
-
 __global__ void __launch_bounds__(kRT)
     k_s1_combine_f32(const DevInst* __restrict__ st, const int* __restrict__ chunk_inst, double* __restrict__ part) {
   __shared__ float4 cs[kBatchMaxKrylov + 2];  // (re.hi, re.lo, im.hi, im.lo)

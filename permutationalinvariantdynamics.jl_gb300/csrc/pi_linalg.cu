@@ -8,6 +8,7 @@
 #include <algorithm>
 
 #include "pi_internal.hpp"
+#include "pi_reduce.cuh"
 
 namespace picuda {
 
@@ -52,93 +53,86 @@ __device__ __forceinline__ double2 load_c(const T2* p) {
 }
 
 // Stage 1 of a multi-dot: block (bx, by) reduces vectors by*8 .. by*8+7 over element chunk
-// bx and writes partial[bx][i].  One block-wide sum per block.
+// bx and writes partial[bx * stride + i].  The columns of a group are counted at compile time
+// (8, then 4, 2, 1): FMAs of absent columns would be issued all the same.  Lane sums exchange
+// halves of the accumulators (16 additions for 8 columns against 80 one by one, which at N = 200
+// took as long as the products); FP32 vectors are summed in double-float until one value per
+// lane is left, as a conversion holds the FP64 pipe like an addition.
 constexpr int kDotGroup = 8;
+
+template <int K>
+__device__ __forceinline__ void dot_cols(const double2* __restrict__ V, long long ldv, const double2* __restrict__ w,
+                                         long long beg, long long end, double* row) {
+  double acc[2 * K];
+#pragma unroll
+  for (int k = 0; k < 2 * K; ++k) acc[k] = 0.0;
+  for (long long e = beg + threadIdx.x; e < end; e += blockDim.x) {
+    const double2 wv = __ldg(w + e);
+#pragma unroll
+    for (int k = 0; k < K; ++k) {
+      const double2 v = __ldg(V + k * ldv + e);
+      acc[2 * k] = fma(v.x, wv.x, acc[2 * k]);
+      acc[2 * k] = fma(v.y, wv.y, acc[2 * k]);
+      acc[2 * k + 1] = fma(v.x, wv.y, acc[2 * k + 1]);
+      acc[2 * k + 1] = fma(-v.y, wv.x, acc[2 * k + 1]);
+    }
+  }
+  warp_transpose_sum<2 * K>(acc);
+  constexpr int span = 32 / (2 * K);
+  const int lane = threadIdx.x & 31;
+  if (lane % span == 0) row[lane / span] = acc[0];
+}
+
+// FP32 vectors: exact products, double-float accumulation.
+template <int K>
+__device__ __forceinline__ void dot_cols(const float2* __restrict__ V, long long ldv, const float2* __restrict__ w,
+                                         long long beg, long long end, double* row) {
+  DF acc[2 * K];
+#pragma unroll
+  for (int k = 0; k < 2 * K; ++k) acc[k] = DF{0.f, 0.f};
+#pragma unroll 2
+  for (long long e = beg + threadIdx.x; e < end; e += blockDim.x) {
+    const float2 wv = __ldg(w + e);
+#pragma unroll
+    for (int k = 0; k < K; ++k) {
+      const float2 v = __ldg(V + k * ldv + e);
+      df_add_prod(acc[2 * k], v.x, wv.x);
+      df_add_prod(acc[2 * k], v.y, wv.y);
+      df_add_prod(acc[2 * k + 1], v.x, wv.y);
+      df_add_prod(acc[2 * k + 1], -v.y, wv.x);
+    }
+  }
+  warp_transpose_sum<2 * K>(acc);
+  constexpr int span = 32 / (2 * K);
+  const int lane = threadIdx.x & 31;
+  if (lane % span == 0) row[lane / span] = (double)acc[0].hi + (double)acc[0].lo;
+}
 
 template <typename T2>
 __global__ void __launch_bounds__(kReduceThreads)
     k_mdot_partial(const T2* __restrict__ V, long long ldv, int nv, const T2* __restrict__ w, long long n,
-                   double2* __restrict__ partial) {
-  __shared__ double smem[32 * 2 * kDotGroup];
+                   double2* __restrict__ partial, int stride) {
+  __shared__ double red[kReduceThreads / 32][2 * kDotGroup];
   long long beg, end;
   chunk_bounds(n, beg, end);
   const int g = blockIdx.y * kDotGroup;
   const int cnt = min(kDotGroup, nv - g);
-  double acc[2 * kDotGroup];
-#pragma unroll
-  for (int k = 0; k < 2 * kDotGroup; ++k) acc[k] = 0.0;
-  for (long long e = beg + threadIdx.x; e < end; e += blockDim.x) {
-    const double2 wv = load_c(w + e);
-#pragma unroll
-    for (int k = 0; k < kDotGroup; ++k) {
-      if (k < cnt) {
-        const double2 v = load_c(V + (long long)(g + k) * ldv + e);
-        acc[2 * k] = fma(v.x, wv.x, acc[2 * k]);
-        acc[2 * k] = fma(v.y, wv.y, acc[2 * k]);
-        acc[2 * k + 1] = fma(v.x, wv.y, acc[2 * k + 1]);
-        acc[2 * k + 1] = fma(-v.y, wv.x, acc[2 * k + 1]);
-      }
-    }
+  V += (long long)g * ldv;
+  double* row = red[threadIdx.x >> 5];
+  if (cnt == 8) {  // uniform
+    dot_cols<8>(V, ldv, w, beg, end, row);
+  } else {
+    int k = 0;
+    if (cnt & 4) dot_cols<4>(V, ldv, w, beg, end, row), k = 4;
+    if (cnt & 2) dot_cols<2>(V + k * ldv, ldv, w, beg, end, row + 2 * k), k += 2;
+    if (cnt & 1) dot_cols<1>(V + k * ldv, ldv, w, beg, end, row + 2 * k);
   }
-  block_sum<2 * kDotGroup>(acc, smem);
-  if (threadIdx.x == 0) {
-    for (int k = 0; k < cnt; ++k)
-      partial[(long long)blockIdx.x * kMaxDots + g + k] = make_double2(acc[2 * k], acc[2 * k + 1]);
-  }
-}
-
-// Double-float accumulator: the pair (hi, lo) carries a ~48-bit significand on the FP32
-// pipes.  Products of two FP32 numbers are split exactly with an FMA (a*b = p + e) and
-// added with Knuth's TwoSum, so a dot of FP32 vectors is accumulated to FP64-class accuracy
-// without the GB300 FP64 pipe (1/64 of the FP32 rate).
-struct DF {
-  float hi, lo;
-};
-__device__ __forceinline__ void df_add_prod(DF& acc, float a, float b) {
-  const float p = a * b;
-  const float e = fmaf(a, b, -p);
-  const float s = acc.hi + p;
-  const float bb = s - acc.hi;
-  const float err = (acc.hi - (s - bb)) + (p - bb);
-  acc.hi = s;
-  acc.lo += err + e;
-}
-
-// Stage 1 of a multi-dot for FP32 vectors with double-float accumulation (grid as above).
-__global__ void __launch_bounds__(kReduceThreads)
-    k_mdot_partial_df(const float2* __restrict__ V, long long ldv, int nv, const float2* __restrict__ w, long long n,
-                      double2* __restrict__ partial) {
-  __shared__ double smem[32 * 2 * kDotGroup];
-  long long beg, end;
-  chunk_bounds(n, beg, end);
-  const int g = blockIdx.y * kDotGroup;
-  const int cnt = min(kDotGroup, nv - g);
-  DF re[kDotGroup], im[kDotGroup];
+  __syncthreads();
+  for (int i = threadIdx.x; i < 2 * cnt; i += blockDim.x) {
+    double t = 0;
 #pragma unroll
-  for (int k = 0; k < kDotGroup; ++k) re[k] = im[k] = DF{0.f, 0.f};
-  for (long long e = beg + threadIdx.x; e < end; e += blockDim.x) {
-    const float2 wv = __ldg(w + e);
-#pragma unroll
-    for (int k = 0; k < kDotGroup; ++k) {
-      if (k < cnt) {
-        const float2 v = __ldg(V + (long long)(g + k) * ldv + e);
-        df_add_prod(re[k], v.x, wv.x);
-        df_add_prod(re[k], v.y, wv.y);
-        df_add_prod(im[k], v.x, wv.y);
-        df_add_prod(im[k], -v.y, wv.x);
-      }
-    }
-  }
-  double acc[2 * kDotGroup];
-#pragma unroll
-  for (int k = 0; k < kDotGroup; ++k) {
-    acc[2 * k] = (double)re[k].hi + (double)re[k].lo;
-    acc[2 * k + 1] = (double)im[k].hi + (double)im[k].lo;
-  }
-  block_sum<2 * kDotGroup>(acc, smem);
-  if (threadIdx.x == 0) {
-    for (int k = 0; k < cnt; ++k)
-      partial[(long long)blockIdx.x * kMaxDots + g + k] = make_double2(acc[2 * k], acc[2 * k + 1]);
+    for (int q = 0; q < kReduceThreads / 32; ++q) t += red[q][i];
+    reinterpret_cast<double*>(partial + (long long)blockIdx.x * stride + g)[i] = t;
   }
 }
 
@@ -192,12 +186,12 @@ __global__ void __launch_bounds__(kReduceThreads)
 
 // Stage 2: one block per dot, fixed-order sum over the partials.
 __global__ void __launch_bounds__(kReduceThreads)
-    k_mdot_final(const double2* __restrict__ partial, int nblocks, double2* __restrict__ out) {
+    k_mdot_final(const double2* __restrict__ partial, int nblocks, int stride, double2* __restrict__ out) {
   __shared__ double smem[32 * 2];
   const int i = blockIdx.x;
   double acc[2] = {0, 0};
   for (int b = threadIdx.x; b < nblocks; b += blockDim.x) {
-    const double2 p = partial[(long long)b * kMaxDots + i];
+    const double2 p = partial[(long long)b * stride + i];
     acc[0] += p.x;
     acc[1] += p.y;
   }
@@ -229,6 +223,7 @@ __global__ void __launch_bounds__(kReduceThreads)
   for (long long e = beg + threadIdx.x; e < end; e += blockDim.x) {
     T2 wr = w[e];
     double wx = (double)wr.x, wy = (double)wr.y;
+#pragma unroll 8
     for (int i = 0; i < nv; ++i) {
       const double2 v = load_c(V + (long long)i * ldv + e);
       const double2 c = hs[i];
@@ -317,22 +312,44 @@ __global__ void __launch_bounds__(kReduceThreads)
   }
 }
 
-// t^H x over all block diagonals; a single block, fixed order.
+// t^H x over all block diagonals: a cluster of blocks, fixed order.  The gathers are latency and
+// the sums FP64 issue, of which one SM had 20 us at N = 200 (10,201 diagonal entries); the blocks
+// hand their sums to the first one through its shared memory.
+constexpr int kTraceBlocks = 8;
+
 template <typename T2>
-__global__ void __launch_bounds__(1024)
+__global__ void __cluster_dims__(kTraceBlocks, 1, 1) __launch_bounds__(kReduceThreads)
     k_trace_dot(const DevSector* __restrict__ sectors, const int* __restrict__ diag_sector,
                 const long long* __restrict__ diag_index, int ndiag, const T2* __restrict__ x, int coords,
                 double2* __restrict__ out) {
   __shared__ double smem[32 * 2];
+  __shared__ double2 parts[kTraceBlocks];
   double acc[2] = {0, 0};
-  for (int i = threadIdx.x; i < ndiag; i += blockDim.x) {
-    const double w = coords ? 1.0 : sectors[diag_sector[i]].sqrt_f;
+#pragma unroll 4
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < ndiag; i += kTraceBlocks * blockDim.x) {
     const double2 v = load_c(x + diag_index[i]);
+    const double w = coords ? 1.0 : sectors[diag_sector[i]].sqrt_f;
     acc[0] = fma(w, v.x, acc[0]);
     acc[1] = fma(w, v.y, acc[1]);
   }
   block_sum<2>(acc, smem);
-  if (threadIdx.x == 0) *out = make_double2(acc[0], acc[1]);
+  // the first block has started before any block writes into its shared memory
+  asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+  if (threadIdx.x == 0) {
+    const unsigned local = (unsigned)__cvta_generic_to_shared(&parts[blockIdx.x]);
+    unsigned remote;
+    asm("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(remote) : "r"(local));
+    asm volatile("st.shared::cluster.v2.f64 [%0], {%1, %2};" ::"r"(remote), "d"(acc[0]), "d"(acc[1]) : "memory");
+  }
+  asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    double2 t = make_double2(0.0, 0.0);
+    for (int b = 0; b < kTraceBlocks; ++b) {
+      t.x += parts[b].x;
+      t.y += parts[b].y;
+    }
+    *out = t;
+  }
 }
 
 // Coordinate change between reference coordinates x and population coordinates z.
@@ -413,8 +430,8 @@ cudaError_t mdot_f64(const double2* V, long long ldv, int nv, const double2* w, 
   if (nv > kMaxDots) return cudaErrorInvalidValue;
   const int gy = (nv + kDotGroup - 1) / kDotGroup;
   const int gx = reduce_blocks(n, gy);
-  k_mdot_partial<double2><<<dim3(gx, gy), kReduceThreads, 0, stream>>>(V, ldv, nv, w, n, rs.partial);
-  k_mdot_final<<<nv, kReduceThreads, 0, stream>>>(rs.partial, gx, h_out);
+  k_mdot_partial<double2><<<dim3(gx, gy), kReduceThreads, 0, stream>>>(V, ldv, nv, w, n, rs.partial, kMaxDots);
+  k_mdot_final<<<nv, kReduceThreads, 0, stream>>>(rs.partial, gx, kMaxDots, h_out);
   return cudaGetLastError();
 }
 
@@ -424,8 +441,8 @@ cudaError_t mdot_f32(const float2* V, long long ldv, int nv, const float2* w, lo
   if (nv > kMaxDots) return cudaErrorInvalidValue;
   const int gy = (nv + kDotGroup - 1) / kDotGroup;
   const int gx = reduce_blocks(n, gy);
-  k_mdot_partial_df<<<dim3(gx, gy), kReduceThreads, 0, stream>>>(V, ldv, nv, w, n, rs.partial);
-  k_mdot_final<<<nv, kReduceThreads, 0, stream>>>(rs.partial, gx, h_out);
+  k_mdot_partial<float2><<<dim3(gx, gy), kReduceThreads, 0, stream>>>(V, ldv, nv, w, n, rs.partial, kMaxDots);
+  k_mdot_final<<<nv, kReduceThreads, 0, stream>>>(rs.partial, gx, kMaxDots, h_out);
   return cudaGetLastError();
 }
 
@@ -488,10 +505,10 @@ cudaError_t combine_f32_to_f64(const float2* V, long long ldv, int nv, const dou
 cudaError_t trace_dot(const DevicePlan& dp, const void* x, int is_f32, int coords, double2* out,
                       cudaStream_t stream) {
   if (is_f32)
-    k_trace_dot<float2><<<1, 1024, 0, stream>>>(dp.sectors, dp.diag_sector, dp.diag_index, dp.ndiag,
+    k_trace_dot<float2><<<kTraceBlocks, kReduceThreads, 0, stream>>>(dp.sectors, dp.diag_sector, dp.diag_index, dp.ndiag,
                                                 (const float2*)x, coords, out);
   else
-    k_trace_dot<double2><<<1, 1024, 0, stream>>>(dp.sectors, dp.diag_sector, dp.diag_index, dp.ndiag,
+    k_trace_dot<double2><<<kTraceBlocks, kReduceThreads, 0, stream>>>(dp.sectors, dp.diag_sector, dp.diag_index, dp.ndiag,
                                                  (const double2*)x, coords, out);
   return cudaGetLastError();
 }
@@ -550,52 +567,6 @@ constexpr int kNoAllocMaxDots = 32;
 
 static __device__ __align__(256) double2 g_noalloc_partials[kNoAllocBlocks * kNoAllocMaxDots];
 
-// Same arithmetic as the plan-owned multi-dot, with the partial stride of the static array.
-__global__ void __launch_bounds__(kReduceThreads)
-    k_mdot_partial_noalloc(const double2* __restrict__ V, long long ldv, int nv, const double2* __restrict__ w,
-                           long long n, double2* __restrict__ partial) {
-  __shared__ double smem[32 * 2 * kDotGroup];
-  long long beg, end;
-  chunk_bounds(n, beg, end);
-  const int g = blockIdx.y * kDotGroup;
-  const int cnt = min(kDotGroup, nv - g);
-  double acc[2 * kDotGroup];
-#pragma unroll
-  for (int k = 0; k < 2 * kDotGroup; ++k) acc[k] = 0.0;
-  for (long long e = beg + threadIdx.x; e < end; e += blockDim.x) {
-    const double2 wv = w[e];
-#pragma unroll
-    for (int k = 0; k < kDotGroup; ++k) {
-      if (k < cnt) {
-        const double2 v = V[(long long)(g + k) * ldv + e];
-        acc[2 * k] = fma(v.x, wv.x, acc[2 * k]);
-        acc[2 * k] = fma(v.y, wv.y, acc[2 * k]);
-        acc[2 * k + 1] = fma(v.x, wv.y, acc[2 * k + 1]);
-        acc[2 * k + 1] = fma(-v.y, wv.x, acc[2 * k + 1]);
-      }
-    }
-  }
-  block_sum<2 * kDotGroup>(acc, smem);
-  if (threadIdx.x == 0) {
-    for (int k = 0; k < cnt; ++k)
-      partial[(long long)blockIdx.x * kNoAllocMaxDots + g + k] = make_double2(acc[2 * k], acc[2 * k + 1]);
-  }
-}
-
-__global__ void __launch_bounds__(kReduceThreads)
-    k_mdot_final_noalloc(const double2* __restrict__ partial, int nblocks, double2* __restrict__ out) {
-  __shared__ double smem[32 * 2];
-  const int i = blockIdx.x;
-  double acc[2] = {0, 0};
-  for (int b = threadIdx.x; b < nblocks; b += blockDim.x) {
-    const double2 p = partial[(long long)b * kNoAllocMaxDots + i];
-    acc[0] += p.x;
-    acc[1] += p.y;
-  }
-  block_sum<2>(acc, smem);
-  if (threadIdx.x == 0) out[i] = make_double2(acc[0], acc[1]);
-}
-
 }  // namespace
 
 }  // namespace picuda
@@ -636,11 +607,11 @@ extern "C" int pi_mdot_f64_noalloc(const double* V_dev, long long ldv, int nv, c
   cudaStream_t s = (cudaStream_t)stream;
   // Every partial that the final pass reads is written by the first pass of the same call,
   // so nothing needs clearing; two calls that overlap on the GPU share the array and race.
-  k_mdot_partial_noalloc<<<dim3((unsigned)gx, gy), kReduceThreads, 0, s>>>(
-      (const double2*)V_dev, ldv, nv, (const double2*)w_dev, n, scratch);
+  k_mdot_partial<double2><<<dim3((unsigned)gx, gy), kReduceThreads, 0, s>>>(
+      (const double2*)V_dev, ldv, nv, (const double2*)w_dev, n, scratch, kNoAllocMaxDots);
   e = cudaGetLastError();
   if (e != cudaSuccess) return cuda_fail(e, "pi_mdot_f64_noalloc partial-sum launch");
-  k_mdot_final_noalloc<<<nv, kReduceThreads, 0, s>>>(scratch, (int)gx, (double2*)h_dev);
+  k_mdot_final<<<nv, kReduceThreads, 0, s>>>(scratch, (int)gx, kNoAllocMaxDots, (double2*)h_dev);
   e = cudaGetLastError();
   if (e != cudaSuccess) return cuda_fail(e, "pi_mdot_f64_noalloc final-sum launch");
   return PI_OK;

@@ -55,11 +55,13 @@
 #include <complex>
 #include <cstring>
 #include <string>
+#include <type_traits>
 #include <vector>
 
 #include "../../include/picuda.h"
 #include "pi_handle.hpp"
 #include "pi_internal.hpp"
+#include "pi_reduce.cuh"
 #include "pi_precond.hpp"
 #include "pi_drive.hpp"
 
@@ -390,6 +392,77 @@ __device__ __forceinline__ void solve_level(const PrecondDev& Pd, const Slot<T, 
   }
 }
 
+// The d = 0 chain's correction z -= k w0 at entries c0 .. c1 and this thread's share of t^H z
+// after it.  One block does it for the whole chain (10,201 entries at N = 200), so eight entries
+// per thread are in flight together: one by one, their two dependent gathers and the FP64
+// arithmetic took a third of the sweep.
+constexpr int kTailUnroll = 8;
+
+template <typename TO>
+__device__ __forceinline__ double2 chain0_correct(const PrecondDev& Pd, TO* z, int c0, int c1, double2 k) {
+  double2 tsum = make_double2(0.0, 0.0);
+  for (int e0 = c0 + threadIdx.x; e0 < c1; e0 += kTailUnroll * kSweepThreads) {
+    int el[kTailUnroll];
+    double2 w[kTailUnroll], v[kTailUnroll];
+    double t[kTailUnroll];
+#pragma unroll
+    for (int q = 0; q < kTailUnroll; ++q) {
+      const int e = e0 + q * kSweepThreads;
+      el[q] = e < c1 ? Pd.elem[e] : -1;
+      w[q] = e < c1 ? Pd.w0[e - c0] : make_double2(0.0, 0.0);
+      t[q] = e < c1 ? Pd.t0[e - c0] : 0.0;
+    }
+#pragma unroll
+    for (int q = 0; q < kTailUnroll; ++q) v[q] = el[q] >= 0 ? load_d2(z + el[q]) : make_double2(0.0, 0.0);
+#pragma unroll
+    for (int q = 0; q < kTailUnroll; ++q) {
+      if (el[q] < 0) continue;
+      v[q].x = fma(-k.x, w[q].x, fma(k.y, w[q].y, v[q].x));
+      v[q].y = fma(-k.x, w[q].y, fma(-k.y, w[q].x, v[q].y));
+      store_as<TO, double2>(z + el[q], v[q]);
+      tsum.x = fma(t[q], v[q].x, tsum.x);
+      tsum.y = fma(t[q], v[q].y, tsum.y);
+    }
+  }
+  return tsum;
+}
+
+// The same for FP32 vectors in population coordinates, where t is one: in double-float, as each
+// conversion and FP64 operation of a warp holds a quarter of the SM's FP64 pipe for 64 cycles.
+__device__ __forceinline__ double2 chain0_correct_df(const PrecondDev& Pd, float2* z, int c0, int c1, double2 k) {
+  const DF kx{(float)k.x, (float)(k.x - (double)(float)k.x)}, ky{(float)k.y, (float)(k.y - (double)(float)k.y)};
+  DF sx{0.f, 0.f}, sy{0.f, 0.f};
+  for (int e0 = c0 + threadIdx.x; e0 < c1; e0 += kTailUnroll * kSweepThreads) {
+    int el[kTailUnroll];
+    float4 w[kTailUnroll];
+    float2 v[kTailUnroll];
+#pragma unroll
+    for (int q = 0; q < kTailUnroll; ++q) {
+      const int e = e0 + q * kSweepThreads;
+      el[q] = e < c1 ? Pd.elem[e] : -1;
+      w[q] = e < c1 ? Pd.w0f[e - c0] : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+#pragma unroll
+    for (int q = 0; q < kTailUnroll; ++q) v[q] = el[q] >= 0 ? z[el[q]] : make_float2(0.f, 0.f);
+#pragma unroll
+    for (int q = 0; q < kTailUnroll; ++q) {
+      if (el[q] < 0) continue;
+      // w = (x.hi, x.lo, y.hi, y.lo)
+      DF zx{v[q].x, 0.f}, zy{v[q].y, 0.f};
+      df_axpy(zx, -kx.hi, -kx.lo, w[q].x);
+      df_axpy(zx, ky.hi, ky.lo, w[q].z);
+      zx.lo = fmaf(-kx.hi, w[q].y, fmaf(ky.hi, w[q].w, zx.lo));
+      df_axpy(zy, -kx.hi, -kx.lo, w[q].z);
+      df_axpy(zy, -ky.hi, -ky.lo, w[q].x);
+      zy.lo = fmaf(-kx.hi, w[q].w, fmaf(-ky.hi, w[q].y, zy.lo));
+      z[el[q]] = make_float2(zx.hi + zx.lo, zy.hi + zy.lo);
+      sx = df_sum(sx, zx);
+      sy = df_sum(sy, zy);
+    }
+  }
+  return make_double2((double)sx.hi + (double)sx.lo, (double)sy.hi + (double)sy.lo);
+}
+
 template <typename T, typename TI, typename TO>
 __global__ void __launch_bounds__(kSweepThreads)
     k_level_sweep(const PrecondDev Pd, const TI* __restrict__ r, TO* __restrict__ z, double s) {
@@ -461,17 +534,10 @@ __global__ void __launch_bounds__(kSweepThreads)
     const double den = rv.x * rv.x + rv.y * rv.y;
     const double2 beta =
         make_double2((rrv.x * rv.x + rrv.y * rv.y) / den, (rrv.y * rv.x - rrv.x * rv.y) / den);
-    for (int e = c0 + tid; e < c1; e += blockDim.x) {
-      const int el = Pd.elem[e];
-      const double2 yv = Pd.w0[e - c0];
-      double2 zv = load_d2(z + el);
-      zv.x -= beta.x * yv.x - beta.y * yv.y;
-      zv.y -= beta.x * yv.y + beta.y * yv.x;
-      store_as<TO, double2>(z + el, zv);
-      const double t = Pd.t0[e - c0];
-      tsum.x = fma(t, zv.x, tsum.x);
-      tsum.y = fma(t, zv.y, tsum.y);
-    }
+    if constexpr (std::is_same<T, float>::value && std::is_same<TO, float2>::value)
+      tsum = chain0_correct_df(Pd, z, c0, c1, beta);
+    else
+      tsum = chain0_correct(Pd, z, c0, c1, beta);
     const double2 tz = block_sum2(tsum, S.red);
     if (tid == 0 && Pd.free_ent >= 0) {
       const double t = Pd.t0[Pd.free_ent - c0];
@@ -482,14 +548,10 @@ __global__ void __launch_bounds__(kSweepThreads)
     const double2 tz = block_sum2(tsum, S.red);
     const double2 kk =
         make_double2(tz.x * Pd.sm_coef.x - tz.y * Pd.sm_coef.y, tz.x * Pd.sm_coef.y + tz.y * Pd.sm_coef.x);
-    for (int e = c0 + tid; e < c1; e += blockDim.x) {
-      const int el = Pd.elem[e];
-      const double2 w0 = Pd.w0[e - c0];
-      double2 zv = load_d2(z + el);
-      zv.x -= w0.x * kk.x - w0.y * kk.y;
-      zv.y -= w0.x * kk.y + w0.y * kk.x;
-      store_as<TO, double2>(z + el, zv);
-    }
+    if constexpr (std::is_same<T, float>::value && std::is_same<TO, float2>::value)
+      (void)chain0_correct_df(Pd, z, c0, c1, kk);
+    else
+      (void)chain0_correct(Pd, z, c0, c1, kk);
   }
 }
 
@@ -930,6 +992,14 @@ int pi_precond_create(pi_plan* plan, int coords, double regularization, double o
   const double2* wp = nullptr;
   if ((rc = upload_vec(P, w0, &wp))) return free_precond(P), rc;
   P->dev.w0 = wp;
+  std::vector<float4> w0f(w0.size());  // the same as double-floats (x.hi, x.lo, y.hi, y.lo)
+  for (size_t k = 0; k < w0.size(); ++k) {
+    const float xh = (float)w0[k].x, yh = (float)w0[k].y;
+    w0f[k] = make_float4(xh, (float)(w0[k].x - (double)xh), yh, (float)(w0[k].y - (double)yh));
+  }
+  const float4* wfp = nullptr;
+  if ((rc = upload_vec(P, w0f, &wfp))) return free_precond(P), rc;
+  P->dev.w0f = wfp;
   P->dev.chain0 = H.chain0;
   P->dev.chain0_ent = H.chain0_ent;
   P->dev.free_ent = H.free_ent;

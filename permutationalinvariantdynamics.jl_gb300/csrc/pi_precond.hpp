@@ -58,6 +58,7 @@ struct PrecondDev {
   const double* t0;
   const double* v0;
   const double2* w0;
+  const float4* w0f;  // w0 as double-floats
   double2 sm_coef;
   int chain0;
   int chain0_ent;

@@ -52,7 +52,8 @@ struct Run {
   cudaError_t err = cudaSuccess;
   int applications = 0;
   int coords = 0;  // PI_COORDS_* of every vector of the solve
-  Planes64 planes;  // merged FP64 coefficients of an FP64 solve (mixed solves apply FP64 once per restart)
+  Planes64 planes;      // merged FP64 coefficients of an FP64 solve (mixed solves apply FP64 once per restart)
+  Planes32 planes_f32;  // merged FP32 coefficients of a mixed solve
   explicit Run(pi_plan* plan, int c = 0) : p(plan), s(plan->stream), n(plan->host.dim), coords(c) {}
   bool ok() const { return err == cudaSuccess; }
   void chk(cudaError_t e) {
@@ -87,7 +88,8 @@ struct Run {
   void apply_bordered_f32(const float2* x, float2* y, double invscale, double2* alpha_dev) {
     chk(trace_dot(p->dev, x, 1, coords, alpha_dev, s));
     BorderArgs b{invscale, alpha_dev, coords};
-    chk(launch_apply_f32(p->dev, (const float*)x, (float*)y, 1, n, b, s));
+    chk(planes_f32.items ? launch_apply_strip<float>(p->dev, planes_f32, (const float*)x, (float*)y, 1, n, b, s)
+                         : launch_apply_f32(p->dev, (const float*)x, (float*)y, 1, n, b, s));
     ++applications;
   }
   // Left preconditioning of the bordered system B = L/s + v t^H.  Stage 0 applies `level`
@@ -623,7 +625,10 @@ int pi_steady_state(pi_plan* plan, double* x_dev, const pi_gmres_opts_t* opts, p
   }
   const int coords = opts->coords;
   Run R(plan, coords);
-  if (opts->precision == PI_FP64) R.planes = planes64(plan, coords);
+  if (opts->precision == PI_FP64)
+    R.planes = planes64(plan, coords);
+  else
+    R.planes_f32 = planes32(plan, coords);
   const long long n = R.n;
   const int m = (int)std::min<long long>(opts->krylovdim, n);
   pi_gmres_info_t loc;
