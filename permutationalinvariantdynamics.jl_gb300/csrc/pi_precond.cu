@@ -35,17 +35,24 @@
 // charge, so y_v, w0 and both corrections stay inside the thread block that sweeps that
 // chain.
 //
-// Device layout: one thread block per charge chain (2 n_max - 1 chains, the longest first),
-// four warps each.  A ring of four shared-memory level slots keeps the sweep fed: warps 1-3
-// copy the factors of level l+3 and gather r at the elements of level l+2 with cp.async
-// (each thread gathers the entries whose indices it copied), while warp 0 solves level l.
-// Warp 0 subtracts the gains from the previous level's solution and runs both Thomas
-// recurrences as warp-wide scans of affine maps (each lane composes a chunk of at most five
-// entries, five shuffle steps combine the lanes), so a level costs a few dozen dependent
-// steps however many sectors it spans.  Population coordinates run in FP32 (the
-// preconditioner is an approximation of L^-1 either way, and every entry is a bounded
-// population); reference coordinates run in FP64, since their entries span many decades at
-// large N.
+// Device layout: one thread block per charge chain (2 n_max - 1 chains, the longest first).  The
+// levels of a chain depend on one another, so the time is the latency of one level on the warp that
+// solves it, and everything that does not depend on the previous level is taken off that warp.  A
+// ring of shared-memory slots holds the levels at hand.  Each stager warp prepares every NS-th level
+// alone: it copies the factors with cp.async, gathers r, replaces r by W s r, and forms the
+// products of Thomas multipliers that the two scans combine with.  The solving warp takes a level
+// when its slot is full, adds the gains of the previous level's solution (premultiplied by -W in
+// the tables), runs both Thomas recurrences as warp-wide scans of affine maps (each lane composes a
+// chunk of at most five entries; FP32 scans step by factors of four) and leaves the solution in
+// the slot, from where the stager that takes the slot next writes it to z.  Full and done
+// mbarriers order the warps; nothing waits for a whole block.  N = 200, FP32, per sweep of
+// FP64 vectors: 235 us with block barriers and the store of z and the products on the solving
+// warp, 160 us now; FP64 sweeps in reference coordinates 1188 us, now 818.  A level of 101 entries
+// takes about 1300 cycles: gains 400, forward and backward scan 270 each, the rest waits and
+// arrivals.  Loading the next level's entries into registers during the backward scan costs more
+// (spills, or fewer stagers: 213 us).  Population coordinates run in FP32 (the preconditioner is an
+// approximation of L^-1 either way, and every entry is a bounded population); reference coordinates
+// run in FP64, since their entries span many decades at large N.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -69,7 +76,6 @@ namespace picuda {
 
 namespace {
 
-constexpr int kSweepThreads = 128;
 constexpr int kNoGain = 1023;
 
 template <typename T>
@@ -148,22 +154,26 @@ __device__ __forceinline__ double2 block_sum2(double2 v, double* red) {
   return out;
 }
 
-constexpr int kStagers = kSweepThreads - 32;  // warps 1.. stage levels ahead of warp 0
-static_assert(kPrecondMaxLevel <= 5 * 32, "warp 0 solves levels of at most five entries per lane");
-// Depth of the level ring: the factors of level k + DF and the gather of r at level k + DG are
-// issued while level k is solved, so copies have DF - DG and gathers DG - 1 levels of time to
-// land.  FP32 sweeps keep six slots (about 70 KB of shared memory, three blocks per SM);
-// FP64 sweeps keep four to stay at two blocks per SM.
+static_assert(kPrecondMaxLevel <= 5 * 32, "the solving warp takes levels of at most five entries per lane");
+// Stager warps, slots and scan coefficients per direction.  A stager has NS levels of time for one
+// of its own, and starts it when the level SLOTS - 1 before it is solved.  A staged FP32 level costs
+// several times the latency of a solved one (two dependent copies, then the products): N = 200
+// takes 192 us with three stagers and six slots, 195 with four and five, 163 with four and six, 160
+// with five and seven, 173 with seven and eight.  An FP64 level is bound by its sub-partition's FP64
+// pipe on either side, and three stagers have a sub-partition each.  Both rings leave room for two
+// blocks per SM.
 template <typename T>
 struct Ring;
 template <>
 struct Ring<float> {
-  static constexpr int DF = 5, DG = 3;
+  static constexpr int NS = 5, SLOTS = 7, COEFS = 7;
 };
 template <>
 struct Ring<double> {
-  static constexpr int DF = 3, DG = 2;
+  static constexpr int NS = 3, SLOTS = 5, COEFS = 5;
 };
+template <typename T>
+constexpr int kSweepThreads = 32 * (1 + Ring<T>::NS);
 constexpr int kMaxChainLevels = 2 * kPrecondMaxLevel + 4;
 
 __device__ __forceinline__ float2 shfl_up_c(float2 v, int d) {
@@ -194,51 +204,116 @@ __device__ __forceinline__ void cpa_wait() {
   asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory");
 }
 
-// One staged level: r at the level's elements (as stored) and the level's factors and gain
-// tables.
 // Slot position of entry i of a level with K = ceil(cnt / 32) entries per lane: lane l's q-th
-// entry (i = l K + q) sits at q * 32 + l, so warp 0's accesses of one q are bank-conflict free.
+// entry (i = l K + q) sits at q * 32 + l, so the solving warp's accesses of one q are bank-conflict free.
 __device__ __forceinline__ int slot_pos(int i, int K) { return (i % K) * 32 + i / K; }
+__device__ __forceinline__ int level_width(int cnt) { return max((cnt + 31) >> 5, 1); }
 
+// One staged level: its right-hand side, factors and gain tables.
 template <typename T, typename TI>
 struct Slot {
   using T2 = typename V2<T>::type;
-  TI rv[kPrecondMaxLevel];    // r at the level's elements
-  T2 w[kPrecondMaxLevel];     // 1 / pivot
-  T2 a[kPrecondMaxLevel];     // forward multiplier
-  T2 c[kPrecondMaxLevel];     // backward multiplier
-  T2 g[3][kPrecondMaxLevel];  // gain coefficients
-  int gp[kPrecondMaxLevel];   // packed gain positions in the previous level
-  int el[kPrecondMaxLevel];   // element index
+  union {
+    TI r[kPrecondMaxLevel];  // r at the level's elements, as stored
+    T2 b[kPrecondMaxLevel];  // then W s r, then the solution
+  };
+  union {
+    T2 w[kPrecondMaxLevel];           // 1 / pivot
+    T2 pf[32 * Ring<T>::COEFS];       // then the forward scan's coefficients
+  };
+  T2 pb[32 * Ring<T>::COEFS];  // the backward scan's coefficients
+  T2 a[kPrecondMaxLevel];      // forward multiplier
+  T2 c[kPrecondMaxLevel];      // backward multiplier
+  T2 g[3][kPrecondMaxLevel];   // gain coefficients times -W
+  int gp[kPrecondMaxLevel];    // packed gain positions in the previous level
+  int el[kPrecondMaxLevel];    // element index
 };
 
 template <typename T, typename TI>
 struct SweepSmem {
   using T2 = typename V2<T>::type;
-  static constexpr int kSlots = Ring<T>::DF + 1;
+  static constexpr int kSlots = Ring<T>::SLOTS;
   Slot<T, TI> slot[kSlots];
-  T2 u[2][kPrecondMaxLevel];     // solution of the previous / current level
-  T2 b[kPrecondMaxLevel];        // W_i (s r_i - gains), slot order
+  unsigned long long full[kSlots], done[kSlots];  // mbarriers
+  double red[2 * (1 + Ring<T>::NS)];
+  T2 none;                       // the first level's previous solution: a finite zero
   int lev_ent[kMaxChainLevels];  // the chain's level bounds
-  double red[2 * (kSweepThreads / 32)];
+  int gave_up;
 };
 
-// Stager thread t copies the factors of entries t, t + kStagers, ... of chain level k into
-// its slot with cp.async (one commit group per call, empty past the chain's end).
+// One direction's affine maps compose from lane to lane as (P, Q)_l <- (P, Q)_l o (P, Q)_{l-D}
+// (forward, UP) or l + D.  A step of N neighbours at distances D, 2D .. N D uses the coefficients
+// out[j] = P_l P_{l-D} .. P_{l-jD}, zero where the neighbour does not exist; P becomes the product
+// over the window of N + 1.
+template <bool UP, int D, int N, typename T2>
+__device__ __forceinline__ void coef_step(T2& P, T2* out, int lane) {
+  const int room = UP ? lane : 31 - lane;  // lanes on the side that is read
+  T2 c = P;
+#pragma unroll
+  for (int j = 0; j < N; ++j) {
+    if (j > 0) c = cmul(c, UP ? shfl_up_c(P, j * D) : shfl_down_c(P, j * D));
+    T2 v = c;
+    if (room < (j + 1) * D) v.x = v.y = 0;
+    out[32 * j + lane] = v;
+  }
+  if (D * (N + 1) < 32) P = cmul(c, UP ? shfl_up_c(P, N * D) : shfl_down_c(P, N * D));
+}
+// The matching step on the constant parts.  A lane without that neighbour reads its own value and a
+// zero coefficient.
+template <bool UP, int D, int N, typename T2>
+__device__ __forceinline__ void scan_step(T2& Q, const T2* coef, int lane) {
+  T2 q[N];
+#pragma unroll
+  for (int j = 0; j < N; ++j) q[j] = UP ? shfl_up_c(Q, (j + 1) * D) : shfl_down_c(Q, (j + 1) * D);
+#pragma unroll
+  for (int j = 0; j < N; ++j) Q = cfma(coef[32 * j + lane], q[j], Q);
+}
+// FP32: two steps by four and one by two (latency counts); FP64: five steps by two (each FP64
+// instruction of a warp holds the pipe for 64 cycles, so their number counts).
+template <bool UP>
+__device__ __forceinline__ void scan_coefs(float2 P, float2* out, int lane) {
+  coef_step<UP, 1, 3>(P, out, lane);
+  coef_step<UP, 4, 3>(P, out + 96, lane);
+  coef_step<UP, 16, 1>(P, out + 192, lane);
+}
+template <bool UP>
+__device__ __forceinline__ void scan(float2& Q, const float2* coef, int lane) {
+  scan_step<UP, 1, 3>(Q, coef, lane);
+  scan_step<UP, 4, 3>(Q, coef + 96, lane);
+  scan_step<UP, 16, 1>(Q, coef + 192, lane);
+}
+template <bool UP>
+__device__ __forceinline__ void scan_coefs(double2 P, double2* out, int lane) {
+  coef_step<UP, 1, 1>(P, out, lane);
+  coef_step<UP, 2, 1>(P, out + 32, lane);
+  coef_step<UP, 4, 1>(P, out + 64, lane);
+  coef_step<UP, 8, 1>(P, out + 96, lane);
+  coef_step<UP, 16, 1>(P, out + 128, lane);
+}
+template <bool UP>
+__device__ __forceinline__ void scan(double2& Q, const double2* coef, int lane) {
+  scan_step<UP, 1, 1>(Q, coef, lane);
+  scan_step<UP, 2, 1>(Q, coef + 32, lane);
+  scan_step<UP, 4, 1>(Q, coef + 64, lane);
+  scan_step<UP, 8, 1>(Q, coef + 96, lane);
+  scan_step<UP, 16, 1>(Q, coef + 128, lane);
+}
+
+// One stager warp prepares a level of cnt entries from e0 in slot L; entries past the level up to
+// the K-th of lane 31 become zeros, so that the solving warp needs no bounds.
 template <typename T, typename TI>
-__device__ __forceinline__ void issue_factors(const PrecondDev& P, SweepSmem<T, TI>& S, int k, int nlev, int t) {
+__device__ __forceinline__ void stage_level(const PrecondDev& P, Slot<T, TI>& L, const TI* __restrict__ r, int e0,
+                                            int cnt, T s, int lane) {
   using T2 = typename V2<T>::type;
-  if (k >= 0 && k < nlev) {
-    Slot<T, TI>& L = S.slot[k % SweepSmem<T, TI>::kSlots];
-    const T2* W = reinterpret_cast<const T2*>(P.W);
-    const T2* A = reinterpret_cast<const T2*>(P.A);
-    const T2* C = reinterpret_cast<const T2*>(P.C);
-    const T2* G = reinterpret_cast<const T2*>(P.G);
-    const int e0 = S.lev_ent[k], cnt = S.lev_ent[k + 1] - e0;
-    const int K = (cnt + 31) >> 5;
-    for (int i = t; i < cnt; i += kStagers) {
-      const int e = e0 + i;
-      const int p = slot_pos(i, K);
+  const T2* W = reinterpret_cast<const T2*>(P.W);
+  const T2* A = reinterpret_cast<const T2*>(P.A);
+  const T2* C = reinterpret_cast<const T2*>(P.C);
+  const T2* G = reinterpret_cast<const T2*>(P.G);
+  const T2 zero = V2<T>::make((T)0, (T)0);
+  const int K = level_width(cnt);
+  for (int i = lane; i < 32 * K; i += 32) {
+    const int p = slot_pos(i, K), e = e0 + i;
+    if (i < cnt) {
       cpa(&L.el[p], P.elem + e, 4);
       cpa(&L.gp[p], P.gsrc + e, 4);
       cpa(&L.w[p], W + e, sizeof(T2));
@@ -246,171 +321,175 @@ __device__ __forceinline__ void issue_factors(const PrecondDev& P, SweepSmem<T, 
       cpa(&L.c[p], C + e, sizeof(T2));
 #pragma unroll
       for (int q = 0; q < 3; ++q) cpa(&L.g[q][p], G + 3LL * e + q, sizeof(T2));
+    } else {
+      L.gp[p] = 0;
+      L.w[p] = L.a[p] = L.c[p] = L.g[0][p] = L.g[1][p] = L.g[2][p] = zero;
     }
   }
   cpa_commit();
-}
-
-// The same stager thread gathers r at the elements whose indices it copied, with cp.async.
-template <typename T, typename TI>
-__device__ __forceinline__ void issue_gather(const TI* __restrict__ r, SweepSmem<T, TI>& S, int k, int nlev, int t) {
-  if (k >= 0 && k < nlev) {
-    Slot<T, TI>& L = S.slot[k % SweepSmem<T, TI>::kSlots];
-    const int cnt = S.lev_ent[k + 1] - S.lev_ent[k];
-    const int K = (cnt + 31) >> 5;
-    for (int i = t; i < cnt; i += kStagers) {
-      const int p = slot_pos(i, K);
-      cpa(&L.rv[p], r + L.el[p], sizeof(TI));
-    }
+  cpa_wait<0>();
+  for (int i = lane; i < cnt; i += 32) {  // the elements whose indices this lane copied
+    const int p = slot_pos(i, K);
+    cpa(&L.r[p], r + L.el[p], sizeof(TI));
   }
   cpa_commit();
-}
-
-// Right-hand sides of one level, all warps: b_i = W_i (s r_i - sum of the gains from the
-// previous level's solution), at slot positions.  Absent gains read slot 0 with a zero
-// coefficient; the thread that meets the free entry keeps its unscaled residual.
-template <typename T, typename TI>
-__device__ __forceinline__ void level_rhs(const PrecondDev& Pd, const Slot<T, TI>& L,
-                                          const typename V2<T>::type* __restrict__ uprev,
-                                          typename V2<T>::type* __restrict__ b, int e0, int cnt, T sT, int tid,
-                                          double2& rho_r, bool& has_rho) {
-  using T2 = typename V2<T>::type;
-  const int K = (cnt + 31) >> 5;
-  for (int p = tid; p < 32 * K; p += kSweepThreads) {
-    const int i = (p & 31) * K + (p >> 5);  // entry of slot p
-    if (i >= cnt) continue;
-    const TI x = L.rv[p];
-    T2 rv = V2<T>::make(sT * (T)x.x, sT * (T)x.y);
-    const int packed = L.gp[p];
+  // meanwhile the chunk products; A and C of a lane were copied by others
+  __syncwarp();
+  T2 PA = L.a[lane], PC = L.c[lane];
+  for (int q = 1; q < K; ++q) {
+    PA = cmul(PA, L.a[q * 32 + lane]);
+    PC = cmul(PC, L.c[q * 32 + lane]);
+  }
+  scan_coefs<false>(PC, L.pb, lane);
+  cpa_wait<0>();
+  __syncwarp();
+  // W s r in place: all of r and W is read before the first write
+  T2 v[5];
 #pragma unroll
-    for (int g3 = 0; g3 < 3; ++g3) {
-      int pos = (packed >> (10 * g3)) & 1023;  // slot position in the previous level
-      pos = pos == kNoGain ? 0 : pos;          // an absent gain has a zero coefficient
-      const T2 g = L.g[g3][p];
-      T2 m;
-      m.x = -g.x;
-      m.y = -g.y;
-      rv = cfma(m, uprev[pos], rv);
+  for (int q = 0; q < 5; ++q) {
+    if (q >= K) break;
+    const int p = q * 32 + lane, i = lane * K + q;
+    if (i < cnt) {
+      const TI x = L.r[p];
+      v[q] = V2<T>::make(s * (T)x.x, s * (T)x.y);
+      if (e0 + i != P.free_ent) v[q] = cmul(L.w[p], v[q]);  // the free entry keeps s r for its residual
+    } else {
+      v[q] = zero;
     }
-    const bool hit = e0 + i == Pd.free_ent;
-    rho_r.x = hit ? (double)rv.x : rho_r.x;
-    rho_r.y = hit ? (double)rv.y : rho_r.y;
-    has_rho = has_rho || hit;
-    b[p] = cmul(L.w[p], rv);
+  }
+  __syncwarp();
+#pragma unroll
+  for (int q = 0; q < 5; ++q)
+    if (q < K) L.b[q * 32 + lane] = v[q];
+  scan_coefs<true>(PA, L.pf, lane);
+}
+
+// t^H z over the entries a thread has written: FP64 with the weights t, or, in population
+// coordinates, where t is one, in double-float.
+struct TraceSum64 {
+  double2 s = make_double2(0.0, 0.0);
+  __device__ __forceinline__ void add(const PrecondDev& P, int e, double2 u) {
+    const double t = P.t0[e - P.chain0_ent];
+    s.x = fma(t, u.x, s.x);
+    s.y = fma(t, u.y, s.y);
+  }
+  __device__ __forceinline__ double2 value() const { return s; }
+};
+struct TraceSumDF {
+  DF x{0.f, 0.f}, y{0.f, 0.f};
+  __device__ __forceinline__ void add(const PrecondDev&, int, float2 u) {
+    df_add(x, u.x);
+    df_add(y, u.y);
+  }
+  __device__ __forceinline__ double2 value() const {
+    return make_double2((double)x.hi + (double)x.lo, (double)y.hi + (double)y.lo);
+  }
+};
+
+// The solution of a level goes from its slot to z, and into the sum t^H z where that is wanted.
+template <typename T, typename TI, typename TO, typename Sum>
+__device__ __forceinline__ void drain_level(const PrecondDev& P, const Slot<T, TI>& L, TO* __restrict__ z, int e0,
+                                            int cnt, bool sum_t, int lane, Sum& sum) {
+  const int K = level_width(cnt);
+  for (int i = lane; i < cnt; i += 32) {
+    const int p = slot_pos(i, K);
+    store_as<TO, typename V2<T>::type>(z + L.el[p], L.b[p]);
+    if (sum_t) sum.add(P, e0 + i, L.b[p]);
   }
 }
 
-// Warp 0's solve of one level of cnt entries, K = ceil(cnt / 32) of them per lane.  Lane l
-// owns the K consecutive entries l K .. l K + K - 1 (slots q 32 + l).  Both Thomas
-// recurrences, y_i = A_i y_{i-1} + b_i and u_i = C_i u_{i+1} + y_i, are affine maps composed
-// over each lane's chunk, combined across lanes by a five-step shuffle scan, then replayed
-// inside the chunk.  Specialised on K so that short levels issue short code.
-template <typename T, typename TI, typename TO, int K>
-__device__ __forceinline__ void solve_level(const PrecondDev& Pd, const Slot<T, TI>& L,
-                                            const typename V2<T>::type* __restrict__ b,
-                                            typename V2<T>::type* __restrict__ ucur, TO* __restrict__ z, int e0,
-                                            int cnt, bool sum_t, int lane, double2& tsum) {
+// ---- mbarriers with bounded waits
+constexpr int kSweepWaitLimit = 1 << 20;  // polls, each of about a microsecond at most
+
+__device__ __forceinline__ unsigned smem_addr(const void* p) { return (unsigned)__cvta_generic_to_shared(p); }
+__device__ __forceinline__ void bar_init(unsigned long long* b, unsigned count) {
+  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_addr(b)), "r"(count) : "memory");
+}
+__device__ __forceinline__ void bar_arrive(unsigned long long* b) {
+  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_addr(b)) : "memory");
+}
+// Waits for the phase with the given parity to complete; false after kSweepWaitLimit polls.
+__device__ __forceinline__ bool bar_wait(unsigned long long* b, unsigned parity) {
+  for (int it = 0; it < kSweepWaitLimit; ++it) {
+    unsigned done;
+    asm volatile(
+        "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n selp.u32 %0, 1, 0, p;\n}\n"
+        : "=r"(done)
+        : "r"(smem_addr(b)), "r"(parity), "r"(1000)  // ns
+        : "memory");
+    if (done) return true;
+  }
+  return false;
+}
+
+// The solve of one staged level, K = ceil(cnt / 32) entries per lane.  Lane l owns the K
+// consecutive entries l K .. l K + K - 1 (positions q 32 + l).  Right-hand sides b_i = W_i (s r_i
+// - gains of the previous level's solution); the lane that meets the free entry keeps its unscaled
+// residual.  Both Thomas recurrences, y_i = A_i y_{i-1} + b_i and u_i = C_i u_{i+1} + y_i, are
+// affine maps composed over each lane's chunk, combined across lanes by a scan, then
+// replayed inside the chunk.  Specialised on K so that short levels issue short code.
+template <typename T, typename TI, int K>
+__device__ __forceinline__ void solve_level(const PrecondDev& Pd, Slot<T, TI>& L, const typename V2<T>::type* uprev,
+                                            int e0, int cnt, int lane, double2& rho_r, bool& has_rho) {
   using T2 = typename V2<T>::type;
-  const int i0 = lane * K;
-  T2 Bv[K], Av[K], Cv[K];
-  bool ok[K];
-  const T2 one = V2<T>::make((T)1, (T)0), zero = V2<T>::make((T)0, (T)0);
+  const T2 zero = V2<T>::make((T)0, (T)0);
+  // the chunk index of the free entry; a level's padding has the next level's entry numbers
+  const int free_q = Pd.free_ent - e0 < cnt ? Pd.free_ent - e0 - lane * K : -1;
+  T2 B[K], A[K], C[K];
 #pragma unroll
   for (int q = 0; q < K; ++q) {
-    ok[q] = i0 + q < cnt;
     const int p = q * 32 + lane;
-    const T2 bb = b[p], a = L.a[p], c = L.c[p];
-    Bv[q] = ok[q] ? bb : zero;
-    Av[q] = ok[q] ? a : zero;
-    Cv[q] = ok[q] ? c : zero;
-  }
-  // the lane's forward map y_out = P y_in + Q
-  T2 P = one, Q = zero;
-#pragma unroll
-  for (int q = 0; q < K; ++q) {
-    const T2 Pq = cmul(Av[q], P), Qq = cfma(Av[q], Q, Bv[q]);
-    P = ok[q] ? Pq : P;
-    Q = ok[q] ? Qq : Q;
-  }
-  // inclusive scan in lane order: (P, Q) <- (P, Q) o (P_prev, Q_prev)
-#pragma unroll
-  for (int d = 1; d < 32; d <<= 1) {
-    const T2 Pn = shfl_up_c(P, d), Qn = shfl_up_c(Q, d);
-    if (lane >= d) {
-      Q = cfma(P, Qn, Q);
-      P = cmul(P, Pn);
+    const int packed = L.gp[p];  // an absent gain reads entry 0 with a zero coefficient
+    T2 b = cfma(L.g[0][p], uprev[packed & 1023], L.b[p]);
+    b = cfma(L.g[1][p], uprev[(packed >> 10) & 1023], b);
+    B[q] = cfma(L.g[2][p], uprev[packed >> 20], b);
+    A[q] = L.a[p];
+    C[q] = L.c[p];
+    if (q == free_q) {
+      rho_r = make_double2((double)B[q].x, (double)B[q].y);
+      has_rho = true;
+      B[q] = zero;
     }
   }
+  T2 Q = B[0];
+#pragma unroll
+  for (int q = 1; q < K; ++q) Q = cfma(A[q], Q, B[q]);
+  scan<true>(Q, L.pf, lane);
   T2 y = shfl_up_c(Q, 1);
   if (lane == 0) y = zero;
 #pragma unroll
   for (int q = 0; q < K; ++q) {
-    y = cfma(Av[q], y, Bv[q]);  // Av = Bv = 0 past the level: harmless zeros
-    Bv[q] = y;                  // Bv now holds y_i
+    y = cfma(A[q], y, B[q]);
+    B[q] = y;
   }
-  // the lane's backward map u_in = P2 u_next + Q2 over its entries of the level
-  T2 P2 = one, Q2 = zero;
+  Q = B[K - 1];
+#pragma unroll
+  for (int q = K - 2; q >= 0; --q) Q = cfma(C[q], Q, B[q]);
+  scan<false>(Q, L.pb, lane);
+  T2 u = shfl_down_c(Q, 1);
+  if (lane == 31) u = zero;
 #pragma unroll
   for (int q = K - 1; q >= 0; --q) {
-    const T2 Pq = cmul(Cv[q], P2), Qq = cfma(Cv[q], Q2, Bv[q]);
-    P2 = ok[q] ? Pq : P2;
-    Q2 = ok[q] ? Qq : Q2;
-  }
-  // suffix scan in reverse lane order
-#pragma unroll
-  for (int d = 1; d < 32; d <<= 1) {
-    const T2 Pn = shfl_down_c(P2, d), Qn = shfl_down_c(Q2, d);
-    if (lane + d < 32) {
-      Q2 = cfma(P2, Qn, Q2);
-      P2 = cmul(P2, Pn);
-    }
-  }
-  T2 uv = shfl_down_c(Q2, 1);
-  if (lane == 31) uv = zero;
-  T2 U[K];
-#pragma unroll
-  for (int q = K - 1; q >= 0; --q) {
-    uv = cfma(Cv[q], uv, Bv[q]);
-    U[q] = uv;
-  }
-#pragma unroll
-  for (int q = 0; q < K; ++q) {
-    if (ok[q]) {
-      ucur[q * 32 + lane] = U[q];
-      store_as<TO, T2>(z + L.el[q * 32 + lane], U[q]);
-    }
-  }
-  if (sum_t) {
-#pragma unroll
-    for (int q = 0; q < K; ++q) {
-      if (ok[q]) {
-        const double t = Pd.t0[e0 + i0 + q - Pd.chain0_ent];
-        tsum.x = fma(t, (double)U[q].x, tsum.x);
-        tsum.y = fma(t, (double)U[q].y, tsum.y);
-      }
-    }
+    u = cfma(C[q], u, B[q]);
+    L.b[q * 32 + lane] = u;
   }
 }
 
-// The d = 0 chain's correction z -= k w0 at entries c0 .. c1 and this thread's share of t^H z
-// after it.  One block does it for the whole chain (10,201 entries at N = 200), so eight entries
-// per thread are in flight together: one by one, their two dependent gathers and the FP64
-// arithmetic took a third of the sweep.
+// The d = 0 chain's correction z -= k w0 at entries c0 .. c1.  One block does it for the whole
+// chain (10,201 entries at N = 200), so eight entries per thread are in flight together: one by
+// one, their two dependent gathers took a third of the sweep.
 constexpr int kTailUnroll = 8;
 
 template <typename TO>
-__device__ __forceinline__ double2 chain0_correct(const PrecondDev& Pd, TO* z, int c0, int c1, double2 k) {
-  double2 tsum = make_double2(0.0, 0.0);
-  for (int e0 = c0 + threadIdx.x; e0 < c1; e0 += kTailUnroll * kSweepThreads) {
+__device__ __forceinline__ void chain0_correct(const PrecondDev& Pd, TO* z, int c0, int c1, double2 k) {
+  for (int e0 = c0 + threadIdx.x; e0 < c1; e0 += kTailUnroll * blockDim.x) {
     int el[kTailUnroll];
     double2 w[kTailUnroll], v[kTailUnroll];
-    double t[kTailUnroll];
 #pragma unroll
     for (int q = 0; q < kTailUnroll; ++q) {
-      const int e = e0 + q * kSweepThreads;
+      const int e = e0 + q * blockDim.x;
       el[q] = e < c1 ? Pd.elem[e] : -1;
       w[q] = e < c1 ? Pd.w0[e - c0] : make_double2(0.0, 0.0);
-      t[q] = e < c1 ? Pd.t0[e - c0] : 0.0;
     }
 #pragma unroll
     for (int q = 0; q < kTailUnroll; ++q) v[q] = el[q] >= 0 ? load_d2(z + el[q]) : make_double2(0.0, 0.0);
@@ -420,25 +499,21 @@ __device__ __forceinline__ double2 chain0_correct(const PrecondDev& Pd, TO* z, i
       v[q].x = fma(-k.x, w[q].x, fma(k.y, w[q].y, v[q].x));
       v[q].y = fma(-k.x, w[q].y, fma(-k.y, w[q].x, v[q].y));
       store_as<TO, double2>(z + el[q], v[q]);
-      tsum.x = fma(t[q], v[q].x, tsum.x);
-      tsum.y = fma(t[q], v[q].y, tsum.y);
     }
   }
-  return tsum;
 }
 
-// The same for FP32 vectors in population coordinates, where t is one: in double-float, as each
-// conversion and FP64 operation of a warp holds a quarter of the SM's FP64 pipe for 64 cycles.
-__device__ __forceinline__ double2 chain0_correct_df(const PrecondDev& Pd, float2* z, int c0, int c1, double2 k) {
+// The same for FP32 vectors: in double-float, as each conversion and FP64 operation of a warp
+// holds a quarter of the SM's FP64 pipe for 64 cycles.
+__device__ __forceinline__ void chain0_correct_df(const PrecondDev& Pd, float2* z, int c0, int c1, double2 k) {
   const DF kx{(float)k.x, (float)(k.x - (double)(float)k.x)}, ky{(float)k.y, (float)(k.y - (double)(float)k.y)};
-  DF sx{0.f, 0.f}, sy{0.f, 0.f};
-  for (int e0 = c0 + threadIdx.x; e0 < c1; e0 += kTailUnroll * kSweepThreads) {
+  for (int e0 = c0 + threadIdx.x; e0 < c1; e0 += kTailUnroll * blockDim.x) {
     int el[kTailUnroll];
     float4 w[kTailUnroll];
     float2 v[kTailUnroll];
 #pragma unroll
     for (int q = 0; q < kTailUnroll; ++q) {
-      const int e = e0 + q * kSweepThreads;
+      const int e = e0 + q * blockDim.x;
       el[q] = e < c1 ? Pd.elem[e] : -1;
       w[q] = e < c1 ? Pd.w0f[e - c0] : make_float4(0.f, 0.f, 0.f, 0.f);
     }
@@ -456,15 +531,12 @@ __device__ __forceinline__ double2 chain0_correct_df(const PrecondDev& Pd, float
       df_axpy(zy, -ky.hi, -ky.lo, w[q].x);
       zy.lo = fmaf(-kx.hi, w[q].w, fmaf(-ky.hi, w[q].y, zy.lo));
       z[el[q]] = make_float2(zx.hi + zx.lo, zy.hi + zy.lo);
-      sx = df_sum(sx, zx);
-      sy = df_sum(sy, zy);
     }
   }
-  return make_double2((double)sx.hi + (double)sx.lo, (double)sy.hi + (double)sy.lo);
 }
 
 template <typename T, typename TI, typename TO>
-__global__ void __launch_bounds__(kSweepThreads)
+__global__ void __launch_bounds__(kSweepThreads<T>, 2)
     k_level_sweep(const PrecondDev Pd, const TI* __restrict__ r, TO* __restrict__ z, double s) {
   using T2 = typename V2<T>::type;
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -474,85 +546,97 @@ __global__ void __launch_bounds__(kSweepThreads)
   const int nlev = lev1 - lev0;
   const bool chain0 = chain == Pd.chain0;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int st = tid - 32;  // stager index
+  constexpr int kSlots = Ring<T>::SLOTS, NS = Ring<T>::NS;
   for (int k = tid; k <= nlev; k += blockDim.x) S.lev_ent[k] = Pd.lev_ent[lev0 + k];
-  for (int i = tid; i < 2 * kPrecondMaxLevel; i += blockDim.x)  // absent gains read finite zeros
-    S.u[i / kPrecondMaxLevel][i % kPrecondMaxLevel] = V2<T>::make((T)0, (T)0);
+  if (tid < kSlots) {
+    bar_init(&S.full[tid], 1);
+    bar_init(&S.done[tid], 1);
+  }
+  if (tid == 0) {
+    S.none = V2<T>::make((T)0, (T)0);
+    S.gave_up = 0;
+  }
   __syncthreads();
-  // Level j's step issues the factors of j + DF, waits until this thread's factors of j + DG
-  // and gather of j + 1 have landed (after the gather of j + 1 it has committed 2 DG - 3
-  // groups, after the factors of j + DG 2 (DF - DG)), and issues the gather of j + DG; steps
-  // j < 0 fill the ring before warp 0 starts (empty groups keep the commit counts uniform).
-  constexpr int DF = Ring<T>::DF, DG = Ring<T>::DG;
   double2 tsum = make_double2(0.0, 0.0);
   double2 rho_r = make_double2(0.0, 0.0);  // residual of the dropped free equation (lane-held)
   bool has_rho = false;
-  int prev = 0, cur = 1;
-  const T sT = (T)s;
-  for (int k = -DF; k < nlev; ++k) {
-    const Slot<T, TI>& L = S.slot[(k + SweepSmem<T, TI>::kSlots) % SweepSmem<T, TI>::kSlots];
-    const int e0 = k >= 0 ? S.lev_ent[k] : 0;
-    const int cnt = k >= 0 ? S.lev_ent[k + 1] - e0 : 0;
-    if (k >= 0) {
-      level_rhs<T, TI>(Pd, L, S.u[prev], S.b, e0, cnt, sT, tid, rho_r, has_rho);
-      __syncthreads();
-    }
-    if (warp > 0) {
-      issue_factors<T, TI>(Pd, S, k + DF, nlev, st);
-      cpa_wait<(2 * DG - 3 < 2 * (DF - DG) ? 2 * DG - 3 : 2 * (DF - DG))>();
-      issue_gather<T, TI>(r, S, k + DG, nlev, st);
-    } else if (k >= 0) {
-      const bool sum_t = chain0 && Pd.mode == 1;
-      switch ((cnt + 31) >> 5) {
-        case 1: solve_level<T, TI, TO, 1>(Pd, L, S.b, S.u[cur], z, e0, cnt, sum_t, lane, tsum); break;
-        case 2: solve_level<T, TI, TO, 2>(Pd, L, S.b, S.u[cur], z, e0, cnt, sum_t, lane, tsum); break;
-        case 3: solve_level<T, TI, TO, 3>(Pd, L, S.b, S.u[cur], z, e0, cnt, sum_t, lane, tsum); break;
-        case 4: solve_level<T, TI, TO, 4>(Pd, L, S.b, S.u[cur], z, e0, cnt, sum_t, lane, tsum); break;
-        default: solve_level<T, TI, TO, 5>(Pd, L, S.b, S.u[cur], z, e0, cnt, sum_t, lane, tsum); break;
+  if (warp > 0) {
+    const T sT = (T)s;
+    typename std::conditional<std::is_same<T, float>::value, TraceSumDF, TraceSum64>::type sum;
+    for (int k = warp - 1; k < nlev + kSlots; k += NS) {
+      // level k takes the slot of level k - kSlots, whose solution level k - kSlots + 1 has read
+      const int out = k - kSlots;
+      if (out >= 0) {
+        const int by = min(out + 1, nlev - 1);
+        if (!bar_wait(&S.done[by % kSlots], (unsigned)(by / kSlots) & 1u)) {
+          S.gave_up = 1;
+          break;
+        }
+        const int e0 = S.lev_ent[out], cnt = S.lev_ent[out + 1] - e0;
+        drain_level<T, TI, TO>(Pd, S.slot[out % kSlots], z, e0, cnt, chain0, lane, sum);
+        __syncwarp();
+      }
+      if (k < nlev) {
+        stage_level<T, TI>(Pd, S.slot[k % kSlots], r, S.lev_ent[k], S.lev_ent[k + 1] - S.lev_ent[k], sT, lane);
+        __syncwarp();
+        if (lane == 0) bar_arrive(&S.full[k % kSlots]);
       }
     }
-    __syncthreads();
-    if (k >= 0) {
-      prev ^= 1;
-      cur ^= 1;
+    tsum = sum.value();
+  } else {
+    const T2* up = &S.none;
+    for (int k = 0; k < nlev; ++k) {
+      const int e0 = S.lev_ent[k], cnt = S.lev_ent[k + 1] - e0;
+      if (!bar_wait(&S.full[k % kSlots], (unsigned)(k / kSlots) & 1u)) {
+        S.gave_up = 1;
+        break;
+      }
+      Slot<T, TI>& L = S.slot[k % kSlots];
+      switch (level_width(cnt)) {
+        case 1: solve_level<T, TI, 1>(Pd, L, up, e0, cnt, lane, rho_r, has_rho); break;
+        case 2: solve_level<T, TI, 2>(Pd, L, up, e0, cnt, lane, rho_r, has_rho); break;
+        case 3: solve_level<T, TI, 3>(Pd, L, up, e0, cnt, lane, rho_r, has_rho); break;
+        case 4: solve_level<T, TI, 4>(Pd, L, up, e0, cnt, lane, rho_r, has_rho); break;
+        default: solve_level<T, TI, 5>(Pd, L, up, e0, cnt, lane, rho_r, has_rho); break;
+      }
+      up = L.b;
+      __syncwarp();  // the level's solution is in place for every lane
+      if (lane == 0) bar_arrive(&S.done[k % kSlots]);
     }
+  }
+  __syncthreads();
+  if (S.gave_up) {  // a wait ran out: leave no number behind
+    if (tid == 0)
+      store_as<TO, double2>(z + Pd.elem[Pd.lev_ent[lev0]], make_double2(nan(""), nan("")));
+    return;
   }
   if (!chain0) return;
   const int c0 = Pd.chain0_ent, c1 = Pd.lev_ent[lev1];
+  const double2 tz = block_sum2(tsum, S.red);  // t^H y, the free entry apart
+  double2 k;
   if (Pd.mode == 0) {
     // beta = rho_r / rho_v; y = y_r - beta y_v; z_f = (beta - t^H y) / t_f
-    double* rr = S.red;  // the lane that met the free entry hands rho_r over
-    __syncthreads();
-    if (has_rho) {
-      rr[0] = rho_r.x;
-      rr[1] = rho_r.y;
+    if (has_rho) {  // one lane
+      const double2 iv = Pd.sm_coef;  // 1 / rho_v
+      const double2 beta = make_double2(rho_r.x * iv.x - rho_r.y * iv.y, rho_r.x * iv.y + rho_r.y * iv.x);
+      const double2 sv = Pd.free_coef;  // (1 + t^H y_v) / t_f
+      const double it = Pd.free_inv;    // 1 / t_f
+      S.red[0] = beta.x;
+      S.red[1] = beta.y;
+      store_as<TO, double2>(z + Pd.elem[Pd.free_ent],
+                            make_double2(fma(beta.x, sv.x, fma(-beta.y, sv.y, -tz.x * it)),
+                                         fma(beta.x, sv.y, fma(beta.y, sv.x, -tz.y * it))));
     }
     __syncthreads();
-    const double2 rrv = make_double2(rr[0], rr[1]);
-    __syncthreads();
-    const double2 rv = Pd.sm_coef;  // rho_v
-    const double den = rv.x * rv.x + rv.y * rv.y;
-    const double2 beta =
-        make_double2((rrv.x * rv.x + rrv.y * rv.y) / den, (rrv.y * rv.x - rrv.x * rv.y) / den);
-    if constexpr (std::is_same<T, float>::value && std::is_same<TO, float2>::value)
-      tsum = chain0_correct_df(Pd, z, c0, c1, beta);
-    else
-      tsum = chain0_correct(Pd, z, c0, c1, beta);
-    const double2 tz = block_sum2(tsum, S.red);
-    if (tid == 0 && Pd.free_ent >= 0) {
-      const double t = Pd.t0[Pd.free_ent - c0];
-      store_as<TO, double2>(z + Pd.elem[Pd.free_ent], make_double2((beta.x - tz.x) / t, (beta.y - tz.y) / t));
-    }
+    k = make_double2(S.red[0], S.red[1]);
   } else {
     // Sherman-Morrison: z -= w0 (t^H y) / (1 + t^H w0)
-    const double2 tz = block_sum2(tsum, S.red);
-    const double2 kk =
-        make_double2(tz.x * Pd.sm_coef.x - tz.y * Pd.sm_coef.y, tz.x * Pd.sm_coef.y + tz.y * Pd.sm_coef.x);
-    if constexpr (std::is_same<T, float>::value && std::is_same<TO, float2>::value)
-      (void)chain0_correct_df(Pd, z, c0, c1, kk);
-    else
-      (void)chain0_correct(Pd, z, c0, c1, kk);
+    k = make_double2(tz.x * Pd.sm_coef.x - tz.y * Pd.sm_coef.y, tz.x * Pd.sm_coef.y + tz.y * Pd.sm_coef.x);
   }
+  if constexpr (std::is_same<T, float>::value && std::is_same<TO, float2>::value)
+    chain0_correct_df(Pd, z, c0, c1, k);
+  else
+    chain0_correct(Pd, z, c0, c1, k);
 }
 
 template <typename T, typename TI, typename TO>
@@ -569,7 +653,7 @@ cudaError_t launch_sweep(const PrecondDev& D, int blocks, const void* r, void* z
     if (e != cudaSuccess) return e;
     configured.fetch_or(bit);
   }
-  k_level_sweep<T, TI, TO><<<blocks, kSweepThreads, smem, stream>>>(D, (const TI*)r, (TO*)z, scale);
+  k_level_sweep<T, TI, TO><<<blocks, kSweepThreads<T>, smem, stream>>>(D, (const TI*)r, (TO*)z, scale);
   return cudaGetLastError();
 }
 
@@ -878,7 +962,12 @@ int upload_factors(pi_precond* P) {
   P->dev.A = p;
   if ((rc = upload_vec(P, conv(H.C), &p))) return rc;
   P->dev.C = p;
-  if ((rc = upload_vec(P, conv(H.G), &p))) return rc;
+  // the gains times -W; the free entry (W = 0) keeps -G for its residual
+  std::vector<cdv> G(H.G.size());
+  for (size_t e = 0; e < H.W.size(); ++e)
+    for (int q = 0; q < 3; ++q)
+      G[3 * e + q] = (long long)e == H.free_ent ? -H.G[3 * e + q] : -H.W[e] * H.G[3 * e + q];
+  if ((rc = upload_vec(P, conv(G), &p))) return rc;
   P->dev.G = p;
   return PI_OK;
 }
@@ -970,7 +1059,7 @@ int pi_precond_create(pi_plan* plan, int coords, double regularization, double o
           int packed = 0;
           for (int q = 0; q < 3; ++q) {
             int pos = (H.gsrc[e] >> (10 * q)) & 1023;
-            if (pos != 1023) pos = (pos % Kp) * 32 + pos / Kp;
+            pos = pos == kNoGain ? 0 : (pos % Kp) * 32 + pos / Kp;  // none: entry 0, coefficient zero
             packed |= pos << (10 * q);
           }
           gslot[e] = packed;
@@ -1004,7 +1093,15 @@ int pi_precond_create(pi_plan* plan, int coords, double regularization, double o
   P->dev.chain0_ent = H.chain0_ent;
   P->dev.free_ent = H.free_ent;
   P->dev.mode = H.mode;
-  P->dev.sm_coef = make_double2(H.sm_coef.real(), H.sm_coef.imag());
+  // mode 0: 1 / rho_v, and z_f = (beta (1 + t^H y_v) - t^H y_r) / t_f
+  const std::complex<double> coef = H.mode == 0 ? 1.0 / H.sm_coef : H.sm_coef;
+  P->dev.sm_coef = make_double2(coef.real(), coef.imag());
+  if (H.mode == 0) {
+    std::complex<double> tv = 1.0;
+    for (size_t i = 0; i < H.w0.size(); ++i) tv += H.t0[i] * H.w0[i];
+    P->dev.free_inv = 1.0 / H.t0[H.free_ent - H.chain0_ent];
+    P->dev.free_coef = make_double2(tv.real() * P->dev.free_inv, tv.imag() * P->dev.free_inv);
+  }
   P->setup_seconds = std::chrono::duration<double>(std::chrono::steady_clock::now() - t0).count();
   *out = P;
   return PI_OK;
