@@ -358,7 +358,12 @@ int rk4_run(pi_plan* plan, double2* rho, int nt, const double* times, int steps,
     StageKernel k[4];
     const Planes64 p64 = mixed ? Planes64{} : planes64(plan, PI_COORDS_REFERENCE);
     chk(stage_kernels(mixed, p64, k));
-    const int gsteps = steps <= 128 ? steps : 64;
+    // A graph of kernel nodes costs about 1.7 us a node to build and instantiate on each call, and a
+    // launch of it some microseconds of the host that run ahead of the device: short graphs
+    // launched more often.  64 steps at N = 120 take 4.79 ms in one graph, 4.34 in graphs of
+    // 8 (4.40 of 16, 4.36 of 2); 1000 steps at N = 20 13.2 ms in graphs of 64, 12.5 of 8, 13.6 of 2.
+    constexpr int kGraphSteps = 8;
+    const int gsteps = std::min(steps, kGraphSteps);
     const int reps = steps / gsteps, rem = steps % gsteps;
     StepGraph main, tail;
     // Only the step size changes between intervals: the graphs read it from hcur.
