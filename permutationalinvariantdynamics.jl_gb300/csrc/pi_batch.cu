@@ -1387,7 +1387,10 @@ __global__ void __launch_bounds__(32) k_step_finish(DevInst* st, int* again) {
 // instructions (64 cycles each per quarter of an SM).
 
 // Grid barrier: arrivals are counted up over the whole launch.  A block that waits in vain
-// raises err, which ends every wait of the launch; the host reads it after the cycle.
+// raises err, which ends every wait of the launch; the host reads it after the cycle.  Without one
+// (bar null) the grid is one cluster and the barrier is the cluster's, in hardware: an interval
+// of N = 8 (seven blocks, 30 steps) takes 0.87 -> 0.73 ms.  Every block leaves the cycle at the
+// same barrier, and a cluster barrier waits for threads that have not exited only.
 struct GridBar {
   unsigned count;
   int err;
@@ -1396,8 +1399,12 @@ constexpr int kGridWaitLimit = 1 << 24;  // polls, several seconds
 
 // Arrival of this block; its writes so far are visible to blocks that wait for it.
 __device__ __forceinline__ void grid_arrive(GridBar* bar, unsigned& target) {
-  __syncthreads();
+  if (bar != nullptr) __syncthreads();
   target += gridDim.x;
+  if (bar == nullptr) {
+    asm volatile("barrier.cluster.arrive.release;" ::: "memory");
+    return;
+  }
   if (gridDim.x > 1 && threadIdx.x == 0) {
     __threadfence();
     atomicAdd(&bar->count, 1u);
@@ -1406,6 +1413,10 @@ __device__ __forceinline__ void grid_arrive(GridBar* bar, unsigned& target) {
 
 // Waits for the arrival of every block; false when the launch has given up.
 __device__ __forceinline__ bool grid_wait(GridBar* bar, unsigned target) {
+  if (bar == nullptr) {
+    asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
+    return true;
+  }
   if (gridDim.x == 1) return true;
   __shared__ int ok;
   if (threadIdx.x == 0) {
@@ -2451,6 +2462,7 @@ void Engine::rebuild() {
   total_strips_ = (int)si.size();
   cycle_kernel_ = canonical && n > 0 && total_elems <= kCycleElems && cycle_max_ > 0 && sm_count_ > 0;
   total_chunks_ = (int)ci.size();
+  plan_cycle();
   reserve(&st_, &st_cap_, sizeof(DevInst) * nn, false);
   reserve(&tile_inst_, &tile_inst_cap_, sizeof(int) * std::max<size_t>(ti.size(), 1), false);
   reserve(&tile_local_, &tile_local_cap_, sizeof(int) * std::max<size_t>(tl.size(), 1), false);
@@ -2663,22 +2675,62 @@ void Engine::arnoldi_step() {
   if (!build_) chk(cudaGetLastError());
 }
 
-// The cycle of a small job set in one cooperative launch: a block more than its longest work
-// list has entries (the finish of a single job), at most what is resident at once.
+// The cycle of a small job set in one launch: a block more than its longest work list has entries
+// (the finish of a single job), at most what is resident at once.  Up to kMaxCluster blocks are a
+// cluster, whose barrier costs less than the grid barrier; larger sets are cooperative launches.
+// Sets that would have to fold onto a cluster lose more than that: N = 14 (22 chunks) takes 6.1 ms
+// as 23 cooperative blocks and 7.1 as a cluster of 16, N = 16 GMRES 15.7 and 19.6.
+static const void* cycle_fn(bool f32) {
+  return f32 ? (const void*)k_cycle<true> : (const void*)k_cycle<false>;
+}
+static cudaLaunchConfig_t cluster_config(int blocks, cudaLaunchAttribute* at) {
+  at->id = cudaLaunchAttributeClusterDimension;
+  at->val.clusterDim.x = blocks;
+  at->val.clusterDim.y = at->val.clusterDim.z = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(blocks);
+  cfg.blockDim = dim3(kRT);
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  return cfg;
+}
+constexpr int kMaxCluster = 16;
+
+void Engine::plan_cycle() {
+  cycle_grid_ = std::max(1, std::min(std::max(total_chunks_, total_strips_) + 1, cycle_max_ * sm_count_));
+  cycle_cluster_ = cycle_kernel_ && cycle_grid_ > 1 && cycle_grid_ <= kMaxCluster;
+  if (!cycle_cluster_) return;
+  cudaLaunchAttribute at{};
+  const cudaLaunchConfig_t cfg = cluster_config(cycle_grid_, &at);
+  int fit = 0;
+  if (cudaFuncSetAttribute(cycle_fn(f32_), cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess ||
+      cudaOccupancyMaxActiveClusters(&fit, cycle_fn(f32_), &cfg) != cudaSuccess) {
+    fit = 0;
+    (void)cudaGetLastError();  // the cooperative launch serves
+  }
+  cycle_cluster_ = fit > 0;
+}
+
 void Engine::launch_cycle() {
   const int n = (int)jobs_.size();
-  const int grid = std::max(1, std::min(std::max(total_chunks_, total_strips_) + 1, cycle_max_ * sm_count_));
+  const int grid = cycle_grid_;
   DevInst* st = (DevInst*)st_;
   const int *ci = (const int*)chunk_inst_, *si = (const int*)strip_inst_, *sl = (const int*)strip_local_;
   const int* nc = (const int*)nchunks_;
   double2* partv = (double2*)partv_;
   double* part = (double*)part1_;
-  GridBar* bar = (GridBar*)bar_;
+  GridBar* bar = cycle_cluster_ ? nullptr : (GridBar*)bar_;
   int nn = n, C = total_chunks_, T = total_strips_, steps = m_, border = any_border_ ? 1 : 0;
-  chk(cudaMemsetAsync(bar, 0, sizeof(GridBar), s_));
+  chk(cudaMemsetAsync(bar_, 0, sizeof(GridBar), s_));
   void* args[] = {&st, &nn, &ci, &C, &si, &sl, &T, &nc, &partv, &part, &steps, &border, &bar};
-  chk(cudaLaunchCooperativeKernel(f32_ ? (const void*)k_cycle<true> : (const void*)k_cycle<false>, dim3(grid),
-                                  dim3(kRT), args, 0, s_));
+  if (cycle_cluster_) {
+    cudaLaunchAttribute at{};
+    cudaLaunchConfig_t cfg = cluster_config(grid, &at);
+    cfg.stream = s_;
+    chk(cudaLaunchKernelExC(&cfg, cycle_fn(f32_), args));
+    return;
+  }
+  chk(cudaLaunchCooperativeKernel(cycle_fn(f32_), dim3(grid), dim3(kRT), args, 0, s_));
 }
 
 void Engine::run_cycle_steps() {

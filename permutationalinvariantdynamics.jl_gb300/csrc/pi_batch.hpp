@@ -353,10 +353,13 @@ class Engine {
   // job-set shape)
   void choose_apply_schedule();
   void launch_step_apply(int schedule);
+  void plan_cycle();
   void launch_cycle();
   int apply_schedule_ = PI_SCHEDULE_PER_TILE;
   bool schedule_chosen_ = false;
   int sm_count_ = 0;
+  int cycle_grid_ = 1;          // blocks of k_cycle
+  bool cycle_cluster_ = false;  // as one cluster
   int cycle_max_ = 0;    // resident blocks per SM of k_cycle
   int persist_max_ = 0;  // resident blocks per SM of the persistent apply (0: unavailable)
 };
