@@ -2733,6 +2733,10 @@ void Engine::launch_cycle() {
   chk(cudaLaunchCooperativeKernel(cycle_fn(f32_), dim3(grid), dim3(kRT), args, 0, s_));
 }
 
+// Steps per graph.  Building and instantiating a graph takes about 1.7 us per node, once per job
+// set, and each step has about ten.
+constexpr int kGraphSteps = 5;
+
 void Engine::run_cycle_steps() {
   // an explicit step-apply schedule asks for the step kernels
   ran_cycle_ = cycle_kernel_ && (!f32_ || g_apply_schedule.load() == PI_SCHEDULE_AUTO);
@@ -2750,7 +2754,7 @@ void Engine::run_cycle_steps() {
     chk(cudaGraphCreate(&build_, 0));
     last_ = nullptr;
     if (build_) {
-      for (int j = 0; j < m_; ++j) arnoldi_step();
+      for (int j = 0; j < std::min(m_, kGraphSteps); ++j) arnoldi_step();
       if (err == cudaSuccess) chk(cudaGraphInstantiate(&graph_, build_, 0));
       cudaGraphDestroy(build_);
     }
@@ -2758,7 +2762,8 @@ void Engine::run_cycle_steps() {
     last_ = nullptr;
     if (err != cudaSuccess) return;
   }
-  chk(cudaGraphLaunch(graph_, s_));
+  for (int j = kGraphSteps; j <= std::max(m_, kGraphSteps); j += kGraphSteps) chk(cudaGraphLaunch(graph_, s_));
+  for (int j = m_ < kGraphSteps ? 0 : m_ % kGraphSteps; j > 0; --j) arnoldi_step();
 }
 
 // f(i) for every job, those in `busy` spread over a few host threads: a cycle's end costs each of
