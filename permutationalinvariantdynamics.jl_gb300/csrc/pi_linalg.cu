@@ -53,19 +53,25 @@ __device__ __forceinline__ double2 load_c(const T2* p) {
 }
 
 // Stage 1 of a multi-dot: block (bx, by) reduces vectors by*8 .. by*8+7 over element chunk
-// bx and writes partial[bx * stride + i].  The columns of a group are counted at compile time
-// (8, then 4, 2, 1): FMAs of absent columns would be issued all the same.  Lane sums exchange
-// halves of the accumulators (16 additions for 8 columns against 80 one by one, which at N = 200
-// took as long as the products); FP32 vectors are summed in double-float until one value per
-// lane is left, as a conversion holds the FP64 pipe like an addition.
+// bx and writes partial[bx * stride + i].  The columns of a group are counted at compile time:
+// FMAs of absent columns would be issued all the same, and a pass per power of two (4, 2, 1)
+// reads w and waits for memory as often.  Lane sums exchange halves of the accumulators (16
+// additions for 8 columns against 80 one by one, which at N = 200 took as long as the products);
+// FP32 vectors are summed in double-float until one value per lane is left, as a conversion holds
+// the FP64 pipe like an addition.  FP32 in 64 registers, so that all 608 blocks are resident at
+// once, and one element at a time: N = 200, 7, 8, 15 and 16 columns 36, 52, 58 and 52 us with
+// passes and 66 registers (three blocks per SM, two rounds), 21, 24, 38 and 34 us now (26 us of
+// memory time for 16); two elements at a time take 24, 33, 56 and 53 us.
 constexpr int kDotGroup = 8;
+__host__ __device__ constexpr int dot_values(int k) { return k > 4 ? 16 : k > 2 ? 8 : 2 * k; }  // a power of two
 
 template <int K>
 __device__ __forceinline__ void dot_cols(const double2* __restrict__ V, long long ldv, const double2* __restrict__ w,
                                          long long beg, long long end, double* row) {
-  double acc[2 * K];
+  constexpr int NV = dot_values(K);
+  double acc[NV];
 #pragma unroll
-  for (int k = 0; k < 2 * K; ++k) acc[k] = 0.0;
+  for (int k = 0; k < NV; ++k) acc[k] = 0.0;
   for (long long e = beg + threadIdx.x; e < end; e += blockDim.x) {
     const double2 wv = __ldg(w + e);
 #pragma unroll
@@ -77,8 +83,8 @@ __device__ __forceinline__ void dot_cols(const double2* __restrict__ V, long lon
       acc[2 * k + 1] = fma(-v.y, wv.x, acc[2 * k + 1]);
     }
   }
-  warp_transpose_sum<2 * K>(acc);
-  constexpr int span = 32 / (2 * K);
+  warp_transpose_sum<NV>(acc);
+  constexpr int span = 32 / NV;
   const int lane = threadIdx.x & 31;
   if (lane % span == 0) row[lane / span] = acc[0];
 }
@@ -87,10 +93,11 @@ __device__ __forceinline__ void dot_cols(const double2* __restrict__ V, long lon
 template <int K>
 __device__ __forceinline__ void dot_cols(const float2* __restrict__ V, long long ldv, const float2* __restrict__ w,
                                          long long beg, long long end, double* row) {
-  DF acc[2 * K];
+  constexpr int NV = dot_values(K);
+  DF acc[NV];
 #pragma unroll
-  for (int k = 0; k < 2 * K; ++k) acc[k] = DF{0.f, 0.f};
-#pragma unroll 2
+  for (int k = 0; k < NV; ++k) acc[k] = DF{0.f, 0.f};
+#pragma unroll 1
   for (long long e = beg + threadIdx.x; e < end; e += blockDim.x) {
     const float2 wv = __ldg(w + e);
 #pragma unroll
@@ -102,14 +109,14 @@ __device__ __forceinline__ void dot_cols(const float2* __restrict__ V, long long
       df_add_prod(acc[2 * k + 1], -v.y, wv.x);
     }
   }
-  warp_transpose_sum<2 * K>(acc);
-  constexpr int span = 32 / (2 * K);
+  warp_transpose_sum<NV>(acc);
+  constexpr int span = 32 / NV;
   const int lane = threadIdx.x & 31;
   if (lane % span == 0) row[lane / span] = (double)acc[0].hi + (double)acc[0].lo;
 }
 
 template <typename T2>
-__global__ void __launch_bounds__(kReduceThreads)
+__global__ void __launch_bounds__(kReduceThreads, sizeof(T2) == 8 ? 4 : 1)
     k_mdot_partial(const T2* __restrict__ V, long long ldv, int nv, const T2* __restrict__ w, long long n,
                    double2* __restrict__ partial, int stride) {
   __shared__ double red[kReduceThreads / 32][2 * kDotGroup];
@@ -119,13 +126,15 @@ __global__ void __launch_bounds__(kReduceThreads)
   const int cnt = min(kDotGroup, nv - g);
   V += (long long)g * ldv;
   double* row = red[threadIdx.x >> 5];
-  if (cnt == 8) {  // uniform
-    dot_cols<8>(V, ldv, w, beg, end, row);
-  } else {
-    int k = 0;
-    if (cnt & 4) dot_cols<4>(V, ldv, w, beg, end, row), k = 4;
-    if (cnt & 2) dot_cols<2>(V + k * ldv, ldv, w, beg, end, row + 2 * k), k += 2;
-    if (cnt & 1) dot_cols<1>(V + k * ldv, ldv, w, beg, end, row + 2 * k);
+  switch (cnt) {  // uniform
+    case 1: dot_cols<1>(V, ldv, w, beg, end, row); break;
+    case 2: dot_cols<2>(V, ldv, w, beg, end, row); break;
+    case 3: dot_cols<3>(V, ldv, w, beg, end, row); break;
+    case 4: dot_cols<4>(V, ldv, w, beg, end, row); break;
+    case 5: dot_cols<5>(V, ldv, w, beg, end, row); break;
+    case 6: dot_cols<6>(V, ldv, w, beg, end, row); break;
+    case 7: dot_cols<7>(V, ldv, w, beg, end, row); break;
+    default: dot_cols<8>(V, ldv, w, beg, end, row);
   }
   __syncthreads();
   for (int i = threadIdx.x; i < 2 * cnt; i += blockDim.x) {
