@@ -231,6 +231,7 @@ int upload_plan(pi_plan* plan) {
   // Built only when every term of every sector sits at one of these positions.
   std::vector<int4> canon;
   int canon_plus = 0;
+  TermCounts canon_terms{};
   if (fast_sr > 0) {
     bool ok = true;
     std::vector<int4> table;
@@ -279,6 +280,7 @@ int upload_plan(pi_plan* plan) {
           if (!ok) break;
         }
       }
+      for (int k = 0; k < 9; ++k) canon_terms.n[k] = std::max(canon_terms.n[k], (signed char)nsand[k]);
       table.insert(table.end(), e.begin(), e.end());
     }
     if (ok && zoff >= 0) canon.swap(table);
@@ -306,6 +308,7 @@ int upload_plan(pi_plan* plan) {
   if (!canon.empty()) {
     if ((rc = upload(plan, canon, &plan->dev.canon))) return rc;
     plan->dev.canon_plus = canon_plus;
+    plan->dev.canon_terms = canon_terms;
   }
   if ((rc = upload(plan, diag_index, &plan->dev.diag_index))) return rc;
   plan->dev.nsectors = S;

@@ -108,6 +108,11 @@ struct alignas(16) StripItem {
 };
 static_assert(sizeof(StripItem) == 48, "strip record layout");
 
+// Sandwich terms in use at each position of the canonical table (the most of any sector).
+struct TermCounts {
+  signed char n[9];
+};
+
 // Real gain position of a canonical plan: source (0 own, 1 smaller, 2 larger sector) at the
 // diagonal shift `shift` from the entry with the same magnetic numbers there, in index terms
 // own (a + shift, b + shift), smaller (a - 1 + shift, ...), larger (a + 1 + shift, ...).

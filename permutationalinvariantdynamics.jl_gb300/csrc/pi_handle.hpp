@@ -78,6 +78,7 @@ struct pi_plan {
   bool planes64_failed[2] = {false, false};
   bool planes32_failed[2] = {false, false};
   const picuda::StripItem* strip_items = nullptr;
+  const int2* strip_first = nullptr;  // per sector: first line, first strip item
   int nstrip_items = 0;
   // Single-instance solves run as one job of a batched engine kept with the plan (created on
   // first use for a Krylov dimension and basis precision, replaced when those change).

@@ -25,6 +25,7 @@ struct DevicePlan {
   int fast_sr = 0;                   // real sandwich terms per sector of the fixed structure (0: none)
   const int4* canon = nullptr;      // canonical-position table (kCanonEntries per sector) or null
   int canon_plus = 0;                // some sandwich term sits at the +1 diagonal shift
+  TermCounts canon_terms{};          // sandwich terms per position of the canonical table
   int nsectors = 0;
   int ntiles = 0;
   int ndiag = 0;
