@@ -223,8 +223,8 @@ int upload_plan(pi_plan* plan) {
       }
     }
   }
-  // Canonical-position table for the register-reuse batched kernel (pi_apply.cu,
-  // k_apply_canon): per sector kCanonEntries int4 (alpha_off, beta_off, 0, 0):
+  // Canonical-position table, from which the merged coefficient planes are built (pi_strip.cu,
+  // pi_apply_em.cu): per sector kCanonEntries int4 (alpha_off, beta_off, 0, 0):
   //   [0] ADD; [1], [2] imaginary LEFT at row shift p = -1, +1; [3], [4] imaginary RIGHT at
   //   column shift q = -1, +1; then, for each source slot (0..2) and diagonal shift
   //   p = q = -1, 0, +1, kCanonPerPos real sandwich terms (zero-padded).
