@@ -589,8 +589,14 @@ __global__ void __launch_bounds__(kTmThreads, 2)
 #pragma unroll
     for (int c = 0; c < 3; ++c) win[qi][c] = rl[slot * SLOT_F4 + 1 * SRC_F4 + c * COL_F4];
   };
-  auto release = [&](int slot) {
-    __syncwarp();
+  // Frees a slot once the reads that x, y and z come from have returned.  An arrival is not ordered
+  // before shared-memory reads in flight as far as the next bulk copy into the slot is concerned:
+  // a warp whose reads queued behind stalled stores let the copy overtake them, about once in 30,000
+  // launches.  So every lane's values go into a vote, and an instruction ahead of the arrival
+  // depends on the vote.
+  auto release = [&](int slot, float x, float y, float z) {
+    const unsigned bits = __float_as_uint(x) & __float_as_uint(y) & __float_as_uint(z);
+    if (__any_sync(0xffffffffu, bits == 0xffffffffu)) asm volatile("nanosleep.u32 0;" ::: "memory");
     if (lane == 0) mbar_arrive(empty0 + 8 * slot);
   };
   float4 hs, hl;  // smaller / larger column w of step r, read one row early
@@ -602,7 +608,7 @@ __global__ void __launch_bounds__(kTmThreads, 2)
     take_own(1, 1);
     hs = rl[0 * SLOT_F4 + 0 * SRC_F4 + 0 * COL_F4];
     hl = rl[0 * SLOT_F4 + 2 * SRC_F4 + 0 * COL_F4];
-    release(0);
+    release(0, hs.w, hl.w, win[0][0].w + win[0][1].w + win[0][2].w);
   }
   uint32_t phase = 0;  // parity of ring pass base / RING
   for (int base = 0; good && base < rows; base += RING, phase ^= 1u) {
@@ -623,11 +629,10 @@ __global__ void __launch_bounds__(kTmThreads, 2)
         xs2 = rl[sl2 * SLOT_F4 + 0 * SRC_F4 + 2 * COL_F4];
         xl2 = rl[sl2 * SLOT_F4 + 2 * SRC_F4 + 2 * COL_F4];
       }
-      const float4 xs1 = rl[sl1 * SLOT_F4 + 0 * SRC_F4 + 1 * COL_F4];
-      const float4 xl1 = rl[sl1 * SLOT_F4 + 2 * SRC_F4 + 1 * COL_F4];
       const float4 ns = rl[sl1 * SLOT_F4 + 0 * SRC_F4 + 0 * COL_F4];
       const float4 nl = rl[sl1 * SLOT_F4 + 2 * SRC_F4 + 0 * COL_F4];
-      release(sl1);  // step r+1 is not read again
+      const float4 xs1 = rl[sl1 * SLOT_F4 + 0 * SRC_F4 + 1 * COL_F4];
+      const float4 xl1 = rl[sl1 * SLOT_F4 + 2 * SRC_F4 + 1 * COL_F4];
       const float4 e0 = ew[r * NE], e1 = ew[r * NE + 1];
       const float4 lv = lrw[r];  // LEFT -1, +1 of row a
       float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -647,6 +652,7 @@ __global__ void __launch_bounds__(kTmThreads, 2)
         rmac2(acc, e2.x, xs2);         // 11 smaller (0,0): step r+2, column w+2
         rmac2(acc, e2.y, xl2);         // 12 larger (2,2): step r+2, column w+2
       }
+      release(sl1, ns.w, nl.w, acc.w);  // step r+1: acc holds xs1 and xl1, and own rows read before
       if (ok) __stcs(y + yi, acc);  // streamed out: keeps L2 for the rows neighbouring sectors reread
       yi += ld4;
       hs = ns;
