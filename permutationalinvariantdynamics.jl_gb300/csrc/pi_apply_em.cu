@@ -411,12 +411,12 @@ __global__ void __launch_bounds__(32 * kEmWarps, 4)
 // so output row a reads the slots of steps a-1, a and a+1; a consumer warp reads each step's
 // own row when it lands and its neighbour columns one row later, then releases the slot.  A
 // tile of R rows takes R + 2 steps (a0-1 .. a0+R).
-constexpr int kTmW = kEmWarps;                      // consumer warps = output columns
-constexpr int kTmCols = kTmW + 2;                   // staged columns per source sector
-constexpr int kTmHalf = 64;                         // complex right-hand sides per block
-constexpr int kTmColBytes = kTmHalf * 8;            // one staged column of one row
-constexpr int kTmSrcBytes = kTmCols * kTmColBytes;  // one source sector of one step
-constexpr int kTmSlotBytes = 3 * kTmSrcBytes;       // one ring slot
+//
+// Narrow batches: a block of G = 64, 32 or 16 right-hand sides, whose warps own 64 / G output
+// columns each (lane l: pair l % (G / 2) of column l / (G / 2)), so a batch of 32 or 16 columns
+// fills the lanes that blocks of 64 would leave idle, and a tile of 16 or 32 columns stages
+// fewer halo columns per output column.  N = 200: 16 right-hand sides 231 -> 101 us, 32 234 -> 155.
+constexpr int kTmW = kEmWarps;                      // consumer warps
 constexpr int kTmThreads = 32 * (kTmW + 1);         // + one producer warp
 constexpr int kTmWaitLimit = 1 << 22;               // mbarrier polls before a wait gives up
 
@@ -436,14 +436,21 @@ struct alignas(16) TmTile {
 };
 static_assert(sizeof(TmTile) == 48, "tile record layout");
 
-template <bool PLUS, int ROWS>
+template <bool PLUS, int ROWS, int G>
 struct TmCfg {
   static constexpr int NE = PLUS ? 3 : 2;  // float4 of the entry plane per entry
   static constexpr int RING = 6;           // two blocks of 8+1 warps per SM
-  static constexpr int ENTRY_BYTES = kTmW * ROWS * NE * 16;  // entry-plane runs of the warps
-  static constexpr int ROW_BYTES = ROWS * 16;                // row-plane run of the tile
-  static constexpr int COL_BYTES = kTmW * 16;                   // column-plane values of the tile
-  static constexpr int SMEM = RING * kTmSlotBytes + ENTRY_BYTES + ROW_BYTES + COL_BYTES + 2 * RING * 8;
+  static constexpr int SUB = 64 / G;       // output columns of a warp
+  static constexpr int W = kTmW * SUB;     // output columns of a block
+  static constexpr int COLS = W + 2;       // staged columns per source sector
+  static constexpr int STAGED_BYTES = G * 8;             // one staged column of one row
+  static constexpr int SRC_BYTES = COLS * STAGED_BYTES;  // one source sector of one step
+  static constexpr int SLOT_BYTES = 3 * SRC_BYTES;       // one ring slot
+  static constexpr int ENTRY_BYTES = W * ROWS * NE * 16;  // entry-plane runs of the columns
+  static constexpr int ROW_BYTES = ROWS * 16;             // row-plane run of the tile
+  static constexpr int COL_BYTES = W * 16;                // column-plane values of the tile
+  static constexpr int SMEM = RING * SLOT_BYTES + ENTRY_BYTES + ROW_BYTES + COL_BYTES + 2 * RING * 8;
+  static_assert(SRC_BYTES % 128 == 0, "TMA destinations start on 128-byte boundaries");
 };
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
@@ -484,21 +491,21 @@ __device__ __forceinline__ void bulk_load(uint32_t dst, const void* src, uint32_
                : "memory");
 }
 
-template <bool PLUS, int MAXS, int ROWS>
+template <bool PLUS, int MAXS, int ROWS, int G>
 __global__ void __launch_bounds__(kTmThreads, 2)
     k_apply_em_tma(const __grid_constant__ EmMaps<MAXS> maps, const TmTile* __restrict__ tiles,
                    const float4* __restrict__ eplane, const float4* __restrict__ lrow,
                    const float4* __restrict__ rcol, float4* __restrict__ y, unsigned ld4, int npairs) {
-  using C = TmCfg<PLUS, ROWS>;
+  using C = TmCfg<PLUS, ROWS, G>;
   constexpr int NE = C::NE;
   constexpr int RING = C::RING;
   static_assert(RING % 3 == 0, "own rows are kept in registers indexed by step modulo three");
   extern __shared__ __align__(1024) unsigned char smem[];
   const float4* ring = reinterpret_cast<const float4*>(smem);
-  const float4* ent = reinterpret_cast<const float4*>(smem + RING * kTmSlotBytes);
-  const float4* lrw = reinterpret_cast<const float4*>(smem + RING * kTmSlotBytes + C::ENTRY_BYTES);
+  const float4* ent = reinterpret_cast<const float4*>(smem + RING * C::SLOT_BYTES);
+  const float4* lrw = reinterpret_cast<const float4*>(smem + RING * C::SLOT_BYTES + C::ENTRY_BYTES);
   const uint32_t ring_u32 = smem_u32(smem);
-  const uint32_t ent_u32 = ring_u32 + RING * kTmSlotBytes;
+  const uint32_t ent_u32 = ring_u32 + RING * C::SLOT_BYTES;
   const uint32_t row_u32 = ent_u32 + C::ENTRY_BYTES;
   const uint32_t col_u32 = row_u32 + C::ROW_BYTES;
   const uint32_t full0 = col_u32 + C::COL_BYTES;  // full[i] at full0 + 8 i
@@ -522,7 +529,7 @@ __global__ void __launch_bounds__(kTmThreads, 2)
   // slot is zeroed once here, so the consumers read zeros without a test per load.
   if (s0 < 0 || s2 < 0) {
     float4* rw = reinterpret_cast<float4*>(smem);
-    constexpr int per_src = kTmSrcBytes / 16;
+    constexpr int per_src = C::SRC_BYTES / 16;
     for (int i = threadIdx.x; i < RING * per_src; i += blockDim.x) {
       const int slot = i / per_src, e = i - slot * per_src;
       if (s0 < 0) rw[(slot * 3 + 0) * per_src + e] = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -534,14 +541,14 @@ __global__ void __launch_bounds__(kTmThreads, 2)
   if (warp == kTmW) {  // producer: one thread issues every copy of the block
     if (lane != 0) return;
     // Step i (relative row a0-1+i): own row, smaller row - 1, larger row + 1, and at step 0
-    // every consumer warp's merged coefficients for all its rows (contiguous in the planes).
+    // every output column's merged coefficients for all its rows (contiguous in the planes).
     // Step i reuses the slot of step i - RING once every consumer warp has released it.
     const CUtensorMap* m_own = &maps.m[tile.sector];
     const CUtensorMap* m_sm = s0 >= 0 ? &maps.m[s0] : nullptr;
     const CUtensorMap* m_lg = s2 >= 0 ? &maps.m[s2] : nullptr;
-    const int xq = blockIdx.y * kTmHalf;
-    const uint32_t step_bytes = kTmSrcBytes * (1u + (m_sm != nullptr) + (m_lg != nullptr));
-    const int nact = min(kTmW, n - b0);
+    const int xq = blockIdx.y * G;
+    const uint32_t step_bytes = C::SRC_BYTES * (1u + (m_sm != nullptr) + (m_lg != nullptr));
+    const int nact = min(C::W, n - b0);
     const uint32_t run_bytes = (uint32_t)rows * NE * 16, row_bytes = (uint32_t)rows * 16;
     const int nsteps = rows + 2;
     for (int i = 0; i < nsteps; ++i) {
@@ -550,11 +557,11 @@ __global__ void __launch_bounds__(kTmThreads, 2)
       if (i >= RING && !mbar_wait(empty0 + 8 * slot, (uint32_t)((i / RING) - 1) & 1u)) return;
       mbar_expect_tx(full, step_bytes + (i == 0 ? (run_bytes + 16u) * (uint32_t)nact + row_bytes : 0u));
       const int k = a0 - 1 + i;
-      const uint32_t dst = ring_u32 + slot * kTmSlotBytes;
-      tma_load_3d(dst + kTmSrcBytes, m_own, xq, k, b0 - 1, full);
+      const uint32_t dst = ring_u32 + slot * C::SLOT_BYTES;
+      tma_load_3d(dst + C::SRC_BYTES, m_own, xq, k, b0 - 1, full);
       if (m_sm) tma_load_3d(dst, m_sm, xq, k - 1, b0 - 2, full);
-      if (m_lg) tma_load_3d(dst + 2 * kTmSrcBytes, m_lg, xq, k + 1, b0, full);
-      if (i == 0) {  // the warps' entry-plane runs (contiguous down a column), row and column planes
+      if (m_lg) tma_load_3d(dst + 2 * C::SRC_BYTES, m_lg, xq, k + 1, b0, full);
+      if (i == 0) {  // the columns' entry-plane runs (contiguous down a column), row and column planes
         for (int w = 0; w < nact; ++w)
           bulk_load(ent_u32 + w * (ROWS * NE * 16), eplane + (size_t)(tile.offset + a0 + (long long)(b0 + w) * n) * NE,
                     run_bytes, full);
@@ -565,16 +572,17 @@ __global__ void __launch_bounds__(kTmThreads, 2)
     return;
   }
 
-  // consumers: warp w owns output column b = b0 + w, lane l the right-hand-side pair q
-  const int b = b0 + warp;
+  // consumers: warp w owns output columns b0 + SUB w .. + SUB - 1; this lane one column and pair q
+  const int w = warp * C::SUB + lane / (G / 2), lq = lane % (G / 2);
+  const int b = b0 + w;
   const bool active = b < n;
-  const int q = blockIdx.y * 32 + lane;
+  const int q = blockIdx.y * (G / 2) + lq;
   const bool ok = active && q < npairs;
   // This lane's float4 in staged column c of source src of slot i is rl[SLOT_F4 i + SRC_F4 src
   // + COL_F4 c]: with the row loop unrolled over the ring, every offset is a constant.
-  constexpr int COL_F4 = kTmColBytes / 16, SRC_F4 = kTmSrcBytes / 16, SLOT_F4 = kTmSlotBytes / 16;
-  const float4* rl = ring + warp * COL_F4 + lane;
-  const float4* ew = ent + warp * (ROWS * NE);
+  constexpr int COL_F4 = C::STAGED_BYTES / 16, SRC_F4 = C::SRC_BYTES / 16, SLOT_F4 = C::SLOT_BYTES / 16;
+  const float4* rl = ring + w * COL_F4 + lq;
+  const float4* ew = ent + w * (ROWS * NE);
   unsigned yi = (unsigned)(tile.offset + a0 + (long long)(active ? b : 0) * n) * ld4 + (unsigned)(ok ? q : 0);
   int r = 0;
   // Step s carries own row s-1 (relative to a0), used by output rows s-2 .. s, and the
@@ -602,7 +610,7 @@ __global__ void __launch_bounds__(kTmThreads, 2)
   float4 hs, hl;  // smaller / larger column w of step r, read one row early
   bool good = mbar_wait(full0, 0) && mbar_wait(full0 + 8, 0);
   // RIGHT -1, +1 of column b (staged with step 0)
-  const float4 rc = reinterpret_cast<const float4*>(smem + RING * kTmSlotBytes + C::ENTRY_BYTES + C::ROW_BYTES)[active ? warp : 0];
+  const float4 rc = reinterpret_cast<const float4*>(smem + RING * C::SLOT_BYTES + C::ENTRY_BYTES + C::ROW_BYTES)[active ? w : 0];
   if (good) {
     take_own(0, 0);
     take_own(1, 1);
@@ -715,12 +723,12 @@ static int em_prepare(pi_plan* plan, int which, const float2** planes_out) {
   return PI_OK;
 }
 
-// Tile records of the TMA-staged kernel for tiles of rows x kTmW (one load per block),
-// built once per plan and tile height.  Caller holds plan->em_mu.
-static int em_tma_tiles(pi_plan* plan, int ri, const TmTile** tiles_out, int* ntiles_out) {
+// Tile records of the TMA-staged kernel for tiles of kRows[ri] rows x (kTmW << gi) columns (one load
+// per block), built once per plan and tile shape.  Caller holds plan->em_mu.
+static int em_tma_tiles(pi_plan* plan, int ri, int gi, const TmTile** tiles_out, int* ntiles_out) {
   static constexpr int kRows[3] = {16, 32, 64};
   const DevicePlan& dp = plan->dev;
-  if (!plan->em_tma_tiles[ri]) {
+  if (!plan->em_tma_tiles[ri][gi]) {
     std::vector<DevSector> secs(dp.nsectors);
     cudaError_t e = cudaMemcpy(secs.data(), dp.sectors, sizeof(DevSector) * secs.size(), cudaMemcpyDeviceToHost);
     if (e != cudaSuccess) return cuda_fail(e, "element-major tile list");
@@ -729,7 +737,7 @@ static int em_tma_tiles(pi_plan* plan, int ri, const TmTile** tiles_out, int* nt
     for (int s = 0; s < dp.nsectors; ++s) {
       const int n = secs[s].n;
       for (int a0 = 0; a0 < n; a0 += kRows[ri])
-        for (int b0 = 0; b0 < n; b0 += kTmW) {
+        for (int b0 = 0; b0 < n; b0 += kTmW << gi) {
           TmTile t{};
           t.offset = secs[s].offset;
           t.sector = s;
@@ -747,11 +755,11 @@ static int em_tma_tiles(pi_plan* plan, int ri, const TmTile** tiles_out, int* nt
     if (!d) return fail(PI_ERR_OUT_OF_MEMORY, "element-major tile list");
     e = cudaMemcpy(d, tiles.data(), sizeof(TmTile) * tiles.size(), cudaMemcpyHostToDevice);
     if (e != cudaSuccess) return cuda_fail(e, "element-major tile list");
-    plan->em_tma_tiles[ri] = d;
-    plan->em_tma_ntiles[ri] = (int)tiles.size();
+    plan->em_tma_tiles[ri][gi] = d;
+    plan->em_tma_ntiles[ri][gi] = (int)tiles.size();
   }
-  *tiles_out = (const TmTile*)plan->em_tma_tiles[ri];
-  *ntiles_out = plan->em_tma_ntiles[ri];
+  *tiles_out = (const TmTile*)plan->em_tma_tiles[ri][gi];
+  *ntiles_out = plan->em_tma_ntiles[ri][gi];
   return PI_OK;
 }
 
@@ -778,7 +786,7 @@ static int em_prepare_split(pi_plan* plan, int which, pi_plan::EmSplit* out) {
   }
   pi_plan::EmSplit& sp = plan->em_split[which];
   if (!sp.eplane) {
-    const int ne = dp.canon_plus ? TmCfg<true, 32>::NE : TmCfg<false, 32>::NE;
+    const int ne = dp.canon_plus ? TmCfg<true, 32, 64>::NE : TmCfg<false, 32, 64>::NE;
     void* e_d = plan_alloc(plan, sizeof(float4) * (size_t)dp.dim * ne);
     void* l_d = plan_alloc(plan, sizeof(float4) * (size_t)plan->em_nlines);
     void* r_d = plan_alloc(plan, sizeof(float4) * (size_t)plan->em_nlines);
@@ -845,13 +853,13 @@ constexpr size_t kTmMapCache = 4;  // source batches whose maps are kept per pla
 
 // Per-sector tensor maps over the batch x: sector s is the 3-D tensor (right-hand side c <
 // ncols, row a < n, column b < n) at x + offset_s * ld with strides (8, 8 ld, 8 ld n) bytes;
-// the box is 64 right-hand sides x 1 row x kTmCols columns.  Encoded on the host once per
-// (x, ld, ncols) and kept for the last few batches.  Returns nullptr when a map cannot be
+// the box is g right-hand sides x 1 row x the staged columns.  Encoded on the host once per
+// (x, ld, ncols, g) and kept for the last few batches.  Returns nullptr when a map cannot be
 // encoded (the caller then uses the kernel with plain loads).
-static const unsigned char* em_tensor_maps(pi_plan* plan, const void* x, long long ld, int ncols) {
+static const unsigned char* em_tensor_maps(pi_plan* plan, const void* x, long long ld, int ncols, int g) {
   std::lock_guard<std::mutex> lk(plan->em_mu);
   for (auto& e : plan->em_maps)
-    if (e.x == x && e.ld == ld && e.ncols == ncols) return e.maps.data();
+    if (e.x == x && e.ld == ld && e.ncols == ncols && e.g == g) return e.maps.data();
   const auto encode = tensor_map_encoder();
   if (!encode) return nullptr;
   const auto& secs = plan->host.sectors;
@@ -860,7 +868,7 @@ static const unsigned char* em_tensor_maps(pi_plan* plan, const void* x, long lo
     const unsigned long long n = (unsigned long long)secs[s].n;
     const cuuint64_t dims[3] = {(cuuint64_t)ncols, n, n};
     const cuuint64_t strides[2] = {(cuuint64_t)ld * 8, (cuuint64_t)ld * 8 * n};
-    const cuuint32_t box[3] = {kTmHalf, 1, kTmCols};
+    const cuuint32_t box[3] = {(cuuint32_t)g, 1, (cuuint32_t)(kTmW * (64 / g) + 2)};
     const cuuint32_t elem[3] = {1, 1, 1};
     CUtensorMap m;
     void* base = (void*)((const char*)x + (size_t)secs[s].offset * (size_t)ld * 8);
@@ -871,42 +879,46 @@ static const unsigned char* em_tensor_maps(pi_plan* plan, const void* x, long lo
     std::memcpy(blob.data() + s * sizeof(CUtensorMap), &m, sizeof(CUtensorMap));
   }
   if (plan->em_maps.size() >= kTmMapCache) plan->em_maps.erase(plan->em_maps.begin());
-  plan->em_maps.push_back(pi_plan::EmMapSet{x, ld, ncols, std::move(blob)});
+  plan->em_maps.push_back(pi_plan::EmMapSet{x, ld, ncols, g, std::move(blob)});
   return plan->em_maps.back().maps.data();
 }
 
-template <bool PLUS, int MAXS, int ROWS>
+template <bool PLUS, int MAXS, int ROWS, int G>
 static cudaError_t launch_em_tma(const unsigned char* blob, int nsectors, const TmTile* tiles, int ntiles,
                                  const pi_plan::EmSplit& sp, float4* y, unsigned ld4, int npairs, cudaStream_t s) {
   EmMaps<MAXS> maps;
   std::memset(&maps, 0, sizeof(maps));
   std::memcpy(maps.m, blob, (size_t)nsectors * sizeof(CUtensorMap));
-  auto kern = k_apply_em_tma<PLUS, MAXS, ROWS>;
-  constexpr int smem = TmCfg<PLUS, ROWS>::SMEM;
+  auto kern = k_apply_em_tma<PLUS, MAXS, ROWS, G>;
+  constexpr int smem = TmCfg<PLUS, ROWS, G>::SMEM;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
   if (e != cudaSuccess) return e;
-  dim3 grid((unsigned)ntiles, (unsigned)((npairs + 31) / 32));
+  dim3 grid((unsigned)ntiles, (unsigned)((npairs + G / 2 - 1) / (G / 2)));
   kern<<<grid, kTmThreads, smem, s>>>(maps, tiles, sp.eplane, sp.lrow, sp.rcol, y, ld4, npairs);
   return cudaGetLastError();
 }
 
-template <int MAXS, int ROWS>
-static cudaError_t launch_em_tma_rows(bool plus, const unsigned char* blob, int nsectors, const TmTile* tiles,
-                                      int ntiles, const pi_plan::EmSplit& sp, float4* y, unsigned ld4, int npairs,
-                                      cudaStream_t s) {
+template <int ROWS, int G>
+static cudaError_t launch_em_tma_shape(bool plus, const unsigned char* blob, int nsectors, const TmTile* tiles,
+                                       int ntiles, const pi_plan::EmSplit& sp, float4* y, unsigned ld4, int npairs,
+                                       cudaStream_t s) {
+  const bool small = nsectors <= kTmMapsSmall;
   if (plus) {
     if constexpr (ROWS <= 32)  // the pumping variant's entry plane leaves no room for 64-row runs
-      return launch_em_tma<true, MAXS, ROWS>(blob, nsectors, tiles, ntiles, sp, y, ld4, npairs, s);
+      return small ? launch_em_tma<true, kTmMapsSmall, ROWS, G>(blob, nsectors, tiles, ntiles, sp, y, ld4, npairs, s)
+                   : launch_em_tma<true, kTmMapsLarge, ROWS, G>(blob, nsectors, tiles, ntiles, sp, y, ld4, npairs, s);
     return cudaErrorInvalidValue;
   }
-  return launch_em_tma<false, MAXS, ROWS>(blob, nsectors, tiles, ntiles, sp, y, ld4, npairs, s);
+  return small ? launch_em_tma<false, kTmMapsSmall, ROWS, G>(blob, nsectors, tiles, ntiles, sp, y, ld4, npairs, s)
+               : launch_em_tma<false, kTmMapsLarge, ROWS, G>(blob, nsectors, tiles, ntiles, sp, y, ld4, npairs, s);
 }
 
-// One element-major kernel choice: TMA-staged with tiles of `rows` rows (kind 0), or plain
-// loads (kind 1).
+// One element-major kernel choice: TMA-staged with tiles of `rows` rows and blocks of g
+// right-hand sides (kind 0), or plain loads (kind 1).
 struct EmCand {
   int kind;
   int rows;
+  int g = 64;
 };
 
 // Runs one candidate.  Returns a PI status.
@@ -917,34 +929,25 @@ static int em_run(pi_plan* plan, EmCand c, float* y_dev, const float* x_dev, int
   const unsigned ld4 = (unsigned)(ld / 2);
   float4* y4 = (float4*)y_dev;
   if (c.kind == 0) {
-    const unsigned char* maps = em_tensor_maps(plan, x_dev, ld, ncols);
+    const unsigned char* maps = em_tensor_maps(plan, x_dev, ld, ncols, c.g);
     if (!maps) return fail(PI_ERR_UNSUPPORTED, "element-major tensor maps could not be encoded");
     pi_plan::EmSplit sp;
     int rc = em_prepare_split(plan, coords, &sp);
     if (rc) return rc;
-    const int ri = c.rows == 16 ? 0 : c.rows == 32 ? 1 : 2;
+    const int ri = c.rows == 16 ? 0 : c.rows == 32 ? 1 : 2, gi = c.g == 64 ? 0 : c.g == 32 ? 1 : 2;
     const TmTile* tiles = nullptr;
     int ntiles = 0;
     {
       std::lock_guard<std::mutex> lk(plan->em_mu);
-      rc = em_tma_tiles(plan, ri, &tiles, &ntiles);
+      rc = em_tma_tiles(plan, ri, gi, &tiles, &ntiles);
     }
     if (rc) return rc;
-    const bool plus = dp.canon_plus != 0, small = dp.nsectors <= kTmMapsSmall;
-    cudaError_t e;
-    switch (ri) {
-      case 0:
-        e = small ? launch_em_tma_rows<kTmMapsSmall, 16>(plus, maps, dp.nsectors, tiles, ntiles, sp, y4, ld4, npairs, s)
-                  : launch_em_tma_rows<kTmMapsLarge, 16>(plus, maps, dp.nsectors, tiles, ntiles, sp, y4, ld4, npairs, s);
-        break;
-      case 1:
-        e = small ? launch_em_tma_rows<kTmMapsSmall, 32>(plus, maps, dp.nsectors, tiles, ntiles, sp, y4, ld4, npairs, s)
-                  : launch_em_tma_rows<kTmMapsLarge, 32>(plus, maps, dp.nsectors, tiles, ntiles, sp, y4, ld4, npairs, s);
-        break;
-      default:
-        e = small ? launch_em_tma_rows<kTmMapsSmall, 64>(plus, maps, dp.nsectors, tiles, ntiles, sp, y4, ld4, npairs, s)
-                  : launch_em_tma_rows<kTmMapsLarge, 64>(plus, maps, dp.nsectors, tiles, ntiles, sp, y4, ld4, npairs, s);
-    }
+    decltype(&launch_em_tma_shape<16, 64>) launch = nullptr;
+    if (c.g == 64)
+      launch = ri == 0 ? launch_em_tma_shape<16, 64> : ri == 1 ? launch_em_tma_shape<32, 64> : launch_em_tma_shape<64, 64>;
+    else
+      launch = gi == 1 ? launch_em_tma_shape<32, 32> : launch_em_tma_shape<16, 16>;
+    const cudaError_t e = launch(dp.canon_plus != 0, maps, dp.nsectors, tiles, ntiles, sp, y4, ld4, npairs, s);
     if (e != cudaSuccess) return cuda_fail(e, "element-major apply launch (TMA)");
     return PI_OK;
   }
@@ -969,13 +972,25 @@ static int em_run(pi_plan* plan, EmCand c, float* y_dev, const float* x_dev, int
 }
 
 // The candidates for a plan: TMA-staged tiles of 16, 32 and (without pumping terms) 64 rows
-// when the plan's tensor maps fit the kernel-parameter table, and plain loads.
-static std::vector<EmCand> em_candidates(const pi_plan* plan) {
+// when the plan's tensor maps fit the kernel-parameter table, and plain loads; for batches of up
+// to 16 columns also blocks of 16 right-hand sides (16 rows x 32 columns), and for 17 to 32 and 65
+// to 96 columns blocks of 32 (32 x 16), which keep the entry planes' size.  Up to 32 columns
+// they stand in for the other tile heights.  Elsewhere they lose: N = 120, 48 columns take 64 us in
+// one block of 64 and 70 in three of 16, 130 columns 194 us in three and 203 in five of 32, while 96
+// take 120 and 109, 32 columns 61 and 46, 16 columns 59 and 30.  ncols = 0 lists the choices that a
+// caller can pin.
+static std::vector<EmCand> em_candidates(const pi_plan* plan, int ncols) {
   std::vector<EmCand> c;
   if (plan->dev.nsectors <= kTmMapsLarge && tensor_map_encoder()) {
     c.push_back({0, 32});
-    c.push_back({0, 16});
-    if (!plan->dev.canon_plus) c.push_back({0, 64});
+    if (ncols == 0 || ncols > 32) {
+      c.push_back({0, 16});
+      if (!plan->dev.canon_plus) c.push_back({0, 64});
+    }
+    if (ncols > 0 && ncols <= 16)
+      c.push_back({0, 16, 16});
+    else if (ncols > 0 && ncols <= 96 && (ncols + 31) / 32 % 2 == 1)
+      c.push_back({0, 32, 32});
   }
   c.push_back({1, 32});
   return c;
@@ -991,7 +1006,7 @@ static int em_tune(pi_plan* plan, float* y_dev, const float* x_dev, int ncols, l
   // a candidate that cannot run on this batch (its tensor maps do not encode, say) drops out
   std::vector<EmCand> cands;
   int first_rc = PI_OK;
-  for (const EmCand& c : em_candidates(plan)) {
+  for (const EmCand& c : em_candidates(plan, ncols)) {
     const int rc = em_run(plan, c, y_dev, x_dev, ncols, ld, coords, s);
     if (rc == PI_OK)
       cands.push_back(c);
@@ -1027,7 +1042,7 @@ static int em_tune(pi_plan* plan, float* y_dev, const float* x_dev, int ncols, l
       }
       if (ms < best_ms) {
         best_ms = ms;
-        best = {ncols, coords, cands[i].kind, cands[i].rows, (double)ms};
+        best = {ncols, coords, cands[i].kind, cands[i].rows, (double)ms, cands[i].g};
       }
     }
   for (auto& f : ev) cudaEventDestroy(f);
@@ -1091,7 +1106,7 @@ extern "C" int pi_apply_f32_em(pi_plan* plan, float* y_dev, const float* x_dev, 
       return PI_OK;  // y already holds L x from the timed runs
     }
   }
-  return em_run(plan, EmCand{ch.kind, ch.rows}, y_dev, x_dev, ncols, ld, coords, s);
+  return em_run(plan, EmCand{ch.kind, ch.rows, ch.g}, y_dev, x_dev, ncols, ld, coords, s);
 }
 
 extern "C" int pi_apply_f32_em_tuning(pi_plan* plan, int ncols, int coords, int* kind, int* rows, double* ms) {
@@ -1112,7 +1127,7 @@ extern "C" int pi_apply_f32_em_select(pi_plan* plan, int ncols, int coords, int 
   if (coords != PI_COORDS_REFERENCE && coords != PI_COORDS_POPULATION)
     return fail(PI_ERR_INVALID_ARGUMENT, "coords must be PI_COORDS_REFERENCE or PI_COORDS_POPULATION");
   bool listed = false;
-  for (const EmCand& c : em_candidates(plan)) listed = listed || (c.kind == kind && (kind == 1 || c.rows == rows));
+  for (const EmCand& c : em_candidates(plan, 0)) listed = listed || (c.kind == kind && (kind == 1 || c.rows == rows));
   if (!listed) return fail(PI_ERR_INVALID_ARGUMENT, "this element-major kernel choice is not available for the plan");
   std::lock_guard<std::mutex> lk(plan->em_mu);
   pi_plan::EmChoice ch{ncols, coords, kind, kind == 1 ? 32 : rows, 0.0};

@@ -1470,7 +1470,9 @@ __global__ void __launch_bounds__(kRT, 2)
     FinishSmem finish;
   } sm;
   __shared__ double2 tr;
-  __shared__ DevInst fixed;  // a single job's control block, for the fields that stay as they are
+  // a single job's control block, for the fields that stay as they are
+  __shared__ __align__(16) unsigned char fixed_raw[sizeof(DevInst)];
+  DevInst& fixed = *reinterpret_cast<DevInst*>(fixed_raw);
   using T2 = typename Vec2<typename std::conditional<F32, float, double>::type>::type;
   const int nblk = gridDim.x, blk = blockIdx.x;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;

@@ -45,7 +45,7 @@ struct pi_plan {
   struct EmMapSet {
     const void* x;
     long long ld;
-    int ncols;
+    int ncols, g;                     // width, right-hand sides per box
     std::vector<unsigned char> maps;  // nsectors x 128 bytes
   };
   std::vector<EmMapSet> em_maps;
@@ -61,13 +61,15 @@ struct pi_plan {
   EmSplit em_split[2];
   const int* em_line_off = nullptr;
   int em_nlines = 0;
-  const void* em_tma_tiles[3] = {nullptr, nullptr, nullptr};  // tile records, tiles of 16 / 32 / 64 rows
-  int em_tma_ntiles[3] = {0, 0, 0};
+  const void* em_tma_tiles[3][3] = {};  // tile records: 16 / 32 / 64 rows x 8 / 16 / 32 columns
+  int em_tma_ntiles[3][3] = {};
   // Element-major kernel chosen by the autotuner (or pinned by the caller) per batch width
-  // and coordinate system: kind 0 TMA-staged with tiles of `rows` rows, 1 plain loads.
+  // and coordinate system: kind 0 TMA-staged with tiles of `rows` rows and blocks of g right-hand
+  // sides, 1 plain loads.
   struct EmChoice {
     int ncols, coords, kind, rows;
     double ms;  // timed duration of one apply (0 when pinned)
+    int g = 64;
   };
   std::vector<EmChoice> em_choices;
   std::mutex em_tune_mu;
