@@ -415,7 +415,7 @@ __global__ void __launch_bounds__(32 * kEmWarps, 4)
 // Narrow batches: a block of G = 64, 32 or 16 right-hand sides, whose warps own 64 / G output
 // columns each (lane l: pair l % (G / 2) of column l / (G / 2)), so a batch of 32 or 16 columns
 // fills the lanes that blocks of 64 would leave idle, and a tile of 16 or 32 columns stages
-// fewer halo columns per output column.  N = 200: 16 right-hand sides 231 -> 101 us, 32 234 -> 155.
+// fewer halo columns per output column.  N = 200: 16 right-hand sides 231 -> 101 us, 32 234 -> 153.
 constexpr int kTmW = kEmWarps;                      // consumer warps
 constexpr int kTmThreads = 32 * (kTmW + 1);         // + one producer warp
 constexpr int kTmWaitLimit = 1 << 22;               // mbarrier polls before a wait gives up
@@ -660,8 +660,8 @@ __global__ void __launch_bounds__(kTmThreads, 2)
         rmac2(acc, e2.x, xs2);         // 11 smaller (0,0): step r+2, column w+2
         rmac2(acc, e2.y, xl2);         // 12 larger (2,2): step r+2, column w+2
       }
-      release(sl1, ns.w, nl.w, acc.w);  // step r+1: acc holds xs1 and xl1, and own rows read before
       if (ok) __stcs(y + yi, acc);  // streamed out: keeps L2 for the rows neighbouring sectors reread
+      release(sl1, ns.w, nl.w, acc.w);  // step r+1: acc holds xs1 and xl1, and own rows read before
       yi += ld4;
       hs = ns;
       hl = nl;
@@ -977,7 +977,7 @@ static int em_run(pi_plan* plan, EmCand c, float* y_dev, const float* x_dev, int
 // to 96 columns blocks of 32 (32 x 16), which keep the entry planes' size.  Up to 32 columns
 // they stand in for the other tile heights.  Elsewhere they lose: N = 120, 48 columns take 64 us in
 // one block of 64 and 70 in three of 16, 130 columns 194 us in three and 203 in five of 32, while 96
-// take 120 and 109, 32 columns 61 and 46, 16 columns 59 and 30.  ncols = 0 lists the choices that a
+// take 120 and 109, 32 columns 61 and 45, 16 columns 59 and 30.  ncols = 0 lists the choices that a
 // caller can pin.
 static std::vector<EmCand> em_candidates(const pi_plan* plan, int ncols) {
   std::vector<EmCand> c;
