@@ -9,6 +9,7 @@
 #include <cstdio>
 #include <cstring>
 #include <limits>
+#include <exception>
 #include <map>
 #include <mutex>
 #include <random>
@@ -2776,8 +2777,15 @@ static void for_jobs(const std::vector<char>& busy, const F& f) {
   const long count = std::count(busy.begin(), busy.end(), 1);
   const int threads = (int)std::min<long>({count / 2, 8, (long)std::thread::hardware_concurrency()});
   std::atomic<int> next{0};
+  std::exception_ptr thrown;
+  std::mutex thrown_mu;
   auto work = [&] {
-    for (int i = next++; i < n; i = next++) f(i);
+    try {
+      for (int i = next++; i < n; i = next++) f(i);
+    } catch (...) {  // goes on in the calling thread, as without helpers
+      std::lock_guard<std::mutex> lk(thrown_mu);
+      if (!thrown) thrown = std::current_exception();
+    }
   };
   std::vector<std::thread> pool;
   try {
@@ -2786,6 +2794,7 @@ static void for_jobs(const std::vector<char>& busy, const F& f) {
   }
   work();
   for (std::thread& t : pool) t.join();
+  if (thrown) std::rethrow_exception(thrown);
 }
 
 bool Engine::tick() {
