@@ -173,10 +173,10 @@ int pi_apply_f32(pi_plan* plan, float* y_dev, const float* x_dev, int ncols, lon
  * both buffers 16-byte aligned.  Needs a plan whose stencil sits at the canonical
  * positions (pi_plan_info_t.batched_kernel == 2).  Kernels: TMA-staged tiles of 16, 32 or
  * (without pumping terms) 64 rows for plans of up to 160 sectors (N <= 318; tensor maps
- * encoded on the host per source pointer, stride and width, the last four kept), and plain
- * loads.  Autotuned: the first call for a batch width and coordinate system runs every
- * candidate on the caller's batch, times them with CUDA events on `stream`, waits for that
- * stream once and keeps the fastest for later calls; all candidates give the same y.  The
+ * encoded on the host per source pointer, stride, width and right-hand sides per block, the last
+ * four kept), and plain loads.  Autotuned: the first call for a batch width and coordinate
+ * system runs every candidate on the caller's batch, times them with CUDA events on `stream`, waits
+ * for that stream once and keeps the fastest for later calls; all candidates give the same y.  The
  * coefficient planes (32-48 bytes per PI coordinate for TMA, 80-112 for plain loads) are
  * built and cached on first use, with a synchronisation of their own.  A caller that
  * captures the apply into a CUDA graph therefore makes one call per batch width and

@@ -849,17 +849,13 @@ static PFN_cuTensorMapEncodeTiled_v12000 tensor_map_encoder() {
 
 constexpr int kTmMapsSmall = 64;   // sectors of N <= 126
 constexpr int kTmMapsLarge = 160;  // sectors of N <= 318
-constexpr size_t kTmMapCache = 4;  // source batches whose maps are kept per plan
+constexpr size_t kTmMapCache = 4;  // map sets kept per plan: one per source batch in use
 
 // Per-sector tensor maps over the batch x: sector s is the 3-D tensor (right-hand side c <
 // ncols, row a < n, column b < n) at x + offset_s * ld with strides (8, 8 ld, 8 ld n) bytes;
-// the box is g right-hand sides x 1 row x the staged columns.  Encoded on the host once per
-// (x, ld, ncols, g) and kept for the last few batches.  Returns nullptr when a map cannot be
-// encoded (the caller then uses the kernel with plain loads).
-static const unsigned char* em_tensor_maps(pi_plan* plan, const void* x, long long ld, int ncols, int g) {
-  std::lock_guard<std::mutex> lk(plan->em_mu);
-  for (auto& e : plan->em_maps)
-    if (e.x == x && e.ld == ld && e.ncols == ncols && e.g == g) return e.maps.data();
+// the box is g right-hand sides x 1 row x the staged columns.  Encoded on the host; null when a map
+// cannot be encoded (the caller then uses the kernel with plain loads).
+static pi_plan::EmMapBlob em_encode_maps(const pi_plan* plan, const void* x, long long ld, int ncols, int g) {
   const auto encode = tensor_map_encoder();
   if (!encode) return nullptr;
   const auto& secs = plan->host.sectors;
@@ -878,9 +874,20 @@ static const unsigned char* em_tensor_maps(pi_plan* plan, const void* x, long lo
       return nullptr;
     std::memcpy(blob.data() + s * sizeof(CUtensorMap), &m, sizeof(CUtensorMap));
   }
+  return std::make_shared<const std::vector<unsigned char>>(std::move(blob));
+}
+
+// The kept maps of a batch; on its first apply `maps`, or newly encoded ones.
+static pi_plan::EmMapBlob em_tensor_maps(pi_plan* plan, const void* x, long long ld, int ncols, int g,
+                                         pi_plan::EmMapBlob maps = nullptr) {
+  std::lock_guard<std::mutex> lk(plan->em_mu);
+  for (const auto& e : plan->em_maps)
+    if (e.x == x && e.ld == ld && e.ncols == ncols && e.g == g) return e.maps;
+  if (!maps) maps = em_encode_maps(plan, x, ld, ncols, g);
+  if (!maps) return nullptr;
   if (plan->em_maps.size() >= kTmMapCache) plan->em_maps.erase(plan->em_maps.begin());
-  plan->em_maps.push_back(pi_plan::EmMapSet{x, ld, ncols, g, std::move(blob)});
-  return plan->em_maps.back().maps.data();
+  plan->em_maps.push_back(pi_plan::EmMapSet{x, ld, ncols, g, maps});
+  return maps;
 }
 
 template <bool PLUS, int MAXS, int ROWS, int G>
@@ -921,15 +928,14 @@ struct EmCand {
   int g = 64;
 };
 
-// Runs one candidate.  Returns a PI status.
-static int em_run(pi_plan* plan, EmCand c, float* y_dev, const float* x_dev, int ncols, long long ld, int coords,
-                  cudaStream_t s) {
+// Runs one candidate, a TMA-staged one with the given maps of the batch.  Returns a PI status.
+static int em_run(pi_plan* plan, EmCand c, const pi_plan::EmMapBlob& maps, float* y_dev, const float* x_dev, int ncols,
+                  long long ld, int coords, cudaStream_t s) {
   const DevicePlan& dp = plan->dev;
   const int npairs = ncols / 2;
   const unsigned ld4 = (unsigned)(ld / 2);
   float4* y4 = (float4*)y_dev;
   if (c.kind == 0) {
-    const unsigned char* maps = em_tensor_maps(plan, x_dev, ld, ncols, c.g);
     if (!maps) return fail(PI_ERR_UNSUPPORTED, "element-major tensor maps could not be encoded");
     pi_plan::EmSplit sp;
     int rc = em_prepare_split(plan, coords, &sp);
@@ -947,7 +953,7 @@ static int em_run(pi_plan* plan, EmCand c, float* y_dev, const float* x_dev, int
       launch = ri == 0 ? launch_em_tma_shape<16, 64> : ri == 1 ? launch_em_tma_shape<32, 64> : launch_em_tma_shape<64, 64>;
     else
       launch = gi == 1 ? launch_em_tma_shape<32, 32> : launch_em_tma_shape<16, 16>;
-    const cudaError_t e = launch(dp.canon_plus != 0, maps, dp.nsectors, tiles, ntiles, sp, y4, ld4, npairs, s);
+    const cudaError_t e = launch(dp.canon_plus != 0, maps->data(), dp.nsectors, tiles, ntiles, sp, y4, ld4, npairs, s);
     if (e != cudaSuccess) return cuda_fail(e, "element-major apply launch (TMA)");
     return PI_OK;
   }
@@ -1003,15 +1009,20 @@ static std::vector<EmCand> em_candidates(const pi_plan* plan, int ncols) {
 // fastest for later calls.
 static int em_tune(pi_plan* plan, float* y_dev, const float* x_dev, int ncols, long long ld, int coords,
                    cudaStream_t s, pi_plan::EmChoice* out) {
-  // a candidate that cannot run on this batch (its tensor maps do not encode, say) drops out
+  // a candidate that cannot run on this batch (its tensor maps do not encode, say) drops out; only
+  // the winner's maps are kept
   std::vector<EmCand> cands;
+  std::vector<pi_plan::EmMapBlob> maps;
   int first_rc = PI_OK;
   for (const EmCand& c : em_candidates(plan, ncols)) {
-    const int rc = em_run(plan, c, y_dev, x_dev, ncols, ld, coords, s);
-    if (rc == PI_OK)
+    const pi_plan::EmMapBlob m = c.kind == 0 ? em_encode_maps(plan, x_dev, ld, ncols, c.g) : nullptr;
+    const int rc = em_run(plan, c, m, y_dev, x_dev, ncols, ld, coords, s);
+    if (rc == PI_OK) {
       cands.push_back(c);
-    else if (first_rc == PI_OK)
+      maps.push_back(m);
+    } else if (first_rc == PI_OK) {
       first_rc = rc;
+    }
   }
   if (cands.empty()) return first_rc;
   std::vector<cudaEvent_t> ev(2 * cands.size() * 2, nullptr);
@@ -1025,7 +1036,7 @@ static int em_tune(pi_plan* plan, float* y_dev, const float* x_dev, int ncols, l
   for (int round = 0; round < 2 && !rc; ++round)
     for (size_t i = 0; i < cands.size() && !rc; ++i) {
       cudaEventRecord(ev[(round * cands.size() + i) * 2], s);
-      rc = em_run(plan, cands[i], y_dev, x_dev, ncols, ld, coords, s);
+      rc = em_run(plan, cands[i], maps[i], y_dev, x_dev, ncols, ld, coords, s);
       cudaEventRecord(ev[(round * cands.size() + i) * 2 + 1], s);
     }
   cudaError_t e = rc ? cudaSuccess : cudaEventSynchronize(ev.back());
@@ -1048,6 +1059,9 @@ static int em_tune(pi_plan* plan, float* y_dev, const float* x_dev, int ncols, l
   for (auto& f : ev) cudaEventDestroy(f);
   if (rc) return rc;
   if (e != cudaSuccess) return cuda_fail(e, "autotuner timing");
+  for (size_t i = 0; i < cands.size(); ++i)
+    if (best.kind == 0 && cands[i].kind == 0 && cands[i].rows == best.rows && cands[i].g == best.g)
+      em_tensor_maps(plan, x_dev, ld, ncols, best.g, maps[i]);
   *out = best;
   return PI_OK;
 }
@@ -1106,7 +1120,8 @@ extern "C" int pi_apply_f32_em(pi_plan* plan, float* y_dev, const float* x_dev, 
       return PI_OK;  // y already holds L x from the timed runs
     }
   }
-  return em_run(plan, EmCand{ch.kind, ch.rows, ch.g}, y_dev, x_dev, ncols, ld, coords, s);
+  const pi_plan::EmMapBlob maps = ch.kind == 0 ? em_tensor_maps(plan, x_dev, ld, ncols, ch.g) : nullptr;
+  return em_run(plan, EmCand{ch.kind, ch.rows, ch.g}, maps, y_dev, x_dev, ncols, ld, coords, s);
 }
 
 extern "C" int pi_apply_f32_em_tuning(pi_plan* plan, int ncols, int coords, int* kind, int* rows, double* ms) {

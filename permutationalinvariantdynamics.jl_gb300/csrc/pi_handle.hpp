@@ -2,6 +2,7 @@
 #pragma once
 
 #include <atomic>
+#include <memory>
 #include <mutex>
 #include <string>
 #include <vector>
@@ -41,12 +42,15 @@ struct pi_plan {
   int em_ntiles = 0;
   const float2* em_planes32[2] = {nullptr, nullptr};
   // Encoded per-sector TMA tensor maps of the last few element-major source batches (host
-  // copies, passed to the kernel by value), keyed by source pointer, stride and width.
+  // copies, passed to the kernel by value), keyed by source pointer, stride, width and right-hand
+  // sides per box.  An apply in another thread may displace a set that this one is about to
+  // launch with, so a set lives as long as somebody holds it.
+  using EmMapBlob = std::shared_ptr<const std::vector<unsigned char>>;  // nsectors x 128 bytes
   struct EmMapSet {
     const void* x;
     long long ld;
-    int ncols, g;                     // width, right-hand sides per box
-    std::vector<unsigned char> maps;  // nsectors x 128 bytes
+    int ncols, g;  // width, right-hand sides per box
+    EmMapBlob maps;
   };
   std::vector<EmMapSet> em_maps;
   // Split coefficient planes of the TMA-staged kernel (entry, row and column planes) per
