@@ -858,6 +858,9 @@ constexpr size_t kTmMapCache = 4;  // map sets kept per plan: one per source bat
 static pi_plan::EmMapBlob em_encode_maps(const pi_plan* plan, const void* x, long long ld, int ncols, int g) {
   const auto encode = tensor_map_encoder();
   if (!encode) return nullptr;
+  // The encoder needs a current context, which a thread without a runtime call so far does not have.
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || cudaSetDevice(dev) != cudaSuccess) return nullptr;
   const auto& secs = plan->host.sectors;
   std::vector<unsigned char> blob(secs.size() * sizeof(CUtensorMap));
   for (size_t s = 0; s < secs.size(); ++s) {

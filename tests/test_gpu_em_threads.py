@@ -11,6 +11,33 @@ from tests import models as M
 pytestmark = pytest.mark.gpu
 
 
+def test_first_apply_of_a_new_thread(lib_built):
+    """A thread whose first CUDA call is an apply of a new batch, pinned to the TMA kernel."""
+    torch = pytest.importorskip("torch")
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    compiled = picuda.compile(M.ensemble_c2(25))
+    x = torch.randn((len(compiled.basis), 16), dtype=torch.complex64, device="cuda")
+    y, ref = torch.zeros_like(x), torch.zeros_like(x)
+    picuda.select_element_major_kernel(compiled, 16, "tma", 32)
+    torch.cuda.synchronize()
+    errors = []
+
+    def worker():
+        try:
+            picuda.apply_element_major_(y, compiled, x)
+        except Exception as err:
+            errors.append(repr(err))
+
+    t = threading.Thread(target=worker)
+    t.start()
+    t.join()
+    picuda.apply_element_major_(ref, compiled, x)
+    torch.cuda.synchronize()
+    assert not errors, errors
+    assert torch.equal(y, ref)
+
+
 @pytest.mark.parametrize("ncols", [16, 64])  # narrow and full blocks
 def test_threads_with_many_batches(lib_built, ncols):
     torch = pytest.importorskip("torch")
