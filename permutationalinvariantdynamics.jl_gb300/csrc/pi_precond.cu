@@ -364,8 +364,8 @@ __device__ __forceinline__ void stage_level(const PrecondDev& P, Slot<T, TI>& L,
   scan_coefs<true>(PA, L.pf, lane);
 }
 
-// t^H z over the entries a thread has written: FP64 with the weights t, or, in population
-// coordinates, where t is one, in double-float.
+// t^H z over a thread's entries: FP64 with the weights t, or, in population coordinates, where t is
+// one, of FP32 values (or double-floats) in triple-float.
 struct TraceSum64 {
   double2 s = make_double2(0.0, 0.0);
   __device__ __forceinline__ void add(const PrecondDev& P, int e, double2 u) {
@@ -375,15 +375,19 @@ struct TraceSum64 {
   }
   __device__ __forceinline__ double2 value() const { return s; }
 };
-struct TraceSumDF {
-  DF x{0.f, 0.f}, y{0.f, 0.f};
+struct TraceSumTF {
+  TF x{0.f, 0.f, 0.f}, y{0.f, 0.f, 0.f};
   __device__ __forceinline__ void add(const PrecondDev&, int, float2 u) {
-    df_add(x, u.x);
-    df_add(y, u.y);
+    tf_add(x, u.x);
+    tf_add(y, u.y);
   }
-  __device__ __forceinline__ double2 value() const {
-    return make_double2((double)x.hi + (double)x.lo, (double)y.hi + (double)y.lo);
+  __device__ __forceinline__ void add(DF u, DF v) {
+    tf_add(x, u.hi);
+    tf_add(x, u.lo);
+    tf_add(y, v.hi);
+    tf_add(y, v.lo);
   }
+  __device__ __forceinline__ double2 value() const { return make_double2(tf_value(x), tf_value(y)); }
 };
 
 // The solution of a level goes from its slot to z, and into the sum t^H z where that is wanted.
@@ -477,11 +481,15 @@ __device__ __forceinline__ void solve_level(const PrecondDev& Pd, Slot<T, TI>& L
 
 // The d = 0 chain's correction z -= k w0 at entries c0 .. c1.  One block does it for the whole
 // chain (10,201 entries at N = 200), so eight entries per thread are in flight together: one by
-// one, their two dependent gathers took a third of the sweep.
+// one, their two dependent gathers took a third of the sweep.  Returns the thread's share of t^H z,
+// summed over the corrected values before they are rounded to TO: the free entry balances the trace
+// of what was stored, and t^H y_r - k t^H w0 from sums of its own is off by the roundings of
+// two large sums (N = 61..128 in FP64: 2e-14 of sum t |z|, against 2e-16).
 constexpr int kTailUnroll = 8;
 
 template <typename TO>
-__device__ __forceinline__ void chain0_correct(const PrecondDev& Pd, TO* z, int c0, int c1, double2 k) {
+__device__ __forceinline__ double2 chain0_correct(const PrecondDev& Pd, TO* z, int c0, int c1, double2 k) {
+  TraceSum64 sum;
   for (int e0 = c0 + threadIdx.x; e0 < c1; e0 += kTailUnroll * blockDim.x) {
     int el[kTailUnroll];
     double2 w[kTailUnroll], v[kTailUnroll];
@@ -499,13 +507,16 @@ __device__ __forceinline__ void chain0_correct(const PrecondDev& Pd, TO* z, int 
       v[q].x = fma(-k.x, w[q].x, fma(k.y, w[q].y, v[q].x));
       v[q].y = fma(-k.x, w[q].y, fma(-k.y, w[q].x, v[q].y));
       store_as<TO, double2>(z + el[q], v[q]);
+      sum.add(Pd, e0 + q * blockDim.x, v[q]);
     }
   }
+  return sum.value();
 }
 
 // The same for FP32 vectors: in double-float, as each conversion and FP64 operation of a warp
 // holds a quarter of the SM's FP64 pipe for 64 cycles.
-__device__ __forceinline__ void chain0_correct_df(const PrecondDev& Pd, float2* z, int c0, int c1, double2 k) {
+__device__ __forceinline__ double2 chain0_correct_df(const PrecondDev& Pd, float2* z, int c0, int c1, double2 k) {
+  TraceSumTF sum;
   const DF kx{(float)k.x, (float)(k.x - (double)(float)k.x)}, ky{(float)k.y, (float)(k.y - (double)(float)k.y)};
   for (int e0 = c0 + threadIdx.x; e0 < c1; e0 += kTailUnroll * blockDim.x) {
     int el[kTailUnroll];
@@ -531,8 +542,10 @@ __device__ __forceinline__ void chain0_correct_df(const PrecondDev& Pd, float2* 
       df_axpy(zy, -ky.hi, -ky.lo, w[q].x);
       zy.lo = fmaf(-kx.hi, w[q].w, fmaf(-ky.hi, w[q].y, zy.lo));
       z[el[q]] = make_float2(zx.hi + zx.lo, zy.hi + zy.lo);
+      sum.add(zx, zy);
     }
   }
+  return sum.value();
 }
 
 template <typename T, typename TI, typename TO>
@@ -545,6 +558,7 @@ __global__ void __launch_bounds__(kSweepThreads<T>, 2)
   const int lev0 = Pd.chain_lev[chain], lev1 = Pd.chain_lev[chain + 1];
   const int nlev = lev1 - lev0;
   const bool chain0 = chain == Pd.chain0;
+  const bool sum_t = chain0 && Pd.mode == 1;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   constexpr int kSlots = Ring<T>::SLOTS, NS = Ring<T>::NS;
   for (int k = tid; k <= nlev; k += blockDim.x) S.lev_ent[k] = Pd.lev_ent[lev0 + k];
@@ -562,7 +576,7 @@ __global__ void __launch_bounds__(kSweepThreads<T>, 2)
   bool has_rho = false;
   if (warp > 0) {
     const T sT = (T)s;
-    typename std::conditional<std::is_same<T, float>::value, TraceSumDF, TraceSum64>::type sum;
+    typename std::conditional<std::is_same<T, float>::value, TraceSumTF, TraceSum64>::type sum;
     for (int k = warp - 1; k < nlev + kSlots; k += NS) {
       // level k takes the slot of level k - kSlots, whose solution level k - kSlots + 1 has read
       const int out = k - kSlots;
@@ -573,7 +587,7 @@ __global__ void __launch_bounds__(kSweepThreads<T>, 2)
           break;
         }
         const int e0 = S.lev_ent[out], cnt = S.lev_ent[out + 1] - e0;
-        drain_level<T, TI, TO>(Pd, S.slot[out % kSlots], z, e0, cnt, chain0, lane, sum);
+        drain_level<T, TI, TO>(Pd, S.slot[out % kSlots], z, e0, cnt, sum_t, lane, sum);
         __syncwarp();
       }
       if (k < nlev) {
@@ -612,31 +626,32 @@ __global__ void __launch_bounds__(kSweepThreads<T>, 2)
   }
   if (!chain0) return;
   const int c0 = Pd.chain0_ent, c1 = Pd.lev_ent[lev1];
-  const double2 tz = block_sum2(tsum, S.red);  // t^H y, the free entry apart
   double2 k;
   if (Pd.mode == 0) {
     // beta = rho_r / rho_v; y = y_r - beta y_v; z_f = (beta - t^H y) / t_f
     if (has_rho) {  // one lane
       const double2 iv = Pd.sm_coef;  // 1 / rho_v
-      const double2 beta = make_double2(rho_r.x * iv.x - rho_r.y * iv.y, rho_r.x * iv.y + rho_r.y * iv.x);
-      const double2 sv = Pd.free_coef;  // (1 + t^H y_v) / t_f
-      const double it = Pd.free_inv;    // 1 / t_f
-      S.red[0] = beta.x;
-      S.red[1] = beta.y;
-      store_as<TO, double2>(z + Pd.elem[Pd.free_ent],
-                            make_double2(fma(beta.x, sv.x, fma(-beta.y, sv.y, -tz.x * it)),
-                                         fma(beta.x, sv.y, fma(beta.y, sv.x, -tz.y * it))));
+      S.red[0] = rho_r.x * iv.x - rho_r.y * iv.y;
+      S.red[1] = rho_r.x * iv.y + rho_r.y * iv.x;
     }
     __syncthreads();
     k = make_double2(S.red[0], S.red[1]);
+    __syncthreads();  // red is free
   } else {
     // Sherman-Morrison: z -= w0 (t^H y) / (1 + t^H w0)
+    const double2 tz = block_sum2(tsum, S.red);
     k = make_double2(tz.x * Pd.sm_coef.x - tz.y * Pd.sm_coef.y, tz.x * Pd.sm_coef.y + tz.y * Pd.sm_coef.x);
   }
+  double2 share;
   if constexpr (std::is_same<T, float>::value && std::is_same<TO, float2>::value)
-    chain0_correct_df(Pd, z, c0, c1, k);
+    share = chain0_correct_df(Pd, z, c0, c1, k);
   else
-    chain0_correct(Pd, z, c0, c1, k);
+    share = chain0_correct(Pd, z, c0, c1, k);
+  if (Pd.mode != 0) return;
+  const double2 tz = block_sum2(share, S.red);  // of every entry but the free one, which is zero so far
+  if (tid == 0 && Pd.free_ent >= 0)
+    store_as<TO, double2>(z + Pd.elem[Pd.free_ent],
+                          make_double2((k.x - tz.x) / Pd.free_t, (k.y - tz.y) / Pd.free_t));
 }
 
 template <typename T, typename TI, typename TO>
@@ -1093,15 +1108,10 @@ int pi_precond_create(pi_plan* plan, int coords, double regularization, double o
   P->dev.chain0_ent = H.chain0_ent;
   P->dev.free_ent = H.free_ent;
   P->dev.mode = H.mode;
-  // mode 0: 1 / rho_v, and z_f = (beta (1 + t^H y_v) - t^H y_r) / t_f
+  // mode 0: 1 / rho_v
   const std::complex<double> coef = H.mode == 0 ? 1.0 / H.sm_coef : H.sm_coef;
   P->dev.sm_coef = make_double2(coef.real(), coef.imag());
-  if (H.mode == 0) {
-    std::complex<double> tv = 1.0;
-    for (size_t i = 0; i < H.w0.size(); ++i) tv += H.t0[i] * H.w0[i];
-    P->dev.free_inv = 1.0 / H.t0[H.free_ent - H.chain0_ent];
-    P->dev.free_coef = make_double2(tv.real() * P->dev.free_inv, tv.imag() * P->dev.free_inv);
-  }
+  if (H.free_ent >= 0) P->dev.free_t = H.t0[H.free_ent - H.chain0_ent];
   P->setup_seconds = std::chrono::duration<double>(std::chrono::steady_clock::now() - t0).count();
   *out = P;
   return PI_OK;

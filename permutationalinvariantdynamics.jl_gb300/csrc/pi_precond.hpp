@@ -60,8 +60,7 @@ struct PrecondDev {
   const double2* w0;
   const float4* w0f;  // w0 as double-floats
   double2 sm_coef;    // 1 / rho_v (mode 0) or 1 / (1 + t^H w0) (mode 1)
-  double2 free_coef;  // mode 0: (1 + t^H y_v) / t_f
-  double free_inv;    // and 1 / t_f
+  double free_t;      // mode 0: t at the free entry
   int chain0;
   int chain0_ent;
   int free_ent;

@@ -51,6 +51,28 @@ __device__ __forceinline__ DF df_sum(DF a, DF b) {
   return DF{s, (a.lo + b.lo) + err};
 }
 
+// Triple-float accumulator: the sum in hi, the rounding errors of its additions in mid, the errors
+// of those in lo (TwoSum twice).  About 70 bits, so a sum of FP32 values or of double-floats is no
+// further off than in FP64, and it stays off the FP64 pipe like a double-float.
+struct TF {
+  float hi, mid, lo;
+};
+__host__ __device__ __forceinline__ float two_sum(float a, float b, float* err) {
+  const float s = a + b;
+  const float bb = s - a;
+  *err = (a - (s - bb)) + (b - bb);
+  return s;
+}
+__host__ __device__ __forceinline__ void tf_add(TF& a, float t) {
+  float e, e2;
+  a.hi = two_sum(a.hi, t, &e);
+  a.mid = two_sum(a.mid, e, &e2);
+  a.lo += e2;
+}
+__host__ __device__ __forceinline__ double tf_value(const TF& a) {
+  return (double)a.hi + ((double)a.mid + (double)a.lo);
+}
+
 // Lane sums of NV values (a power of two) by exchanging halves of the values: NV - 1 additions
 // and a few more, against 5 NV one value at a time.  Afterwards v[0] of lane l is the total of
 // value l / (32 / NV).
