@@ -57,8 +57,9 @@ __device__ __forceinline__ double2 load_c(const T2* p) {
 // FMAs of absent columns would be issued all the same, and a pass per power of two (4, 2, 1)
 // reads w and waits for memory as often.  Lane sums exchange halves of the accumulators (16
 // additions for 8 columns against 80 one by one, which at N = 200 took as long as the products);
-// FP32 vectors are summed in double-float until one value per lane is left, as a conversion holds
-// the FP64 pipe like an addition.  FP32 in 64 registers, so that all 608 blocks are resident at
+// those of FP32 vectors are triple-float until one value per lane is left, as a conversion holds
+// the FP64 pipe like an addition (double-float lane sums lose ten times what the accumulators do
+// at a few thousand elements: 2e-16 of |v| |w| against 6e-18).  FP32 in 64 registers, so that all 608 blocks are resident at
 // once, and one element at a time: N = 200, 7, 8, 15 and 16 columns 36, 52, 58 and 52 us with
 // passes and 66 registers (three blocks per SM, two rounds), 21, 24, 38 and 34 us now (26 us of
 // memory time for 16); two elements at a time take 24, 33, 56 and 53 us.
@@ -109,10 +110,10 @@ __device__ __forceinline__ void dot_cols(const float2* __restrict__ V, long long
       df_add_prod(acc[2 * k + 1], -v.y, wv.x);
     }
   }
-  warp_transpose_sum<NV>(acc);
+  const TF total = warp_transpose_total<NV>(acc);
   constexpr int span = 32 / NV;
   const int lane = threadIdx.x & 31;
-  if (lane % span == 0) row[lane / span] = (double)acc[0].hi + (double)acc[0].lo;
+  if (lane % span == 0) row[lane / span] = tf_value(total);
 }
 
 template <typename T2>

@@ -4,74 +4,9 @@
 
 #include <cuda_runtime.h>
 
+#include "pi_float.cuh"
+
 namespace picuda {
-
-// Double-float accumulator: the pair (hi, lo) carries a ~48-bit significand on the FP32
-// pipes (GB300 issues FP64 at 1/64 of the FP32 rate).
-struct DF {
-  float hi, lo;
-};
-
-// a += t, the rounding error of the addition carried in a.lo (Knuth's TwoSum).
-__device__ __forceinline__ void df_add(DF& a, float t) {
-  const float s = a.hi + t;
-  const float bb = s - a.hi;
-  const float err = (a.hi - (s - bb)) + (t - bb);
-  a.hi = s;
-  a.lo += err;
-}
-
-// acc += a b, the product split exactly with an FMA.
-__device__ __forceinline__ void df_add_prod(DF& acc, float a, float b) {
-  const float p = a * b;
-  const float e = fmaf(a, b, -p);
-  const float s = acc.hi + p;
-  const float bb = s - acc.hi;
-  const float err = (acc.hi - (s - bb)) + (p - bb);
-  acc.hi = s;
-  acc.lo += err + e;
-}
-
-// acc += (ch + cl) v.
-__device__ __forceinline__ void df_axpy(DF& acc, float ch, float cl, float v) {
-  const float p = ch * v;
-  const float e = fmaf(ch, v, -p);
-  const float s = acc.hi + p;
-  const float bb = s - acc.hi;
-  const float err = (acc.hi - (s - bb)) + (p - bb);
-  acc.hi = s;
-  acc.lo += err + fmaf(cl, v, e);
-}
-
-// a + b (TwoSum of the leading parts).
-__device__ __forceinline__ DF df_sum(DF a, DF b) {
-  const float s = a.hi + b.hi;
-  const float bb = s - a.hi;
-  const float err = (a.hi - (s - bb)) + (b.hi - bb);
-  return DF{s, (a.lo + b.lo) + err};
-}
-
-// Triple-float accumulator: the sum in hi, the rounding errors of its additions in mid, the errors
-// of those in lo (TwoSum twice).  About 70 bits, so a sum of FP32 values or of double-floats is no
-// further off than in FP64, and it stays off the FP64 pipe like a double-float.
-struct TF {
-  float hi, mid, lo;
-};
-__host__ __device__ __forceinline__ float two_sum(float a, float b, float* err) {
-  const float s = a + b;
-  const float bb = s - a;
-  *err = (a - (s - bb)) + (b - bb);
-  return s;
-}
-__host__ __device__ __forceinline__ void tf_add(TF& a, float t) {
-  float e, e2;
-  a.hi = two_sum(a.hi, t, &e);
-  a.mid = two_sum(a.mid, e, &e2);
-  a.lo += e2;
-}
-__host__ __device__ __forceinline__ double tf_value(const TF& a) {
-  return (double)a.hi + ((double)a.mid + (double)a.lo);
-}
 
 // Lane sums of NV values (a power of two) by exchanging halves of the values: NV - 1 additions
 // and a few more, against 5 NV one value at a time.  Afterwards v[0] of lane l is the total of
@@ -108,6 +43,40 @@ __device__ __forceinline__ void warp_transpose_sum(DF (&v)[NV]) {
   }
   for (; off >= 1; off >>= 1)
     v[0] = df_sum(v[0], DF{__shfl_xor_sync(0xffffffffu, v[0].hi, off), __shfl_xor_sync(0xffffffffu, v[0].lo, off)});
+}
+
+// The same for double-floats, exactly enough that the lane sums add nothing to the error of the
+// accumulators (pi_float.cuh): v[0] of lane l in triple-float.
+template <int NV>
+__device__ __forceinline__ TF warp_transpose_total(const DF (&v)[NV]) {
+  static_assert(NV >= 2, "the first exchange halves the values");
+  const int lane = threadIdx.x & 31;
+  const bool up = lane & 16;
+  TF t[NV / 2];
+#pragma unroll
+  for (int i = 0; i < NV / 2; ++i) {
+    const DF send = up ? v[i] : v[i + NV / 2], keep = up ? v[i + NV / 2] : v[i];
+    t[i] = tf_pair(keep, DF{__shfl_xor_sync(0xffffffffu, send.hi, 16), __shfl_xor_sync(0xffffffffu, send.lo, 16)});
+  }
+  auto other = [](const TF& a, int off) {
+    return TF{__shfl_xor_sync(0xffffffffu, a.hi, off), __shfl_xor_sync(0xffffffffu, a.mid, off),
+              __shfl_xor_sync(0xffffffffu, a.lo, off)};
+  };
+#pragma unroll
+  for (int step = 1; step < 5; ++step) {
+    const int off = 16 >> step, left = NV >> (step + 1);  // values left after this step (0: one, summed on)
+    const bool high = lane & off;
+    if (left == 0) {
+      t[0] = tf_sum(t[0], other(t[0], off));
+      continue;
+    }
+#pragma unroll
+    for (int i = 0; i < left; ++i) {
+      const TF send = high ? t[i] : t[i + left], keep = high ? t[i + left] : t[i];
+      t[i] = tf_sum(keep, other(send, off));
+    }
+  }
+  return t[0];
 }
 
 }  // namespace picuda
