@@ -96,8 +96,9 @@ int pi_plan_adjoint(const pi_plan* plan, pi_plan** out);
  * MatrixFreeLiouvillian does for shared tasks (liouvillian.jl:35-60).  PI_CONCURRENCY_REJECT
  * makes a call that finds the plan in use return PI_ERR_BUSY at once, the rule of the
  * reference's per-task workspaces (threaded_apply.jl:575).  The device-pointer applies
- * (pi_apply_f64, pi_apply_f32, pi_apply_f32_em) only read the plan and run on the caller's
- * stream, so they never wait. */
+ * (pi_apply_f64, pi_apply_f32, pi_apply_f32_em) run on the caller's stream and never wait for
+ * those calls.  What they share is the coefficient planes, which the first apply of a precision
+ * and coordinate system lays out and later ones only read (see pi_apply_f64). */
 #define PI_CONCURRENCY_WAIT 0
 #define PI_CONCURRENCY_REJECT 1
 int pi_plan_set_concurrency(pi_plan* plan, int mode);
@@ -111,7 +112,9 @@ typedef struct {
   long long stencil_terms; /* total stencil terms over all sectors */
   size_t device_bytes;     /* device memory owned by the plan tables */
   int batched_kernel;      /* applies with >= 2 columns: 0 general tile kernel, 1 fixed-structure
-                              register kernel, 2 canonical-position register-reuse kernel */
+                              register kernel, 2 canonical positions: every apply runs from merged
+                              coefficient planes, one thread per entry (where they have no room,
+                              from the kernel of 1) */
 } pi_plan_info_t;
 int pi_plan_info(const pi_plan* plan, pi_plan_info_t* out);
 
@@ -158,7 +161,12 @@ int pi_sector_multiplicity(int N, int k, double* f, double* sqrt_f);
 /* y = L x for ncols right-hand sides with leading dimension ld (elements), device
  * buffers, complex FP64 reference coordinates, enqueued on `stream` (a cudaStream_t;
  * NULL is the CUDA default stream) without synchronizing.
- * Aliasing of x and y is rejected (liouvillian.jl:3220-3221). */
+ * Aliasing of x and y is rejected (liouvillian.jl:3220-3221).
+ * On a plan with batched_kernel == 2 the first apply of a precision and coordinate system lays
+ * out its merged coefficient planes: it allocates them (8 bytes in FP64, 4 in FP32, per PI
+ * coordinate and plane, with two planes and one per gain position of the stencil, at most ten) and
+ * fills them on a stream that the plan uses for nothing else, for which `stream` waits on the GPU.
+ * The host waits for that fill only when `stream` is being captured into a graph. */
 int pi_apply_f64(pi_plan* plan, double* y_dev, const double* x_dev, int ncols, long long ld,
                  void* stream);
 /* Same action in complex FP32, in reference (x) or population (z = sqrt(f) x)

@@ -71,7 +71,7 @@ int pi_arnoldi(pi_plan* plan, const double* v0_dev, int m, double* V_dev, long l
   if (rc == PI_OK) z.chk(scale_f64(reinterpret_cast<const double2*>(v0_dev), col(0), n, make_double2(1.0 / nq, 0.0), 0, s));
   const double breakfactor = std::numeric_limits<double>::epsilon();
   const BorderArgs none{1.0, nullptr, 0};
-  const Planes64 P = planes64(plan, PI_COORDS_REFERENCE);
+  const Planes64 P = planes64(plan, PI_COORDS_REFERENCE, s);
   for (int j = 0; j < m && rc == PI_OK && z.err == cudaSuccess; ++j) {
     double2* w = col(j + 1);
     const double* vj = reinterpret_cast<const double*>(col(j));

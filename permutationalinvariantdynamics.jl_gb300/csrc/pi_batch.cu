@@ -2391,12 +2391,12 @@ void Engine::rebuild() {
     int strips = 0;
     if (f32_) {
       if (plan->dev.canon && em_split_planes(plan, jobs_[i]->bordered ? 0 : 1, &p32[i]) == PI_OK)
-        it32[i] = strip_items(plan);
+        it32[i] = strip_items(plan, s_);
       else
         p32[i] = SplitPlanes{nullptr, nullptr, nullptr, nullptr, 0};
       strips = it32[i].n;
     } else {
-      p64[i] = planes64(plan, PI_COORDS_REFERENCE);
+      p64[i] = planes64(plan, PI_COORDS_REFERENCE, s_);
       strips = p64[i].nitems;
     }
     const int ntiles = plan->dev.ntiles;

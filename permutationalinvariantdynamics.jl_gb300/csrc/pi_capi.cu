@@ -62,6 +62,7 @@ void free_plan(pi_plan* plan) {
   cudaGetDevice(&cur);
   cudaSetDevice(plan->device);
   if (plan->stream) cudaStreamSynchronize(plan->stream);
+  if (plan->fill_stream) cudaStreamSynchronize(plan->fill_stream);
   release_plan_engine(plan);
   for (void* p : plan->allocations) cudaFree(p);
   if (plan->stage_x) cudaFree(plan->stage_x);
@@ -70,6 +71,10 @@ void free_plan(pi_plan* plan) {
     if (ps) cudaStreamDestroy(ps);
   if (plan->host_pinned) cudaFreeHost(plan->host_pinned);
   if (plan->stream) cudaStreamDestroy(plan->stream);
+  for (TableFill* f : {&plan->items_fill, &plan->planes64_fill[0], &plan->planes64_fill[1], &plan->planes32_fill[0],
+                       &plan->planes32_fill[1]})
+    if (f->ready) cudaEventDestroy(f->ready);
+  if (plan->fill_stream) cudaStreamDestroy(plan->fill_stream);
   cudaSetDevice(cur);
   delete plan;
 }
@@ -104,6 +109,7 @@ int upload_plan(pi_plan* plan) {
   };
   // grouped terms of every sector, kept for the fixed-structure table below
   std::vector<std::array<std::vector<DevTerm>, G_COUNT>> by_group(S);
+  int lines = 0, items = 0;
   for (int s = 0; s < S; ++s) {
     const Sector& sec = hp.sectors[s];
     DevSector& ds = sectors[s];
@@ -114,6 +120,10 @@ int upload_plan(pi_plan* plan) {
     ds.border_x = sec.sqrt_f / hp.trace_norm2;
     ds.border_z = sec.f / hp.trace_norm2;
     ds.sqrt_f = sec.sqrt_f;
+    ds.line0 = lines;
+    ds.item0 = items;
+    lines += sec.n;
+    items += (int)(((long long)sec.n * sec.n + 31) / 32);
     if ((int)sec.terms.size() > kMaxSectorTerms)
       return fail(PI_ERR_UNSUPPORTED, "a sector has more stencil terms than the apply kernel stages");
     ds.src[0] = ds.src[1] = ds.src[2] = -1;
@@ -315,6 +325,8 @@ int upload_plan(pi_plan* plan) {
   plan->dev.ntiles = (int)tiles.size();
   plan->dev.ndiag = (int)diag_index.size();
   plan->dev.dim = hp.dim;
+  plan->nlines = lines;
+  plan->nstrip_items = items;
   plan->stencil_terms = (long long)terms.size();
   plan->rs.partial = (double2*)plan_alloc(plan, sizeof(double2) * kReduceBlocks * kMaxDots);
   plan->rs.result = (double2*)plan_alloc(plan, sizeof(double2) * kMaxDots);
@@ -585,6 +597,13 @@ static int finish_plan(pi_plan* plan, pi_plan** out) {
     delete plan;
     return cuda_fail(e, "cudaStreamCreate");
   }
+  int lowest = 0, highest = 0;
+  cudaDeviceGetStreamPriorityRange(&lowest, &highest);
+  e = cudaStreamCreateWithPriority(&plan->fill_stream, cudaStreamNonBlocking, highest);
+  if (e != cudaSuccess) {
+    free_plan(plan);
+    return cuda_fail(e, "cudaStreamCreate");
+  }
   for (auto& ps : plan->pipe) {
     e = cudaStreamCreateWithFlags(&ps, cudaStreamNonBlocking);
     if (e != cudaSuccess) {
@@ -748,7 +767,7 @@ int pi_apply_f64(pi_plan* plan, double* y_dev, const double* x_dev, int ncols, l
   if (rc) return rc;
   BorderArgs border{1.0, nullptr, 0};
   cudaStream_t s = (cudaStream_t)stream;  // NULL is the CUDA default stream
-  const Planes64 P = planes64(plan, PI_COORDS_REFERENCE);
+  const Planes64 P = planes64(plan, PI_COORDS_REFERENCE, s);
   cudaError_t e = P.items ? launch_apply_strip<double>(plan->dev, P, x_dev, y_dev, ncols, ld, border, s)
                           : launch_apply_f64(plan->dev, x_dev, y_dev, ncols, ld, border, s);
   if (e != cudaSuccess) return cuda_fail(e, "apply launch");
@@ -763,7 +782,7 @@ int pi_apply_f32(pi_plan* plan, float* y_dev, const float* x_dev, int ncols, lon
     return fail(PI_ERR_INVALID_ARGUMENT, "coords must be PI_COORDS_REFERENCE or PI_COORDS_POPULATION");
   BorderArgs border{1.0, nullptr, coords};
   cudaStream_t s = (cudaStream_t)stream;  // NULL is the CUDA default stream
-  const Planes32 P = planes32(plan, coords);
+  const Planes32 P = planes32(plan, coords, s);
   cudaError_t e = P.items ? launch_apply_strip<float>(plan->dev, P, x_dev, y_dev, ncols, ld, border, s)
                           : launch_apply_f32(plan->dev, x_dev, y_dev, ncols, ld, border, s);
   if (e != cudaSuccess) return cuda_fail(e, "apply launch");
@@ -811,10 +830,11 @@ static int apply_host(pi_plan* plan, void* y_host, const void* x_host, int ncols
   const int chunk = std::max(1, (ncols + nchunks - 1) / nchunks);
   BorderArgs border{1.0, nullptr, coords};
   StripPlanes<T> P;
-  if constexpr (sizeof(T) == sizeof(double))
-    P = planes64(plan, coords);
-  else
-    P = planes32(plan, coords);
+  for (const auto& ps : plan->pipe)
+    if constexpr (sizeof(T) == sizeof(double))
+      P = planes64(plan, coords, ps);
+    else
+      P = planes32(plan, coords, ps);
   int k = 0;
   for (int c0 = 0; c0 < ncols && e == cudaSuccess; c0 += chunk, ++k) {
     const int nc = std::min(chunk, ncols - c0);

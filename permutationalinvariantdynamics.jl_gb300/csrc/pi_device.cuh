@@ -32,6 +32,7 @@ struct DevSector {
   double border_x;     // normalized trace vector v = t/|t|^2 on the diagonal, x coordinates
   double border_z;     // the same vector in population coordinates (f / |t|^2)
   double sqrt_f;       // sqrt(f^nu): z = sqrt_f * x
+  int line0, item0;    // first line and first strip item of the block (pi_strip.cu)
 };
 
 // One separable stencil term (see pi_plan.hpp); its group fixes kind and class.  The

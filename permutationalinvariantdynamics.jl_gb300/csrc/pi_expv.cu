@@ -407,7 +407,7 @@ int pi_expv(pi_plan* plan, double* x_dev, double t, const pi_expv_opts_t* opts, 
   pi_expv_info_t loc;
   ExpvWork W{plan, plan->stream, plan->host.dim, (int)std::min<long long>(opts->krylovdim, plan->host.dim),
              opts->precision == PI_FP32};
-  if (!W.mixed) W.planes = planes64(plan, PI_COORDS_REFERENCE);
+  if (!W.mixed) W.planes = planes64(plan, PI_COORDS_REFERENCE, W.s);
   {
     Bufs B;
     B.s = W.s;
@@ -452,7 +452,7 @@ int pi_solve_dynamics(pi_plan* plan, double* rho_dev, int nt, const double* time
   }
   ExpvWork W{plan, plan->stream, plan->host.dim, (int)std::min<long long>(opts->krylovdim, plan->host.dim),
              opts->precision == PI_FP32};
-  if (!W.mixed) W.planes = planes64(plan, PI_COORDS_REFERENCE);
+  if (!W.mixed) W.planes = planes64(plan, PI_COORDS_REFERENCE, W.s);
   pi_expv_info_t total;
   std::memset(&total, 0, sizeof(total));
   total.converged = 1;

@@ -12,7 +12,14 @@
 
 namespace picuda {
 class Engine;
-}
+
+// A table that is filled on the plan's fill stream: `ready` is recorded behind the fill, `done` once
+// it is known to have passed.
+struct TableFill {
+  cudaEvent_t ready = nullptr;
+  bool done = false;
+};
+}  // namespace picuda
 
 struct pi_plan {
   picuda::QubitPlan host;
@@ -77,15 +84,18 @@ struct pi_plan {
   };
   std::vector<EmChoice> em_choices;
   std::mutex em_tune_mu;
-  // Merged coefficient planes per coordinate system, built on first use (guarded by em_mu); a
-  // plan without room for them keeps the general kernels.
+  // Strip items and merged coefficient planes per coordinate system, built on first use (guarded by
+  // em_mu); a plan without room for them keeps the general kernels.  They are filled on a stream
+  // of their own, on which nothing else runs: a first apply waits on the GPU for the fill only, not
+  // for the solves that `stream` has queued.
+  cudaStream_t fill_stream = nullptr;
+  const picuda::StripItem* strip_items = nullptr;
+  int nstrip_items = 0, nlines = 0;
   picuda::Planes64 planes64[2];
   picuda::Planes32 planes32[2];
+  picuda::TableFill items_fill, planes64_fill[2], planes32_fill[2];
   bool planes64_failed[2] = {false, false};
   bool planes32_failed[2] = {false, false};
-  const picuda::StripItem* strip_items = nullptr;
-  const int2* strip_first = nullptr;  // per sector: first line, first strip item
-  int nstrip_items = 0;
   // Single-instance solves run as one job of a batched engine kept with the plan (created on
   // first use for a Krylov dimension and basis precision, replaced when those change).
   picuda::Engine* engine = nullptr;
@@ -128,17 +138,17 @@ void* plan_alloc(pi_plan* plan, size_t bytes);
 int em_split_planes(pi_plan* plan, int which, SplitPlanes* out);
 
 // Strip items of a plan (32 consecutive entries of one sector block each), built on first use;
-// items == nullptr without room for them.
+// items == nullptr without room for them.  Work that stream s gets after the call may read them.
 struct StripItems {
   const StripItem* items = nullptr;
   int n = 0;
 };
-StripItems strip_items(pi_plan* plan);
+StripItems strip_items(pi_plan* plan, cudaStream_t s);
 
 // Merged coefficient planes of a canonical plan in reference (coords 0) or population (1)
-// coordinates, built on first use (pi_strip.cu); items == nullptr when the plan is not canonical
-// or has no room for them.
-Planes64 planes64(pi_plan* plan, int coords);
-Planes32 planes32(pi_plan* plan, int coords);
+// coordinates, built on first use (pi_strip.cu), for work that stream s gets after the call;
+// items == nullptr when the plan is not canonical or has no room for them.
+Planes64 planes64(pi_plan* plan, int coords, cudaStream_t s);
+Planes32 planes32(pi_plan* plan, int coords, cudaStream_t s);
 
 }  // namespace picuda

@@ -356,7 +356,7 @@ int rk4_run(pi_plan* plan, double2* rho, int nt, const double* times, int steps,
     };
     record(0);
     StageKernel k[4];
-    const Planes64 p64 = mixed ? Planes64{} : planes64(plan, PI_COORDS_REFERENCE);
+    const Planes64 p64 = mixed ? Planes64{} : planes64(plan, PI_COORDS_REFERENCE, s);
     chk(stage_kernels(mixed, p64, k));
     // A graph of kernel nodes costs about 1.7 us a node to build and instantiate on each call, and a
     // launch of it some microseconds of the host that run ahead of the device: short graphs

@@ -626,9 +626,9 @@ int pi_steady_state(pi_plan* plan, double* x_dev, const pi_gmres_opts_t* opts, p
   const int coords = opts->coords;
   Run R(plan, coords);
   if (opts->precision == PI_FP64)
-    R.planes = planes64(plan, coords);
+    R.planes = planes64(plan, coords, R.s);
   else
-    R.planes_f32 = planes32(plan, coords);
+    R.planes_f32 = planes32(plan, coords, R.s);
   const long long n = R.n;
   const int m = (int)std::min<long long>(opts->krylovdim, n);
   pi_gmres_info_t loc;

@@ -1,6 +1,5 @@
 // Coefficient planes of the strip apply (pi_strip.cuh) and its launches.
 #include <algorithm>
-#include <vector>
 
 #include "../../include/picuda.h"
 #include "pi_strip.cuh"
@@ -10,9 +9,8 @@
 namespace picuda {
 namespace {
 
-// Strip items of sector blockIdx.y; first[s] = (first line, first item) of sector s.
-__global__ void k_strip_items(const DevSector* __restrict__ sectors, const int2* __restrict__ first,
-                              StripItem* __restrict__ items) {
+// Strip items of sector blockIdx.y.
+__global__ void k_strip_items(const DevSector* __restrict__ sectors, StripItem* __restrict__ items) {
   const int s = blockIdx.y;
   const DevSector& sec = sectors[s];
   const int n = sec.n;
@@ -21,21 +19,20 @@ __global__ void k_strip_items(const DevSector* __restrict__ sectors, const int2*
   it.n = n;
   if (sec.src[0] >= 0) it.off0 = (int)sectors[sec.src[0]].offset, it.m0 = sectors[sec.src[0]].n;
   if (sec.src[2] >= 0) it.off2 = (int)sectors[sec.src[2]].offset, it.m2 = sectors[sec.src[2]].n;
-  it.loff = first[s].x;
+  it.loff = sec.line0;
   it.sector = s;
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; 32LL * i < (long long)n * n; i += gridDim.x * blockDim.x) {
     it.local0 = 32 * i;
-    items[first[s].y + i] = it;
+    items[sec.item0 + i] = it;
   }
 }
 
 // Planes and line tables of sector blockIdx.y, merged in FP64 for either precision.  The sums run
-// over the terms in use, not the table's zero padding.  First apply of a plan, with the planes and
-// without the second table copy and wait: N = 8 100 -> 90 us, N = 97 FP32 230 -> 218.
+// over the terms in use, not the table's zero padding.
 template <typename T>
 __global__ void k_planes(const DevSector* __restrict__ sectors, const int4* __restrict__ canon,
-                         const double2* __restrict__ coef, const int2* __restrict__ first, const StripPlanes<T> P,
-                         int nr, const TermCounts terms, T* __restrict__ plane, typename Vec2<T>::type* __restrict__ lrow,
+                         const double2* __restrict__ coef, const StripPlanes<T> P, int nr, const TermCounts terms,
+                         T* __restrict__ plane, typename Vec2<T>::type* __restrict__ lrow,
                          typename Vec2<T>::type* __restrict__ rcol) {
   using T2 = typename Vec2<T>::type;
   const int s = blockIdx.y;
@@ -66,8 +63,8 @@ __global__ void k_planes(const DevSector* __restrict__ sectors, const int4* __re
   }
   if (blockIdx.x == 0)
     for (int i = threadIdx.x; i < n; i += blockDim.x) {
-      lrow[first[s].x + i] = T2{(T)coef[ct[1].x + i].y, (T)coef[ct[2].x + i].y};
-      rcol[first[s].x + i] = T2{(T)coef[ct[3].y + i].y, (T)coef[ct[4].y + i].y};
+      lrow[sec.line0 + i] = T2{(T)coef[ct[1].x + i].y, (T)coef[ct[2].x + i].y};
+      rcol[sec.line0 + i] = T2{(T)coef[ct[3].y + i].y, (T)coef[ct[4].y + i].y};
     }
 }
 
@@ -123,15 +120,27 @@ struct RelaxedCapture {
 
 }  // namespace
 
-// Per sector (first line, first strip item); returns the totals.
-static int2 strip_starts(const pi_plan* plan, std::vector<int2>* first) {
-  int lines = 0, nitems = 0;
-  for (const Sector& sec : plan->host.sectors) {
-    first->push_back(make_int2(lines, nitems));
-    lines += sec.n;
-    nitems += (sec.n * sec.n + 31) / 32;
-  }
-  return make_int2(lines, nitems);
+// Records the fill that the fill stream has just been given.
+static cudaError_t record_fill(pi_plan* plan, TableFill& f) {
+  cudaError_t e = f.ready ? cudaSuccess : cudaEventCreateWithFlags(&f.ready, cudaEventDisableTiming);
+  return e == cudaSuccess ? cudaEventRecord(f.ready, plan->fill_stream) : e;
+}
+
+// Lets work that s gets from now on read the table: s waits for the fill on the GPU while it may be
+// running.  A capture must not depend on work outside it, so under one the host waits instead, for
+// the fill alone.  Caller holds em_mu.
+static bool order_after(TableFill& f, cudaStream_t s) {
+  if (f.done) return true;
+  RelaxedCapture relaxed;
+  const cudaError_t q = cudaEventQuery(f.ready);
+  if (q == cudaSuccess) return f.done = true;
+  (void)cudaGetLastError();
+  if (q != cudaErrorNotReady) return false;
+  cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(s, &st) == cudaSuccess && st == cudaStreamCaptureStatusNone)
+    return cudaStreamWaitEvent(s, f.ready, 0) == cudaSuccess;
+  (void)cudaGetLastError();
+  return f.done = cudaEventSynchronize(f.ready) == cudaSuccess;
 }
 
 // Keeps `d` with the plan when e is success; otherwise releases it.
@@ -146,55 +155,44 @@ static bool adopt(pi_plan* plan, void* d, size_t bytes, cudaError_t e) {
   return true;
 }
 
-// Caller holds em_mu.  The items are written on the plan's stream; with `wait` they are there on
-// return, otherwise the caller waits for that stream before it lets go of em_mu.
-static StripItems strip_items_locked(pi_plan* plan, bool wait) {
+// Builds the strip items; the fill stream writes them.  Caller holds em_mu.
+static bool build_items(pi_plan* plan) {
   const DevicePlan& dp = plan->dev;
   // 32-bit element indices within a vector
-  if (dp.dim == 0 || dp.dim > 0x3fffffffLL) return StripItems{};
-  if (plan->strip_items) return StripItems{plan->strip_items, plan->nstrip_items};
+  if (dp.dim == 0 || dp.dim > 0x3fffffffLL) return false;
+  if (plan->strip_items) return true;
   RelaxedCapture relaxed;
-  std::vector<int2> first;
-  const int nitems = strip_starts(plan, &first).y;
-  const size_t bytes = sizeof(StripItem) * (size_t)nitems + sizeof(int2) * first.size();
-  char* d = nullptr;
+  const size_t bytes = sizeof(StripItem) * (size_t)plan->nstrip_items;
+  StripItem* d = nullptr;
   cudaError_t e = cudaMalloc((void**)&d, bytes);
   if (e == cudaSuccess) {
-    int2* d_first = (int2*)(d + sizeof(StripItem) * (size_t)nitems);
-    e = cudaMemcpyAsync(d_first, first.data(), sizeof(int2) * first.size(), cudaMemcpyHostToDevice, plan->stream);
-    if (e == cudaSuccess) {
-      k_strip_items<<<dim3(8, (unsigned)first.size()), 256, 0, plan->stream>>>(dp.sectors, d_first, (StripItem*)d);
-      e = cudaGetLastError();
-    }
-    if (e == cudaSuccess && wait) e = cudaStreamSynchronize(plan->stream);
+    k_strip_items<<<dim3(8, (unsigned)dp.nsectors), 256, 0, plan->fill_stream>>>(dp.sectors, d);
+    e = cudaGetLastError();
+    if (e == cudaSuccess) e = record_fill(plan, plan->items_fill);
   }
-  if (!adopt(plan, d, bytes, e)) return StripItems{};
-  plan->strip_first = (const int2*)(d + sizeof(StripItem) * (size_t)nitems);
-  plan->strip_items = (const StripItem*)d;
-  plan->nstrip_items = nitems;
-  return StripItems{plan->strip_items, nitems};
+  if (!adopt(plan, d, bytes, e)) return false;
+  plan->strip_items = d;
+  return true;
 }
 
-StripItems strip_items(pi_plan* plan) {
+StripItems strip_items(pi_plan* plan, cudaStream_t s) {
   std::lock_guard<std::mutex> lk(plan->em_mu);
-  return strip_items_locked(plan, true);
+  if (!build_items(plan) || !order_after(plan->items_fill, s)) return StripItems{};
+  return StripItems{plan->strip_items, plan->nstrip_items};
 }
 
 template <typename T>
-static StripPlanes<T> build_planes(pi_plan* plan, int coords, StripPlanes<T> (&kept)[2], bool (&failed)[2]) {
+static StripPlanes<T> build_planes(pi_plan* plan, int coords, cudaStream_t s, StripPlanes<T> (&kept)[2],
+                                   TableFill (&fill)[2], bool (&failed)[2]) {
   using T2 = typename Vec2<T>::type;
   const DevicePlan& dp = plan->dev;
   if (!dp.canon) return StripPlanes<T>{};
   std::lock_guard<std::mutex> lk(plan->em_mu);
   const int which = coords ? 1 : 0;
   StripPlanes<T>& P = kept[which];
-  if (P.items || failed[which]) return P;
-  const StripItems strips = strip_items_locked(plan, false);
-  if (!strips.items) return StripPlanes<T>{};
+  if (P.items) return order_after(fill[which], s) ? P : StripPlanes<T>{};
+  if (failed[which] || !build_items(plan)) return StripPlanes<T>{};
   RelaxedCapture relaxed;
-  const int S = (int)plan->host.sectors.size();
-  int lines = 0;
-  for (const Sector& sec : plan->host.sectors) lines += sec.n;
   // gain positions that some sector uses, in the order of the canonical kernels: own, smaller,
   // larger sector
   bool drive = false, used[3][3] = {};
@@ -206,7 +204,7 @@ static StripPlanes<T> build_planes(pi_plan* plan, int coords, StripPlanes<T> (&k
   used[0][1] = false;  // joins the centre
   StripPlanes<T> Q;
   Q.dim = dp.dim;
-  Q.nitems = strips.n;
+  Q.nitems = plan->nstrip_items;
   for (GainPos& g : Q.gain) g = GainPos{-1, 0};
   int nr = 0;
   for (int src = 0; src < 3; ++src)
@@ -215,7 +213,7 @@ static StripPlanes<T> build_planes(pi_plan* plan, int coords, StripPlanes<T> (&k
   Q.variant = drive ? (nr <= 1 ? 0 : nr <= 3 ? 1 : nr <= 5 ? 2 : nr <= 6 ? 3 : 4) : (nr <= 5 ? 5 : 6);
   const int np = 2 + nr;
   // one allocation: line tables, planes
-  const size_t line_bytes = (sizeof(T2) * (size_t)lines + 15) / 16 * 16;
+  const size_t line_bytes = (sizeof(T2) * (size_t)plan->nlines + 15) / 16 * 16;
   const size_t plane_bytes = (sizeof(T) * (size_t)dp.dim * np + 15) / 16 * 16;
   const size_t bytes = 2 * line_bytes + plane_bytes;
   char* d = nullptr;
@@ -223,32 +221,31 @@ static StripPlanes<T> build_planes(pi_plan* plan, int coords, StripPlanes<T> (&k
   if (e == cudaSuccess) {
     char* d_plane = d + 2 * line_bytes;
     const dim3 grid((unsigned)std::min<long long>(64, ((long long)plan->host.max_n * plan->host.max_n + 255) / 256),
-                    (unsigned)S);
-    k_planes<T><<<grid, 256, 0, plan->stream>>>(dp.sectors, dp.canon, coords ? dp.coef64z : dp.coef64,
-                                                plan->strip_first, Q, nr, dp.canon_terms, (T*)d_plane, (T2*)d,
-                                                (T2*)(d + line_bytes));
+                    (unsigned)dp.nsectors);
+    // behind the items on the same stream, so its event covers both
+    k_planes<T><<<grid, 256, 0, plan->fill_stream>>>(dp.sectors, dp.canon, coords ? dp.coef64z : dp.coef64, Q, nr,
+                                                     dp.canon_terms, (T*)d_plane, (T2*)d, (T2*)(d + line_bytes));
     e = cudaGetLastError();
-    Q.items = strips.items;
+    if (e == cudaSuccess) e = record_fill(plan, fill[which]);
+    Q.items = plan->strip_items;
     Q.lrow = (const T2*)d;
     Q.rcol = (const T2*)(d + line_bytes);
     Q.plane = (const T*)d_plane;
   }
-  const cudaError_t done = cudaStreamSynchronize(plan->stream);  // the items also without planes
-  if (e == cudaSuccess) e = done;
   if (!adopt(plan, d, bytes, e)) {  // no room: the plan keeps the general kernels
     failed[which] = true;
     return StripPlanes<T>{};
   }
   P = Q;
-  return P;
+  return order_after(fill[which], s) ? P : StripPlanes<T>{};
 }
 
-Planes64 planes64(pi_plan* plan, int coords) {
-  return build_planes<double>(plan, coords, plan->planes64, plan->planes64_failed);
+Planes64 planes64(pi_plan* plan, int coords, cudaStream_t s) {
+  return build_planes<double>(plan, coords, s, plan->planes64, plan->planes64_fill, plan->planes64_failed);
 }
 
-Planes32 planes32(pi_plan* plan, int coords) {
-  return build_planes<float>(plan, coords, plan->planes32, plan->planes32_failed);
+Planes32 planes32(pi_plan* plan, int coords, cudaStream_t s) {
+  return build_planes<float>(plan, coords, s, plan->planes32, plan->planes32_fill, plan->planes32_failed);
 }
 
 namespace {
