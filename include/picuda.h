@@ -90,6 +90,14 @@ int pi_plan_destroy(pi_plan* plan);
  * and solver entry point runs it; destroy it with pi_plan_destroy. */
 int pi_plan_adjoint(const pi_plan* plan, pi_plan** out);
 
+/* memory_budget of compile (liouvillian.jl:4040-4098), in bytes of device memory: merged coefficient
+ * planes that would take device_bytes (pi_plan_info) past it are not laid out, and the calls that
+ * would use them run the general kernels.  A new plan has no budget (INFINITY); an adjoint plan
+ * starts with its parent's, for itself.  Tables that a call cannot do without (the plan's own, those
+ * of pi_apply_f32_em and of FP32 solves) are not held back, and none is given up when the budget
+ * falls below what there is. */
+int pi_plan_set_memory_budget(pi_plan* plan, double bytes);
+
 /* Concurrent calls on one plan (solves, Arnoldi, RK4, host-buffer applies: every call that
  * uses the plan's own stream, staging buffers or engine).  PI_CONCURRENCY_WAIT (the default)
  * serializes them: a second host thread waits for the first, as the reference's locked
@@ -110,7 +118,7 @@ typedef struct {
   int max_block;     /* largest block dimension */
   int max_terms;     /* stencil terms of the busiest sector */
   long long stencil_terms; /* total stencil terms over all sectors */
-  size_t device_bytes;     /* device memory owned by the plan tables */
+  size_t device_bytes;     /* device memory owned by the plan tables laid out so far */
   int batched_kernel;      /* applies with >= 2 columns: 0 general tile kernel, 1 fixed-structure
                               register kernel, 2 canonical positions: every apply runs from merged
                               coefficient planes, one thread per entry (where they have no room,

@@ -682,7 +682,17 @@ int pi_plan_adjoint(const pi_plan* plan, pi_plan** out) {
   pi_plan* adj = new (std::nothrow) pi_plan();
   if (!adj) return fail(PI_ERR_OUT_OF_MEMORY, "host allocation failed");
   adj->host = adjoint_host_plan(plan->host);
+  adj->memory_budget = plan->memory_budget;
   return finish_plan(adj, out);
+}
+
+int pi_plan_set_memory_budget(pi_plan* plan, double bytes) {
+  if (!plan) return fail(PI_ERR_INVALID_ARGUMENT, "null argument");
+  if (!(bytes >= 0)) return fail(PI_ERR_INVALID_ARGUMENT, "memory_budget must not be negative");
+  std::lock_guard<std::mutex> lk(plan->em_mu);
+  plan->memory_budget = bytes;
+  for (int c = 0; c < 2; ++c) plan->planes64_failed[c] = plan->planes32_failed[c] = false;
+  return PI_OK;
 }
 
 int pi_plan_destroy(pi_plan* plan) {
@@ -706,7 +716,10 @@ int pi_plan_info(const pi_plan* plan, pi_plan_info_t* out) {
   out->max_block = plan->host.max_n;
   out->max_terms = plan->host.max_terms;
   out->stencil_terms = plan->stencil_terms;
-  out->device_bytes = plan->device_bytes;
+  {
+    std::lock_guard<std::mutex> lk(const_cast<pi_plan*>(plan)->em_mu);
+    out->device_bytes = plan->device_bytes;
+  }
   out->batched_kernel = plan->dev.canon ? 2 : (plan->dev.fast_sr > 0 ? 1 : 0);
   return PI_OK;
 }

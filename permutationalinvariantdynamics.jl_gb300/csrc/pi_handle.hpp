@@ -2,6 +2,7 @@
 #pragma once
 
 #include <atomic>
+#include <limits>
 #include <memory>
 #include <mutex>
 #include <string>
@@ -26,6 +27,7 @@ struct pi_plan {
   picuda::DevicePlan dev;
   std::vector<void*> allocations;  // device buffers owned by the plan tables
   size_t device_bytes = 0;
+  double memory_budget = std::numeric_limits<double>::infinity();  // of device_bytes, for optional tables
   long long stencil_terms = 0;
   cudaStream_t stream = nullptr;
   int device = 0;
@@ -85,7 +87,7 @@ struct pi_plan {
   std::vector<EmChoice> em_choices;
   std::mutex em_tune_mu;
   // Strip items and merged coefficient planes per coordinate system, built on first use (guarded by
-  // em_mu); a plan without room for them keeps the general kernels.  They are filled on a stream
+  // em_mu); a plan without room for them, in memory or in its budget, keeps the general kernels.  They are filled on a stream
   // of their own, on which nothing else runs: a first apply waits on the GPU for the fill only, not
   // for the solves that `stream` has queued.
   cudaStream_t fill_stream = nullptr;

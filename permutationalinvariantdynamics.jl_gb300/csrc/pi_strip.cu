@@ -143,6 +143,12 @@ static bool order_after(TableFill& f, cudaStream_t s) {
   return f.done = cudaEventSynchronize(f.ready) == cudaSuccess;
 }
 
+// Device memory for an optional table, within the plan's budget.
+static cudaError_t table_alloc(const pi_plan* plan, size_t bytes, char** d) {
+  if ((double)plan->device_bytes + (double)bytes > plan->memory_budget) return cudaErrorMemoryAllocation;
+  return cudaMalloc((void**)d, bytes);
+}
+
 // Keeps `d` with the plan when e is success; otherwise releases it.
 static bool adopt(pi_plan* plan, void* d, size_t bytes, cudaError_t e) {
   if (e != cudaSuccess) {
@@ -163,15 +169,15 @@ static bool build_items(pi_plan* plan) {
   if (plan->strip_items) return true;
   RelaxedCapture relaxed;
   const size_t bytes = sizeof(StripItem) * (size_t)plan->nstrip_items;
-  StripItem* d = nullptr;
-  cudaError_t e = cudaMalloc((void**)&d, bytes);
+  char* d = nullptr;
+  cudaError_t e = table_alloc(plan, bytes, &d);
   if (e == cudaSuccess) {
-    k_strip_items<<<dim3(8, (unsigned)dp.nsectors), 256, 0, plan->fill_stream>>>(dp.sectors, d);
+    k_strip_items<<<dim3(8, (unsigned)dp.nsectors), 256, 0, plan->fill_stream>>>(dp.sectors, (StripItem*)d);
     e = cudaGetLastError();
     if (e == cudaSuccess) e = record_fill(plan, plan->items_fill);
   }
   if (!adopt(plan, d, bytes, e)) return false;
-  plan->strip_items = d;
+  plan->strip_items = (const StripItem*)d;
   return true;
 }
 
@@ -217,7 +223,7 @@ static StripPlanes<T> build_planes(pi_plan* plan, int coords, cudaStream_t s, St
   const size_t plane_bytes = (sizeof(T) * (size_t)dp.dim * np + 15) / 16 * 16;
   const size_t bytes = 2 * line_bytes + plane_bytes;
   char* d = nullptr;
-  cudaError_t e = cudaMalloc((void**)&d, bytes);
+  cudaError_t e = table_alloc(plan, bytes, &d);
   if (e == cudaSuccess) {
     char* d_plane = d + 2 * line_bytes;
     const dim3 grid((unsigned)std::min<long long>(64, ((long long)plan->host.max_n * plan->host.max_n + 255) / 256),

@@ -222,6 +222,7 @@ PROTOTYPES = {
     "pi_solve_dynamics": (C.c_int, [_P, _P, C.c_int, _D, C.c_int, _P, _D,
                                     C.POINTER(pi_expv_opts_t), C.POINTER(pi_expv_info_t)]),
     "pi_plan_adjoint": (C.c_int, [_P, C.POINTER(C.c_void_p)]),
+    "pi_plan_set_memory_budget": (C.c_int, [_P, C.c_double]),
     "pi_stencil_export_adjoint": (C.c_int, [C.c_int, C.c_int, C.c_int, _I, C.c_int, _I, _D, _D, _D, _LL,
                                             _I, _D]),
     "pi_arnoldi": (C.c_int, [_P, _P, C.c_int, _P, C.c_longlong, _D, C.POINTER(pi_arnoldi_info_t)]),

@@ -110,14 +110,25 @@ class CompiledPIModel:
                                       _lib.dptr(rates), _lib.dptr(hbar), C.byref(handle)),
                    "compile(model; backend=:cuda)")
         self._handle = handle
-        info = _lib.pi_plan_info_t()
-        _lib.check(lib.pi_plan_info(handle, C.byref(info)), "pi_plan_info")
-        self.info = {f: getattr(info, f) for f, _ in info._fields_}
-        if len(self.basis) != info.dim:
+        info = self.info
+        if len(self.basis) != info["dim"]:
             raise PiDimensionMismatch("library and host bases disagree")
-        if memory_budget is not None and np.isfinite(memory_budget) and info.device_bytes > memory_budget:
-            self.close()
-            raise PiArgumentError("the prepared CUDA plan exceeds memory_budget")
+        if memory_budget is not None and np.isfinite(memory_budget):
+            if info["device_bytes"] > memory_budget:
+                self.close()
+                raise PiArgumentError("the prepared CUDA plan exceeds memory_budget")
+            _lib.check(lib.pi_plan_set_memory_budget(handle, float(memory_budget)), "memory_budget")
+
+    @property
+    def info(self):
+        """Plan information (pi_plan_info); device_bytes grows with the coefficient planes that the
+        first applies and solves lay out, as far as memory_budget lets them."""
+        out = self.__dict__.setdefault("_info", {})
+        if self._handle is not None:
+            info = _lib.pi_plan_info_t()
+            _lib.check(_lib.load().pi_plan_info(self._handle, C.byref(info)), "pi_plan_info")
+            out.update((f, getattr(info, f)) for f, _ in info._fields_)
+        return out
 
     @property
     def handle(self):
@@ -169,9 +180,6 @@ class CompiledPIModel:
             _lib.check(_lib.load().pi_plan_adjoint(self.handle, C.byref(handle)), "apply_adjoint!")
             adj = CompiledPIModel.__new__(CompiledPIModel)
             adj.model, adj.basis, adj.backend, adj._handle = self.model, self.basis, "cuda", handle
-            info = _lib.pi_plan_info_t()
-            _lib.check(_lib.load().pi_plan_info(handle, C.byref(info)), "pi_plan_info")
-            adj.info = {f: getattr(info, f) for f, _ in info._fields_}
             adj._primary = self  # keeps the forward plan alive while the adjoint is in use
             self._adjoint = adj
         return adj
@@ -211,7 +219,13 @@ class CompiledPIModel:
 
 
 def compile(model: PIModel, backend: str = "cuda", memory_budget=_DEFAULT_MEMORY_BUDGET):
-    """compile(model; backend=:cuda) (liouvillian.jl:4040-4098)."""
+    """compile(model; backend=:cuda) (liouvillian.jl:4040-4098).
+
+    memory_budget (bytes, None for none) bounds the plan's device tables: a plan whose own tables
+    exceed it is refused, and merged coefficient planes (up to 80 bytes per PI coordinate in FP64, 40
+    in FP32, laid out by the first apply or solve that uses them) that would exceed it are not laid
+    out -- those calls then run the general kernels, at about half the speed.  The adjoint has a
+    budget of the same size for itself."""
     if backend != "cuda":
         raise PiArgumentError("this package implements backend=:cuda only")
     if not isinstance(model, PIModel):

@@ -1,0 +1,90 @@
+"""memory_budget of compile: coefficient planes that do not fit are not laid out, and every call that
+would use them gives the same result from the general kernels.
+
+Per output entry at most 11 products are summed, so two orders of summation differ by at most 64
+rounding units of the sum of the products' magnitudes (32 for each side, as against the tables)."""
+import numpy as np
+import pytest
+
+import picuda
+from tests import models as M
+from tests.stencil_eval import evaluate
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def torch_cuda(lib_built):
+    torch = pytest.importorskip("torch")
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    return torch
+
+
+def table_bytes(model):
+    """Device memory of the tables that a plan cannot do without."""
+    held = picuda.compile(model).info["device_bytes"]
+    try:
+        return picuda.compile(model, memory_budget=held - 1).info["device_bytes"]
+    except picuda.PiArgumentError:  # nothing optional so far
+        return held
+
+
+def test_planes_within_the_budget_only(torch_cuda):
+    torch = torch_cuda
+    model = M.ensemble_c2(40)
+    n = len(model.basis)
+    free = picuda.compile(model)
+    own = table_bytes(model)
+    table, coef = picuda.stencil_tables(model)
+    X = np.stack([M.random_state_vector(n, c) for c in range(5)])
+    bound = np.stack([evaluate(model.basis, table, np.abs(coef).astype(complex), np.abs(x)).real for x in X])
+    x = torch.from_numpy(X).cuda()
+    y = picuda.apply_(torch.empty_like(x), free, x).cpu().numpy()
+    used = free.info["device_bytes"]
+    assert used >= own + 7 * 8 * n  # two planes and five gain positions
+    # room for the tables, for the strip items as well, for all but a byte of the planes
+    for budget in (own, own + 3 * n, used - 1):
+        tight = picuda.compile(model, memory_budget=budget)
+        for form in (x, x[0]):
+            got = picuda.apply_(torch.full_like(form, float("nan")), tight, form).cpu().numpy().reshape(-1, n)
+            m = len(got)
+            assert (np.abs(got - y[:m]) <= 64 * 2.0**-52 * bound[:m]).all()
+        host = np.empty_like(X)
+        picuda.apply_(host, tight, X)
+        assert (np.abs(host - y) <= 64 * 2.0**-52 * bound).all()
+        assert tight.info["device_bytes"] <= budget
+    exact = picuda.compile(model, memory_budget=used)
+    assert torch.equal(picuda.apply_(torch.empty_like(x), exact, x).cpu(), torch.from_numpy(y))
+    assert exact.info["device_bytes"] == used
+    # FP32 planes take half the room
+    half = picuda.compile(model, memory_budget=used - 1)
+    x32 = x.to(torch.complex64)
+    ref32 = picuda.apply_(torch.empty_like(x32), free, x32, precision="fp32")
+    assert torch.equal(picuda.apply_(torch.empty_like(x32), half, x32, precision="fp32"), ref32)
+    assert own < half.info["device_bytes"] < used
+    with pytest.raises(picuda.PiArgumentError):
+        picuda.compile(model, memory_budget=own - 1)
+
+
+def test_adjoint_and_solvers_under_a_tight_budget(torch_cuda):
+    torch = torch_cuda
+    model = M.ensemble_c2(24)
+    n = len(model.basis)
+    free = picuda.compile(model)
+    own = table_bytes(model)
+    tight = picuda.compile(model, memory_budget=own)
+    x = torch.from_numpy(M.random_state_vector(n, 9)).cuda()
+    a = picuda.apply_adjoint_(torch.empty_like(x), free, x)
+    b = picuda.apply_adjoint_(torch.empty_like(x), tight, x)
+    table, coef = picuda.stencil_tables(model, adjoint=True)
+    bound = evaluate(model.basis, table, np.abs(coef).astype(complex), x.abs().cpu().numpy().astype(complex)).real
+    assert (np.abs((a - b).cpu().numpy()) <= 64 * 2.0**-52 * bound).all()
+    assert tight.adjoint().info["device_bytes"] <= own
+    rho = picuda.computational_product_state(model.basis, 2)
+    # solvers of the same tolerance: the RK4 steps round differently, the Krylov steps stop at 1e-10
+    for solve, tol in ((lambda c: picuda.time_evolve(c, rho, (0.0, 0.2), steps=40).data, 1e-12),
+                       (lambda c: picuda.krylov_expv(c, rho, 0.2), 1e-9)):
+        p, q = solve(free), solve(tight)
+        assert np.abs(p - q).max() <= tol * np.abs(p).max()
+    assert tight.info["device_bytes"] <= own
