@@ -95,7 +95,9 @@ int pi_plan_adjoint(const pi_plan* plan, pi_plan** out);
  * would use them run the general kernels.  A new plan has no budget (INFINITY); an adjoint plan
  * starts with its parent's, for itself.  Tables that a call cannot do without (the plan's own, those
  * of pi_apply_f32_em and of FP32 solves) are not held back, and none is given up when the budget
- * falls below what there is. */
+ * falls below what there is.  The first call also reserves memory for the planes of a first FP64
+ * apply, where they fit: that apply then allocates nothing.  device_bytes counts what is reserved;
+ * plans that have not used theirs give it back when an allocation of the library fails. */
 int pi_plan_set_memory_budget(pi_plan* plan, double bytes);
 
 /* Concurrent calls on one plan (solves, Arnoldi, RK4, host-buffer applies: every call that
@@ -171,7 +173,7 @@ int pi_sector_multiplicity(int N, int k, double* f, double* sqrt_f);
  * NULL is the CUDA default stream) without synchronizing.
  * Aliasing of x and y is rejected (liouvillian.jl:3220-3221).
  * On a plan with batched_kernel == 2 the first apply of a precision and coordinate system lays
- * out its merged coefficient planes: it allocates them (8 bytes in FP64, 4 in FP32, per PI
+ * out its merged coefficient planes: it allocates them where no memory was reserved (8 bytes in FP64, 4 in FP32, per PI
  * coordinate and plane, with two planes and one per gain position of the stencil, at most ten) and
  * fills them on a stream that the plan uses for nothing else, for which `stream` waits on the GPU.
  * The host waits for that fill only when `stream` is being captured into a graph. */

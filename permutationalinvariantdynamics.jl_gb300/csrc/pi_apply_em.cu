@@ -703,7 +703,7 @@ static int em_tiles(pi_plan* plan) {
 // Builds (once per plan and coefficient set) the merged coefficient planes of the kernel
 // with plain loads.  which: 0 FP32 reference coordinates, 1 FP32 population coordinates.
 static int em_prepare(pi_plan* plan, int which, const float2** planes_out) {
-  std::lock_guard<std::mutex> lk(plan->em_mu);
+  std::lock_guard<std::recursive_mutex> lk(plan->em_mu);
   const DevicePlan& dp = plan->dev;
   int rc = em_tiles(plan);
   if (rc) return rc;
@@ -766,7 +766,7 @@ static int em_tma_tiles(pi_plan* plan, int ri, int gi, const TmTile** tiles_out,
 // Builds (once per plan and coefficient set) the split coefficient planes of the TMA-staged
 // kernel and the per-sector line offsets of its row and column planes.
 static int em_prepare_split(pi_plan* plan, int which, pi_plan::EmSplit* out) {
-  std::lock_guard<std::mutex> lk(plan->em_mu);
+  std::lock_guard<std::recursive_mutex> lk(plan->em_mu);
   const DevicePlan& dp = plan->dev;
   int rc = em_tiles(plan);
   if (rc) return rc;
@@ -883,7 +883,7 @@ static pi_plan::EmMapBlob em_encode_maps(const pi_plan* plan, const void* x, lon
 // The kept maps of a batch; on its first apply `maps`, or newly encoded ones.
 static pi_plan::EmMapBlob em_tensor_maps(pi_plan* plan, const void* x, long long ld, int ncols, int g,
                                          pi_plan::EmMapBlob maps = nullptr) {
-  std::lock_guard<std::mutex> lk(plan->em_mu);
+  std::lock_guard<std::recursive_mutex> lk(plan->em_mu);
   for (const auto& e : plan->em_maps)
     if (e.x == x && e.ld == ld && e.ncols == ncols && e.g == g) return e.maps;
   if (!maps) maps = em_encode_maps(plan, x, ld, ncols, g);
@@ -947,7 +947,7 @@ static int em_run(pi_plan* plan, EmCand c, const pi_plan::EmMapBlob& maps, float
     const TmTile* tiles = nullptr;
     int ntiles = 0;
     {
-      std::lock_guard<std::mutex> lk(plan->em_mu);
+      std::lock_guard<std::recursive_mutex> lk(plan->em_mu);
       rc = em_tma_tiles(plan, ri, gi, &tiles, &ntiles);
     }
     if (rc) return rc;
@@ -1098,7 +1098,7 @@ extern "C" int pi_apply_f32_em(pi_plan* plan, float* y_dev, const float* x_dev, 
   pi_plan::EmChoice ch{};
   bool known = false;
   {
-    std::lock_guard<std::mutex> lk(plan->em_mu);
+    std::lock_guard<std::recursive_mutex> lk(plan->em_mu);
     for (const auto& c : plan->em_choices)
       if (c.ncols == ncols && c.coords == coords) {
         ch = c;
@@ -1108,7 +1108,7 @@ extern "C" int pi_apply_f32_em(pi_plan* plan, float* y_dev, const float* x_dev, 
   if (!known) {
     std::lock_guard<std::mutex> tl(plan->em_tune_mu);  // one tuning pass per key
     {
-      std::lock_guard<std::mutex> lk(plan->em_mu);
+      std::lock_guard<std::recursive_mutex> lk(plan->em_mu);
       for (const auto& c : plan->em_choices)
         if (c.ncols == ncols && c.coords == coords) {
           ch = c;
@@ -1118,7 +1118,7 @@ extern "C" int pi_apply_f32_em(pi_plan* plan, float* y_dev, const float* x_dev, 
     if (!known) {
       int rc = em_tune(plan, y_dev, x_dev, ncols, ld, coords, s, &ch);
       if (rc) return rc;
-      std::lock_guard<std::mutex> lk(plan->em_mu);
+      std::lock_guard<std::recursive_mutex> lk(plan->em_mu);
       plan->em_choices.push_back(ch);
       return PI_OK;  // y already holds L x from the timed runs
     }
@@ -1129,7 +1129,7 @@ extern "C" int pi_apply_f32_em(pi_plan* plan, float* y_dev, const float* x_dev, 
 
 extern "C" int pi_apply_f32_em_tuning(pi_plan* plan, int ncols, int coords, int* kind, int* rows, double* ms) {
   if (!plan || !kind || !rows || !ms) return fail(PI_ERR_INVALID_ARGUMENT, "null argument");
-  std::lock_guard<std::mutex> lk(plan->em_mu);
+  std::lock_guard<std::recursive_mutex> lk(plan->em_mu);
   for (const auto& c : plan->em_choices)
     if (c.ncols == ncols && c.coords == coords) {
       *kind = c.kind;
@@ -1147,7 +1147,7 @@ extern "C" int pi_apply_f32_em_select(pi_plan* plan, int ncols, int coords, int 
   bool listed = false;
   for (const EmCand& c : em_candidates(plan, 0)) listed = listed || (c.kind == kind && (kind == 1 || c.rows == rows));
   if (!listed) return fail(PI_ERR_INVALID_ARGUMENT, "this element-major kernel choice is not available for the plan");
-  std::lock_guard<std::mutex> lk(plan->em_mu);
+  std::lock_guard<std::recursive_mutex> lk(plan->em_mu);
   pi_plan::EmChoice ch{ncols, coords, kind, kind == 1 ? 32 : rows, 0.0};
   for (auto& c : plan->em_choices)
     if (c.ncols == ncols && c.coords == coords) {

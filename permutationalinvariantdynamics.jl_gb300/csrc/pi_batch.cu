@@ -1703,7 +1703,11 @@ Job::~Job() {
 
 void* Job::alloc(size_t b, cudaError_t* err) {
   void* p = nullptr;
-  const cudaError_t e = cudaMallocAsync(&p, b ? b : 16, s_);
+  cudaError_t e = cudaMallocAsync(&p, b ? b : 16, s_);
+  if (e == cudaErrorMemoryAllocation && reclaim_reserves()) {
+    (void)cudaGetLastError();
+    e = cudaMallocAsync(&p, b ? b : 16, s_);
+  }
   if (e != cudaSuccess) {
     *err = e;
     return nullptr;

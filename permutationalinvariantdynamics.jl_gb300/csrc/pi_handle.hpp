@@ -14,11 +14,24 @@
 namespace picuda {
 class Engine;
 
+// A device buffer that tables are cut from, at 256-byte boundaries.
+struct TableRoom {
+  char* base = nullptr;
+  size_t size = 0, used = 0;
+  static size_t padded(size_t bytes) { return (bytes + 255) / 256 * 256; }
+  char* take(size_t bytes) {  // null when there is no room left
+    if (used + padded(bytes) > size) return nullptr;
+    char* p = base + used;
+    used += padded(bytes);
+    return p;
+  }
+};
+
 // A table that is filled on the plan's fill stream: `ready` is recorded behind the fill, `done` once
 // it is known to have passed.
 struct TableFill {
   cudaEvent_t ready = nullptr;
-  bool done = false;
+  bool recorded = false, done = false;
 };
 }  // namespace picuda
 
@@ -26,6 +39,9 @@ struct pi_plan {
   picuda::QubitPlan host;
   picuda::DevicePlan dev;
   std::vector<void*> allocations;  // device buffers owned by the plan tables
+  picuda::TableRoom own_room;      // the tables that the plan is made with
+  bool reserves = false;           // pi_plan_set_memory_budget has been called
+  picuda::TableRoom lazy_room;     // reserved for those that first applies lay out (guarded by em_mu)
   size_t device_bytes = 0;
   double memory_budget = std::numeric_limits<double>::infinity();  // of device_bytes, for optional tables
   long long stencil_terms = 0;
@@ -46,7 +62,7 @@ struct pi_plan {
   std::atomic<int> reject_concurrent{0};
   // Element-major batched apply (pi_apply_em.cu): tile list and merged coefficient planes,
   // built on first use (FP32 reference / population coordinates).
-  std::mutex em_mu;
+  std::recursive_mutex em_mu;  // recursive: an allocation under it may reclaim this plan's reserve
   const picuda::DevTile* em_tiles = nullptr;
   int em_ntiles = 0;
   const float2* em_planes32[2] = {nullptr, nullptr};
@@ -87,11 +103,12 @@ struct pi_plan {
   std::vector<EmChoice> em_choices;
   std::mutex em_tune_mu;
   // Strip items and merged coefficient planes per coordinate system, built on first use (guarded by
-  // em_mu); a plan without room for them, in memory or in its budget, keeps the general kernels.  They are filled on a stream
-  // of their own, on which nothing else runs: a first apply waits on the GPU for the fill only, not
-  // for the solves that `stream` has queued.
+  // em_mu); a plan without room for them, in memory or in its budget, keeps the general kernels.
+  // They are filled on a stream of their own, on which nothing else runs: a first apply waits on
+  // the GPU for the fill only, not for the solves that `stream` has queued.
   cudaStream_t fill_stream = nullptr;
-  const picuda::StripItem* strip_items = nullptr;
+  picuda::StripItem* items_mem = nullptr;
+  const picuda::StripItem* strip_items = nullptr;  // items_mem once its fill is queued
   int nstrip_items = 0, nlines = 0;
   picuda::Planes64 planes64[2];
   picuda::Planes32 planes32[2];
@@ -133,6 +150,14 @@ struct BusyGuard {
 
 // Device allocation tracked by the plan; returns nullptr on failure.
 void* plan_alloc(pi_plan* plan, size_t bytes);
+
+// Reserves device memory for the strip items and the first merged coefficient planes of a canonical
+// plan, as far as its budget lets it (pi_strip.cu).  What a plan has reserved and not used is given
+// back when an allocation fails: reclaim_reserves() frees it on every listed plan and says whether
+// there was any.
+void reserve_planes(pi_plan* plan);
+void list_reserve(pi_plan* plan);
+bool reclaim_reserves();
 
 // Split coefficient planes of a canonical plan in reference (which 0) or population (which 1)
 // FP32 coordinates, built on first use (pi_apply_em.cu); PI_ERR_UNSUPPORTED for a plan whose

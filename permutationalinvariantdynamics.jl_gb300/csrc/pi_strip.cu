@@ -9,9 +9,8 @@
 namespace picuda {
 namespace {
 
-// Strip items of sector blockIdx.y.
-__global__ void k_strip_items(const DevSector* __restrict__ sectors, StripItem* __restrict__ items) {
-  const int s = blockIdx.y;
+// Strip items of sector s by the blocks of one grid row.
+__device__ __forceinline__ void fill_items(const DevSector* __restrict__ sectors, int s, StripItem* __restrict__ items) {
   const DevSector& sec = sectors[s];
   const int n = sec.n;
   StripItem it{};
@@ -27,18 +26,23 @@ __global__ void k_strip_items(const DevSector* __restrict__ sectors, StripItem* 
   }
 }
 
-// Planes and line tables of sector blockIdx.y, merged in FP64 for either precision.  The sums run
+__global__ void k_strip_items(const DevSector* __restrict__ sectors, StripItem* __restrict__ items) {
+  fill_items(sectors, blockIdx.y, items);
+}
+
+// Planes and line tables of sector blockIdx.y, and its strip items unless they are there, merged in FP64 for either precision.  The sums run
 // over the terms in use, not the table's zero padding.
 template <typename T>
 __global__ void k_planes(const DevSector* __restrict__ sectors, const int4* __restrict__ canon,
                          const double2* __restrict__ coef, const StripPlanes<T> P, int nr, const TermCounts terms,
                          T* __restrict__ plane, typename Vec2<T>::type* __restrict__ lrow,
-                         typename Vec2<T>::type* __restrict__ rcol) {
+                         typename Vec2<T>::type* __restrict__ rcol, StripItem* __restrict__ items) {
   using T2 = typename Vec2<T>::type;
   const int s = blockIdx.y;
+  if (items != nullptr) fill_items(sectors, s, items);
   const DevSector& sec = sectors[s];
   const int n = sec.n;
-  const long long cnt = (long long)n * n;
+  const unsigned cnt = (unsigned)n * n;  // below 2^30, as the plan's dimension
   const int4* ct = canon + (long long)s * kCanonEntries;
   // sum of the real products at one sandwich position of the canonical table
   auto sand = [&](int pos, int a, int b) {
@@ -49,8 +53,8 @@ __global__ void k_planes(const DevSector* __restrict__ sectors, const int4* __re
     }
     return v;
   };
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < cnt; i += (long long)gridDim.x * blockDim.x) {
-    const int b = (int)(i / n), a = (int)(i - (long long)b * n);
+  for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < cnt; i += gridDim.x * blockDim.x) {
+    const int b = (int)(i / (unsigned)n), a = (int)i - b * n;
     const double2 al = coef[ct[0].x + a], be = coef[ct[0].y + b];
     T* out = plane + sec.offset + i;
     out[0] = (T)((al.x + be.x) + sand(4, a, b));  // the own-sector centre gain joins the ADD term
@@ -123,19 +127,23 @@ struct RelaxedCapture {
 // Records the fill that the fill stream has just been given.
 static cudaError_t record_fill(pi_plan* plan, TableFill& f) {
   cudaError_t e = f.ready ? cudaSuccess : cudaEventCreateWithFlags(&f.ready, cudaEventDisableTiming);
-  return e == cudaSuccess ? cudaEventRecord(f.ready, plan->fill_stream) : e;
+  if (e == cudaSuccess) e = cudaEventRecord(f.ready, plan->fill_stream);
+  f.recorded = e == cudaSuccess;
+  return e;
 }
 
 // Lets work that s gets from now on read the table: s waits for the fill on the GPU while it may be
 // running.  A capture must not depend on work outside it, so under one the host waits instead, for
-// the fill alone.  Caller holds em_mu.
-static bool order_after(TableFill& f, cudaStream_t s) {
+// the fill alone.  `fresh`: the fill has just been recorded.  Caller holds em_mu.
+static bool order_after(TableFill& f, cudaStream_t s, bool fresh) {
   if (f.done) return true;
   RelaxedCapture relaxed;
-  const cudaError_t q = cudaEventQuery(f.ready);
-  if (q == cudaSuccess) return f.done = true;
-  (void)cudaGetLastError();
-  if (q != cudaErrorNotReady) return false;
+  if (!fresh) {
+    const cudaError_t q = cudaEventQuery(f.ready);
+    if (q == cudaSuccess) return f.done = true;
+    (void)cudaGetLastError();
+    if (q != cudaErrorNotReady) return false;
+  }
   cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
   if (cudaStreamIsCapturing(s, &st) == cudaSuccess && st == cudaStreamCaptureStatusNone)
     return cudaStreamWaitEvent(s, f.ready, 0) == cudaSuccess;
@@ -143,48 +151,90 @@ static bool order_after(TableFill& f, cudaStream_t s) {
   return f.done = cudaEventSynchronize(f.ready) == cudaSuccess;
 }
 
-// Device memory for an optional table, within the plan's budget.
-static cudaError_t table_alloc(const pi_plan* plan, size_t bytes, char** d) {
-  if ((double)plan->device_bytes + (double)bytes > plan->memory_budget) return cudaErrorMemoryAllocation;
-  return cudaMalloc((void**)d, bytes);
+// Device memory for an optional table: from the reserved room, otherwise new within the plan's budget.
+static char* table_alloc(pi_plan* plan, size_t bytes) {
+  if (char* p = plan->lazy_room.take(bytes)) return p;
+  if ((double)plan->device_bytes + (double)bytes > plan->memory_budget) return nullptr;
+  char* p = (char*)plan_alloc(plan, bytes);
+  if (!p) (void)cudaGetLastError();
+  return p;
 }
 
-// Keeps `d` with the plan when e is success; otherwise releases it.
-static bool adopt(pi_plan* plan, void* d, size_t bytes, cudaError_t e) {
-  if (e != cudaSuccess) {
-    (void)cudaGetLastError();
-    if (d) cudaFree(d);
-    return false;
-  }
-  plan->allocations.push_back(d);
-  plan->device_bytes += bytes;
-  return true;
-}
+static size_t items_bytes(const pi_plan* plan) { return sizeof(StripItem) * (size_t)plan->nstrip_items; }
 
-// Builds the strip items; the fill stream writes them.  Caller holds em_mu.
-static bool build_items(pi_plan* plan) {
-  const DevicePlan& dp = plan->dev;
-  // 32-bit element indices within a vector
-  if (dp.dim == 0 || dp.dim > 0x3fffffffLL) return false;
-  if (plan->strip_items) return true;
-  RelaxedCapture relaxed;
-  const size_t bytes = sizeof(StripItem) * (size_t)plan->nstrip_items;
-  char* d = nullptr;
-  cudaError_t e = table_alloc(plan, bytes, &d);
-  if (e == cudaSuccess) {
-    k_strip_items<<<dim3(8, (unsigned)dp.nsectors), 256, 0, plan->fill_stream>>>(dp.sectors, (StripItem*)d);
-    e = cudaGetLastError();
-    if (e == cudaSuccess) e = record_fill(plan, plan->items_fill);
-  }
-  if (!adopt(plan, d, bytes, e)) return false;
-  plan->strip_items = (const StripItem*)d;
-  return true;
+// 32-bit element indices within a vector
+static bool has_items(const DevicePlan& dp) { return dp.dim > 0 && dp.dim <= 0x3fffffffLL; }
+
+static bool items_memory(pi_plan* plan) {
+  if (!plan->items_mem) plan->items_mem = (StripItem*)table_alloc(plan, items_bytes(plan));
+  return plan->items_mem != nullptr;
 }
 
 StripItems strip_items(pi_plan* plan, cudaStream_t s) {
-  std::lock_guard<std::mutex> lk(plan->em_mu);
-  if (!build_items(plan) || !order_after(plan->items_fill, s)) return StripItems{};
+  std::lock_guard<std::recursive_mutex> lk(plan->em_mu);
+  const DevicePlan& dp = plan->dev;
+  const bool fresh = !plan->items_fill.recorded;
+  if (fresh) {
+    RelaxedCapture relaxed;
+    if (!plan->strip_items) {
+      if (!has_items(dp)) return StripItems{};
+      if (!items_memory(plan)) return StripItems{};
+      k_strip_items<<<dim3(8, (unsigned)dp.nsectors), 256, 0, plan->fill_stream>>>(dp.sectors, plan->items_mem);
+      if (cudaGetLastError() != cudaSuccess) return StripItems{};
+      plan->strip_items = plan->items_mem;
+    }
+    if (record_fill(plan, plan->items_fill) != cudaSuccess) return StripItems{};
+  }
+  if (!order_after(plan->items_fill, s, fresh)) return StripItems{};
   return StripItems{plan->strip_items, plan->nstrip_items};
+}
+
+// Line tables and planes of one precision: [row shifts][column shifts][2 + nr planes].
+template <typename T>
+struct PlaneBytes {
+  size_t line, all;
+  PlaneBytes(const pi_plan* plan, int nr)
+      : line((2 * sizeof(T) * (size_t)plan->nlines + 15) / 16 * 16),
+        all(2 * line + (sizeof(T) * (size_t)plan->dev.dim * (2 + nr) + 15) / 16 * 16) {}
+};
+
+// Gain positions that some sector uses, in the order of the canonical kernels: own, smaller, larger
+// sector.  Returns their number; *drive: some sector has line shifts.
+static int gain_positions(const pi_plan* plan, GainPos (&gain)[kMaxGains], bool* drive) {
+  bool used[3][3] = {};
+  *drive = false;
+  for (const Sector& sec : plan->host.sectors)
+    for (const StencilTerm& t : sec.terms) {
+      *drive = *drive || t.kind == ST_LEFT || t.kind == ST_RIGHT;
+      if (t.kind == ST_SAND) used[t.e == 0 ? 0 : t.e < 0 ? 1 : 2][t.p + 1] = true;
+    }
+  used[0][1] = false;  // joins the centre
+  for (GainPos& g : gain) g = GainPos{-1, 0};
+  int nr = 0;
+  for (int src = 0; src < 3; ++src)
+    for (int p = -1; p <= 1; ++p)
+      if (used[src][p + 1]) gain[nr++] = GainPos{(signed char)src, (signed char)p};
+  return nr;
+}
+
+// Room for the items and the first FP64 planes (or FP32 ones of both coordinate systems).  The
+// allocation is a small part of compile(), and most of a first apply that has to make it: 0.17 ms
+// of 0.34 at N = 200, where compile() takes 78.
+void reserve_planes(pi_plan* plan) {
+  const DevicePlan& dp = plan->dev;
+  if (!dp.canon || !has_items(dp) || plan->lazy_room.base || plan->strip_items) return;
+  GainPos gain[kMaxGains];
+  bool drive;
+  const int nr = gain_positions(plan, gain, &drive);
+  const size_t bytes =
+      TableRoom::padded(items_bytes(plan)) + TableRoom::padded(PlaneBytes<double>(plan, nr).all);
+  if ((double)plan->device_bytes + (double)bytes > plan->memory_budget) return;
+  plan->lazy_room.base = (char*)plan_alloc(plan, bytes);
+  if (!plan->lazy_room.base) return (void)cudaGetLastError();
+  plan->lazy_room.size = bytes;
+  list_reserve(plan);
+  for (TableFill* f : {&plan->planes64_fill[0], &plan->planes32_fill[0]})  // a first apply's only event
+    if (cudaEventCreateWithFlags(&f->ready, cudaEventDisableTiming) != cudaSuccess) (void)cudaGetLastError();
 }
 
 template <typename T>
@@ -193,57 +243,39 @@ static StripPlanes<T> build_planes(pi_plan* plan, int coords, cudaStream_t s, St
   using T2 = typename Vec2<T>::type;
   const DevicePlan& dp = plan->dev;
   if (!dp.canon) return StripPlanes<T>{};
-  std::lock_guard<std::mutex> lk(plan->em_mu);
+  std::lock_guard<std::recursive_mutex> lk(plan->em_mu);
   const int which = coords ? 1 : 0;
   StripPlanes<T>& P = kept[which];
-  if (P.items) return order_after(fill[which], s) ? P : StripPlanes<T>{};
-  if (failed[which] || !build_items(plan)) return StripPlanes<T>{};
+  if (P.items) return order_after(fill[which], s, false) ? P : StripPlanes<T>{};
+  if (failed[which] || !has_items(dp)) return StripPlanes<T>{};
   RelaxedCapture relaxed;
-  // gain positions that some sector uses, in the order of the canonical kernels: own, smaller,
-  // larger sector
-  bool drive = false, used[3][3] = {};
-  for (const Sector& sec : plan->host.sectors)
-    for (const StencilTerm& t : sec.terms) {
-      drive = drive || t.kind == ST_LEFT || t.kind == ST_RIGHT;
-      if (t.kind == ST_SAND) used[t.e == 0 ? 0 : t.e < 0 ? 1 : 2][t.p + 1] = true;
-    }
-  used[0][1] = false;  // joins the centre
   StripPlanes<T> Q;
   Q.dim = dp.dim;
   Q.nitems = plan->nstrip_items;
-  for (GainPos& g : Q.gain) g = GainPos{-1, 0};
-  int nr = 0;
-  for (int src = 0; src < 3; ++src)
-    for (int p = -1; p <= 1; ++p)
-      if (used[src][p + 1]) Q.gain[nr++] = GainPos{(signed char)src, (signed char)p};
+  bool drive;
+  const int nr = gain_positions(plan, Q.gain, &drive);
   Q.variant = drive ? (nr <= 1 ? 0 : nr <= 3 ? 1 : nr <= 5 ? 2 : nr <= 6 ? 3 : 4) : (nr <= 5 ? 5 : 6);
-  const int np = 2 + nr;
-  // one allocation: line tables, planes
-  const size_t line_bytes = (sizeof(T2) * (size_t)plan->nlines + 15) / 16 * 16;
-  const size_t plane_bytes = (sizeof(T) * (size_t)dp.dim * np + 15) / 16 * 16;
-  const size_t bytes = 2 * line_bytes + plane_bytes;
-  char* d = nullptr;
-  cudaError_t e = table_alloc(plan, bytes, &d);
-  if (e == cudaSuccess) {
-    char* d_plane = d + 2 * line_bytes;
-    const dim3 grid((unsigned)std::min<long long>(64, ((long long)plan->host.max_n * plan->host.max_n + 255) / 256),
-                    (unsigned)dp.nsectors);
-    // behind the items on the same stream, so its event covers both
-    k_planes<T><<<grid, 256, 0, plan->fill_stream>>>(dp.sectors, dp.canon, coords ? dp.coef64z : dp.coef64, Q, nr,
-                                                     dp.canon_terms, (T*)d_plane, (T2*)d, (T2*)(d + line_bytes));
-    e = cudaGetLastError();
-    if (e == cudaSuccess) e = record_fill(plan, fill[which]);
-    Q.items = plan->strip_items;
-    Q.lrow = (const T2*)d;
-    Q.rcol = (const T2*)(d + line_bytes);
-    Q.plane = (const T*)d_plane;
-  }
-  if (!adopt(plan, d, bytes, e)) {  // no room: the plan keeps the general kernels
+  const PlaneBytes<T> bytes(plan, nr);
+  char* d = items_memory(plan) ? table_alloc(plan, bytes.all) : nullptr;
+  failed[which] = d == nullptr;  // no room: the plan keeps the general kernels
+  if (!d) return StripPlanes<T>{};
+  Q.items = plan->items_mem;
+  Q.lrow = (const T2*)d;
+  Q.rcol = (const T2*)(d + bytes.line);
+  Q.plane = (const T*)(d + 2 * bytes.line);
+  const dim3 grid((unsigned)std::min<long long>(64, ((long long)plan->host.max_n * plan->host.max_n + 255) / 256),
+                  (unsigned)dp.nsectors);
+  // behind items filled before on the same stream, so its event covers them
+  k_planes<T><<<grid, 256, 0, plan->fill_stream>>>(dp.sectors, dp.canon, coords ? dp.coef64z : dp.coef64, Q, nr,
+                                                   dp.canon_terms, (T*)Q.plane, (T2*)Q.lrow, (T2*)Q.rcol,
+                                                   plan->strip_items ? nullptr : plan->items_mem);
+  if (cudaGetLastError() != cudaSuccess || record_fill(plan, fill[which]) != cudaSuccess) {
     failed[which] = true;
     return StripPlanes<T>{};
   }
+  plan->strip_items = plan->items_mem;
   P = Q;
-  return order_after(fill[which], s) ? P : StripPlanes<T>{};
+  return order_after(fill[which], s, true) ? P : StripPlanes<T>{};
 }
 
 Planes64 planes64(pi_plan* plan, int coords, cudaStream_t s) {

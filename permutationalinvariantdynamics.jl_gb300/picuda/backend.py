@@ -113,11 +113,11 @@ class CompiledPIModel:
         info = self.info
         if len(self.basis) != info["dim"]:
             raise PiDimensionMismatch("library and host bases disagree")
-        if memory_budget is not None and np.isfinite(memory_budget):
-            if info["device_bytes"] > memory_budget:
-                self.close()
-                raise PiArgumentError("the prepared CUDA plan exceeds memory_budget")
-            _lib.check(lib.pi_plan_set_memory_budget(handle, float(memory_budget)), "memory_budget")
+        budget = float("inf") if memory_budget is None or not np.isfinite(memory_budget) else float(memory_budget)
+        if info["device_bytes"] > budget:
+            self.close()
+            raise PiArgumentError("the prepared CUDA plan exceeds memory_budget")
+        _lib.check(lib.pi_plan_set_memory_budget(handle, budget), "memory_budget")
 
     @property
     def info(self):

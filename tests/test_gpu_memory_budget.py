@@ -88,3 +88,42 @@ def test_adjoint_and_solvers_under_a_tight_budget(torch_cuda):
         p, q = solve(free), solve(tight)
         assert np.abs(p - q).max() <= tol * np.abs(p).max()
     assert tight.info["device_bytes"] <= own
+
+
+@pytest.mark.parametrize("N", [8, 97, 160])
+def test_first_fp64_apply_allocates_nothing(torch_cuda, N):
+    """compile reserves the planes of a first FP64 apply; those of FP32 take half of it."""
+    torch = torch_cuda
+    model = M.ensemble_c2(N)
+    n = len(model.basis)
+    for dtype, precision in ((torch.complex128, "fp64"), (torch.complex64, "fp32")):
+        compiled = picuda.compile(model)
+        held = compiled.info["device_bytes"]
+        assert held >= table_bytes(model) + 7 * 8 * n
+        x = torch.zeros(n, dtype=dtype, device="cuda")
+        picuda.apply_(torch.empty_like(x), compiled, x, precision=precision)
+        assert compiled.info["device_bytes"] == held
+        x = torch.zeros(n, dtype=torch.complex128, device="cuda")
+        picuda.apply_adjoint_(torch.empty_like(x), compiled, x)
+        assert compiled.info["device_bytes"] == held  # the adjoint has its own
+    assert compiled.adjoint().info["device_bytes"] >= table_bytes(model) + 7 * 8 * n
+
+
+def test_unused_reserves_are_given_back(torch_cuda):
+    """What an allocation that fails does first: the room of plans that have not used it is freed, those
+    plans allocate later, and a plan that has used its room keeps it."""
+    torch = torch_cuda
+    reclaim = picuda.load_library()._ZN6picuda16reclaim_reservesEv
+    model = M.ensemble_c2(30)
+    used, unused = picuda.compile(model), picuda.compile(model)
+    x = torch.from_numpy(M.random_state_vector(len(model.basis), 1)).cuda()
+    ref = picuda.apply_(torch.empty_like(x), used, x)
+    held = used.info["device_bytes"]
+    assert unused.info["device_bytes"] == held
+    assert reclaim() & 0xFF
+    assert used.info["device_bytes"] == held and unused.info["device_bytes"] == table_bytes(model)
+    for compiled in (used, unused):
+        assert torch.equal(picuda.apply_(torch.empty_like(x), compiled, x), ref)
+    gone = picuda.compile(model)
+    gone.close()
+    reclaim()  # a closed plan is no longer listed
