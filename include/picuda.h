@@ -512,22 +512,24 @@ int pi_steady_state_batch(int ninst, pi_plan* const* plans, double* const* x_dev
                           const pi_gmres_opts_t* opts, pi_gmres_info_t* infos);
 
 /* Schedule of the FP32 Arnoldi-step apply of the batched engine (the batched entry points
- * above and PI_FP32 servers).  PI_SCHEDULE_PER_TILE launches one block per (instance,
- * sector-tile) item; k >= 1 launches k blocks per SM (clamped to the resident limit) that
+ * above and PI_FP32 servers).  PI_SCHEDULE_PER_TILE launches one block per work item (a
+ * sector-tile, or a run of strips of a plan with batched_kernel == 2, of one instance); k >= 1 launches k blocks per SM (clamped to the resident limit) that
  * walk the item list persistently, prefetching each next tile's staged windows while
  * computing the current one.  PI_SCHEDULE_AUTO (the default) times every candidate with
  * CUDA events on the engine stream before the first Krylov cycle of a job set whose shape
  * (work-list size class, canonical or general stencils) has not been seen by that engine,
  * and keeps the fastest; the timed launches write only the step's scratch column, which
- * the cycle recomputes.  Every schedule gives bitwise the same results.  Process-wide;
- * applies to engines that choose a schedule after the call. */
-enum { PI_SCHEDULE_AUTO = 0, PI_SCHEDULE_PER_TILE = -1 };
+ * the cycle recomputes.  Small job sets (up to 2^19 elements, all of plans with batched_kernel ==
+ * 2) run a whole Krylov cycle in one launch under PI_SCHEDULE_AUTO and time nothing; the record
+ * shows PI_SCHEDULE_ONE_LAUNCH, which cannot be set.  Every schedule gives bitwise the same
+ * results.  Process-wide; applies to engines that choose a schedule after the call. */
+enum { PI_SCHEDULE_AUTO = 0, PI_SCHEDULE_PER_TILE = -1, PI_SCHEDULE_ONE_LAUNCH = -2 };
 int pi_engine_set_apply_schedule(int schedule);
 
 typedef struct {
   int choices;        /* schedules chosen so far, process-wide (tuned or cached or set) */
   int tunings;        /* of which timed */
-  int schedule;       /* the last choice: PI_SCHEDULE_PER_TILE or blocks per SM */
+  int schedule;       /* the last choice: PI_SCHEDULE_PER_TILE, _ONE_LAUNCH or blocks per SM */
   int items;          /* work-list items of the job set it was made for */
   int resident_max;   /* resident blocks per SM of the persistent launch */
   int ncand;          /* candidates of the last timing (0 if the last choice was not timed) */

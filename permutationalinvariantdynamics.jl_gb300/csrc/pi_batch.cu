@@ -2498,7 +2498,7 @@ void Engine::rebuild() {
     cudaGraphExecDestroy(graph_);
     graph_ = nullptr;
   }
-  schedule_chosen_ = false;
+  schedule_chosen_ = cycle_recorded_ = false;
   dirty_ = false;
 }
 
@@ -2509,6 +2509,15 @@ std::atomic<int> g_apply_schedule{PI_SCHEDULE_AUTO};
 std::mutex g_schedule_mu;
 std::map<long long, int> g_schedule_cache;  // (device, job-set shape) -> schedule
 pi_schedule_info_t g_schedule_info{};
+
+// `rec` (work list, resident limit, candidates) becomes the record of the last choice.
+void record_schedule(pi_schedule_info_t rec, int schedule) {
+  std::lock_guard<std::mutex> lk(g_schedule_mu);
+  rec.choices = g_schedule_info.choices + 1;
+  rec.tunings = g_schedule_info.tunings;
+  rec.schedule = schedule;
+  g_schedule_info = rec;
+}
 
 }  // namespace
 
@@ -2593,11 +2602,7 @@ void Engine::choose_apply_schedule() {
       }
     }
   }
-  std::lock_guard<std::mutex> lk(g_schedule_mu);
-  rec.choices = g_schedule_info.choices + 1;
-  rec.tunings = g_schedule_info.tunings;
-  rec.schedule = apply_schedule_;
-  g_schedule_info = rec;
+  record_schedule(rec, apply_schedule_);
 }
 
 // Launches a kernel on the engine stream, or appends it as the next node of the graph under
@@ -2748,6 +2753,13 @@ void Engine::run_cycle_steps() {
   // an explicit step-apply schedule asks for the step kernels
   ran_cycle_ = cycle_kernel_ && (!f32_ || g_apply_schedule.load() == PI_SCHEDULE_AUTO);
   if (ran_cycle_) {
+    if (f32_ && !cycle_recorded_) {  // once per job set, like a choice among the step schedules
+      pi_schedule_info_t rec{};
+      rec.items = total_strips_;
+      rec.resident_max = persist_max_;
+      record_schedule(rec, PI_SCHEDULE_ONE_LAUNCH);
+      cycle_recorded_ = true;
+    }
     launch_cycle();
     return;
   }

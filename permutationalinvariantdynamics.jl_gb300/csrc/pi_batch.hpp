@@ -357,6 +357,7 @@ class Engine {
   void launch_cycle();
   int apply_schedule_ = PI_SCHEDULE_PER_TILE;
   bool schedule_chosen_ = false;
+  bool cycle_recorded_ = false;  // the current set's one-launch cycle is in the schedule record
   int sm_count_ = 0;
   int cycle_grid_ = 1;          // blocks of k_cycle
   bool cycle_cluster_ = false;  // as one cluster

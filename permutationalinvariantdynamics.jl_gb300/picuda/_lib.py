@@ -36,6 +36,7 @@ PI_SCHEDULE_AUTO = 0
 PI_PRECOND_LEVEL = 0
 PI_PRECOND_DRIVE = 1
 PI_SCHEDULE_PER_TILE = -1
+PI_SCHEDULE_ONE_LAUNCH = -2
 PI_COORDS_POPULATION = 1
 
 

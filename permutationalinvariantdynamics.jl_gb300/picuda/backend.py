@@ -1768,14 +1768,16 @@ def set_engine_schedule(schedule="auto"):
 
 
 def engine_schedule_info():
-    """The batched engine's last step-apply schedule choice: the schedule ("per_tile" or
-    blocks per SM), the work-list size it was made for, the resident-block limit, and the
-    median time of every candidate when the choice was timed."""
+    """The batched engine's last step-apply schedule choice: the schedule ("per_tile", blocks per
+    SM, or "one_launch" for a small job set whose Krylov cycles run in one launch each), the
+    work-list size it was made for, the resident-block limit, and the median time of every
+    candidate when the choice was timed."""
     info = _lib.pi_schedule_info_t()
     _lib.check(_lib.load().pi_engine_schedule_info(C.byref(info)), "engine_schedule_info")
 
     def name(k):
-        return "per_tile" if k == _lib.PI_SCHEDULE_PER_TILE else int(k)
+        names = {_lib.PI_SCHEDULE_PER_TILE: "per_tile", _lib.PI_SCHEDULE_ONE_LAUNCH: "one_launch"}
+        return names.get(k, int(k))
 
     return {"choices": info.choices, "tunings": info.tunings, "schedule": name(info.schedule),
             "items": info.items, "resident_max": info.resident_max,
