@@ -206,10 +206,15 @@ int pi_apply_f32_em(pi_plan* plan, float* y_dev, const float* x_dev, int ncols, 
  * choice was pinned).  PI_ERR_INVALID_ARGUMENT before the first call with that width and
  * coordinate system.  No counterpart in the reference (its autotuner-free CPU path). */
 int pi_apply_f32_em_tuning(pi_plan* plan, int ncols, int coords, int* kind, int* rows, double* ms);
+/* The right-hand sides per block of that kernel: 64, or 32 and 16 of the TMA-staged kernels for
+ * narrow batches (tiles of 32 and 16 rows). */
+int pi_apply_f32_em_block(pi_plan* plan, int ncols, int coords, int* rhs);
 /* Pins the element-major kernel for (ncols, coords) instead of autotuning it (kind and rows
- * as above; PI_ERR_INVALID_ARGUMENT for a choice the plan does not offer).  No counterpart
- * in the reference. */
+ * as above, with blocks of 64 right-hand sides; PI_ERR_INVALID_ARGUMENT for a choice the plan does
+ * not offer).  No counterpart in the reference. */
 int pi_apply_f32_em_select(pi_plan* plan, int ncols, int coords, int kind, int rows);
+/* The same with the block's right-hand sides: what the two calls above report can be pinned. */
+int pi_apply_f32_em_select_block(pi_plan* plan, int ncols, int coords, int kind, int rows, int rhs);
 /* Convenience with host buffers: copies x in, applies, copies y out (pinned host memory
  * gives full link bandwidth).  The FP32 variant takes PI_COORDS_* like pi_apply_f32. */
 int pi_apply_host_f64(pi_plan* plan, double* y_host, const double* x_host, int ncols);

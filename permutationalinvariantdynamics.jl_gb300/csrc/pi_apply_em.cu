@@ -986,20 +986,30 @@ static int em_run(pi_plan* plan, EmCand c, const pi_plan::EmMapBlob& maps, float
 // to 96 columns blocks of 32 (32 x 16), which keep the entry planes' size.  Up to 32 columns
 // they stand in for the other tile heights.  Elsewhere they lose: N = 120, 48 columns take 64 us in
 // one block of 64 and 70 in three of 16, 130 columns 194 us in three and 203 in five of 32, while 96
-// take 120 and 109, 32 columns 61 and 45, 16 columns 59 and 30.  ncols = 0 lists the choices that a
-// caller can pin.
+// take 120 and 109, 32 columns 61 and 45, 16 columns 59 and 30.
 static std::vector<EmCand> em_candidates(const pi_plan* plan, int ncols) {
   std::vector<EmCand> c;
   if (plan->dev.nsectors <= kTmMapsLarge && tensor_map_encoder()) {
     c.push_back({0, 32});
-    if (ncols == 0 || ncols > 32) {
+    if (ncols > 32) {
       c.push_back({0, 16});
       if (!plan->dev.canon_plus) c.push_back({0, 64});
     }
-    if (ncols > 0 && ncols <= 16)
+    if (ncols <= 16)
       c.push_back({0, 16, 16});
-    else if (ncols > 0 && ncols <= 96 && (ncols + 31) / 32 % 2 == 1)
+    else if (ncols <= 96 && (ncols + 31) / 32 % 2 == 1)
       c.push_back({0, 32, 32});
+  }
+  c.push_back({1, 32});
+  return c;
+}
+
+// Every kernel that the plan has, for a caller's choice; any of them takes any width.
+static std::vector<EmCand> em_kernels(const pi_plan* plan) {
+  std::vector<EmCand> c;
+  if (plan->dev.nsectors <= kTmMapsLarge && tensor_map_encoder()) {
+    c = {{0, 32}, {0, 16}, {0, 32, 32}, {0, 16, 16}};
+    if (!plan->dev.canon_plus) c.push_back({0, 64});
   }
   c.push_back({1, 32});
   return c;
@@ -1140,15 +1150,27 @@ extern "C" int pi_apply_f32_em_tuning(pi_plan* plan, int ncols, int coords, int*
   return fail(PI_ERR_INVALID_ARGUMENT, "no element-major apply with this width and coordinate system has run yet");
 }
 
-extern "C" int pi_apply_f32_em_select(pi_plan* plan, int ncols, int coords, int kind, int rows) {
+extern "C" int pi_apply_f32_em_block(pi_plan* plan, int ncols, int coords, int* rhs) {
+  if (!plan || !rhs) return fail(PI_ERR_INVALID_ARGUMENT, "null argument");
+  std::lock_guard<std::recursive_mutex> lk(plan->em_mu);
+  for (const auto& c : plan->em_choices)
+    if (c.ncols == ncols && c.coords == coords) {
+      *rhs = c.g;
+      return PI_OK;
+    }
+  return fail(PI_ERR_INVALID_ARGUMENT, "no element-major apply with this width and coordinate system has run yet");
+}
+
+extern "C" int pi_apply_f32_em_select_block(pi_plan* plan, int ncols, int coords, int kind, int rows, int rhs) {
   if (!plan) return fail(PI_ERR_INVALID_ARGUMENT, "null argument");
   if (coords != PI_COORDS_REFERENCE && coords != PI_COORDS_POPULATION)
     return fail(PI_ERR_INVALID_ARGUMENT, "coords must be PI_COORDS_REFERENCE or PI_COORDS_POPULATION");
   bool listed = false;
-  for (const EmCand& c : em_candidates(plan, 0)) listed = listed || (c.kind == kind && (kind == 1 || c.rows == rows));
+  for (const EmCand& c : em_kernels(plan))
+    listed = listed || (c.kind == kind && (kind == 1 || (c.rows == rows && c.g == rhs)));
   if (!listed) return fail(PI_ERR_INVALID_ARGUMENT, "this element-major kernel choice is not available for the plan");
   std::lock_guard<std::recursive_mutex> lk(plan->em_mu);
-  pi_plan::EmChoice ch{ncols, coords, kind, kind == 1 ? 32 : rows, 0.0};
+  pi_plan::EmChoice ch{ncols, coords, kind, kind == 1 ? 32 : rows, 0.0, kind == 1 ? 64 : rhs};
   for (auto& c : plan->em_choices)
     if (c.ncols == ncols && c.coords == coords) {
       c = ch;
@@ -1156,4 +1178,8 @@ extern "C" int pi_apply_f32_em_select(pi_plan* plan, int ncols, int coords, int 
     }
   plan->em_choices.push_back(ch);
   return PI_OK;
+}
+
+extern "C" int pi_apply_f32_em_select(pi_plan* plan, int ncols, int coords, int kind, int rows) {
+  return pi_apply_f32_em_select_block(plan, ncols, coords, kind, rows, 64);
 }

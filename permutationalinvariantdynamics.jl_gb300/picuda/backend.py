@@ -1006,18 +1006,25 @@ def element_major_tuning(compiled: CompiledPIModel, ncols, coords="population"):
     """The element-major kernel in use for a batch width and coordinate system, as chosen by
     the autotuner on the first apply_element_major_ call (or pinned with
     select_element_major_kernel): {"kernel": "tma" | "plain", "rows": tile rows, "ms": timed
-    duration of one apply (0 when pinned)}."""
+    duration of one apply (0 when pinned)}, and "rhs", the right-hand sides per block, for the
+    narrow blocks (16 or 32; 64 otherwise)."""
     lib = _lib.load()
     cc = _lib.PI_COORDS_POPULATION if coords == "population" else _lib.PI_COORDS_REFERENCE
     kind, rows, ms = C.c_int(), C.c_int(), C.c_double()
     _lib.check(lib.pi_apply_f32_em_tuning(compiled.handle, int(ncols), cc, C.byref(kind), C.byref(rows),
                                           C.byref(ms)), "element-major tuning")
-    return {"kernel": EM_KERNELS[kind.value], "rows": rows.value, "ms": ms.value}
+    rhs = C.c_int()
+    _lib.check(lib.pi_apply_f32_em_block(compiled.handle, int(ncols), cc, C.byref(rhs)), "element-major tuning")
+    out = {"kernel": EM_KERNELS[kind.value], "rows": rows.value, "ms": ms.value}
+    if rhs.value != 64:
+        out["rhs"] = rhs.value
+    return out
 
 
-def select_element_major_kernel(compiled: CompiledPIModel, ncols, kernel="tma", rows=32, coords="population"):
+def select_element_major_kernel(compiled: CompiledPIModel, ncols, kernel="tma", rows=32, coords="population", rhs=64):
     """Pins the element-major kernel for a batch width and coordinate system instead of
-    autotuning it: kernel "tma" (tile rows 16, 32 or, without pumping terms, 64) or "plain"."""
+    autotuning it: kernel "tma" (tile rows 16, 32 or, without pumping terms, 64, in blocks of 64
+    right-hand sides; or rows 32 with rhs=32, rows 16 with rhs=16) or "plain"."""
     kinds = {v: k for k, v in EM_KERNELS.items()}
     if kernel not in kinds:
         raise PiArgumentError(f"element-major kernel must be one of {sorted(kinds)}, got {kernel!r}")
@@ -1025,7 +1032,7 @@ def select_element_major_kernel(compiled: CompiledPIModel, ncols, kernel="tma", 
         raise PiArgumentError(f"coords must be 'population' or 'reference', got {coords!r}")
     lib = _lib.load()
     cc = _lib.PI_COORDS_POPULATION if coords == "population" else _lib.PI_COORDS_REFERENCE
-    _lib.check(lib.pi_apply_f32_em_select(compiled.handle, int(ncols), cc, kinds[kernel], int(rows)),
+    _lib.check(lib.pi_apply_f32_em_select_block(compiled.handle, int(ncols), cc, kinds[kernel], int(rows), int(rhs)),
                "element-major kernel choice")
 
 
