@@ -984,17 +984,17 @@ static int em_run(pi_plan* plan, EmCand c, const pi_plan::EmMapBlob& maps, float
 // when the plan's tensor maps fit the kernel-parameter table, and plain loads; for batches of up
 // to 16 columns also blocks of 16 right-hand sides (16 rows x 32 columns), and for 17 to 32 and 65
 // to 96 columns blocks of 32 (32 x 16), which keep the entry planes' size.  Up to 32 columns
-// they stand in for the other tile heights.  Elsewhere they lose: N = 120, 48 columns take 64 us in
-// one block of 64 and 70 in three of 16, 130 columns 194 us in three and 203 in five of 32, while 96
-// take 120 and 109, 32 columns 61 and 45, 16 columns 59 and 30.
+// they stand in for the 64-row tiles.  Small ensembles fill few SMs, so there the shortest tiles win
+// at any width: N = 40, 32 columns 6.7 us in tiles of 16 rows, 10.6 of 32, 10.8 in blocks of 32.
+// Elsewhere narrow blocks lose: N = 120, 48 columns take 64 us in one block of 64 and 70 in three of
+// 16, 130 columns 194 us in three and 203 in five of 32, while 96 take 120 and 109, 32 columns 61
+// and 45, 16 columns 59 and 30.
 static std::vector<EmCand> em_candidates(const pi_plan* plan, int ncols) {
   std::vector<EmCand> c;
   if (plan->dev.nsectors <= kTmMapsLarge && tensor_map_encoder()) {
     c.push_back({0, 32});
-    if (ncols > 32) {
-      c.push_back({0, 16});
-      if (!plan->dev.canon_plus) c.push_back({0, 64});
-    }
+    c.push_back({0, 16});
+    if (ncols > 32 && !plan->dev.canon_plus) c.push_back({0, 64});
     if (ncols <= 16)
       c.push_back({0, 16, 16});
     else if (ncols <= 96 && (ncols + 31) / 32 % 2 == 1)

@@ -65,3 +65,16 @@ def test_shapes_that_do_not_exist_are_refused(torch_cuda):
     for rows, rhs in ((16, 32), (64, 32), (32, 16), (48, 64), (32, 8)):
         with pytest.raises(picuda.PiArgumentError):
             picuda.select_element_major_kernel(compiled, 16, "tma", rows, rhs=rhs)
+
+
+@pytest.mark.parametrize("make", [lambda: M.ensemble_c2(40),
+                                  lambda: picuda.Models.local_pump_decay(40, down=1.0, up=0.3)])
+def test_tuner_takes_short_tiles_for_small_ensembles(torch_cuda, make):
+    """At N = 40 and 32 columns tiles of 16 rows take two thirds of the time of every other kernel, more
+    than timings of one launch differ by."""
+    torch = torch_cuda
+    compiled = picuda.compile(make())
+    x = torch.randn((len(compiled.basis), 32), dtype=torch.complex64, device="cuda")
+    picuda.apply_element_major_(torch.empty_like(x), compiled, x)
+    found = picuda.element_major_tuning(compiled, 32)
+    assert (found["kernel"], found["rows"], found.get("rhs", 64)) == ("tma", 16, 64)
