@@ -2446,8 +2446,6 @@ void Engine::rebuild() {
     d.items32 = it32[i].items;
     d.nitems32 = it32[i].n;
     d.p64 = p64[i];
-    if (f32_ && dp.canon && em_split_planes(J->plan, d.pwhich, &d.planes) != PI_OK)
-      d.planes = SplitPlanes{nullptr, nullptr, nullptr, nullptr, 0};
     for (int c = 0; c < nc[i]; ++c) ci.push_back(i);
     d.V = J->V;
     d.w = J->w;
