@@ -151,10 +151,11 @@ static bool order_after(TableFill& f, cudaStream_t s, bool fresh) {
   return f.done = cudaEventSynchronize(f.ready) == cudaSuccess;
 }
 
-// Device memory for an optional table: from the reserved room, otherwise new within the plan's budget.
-static char* table_alloc(pi_plan* plan, size_t bytes) {
+// Device memory for a table: from the reserved room, otherwise new, an optional one within the plan's
+// budget.
+static char* table_alloc(pi_plan* plan, size_t bytes, bool optional = true) {
   if (char* p = plan->lazy_room.take(bytes)) return p;
-  if ((double)plan->device_bytes + (double)bytes > plan->memory_budget) return nullptr;
+  if (optional && (double)plan->device_bytes + (double)bytes > plan->memory_budget) return nullptr;
   char* p = (char*)plan_alloc(plan, bytes);
   if (!p) (void)cudaGetLastError();
   return p;
@@ -165,8 +166,8 @@ static size_t items_bytes(const pi_plan* plan) { return sizeof(StripItem) * (siz
 // 32-bit element indices within a vector
 static bool has_items(const DevicePlan& dp) { return dp.dim > 0 && dp.dim <= 0x3fffffffLL; }
 
-static bool items_memory(pi_plan* plan) {
-  if (!plan->items_mem) plan->items_mem = (StripItem*)table_alloc(plan, items_bytes(plan));
+static bool items_memory(pi_plan* plan, bool optional) {
+  if (!plan->items_mem) plan->items_mem = (StripItem*)table_alloc(plan, items_bytes(plan), optional);
   return plan->items_mem != nullptr;
 }
 
@@ -178,7 +179,9 @@ StripItems strip_items(pi_plan* plan, cudaStream_t s) {
     RelaxedCapture relaxed;
     if (!plan->strip_items) {
       if (!has_items(dp)) return StripItems{};
-      if (!items_memory(plan)) return StripItems{};
+      // An FP32 step by strips needs them beside its split planes, which have no budget either: by
+      // tiles from the general terms it would round differently from the persistent schedules.
+      if (!items_memory(plan, false)) return StripItems{};
       k_strip_items<<<dim3(8, (unsigned)dp.nsectors), 256, 0, plan->fill_stream>>>(dp.sectors, plan->items_mem);
       if (cudaGetLastError() != cudaSuccess) return StripItems{};
       plan->strip_items = plan->items_mem;
@@ -256,7 +259,7 @@ static StripPlanes<T> build_planes(pi_plan* plan, int coords, cudaStream_t s, St
   const int nr = gain_positions(plan, Q.gain, &drive);
   Q.variant = drive ? (nr <= 1 ? 0 : nr <= 3 ? 1 : nr <= 5 ? 2 : nr <= 6 ? 3 : 4) : (nr <= 5 ? 5 : 6);
   const PlaneBytes<T> bytes(plan, nr);
-  char* d = items_memory(plan) ? table_alloc(plan, bytes.all) : nullptr;
+  char* d = items_memory(plan, true) ? table_alloc(plan, bytes.all) : nullptr;
   failed[which] = d == nullptr;  // no room: the plan keeps the general kernels
   if (!d) return StripPlanes<T>{};
   Q.items = plan->items_mem;

@@ -127,3 +127,23 @@ def test_unused_reserves_are_given_back(torch_cuda):
     gone = picuda.compile(model)
     gone.close()
     reclaim()  # a closed plan is no longer listed
+
+
+def test_mixed_solves_round_alike_under_any_budget(torch_cuda):
+    """FP32 steps by strips whatever the budget, so that every engine schedule gives the same bits."""
+    model = M.ensemble_c2(30)
+    rho = picuda.computational_product_state(model.basis, 2)
+    alg = picuda.ExpvAlgorithm(krylovdim=20, precision="mixed")
+    out = {}
+    try:
+        for budget in (None, table_bytes(model)):
+            for schedule in ("auto", "per_tile", 1):
+                picuda.set_engine_schedule(schedule)
+                compiled = picuda.compile(model, memory_budget=budget)
+                _, finals = picuda.solve_dynamics_batch([compiled], [rho], (0.0, 0.2), saveat=0.1, algorithm=alg)
+                out[budget, schedule] = np.asarray(finals[0])
+    finally:
+        picuda.set_engine_schedule("auto")
+    ref = out[None, "auto"]
+    for key, got in out.items():
+        assert np.array_equal(got, ref), key
