@@ -47,7 +47,7 @@
 // the slot, from where the stager that takes the slot next writes it to z.  Full and done
 // mbarriers order the warps; nothing waits for a whole block.  N = 200, FP32, per sweep of
 // FP64 vectors: 235 us with block barriers and the store of z and the products on the solving
-// warp, 160 us now; FP64 sweeps in reference coordinates 1188 us, now 818.  A level of 101 entries
+// warp, 161 us now; FP64 sweeps in reference coordinates 1188 us, now 822.  A level of 101 entries
 // takes about 1300 cycles: gains 400, forward and backward scan 270 each, the rest waits and
 // arrivals.  Loading the next level's entries into registers during the backward scan costs more
 // (spills, or fewer stagers: 213 us).  Population coordinates run in FP32 (the preconditioner is an
@@ -487,17 +487,19 @@ __device__ __forceinline__ void solve_level(const PrecondDev& Pd, Slot<T, TI>& L
 // two large sums (N = 61..128 in FP64: 2e-14 of sum t |z|, against 2e-16).
 constexpr int kTailUnroll = 8;
 
-template <typename TO>
+template <bool POP, typename TO>  // POP: population coordinates, where t is one
 __device__ __forceinline__ double2 chain0_correct(const PrecondDev& Pd, TO* z, int c0, int c1, double2 k) {
-  TraceSum64 sum;
+  double2 sum = make_double2(0.0, 0.0);
   for (int e0 = c0 + threadIdx.x; e0 < c1; e0 += kTailUnroll * blockDim.x) {
     int el[kTailUnroll];
     double2 w[kTailUnroll], v[kTailUnroll];
+    double t[kTailUnroll];
 #pragma unroll
     for (int q = 0; q < kTailUnroll; ++q) {
       const int e = e0 + q * blockDim.x;
       el[q] = e < c1 ? Pd.elem[e] : -1;
       w[q] = e < c1 ? Pd.w0[e - c0] : make_double2(0.0, 0.0);
+      t[q] = !POP && e < c1 ? Pd.t0[e - c0] : 1.0;
     }
 #pragma unroll
     for (int q = 0; q < kTailUnroll; ++q) v[q] = el[q] >= 0 ? load_d2(z + el[q]) : make_double2(0.0, 0.0);
@@ -507,10 +509,11 @@ __device__ __forceinline__ double2 chain0_correct(const PrecondDev& Pd, TO* z, i
       v[q].x = fma(-k.x, w[q].x, fma(k.y, w[q].y, v[q].x));
       v[q].y = fma(-k.x, w[q].y, fma(-k.y, w[q].x, v[q].y));
       store_as<TO, double2>(z + el[q], v[q]);
-      sum.add(Pd, e0 + q * blockDim.x, v[q]);
+      sum.x = POP ? sum.x + v[q].x : fma(t[q], v[q].x, sum.x);
+      sum.y = POP ? sum.y + v[q].y : fma(t[q], v[q].y, sum.y);
     }
   }
-  return sum.value();
+  return sum;
 }
 
 // The same for FP32 vectors: in double-float, as each conversion and FP64 operation of a warp
@@ -646,7 +649,7 @@ __global__ void __launch_bounds__(kSweepThreads<T>, 2)
   if constexpr (std::is_same<T, float>::value && std::is_same<TO, float2>::value)
     share = chain0_correct_df(Pd, z, c0, c1, k);
   else
-    share = chain0_correct(Pd, z, c0, c1, k);
+    share = chain0_correct<std::is_same<T, float>::value>(Pd, z, c0, c1, k);
   if (Pd.mode != 0) return;
   const double2 tz = block_sum2(share, S.red);  // of every entry but the free one, which is zero so far
   if (tid == 0 && Pd.free_ent >= 0)
