@@ -676,13 +676,15 @@ __global__ void __launch_bounds__(kTmThreads, 2)
 
 }  // namespace
 
+static int em_check(const pi_plan* plan) {
+  if (plan->dev.canon) return PI_OK;
+  return fail(PI_ERR_UNSUPPORTED,
+              "element-major batched apply needs a plan whose stencil sits at the canonical positions "
+              "(qubit models with real one-body operators)");
+}
+
 // Builds (once per plan) the element-major tile list.  Caller holds plan->em_mu.
 static int em_tiles(pi_plan* plan) {
-  const DevicePlan& dp = plan->dev;
-  if (!dp.canon)
-    return fail(PI_ERR_UNSUPPORTED,
-                "element-major batched apply needs a plan whose stencil sits at the canonical positions "
-                "(qubit models with real one-body operators)");
   if (!plan->em_tiles) {
     std::vector<DevTile> tiles;
     for (int s = 0; s < (int)plan->host.sectors.size(); ++s) {
@@ -705,7 +707,8 @@ static int em_tiles(pi_plan* plan) {
 static int em_prepare(pi_plan* plan, int which, const float2** planes_out) {
   std::lock_guard<std::recursive_mutex> lk(plan->em_mu);
   const DevicePlan& dp = plan->dev;
-  int rc = em_tiles(plan);
+  int rc = em_check(plan);
+  if (rc == PI_OK) rc = em_tiles(plan);
   if (rc) return rc;
   if (!plan->em_planes32[which]) {
     const int np = dp.canon_plus ? kEmPosPlus : kEmPos;
@@ -763,57 +766,34 @@ static int em_tma_tiles(pi_plan* plan, int ri, int gi, const TmTile** tiles_out,
   return PI_OK;
 }
 
-// Builds (once per plan and coefficient set) the split coefficient planes of the TMA-staged
-// kernel and the per-sector line offsets of its row and column planes.
+// Builds (once per plan and coefficient set) the split coefficient planes of the TMA-staged kernel.
 static int em_prepare_split(pi_plan* plan, int which, pi_plan::EmSplit* out) {
   std::lock_guard<std::recursive_mutex> lk(plan->em_mu);
   const DevicePlan& dp = plan->dev;
-  int rc = em_tiles(plan);
+  const int rc = em_check(plan);
   if (rc) return rc;
-  if (!plan->em_line_off) {
-    std::vector<int> off(plan->host.sectors.size());
-    int acc = 0;
-    for (size_t s = 0; s < off.size(); ++s) {
-      off[s] = acc;
-      acc += plan->host.sectors[s].n;
-    }
-    void* d = plan_alloc(plan, sizeof(int) * off.size());
-    if (!d) return fail(PI_ERR_OUT_OF_MEMORY, "element-major line offsets");
-    cudaError_t e = cudaMemcpy(d, off.data(), sizeof(int) * off.size(), cudaMemcpyHostToDevice);
-    if (e != cudaSuccess) return cuda_fail(e, "element-major line offsets");
-    plan->em_line_off = (const int*)d;
-    plan->em_nlines = acc;
-  }
   pi_plan::EmSplit& sp = plan->em_split[which];
   if (!sp.eplane) {
+    // one allocation and one wait for all of a coordinate system's tables: each costs a host call
     const int ne = dp.canon_plus ? TmCfg<true, 32, 64>::NE : TmCfg<false, 32, 64>::NE;
-    void* e_d = plan_alloc(plan, sizeof(float4) * (size_t)dp.dim * ne);
-    void* l_d = plan_alloc(plan, sizeof(float4) * (size_t)plan->em_nlines);
-    void* r_d = plan_alloc(plan, sizeof(float4) * (size_t)plan->em_nlines);
-    if (!e_d || !l_d || !r_d) return fail(PI_ERR_OUT_OF_MEMORY, "element-major coefficient planes");
-    dim3 grid(64, (unsigned)dp.nsectors);
-    k_em_split_planes<<<grid, 256, 0, plan->stream>>>(dp.sectors, dp.canon, which ? dp.coef32z : dp.coef32x,
-                                                      plan->em_line_off, ne, (float4*)e_d, (float4*)l_d, (float4*)r_d);
+    const int nf4 = dp.canon_plus ? kSepF4Plus : kSepF4;
+    const size_t entries = (size_t)dp.dim * ne, lines = (size_t)plan->nlines;
+    float4* ep = (float4*)plan_alloc(plan, sizeof(float4) * (entries + lines * (2 + 2 * nf4)));
+    if (!ep) return fail(PI_ERR_OUT_OF_MEMORY, "element-major coefficient planes");
+    float4 *lr = ep + entries, *rc = lr + lines, *sr = rc + lines, *sc = sr + lines * nf4;
+    const float2* coef = which ? dp.coef32z : dp.coef32x;
+    k_em_split_planes<<<dim3(64, (unsigned)dp.nsectors), 256, 0, plan->stream>>>(dp.sectors, dp.canon, coef,
+                                                                                 dp.line_off, ne, ep, lr, rc);
+    k_sep_planes<<<dim3(4, (unsigned)dp.nsectors), 128, 0, plan->stream>>>(dp.sectors, dp.canon, coef,
+                                                                           dp.line_off, nf4, sr, sc);
     cudaError_t e = cudaGetLastError();
     if (e == cudaSuccess) e = cudaStreamSynchronize(plan->stream);
     if (e != cudaSuccess) return cuda_fail(e, "element-major coefficient planes");
-    sp.eplane = (const float4*)e_d;
-    sp.lrow = (const float4*)l_d;
-    sp.rcol = (const float4*)r_d;
-  }
-  if (!sp.srow) {
-    const int nf4 = dp.canon_plus ? kSepF4Plus : kSepF4;
-    void* sr = plan_alloc(plan, sizeof(float4) * (size_t)plan->em_nlines * nf4);
-    void* sc = plan_alloc(plan, sizeof(float4) * (size_t)plan->em_nlines * nf4);
-    if (!sr || !sc) return fail(PI_ERR_OUT_OF_MEMORY, "separable line planes");
-    dim3 grid(4, (unsigned)dp.nsectors);
-    k_sep_planes<<<grid, 128, 0, plan->stream>>>(dp.sectors, dp.canon, which ? dp.coef32z : dp.coef32x,
-                                                 plan->em_line_off, nf4, (float4*)sr, (float4*)sc);
-    cudaError_t e = cudaGetLastError();
-    if (e == cudaSuccess) e = cudaStreamSynchronize(plan->stream);
-    if (e != cudaSuccess) return cuda_fail(e, "separable line planes");
-    sp.srow = (const float4*)sr;
-    sp.scol = (const float4*)sc;
+    sp.eplane = ep;
+    sp.lrow = lr;
+    sp.rcol = rc;
+    sp.srow = sr;
+    sp.scol = sc;
   }
   *out = sp;
   return PI_OK;
@@ -826,7 +806,7 @@ int em_split_planes(pi_plan* plan, int which, SplitPlanes* out) {
   out->eplane = sp.eplane;
   out->lrow = sp.lrow;
   out->rcol = sp.rcol;
-  out->line_off = plan->em_line_off;
+  out->line_off = plan->dev.line_off;
   out->plus = plan->dev.canon_plus ? 1 : 0;
   out->srow = sp.srow;
   out->scol = sp.scol;
@@ -1100,10 +1080,7 @@ extern "C" int pi_apply_f32_em(pi_plan* plan, float* y_dev, const float* x_dev, 
     return fail(PI_ERR_INVALID_ARGUMENT, "source and destination must not share storage");
   if ((unsigned long long)plan->host.dim * (unsigned long long)(ld / 2) >= (1ULL << 32))
     return fail(PI_ERR_UNSUPPORTED, "element-major batch larger than 2^32 16-byte rows; split the batch");
-  if (!plan->dev.canon)
-    return fail(PI_ERR_UNSUPPORTED,
-                "element-major batched apply needs a plan whose stencil sits at the canonical positions "
-                "(qubit models with real one-body operators)");
+  if (const int rc = em_check(plan)) return rc;
   cudaStream_t s = (cudaStream_t)stream;
   pi_plan::EmChoice ch{};
   bool known = false;

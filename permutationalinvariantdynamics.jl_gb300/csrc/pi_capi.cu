@@ -80,12 +80,18 @@ void* plan_alloc(pi_plan* plan, size_t bytes) {
 
 namespace {
 
+// Copies a table into the plan's own room; into `staged` first, while that has its place, for one copy
+// of all tables.
 template <typename T>
-int upload(pi_plan* plan, const std::vector<T>& host, const T** out) {
-  void* d = plan->own_room.take(host.size() * sizeof(T));
+int upload(pi_plan* plan, std::vector<char>& staged, const std::vector<T>& host, const T** out) {
+  const size_t bytes = host.size() * sizeof(T);
+  char* d = plan->own_room.take(bytes);
   if (!d) return fail(PI_ERR_OUT_OF_MEMORY, "device allocation of plan tables failed");
-  if (!host.empty()) {
-    cudaError_t e = cudaMemcpy(d, host.data(), host.size() * sizeof(T), cudaMemcpyHostToDevice);
+  const size_t at = d - plan->own_room.base;
+  if (at + bytes <= staged.size()) {
+    if (bytes) std::memcpy(staged.data() + at, host.data(), bytes);
+  } else if (bytes) {
+    cudaError_t e = cudaMemcpy(d, host.data(), bytes, cudaMemcpyHostToDevice);
     if (e != cudaSuccess) return cuda_fail(e, "plan upload");
   }
   *out = (const T*)d;
@@ -124,6 +130,8 @@ bool overlap(const void* a, size_t abytes, const void* b, size_t bbytes) {
 
 }  // namespace
 
+constexpr size_t kSpareRoom = 256 << 10;  // N <= 27 with a drive, decay and dephasing
+
 // Flattens the host plan into device tables (explicit_once transfer policy,
 // accelerators.jl:9-11: the plan is uploaded once; applies move no host data).
 int upload_plan(pi_plan* plan) {
@@ -134,7 +142,7 @@ int upload_plan(pi_plan* plan) {
   std::vector<double2> coef64, coef64z;
   std::vector<float2> coef32x, coef32z;
   std::vector<DevTile> tiles;
-  std::vector<int> diag_sector;
+  std::vector<int> diag_sector, line_off;
   std::vector<long long> diag_index;
   auto group_of = [](const StencilTerm& t) -> int {
     switch (t.kind) {
@@ -158,6 +166,7 @@ int upload_plan(pi_plan* plan) {
     ds.border_z = sec.f / hp.trace_norm2;
     ds.sqrt_f = sec.sqrt_f;
     ds.line0 = lines;
+    line_off.push_back(lines);
     ds.item0 = items;
     lines += sec.n;
     items += (int)(((long long)sec.n * sec.n + 31) / 32);
@@ -337,49 +346,61 @@ int upload_plan(pi_plan* plan) {
     return hp.sectors[x.sector].n > hp.sectors[y.sector].n;
   });
   if (coef64.size() > (size_t)0x7fffffff) return fail(PI_ERR_UNSUPPORTED, "coefficient pool too large");
-  // One allocation for all tables: a cudaMalloc takes about 35 us on the host once the driver's pages are
-  // used up, a cudaFree as much, and each of the 15 tables had its own.  compile() takes what it took
-  // with the planes' memory reserved beside (N = 8 427 us, 433 before; N = 120 27.6 ms, 28.0), closing
-  // a plan less (N = 8 164 -> 118 us, N = 120 339 -> 255).
+  plan->dev.nsectors = S;
+  plan->dev.dim = hp.dim;
+  plan->nlines = lines;
+  plan->nstrip_items = items;
+  // One allocation for all tables: a cudaMalloc takes about 35 us on the host once the driver's pages
+  // are used up, a cudaFree as much, and each of the 15 tables had its own.  With the planes' memory
+  // reserved beside, compile() takes 0.33 ms at N = 8 (0.42 with an allocation and a copy each), 27.8
+  // at N = 120 (28.0), and closing a plan less (N = 8 140 -> 110 us, N = 120 340 -> 260).
+  size_t tables = 0;
   {
     size_t bytes = 0;
     auto need = [&](size_t b) { bytes += TableRoom::padded(b); };
     auto table = [&](const auto& v) { need(v.size() * sizeof(v[0])); };
     table(sectors), table(terms), table(tiles), table(coef64), table(coef64z), table(coef32x), table(coef32z);
-    table(diag_sector), table(fterms), table(canon), table(diag_index);
+    table(diag_sector), table(fterms), table(canon), table(line_off), table(diag_index);
+    tables = bytes;
     need(sizeof(double2) * kReduceBlocks * kMaxDots), need(sizeof(double2) * kMaxDots);
     need(sizeof(double) * kReduceBlocks), need(sizeof(double) * 16);
-    plan->own_room.base = (char*)plan_alloc(plan, bytes);
+    // small plans: room for the first planes as well, not counted before it is reserved
+    const size_t planes = canon.empty() ? 0 : reserve_bytes(plan), spare = planes <= kSpareRoom ? planes : 0;
+    plan->own_room.base = (char*)plan_alloc(plan, bytes + spare);
     if (!plan->own_room.base) return fail(PI_ERR_OUT_OF_MEMORY, "device allocation of plan tables failed");
-    plan->own_room.size = bytes;
+    plan->own_room.size = bytes + spare;
+    plan->device_bytes -= spare;
   }
+  // Small tables go up in one copy (about 7 us each otherwise).
+  std::vector<char> staged(tables <= (1u << 20) ? tables : 0);
   int rc;
-  if ((rc = upload(plan, sectors, &plan->dev.sectors))) return rc;
-  if ((rc = upload(plan, terms, &plan->dev.terms))) return rc;
-  if ((rc = upload(plan, tiles, &plan->dev.tiles))) return rc;
-  if ((rc = upload(plan, coef64, &plan->dev.coef64))) return rc;
-  if ((rc = upload(plan, coef64z, &plan->dev.coef64z))) return rc;
-  if ((rc = upload(plan, coef32x, &plan->dev.coef32x))) return rc;
-  if ((rc = upload(plan, coef32z, &plan->dev.coef32z))) return rc;
-  if ((rc = upload(plan, diag_sector, &plan->dev.diag_sector))) return rc;
+  if ((rc = upload(plan, staged, sectors, &plan->dev.sectors))) return rc;
+  if ((rc = upload(plan, staged, terms, &plan->dev.terms))) return rc;
+  if ((rc = upload(plan, staged, tiles, &plan->dev.tiles))) return rc;
+  if ((rc = upload(plan, staged, coef64, &plan->dev.coef64))) return rc;
+  if ((rc = upload(plan, staged, coef64z, &plan->dev.coef64z))) return rc;
+  if ((rc = upload(plan, staged, coef32x, &plan->dev.coef32x))) return rc;
+  if ((rc = upload(plan, staged, coef32z, &plan->dev.coef32z))) return rc;
+  if ((rc = upload(plan, staged, diag_sector, &plan->dev.diag_sector))) return rc;
   if (fast_sr > 0) {
     const DevTerm* ft = nullptr;
-    if ((rc = upload(plan, fterms, &ft))) return rc;
+    if ((rc = upload(plan, staged, fterms, &ft))) return rc;
     plan->dev.fterms = reinterpret_cast<const int4*>(ft);
     plan->dev.fast_sr = fast_sr;
   }
   if (!canon.empty()) {
-    if ((rc = upload(plan, canon, &plan->dev.canon))) return rc;
+    if ((rc = upload(plan, staged, canon, &plan->dev.canon))) return rc;
+    if ((rc = upload(plan, staged, line_off, &plan->dev.line_off))) return rc;
     plan->dev.canon_plus = canon_plus;
     plan->dev.canon_terms = canon_terms;
   }
-  if ((rc = upload(plan, diag_index, &plan->dev.diag_index))) return rc;
-  plan->dev.nsectors = S;
+  if ((rc = upload(plan, staged, diag_index, &plan->dev.diag_index))) return rc;
+  if (!staged.empty()) {
+    cudaError_t e = cudaMemcpy(plan->own_room.base, staged.data(), plan->own_room.used, cudaMemcpyHostToDevice);
+    if (e != cudaSuccess) return cuda_fail(e, "plan upload");
+  }
   plan->dev.ntiles = (int)tiles.size();
   plan->dev.ndiag = (int)diag_index.size();
-  plan->dev.dim = hp.dim;
-  plan->nlines = lines;
-  plan->nstrip_items = items;
   plan->stencil_terms = (long long)terms.size();
   plan->rs.partial = (double2*)plan->own_room.take(sizeof(double2) * kReduceBlocks * kMaxDots);
   plan->rs.result = (double2*)plan->own_room.take(sizeof(double2) * kMaxDots);

@@ -79,7 +79,7 @@ struct pi_plan {
   };
   std::vector<EmMapSet> em_maps;
   // Split coefficient planes of the TMA-staged kernel (entry, row and column planes) per
-  // coordinate system, and the per-sector offsets of the row and column planes.
+  // coordinate system.
   struct EmSplit {
     const float4* eplane = nullptr;
     const float4* lrow = nullptr;
@@ -88,8 +88,6 @@ struct pi_plan {
     const float4* scol = nullptr;
   };
   EmSplit em_split[2];
-  const int* em_line_off = nullptr;
-  int em_nlines = 0;
   const void* em_tma_tiles[3][3] = {};  // tile records: 16 / 32 / 64 rows x 8 / 16 / 32 columns
   int em_tma_ntiles[3][3] = {};
   // Element-major kernel chosen by the autotuner (or pinned by the caller) per batch width
@@ -156,6 +154,7 @@ void* plan_alloc(pi_plan* plan, size_t bytes);
 // back when an allocation fails: reclaim_reserves() frees it on every listed plan and says whether
 // there was any.
 void reserve_planes(pi_plan* plan);
+size_t reserve_bytes(const pi_plan* plan);  // what that takes on a canonical plan
 void list_reserve(pi_plan* plan);
 bool reclaim_reserves();
 

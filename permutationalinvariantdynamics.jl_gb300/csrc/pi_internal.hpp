@@ -26,6 +26,7 @@ struct DevicePlan {
   const int4* canon = nullptr;      // canonical-position table (kCanonEntries per sector) or null
   int canon_plus = 0;                // some sandwich term sits at the +1 diagonal shift
   TermCounts canon_terms{};          // sandwich terms per position of the canonical table
+  const int* line_off = nullptr;     // per sector of a canonical plan: start of its rows and columns in line tables
   int nsectors = 0;
   int ntiles = 0;
   int ndiag = 0;

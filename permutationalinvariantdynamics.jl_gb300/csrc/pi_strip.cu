@@ -220,22 +220,31 @@ static int gain_positions(const pi_plan* plan, GainPos (&gain)[kMaxGains], bool*
   return nr;
 }
 
-// Room for the items and the first FP64 planes (or FP32 ones of both coordinate systems).  The
-// allocation is a small part of compile(), and most of a first apply that has to make it: 0.17 ms
-// of 0.34 at N = 200, where compile() takes 78.
-void reserve_planes(pi_plan* plan) {
-  const DevicePlan& dp = plan->dev;
-  if (!dp.canon || !has_items(dp) || plan->lazy_room.base || plan->strip_items) return;
+size_t reserve_bytes(const pi_plan* plan) {
+  if (!has_items(plan->dev)) return 0;
   GainPos gain[kMaxGains];
   bool drive;
   const int nr = gain_positions(plan, gain, &drive);
-  const size_t bytes =
-      TableRoom::padded(items_bytes(plan)) + TableRoom::padded(PlaneBytes<double>(plan, nr).all);
+  return TableRoom::padded(items_bytes(plan)) + TableRoom::padded(PlaneBytes<double>(plan, nr).all);
+}
+
+// Room for the items and the first FP64 planes (or FP32 ones of both coordinate systems).  The
+// allocation is a small part of compile(), and most of a first apply that has to make it: 0.17 ms
+// of 0.34 at N = 200, where compile() takes 78.  Small plans have the room at the end of their
+// tables' allocation.
+void reserve_planes(pi_plan* plan) {
+  const size_t bytes = plan->dev.canon ? reserve_bytes(plan) : 0;
+  if (bytes == 0 || plan->lazy_room.base || plan->strip_items) return;
   if ((double)plan->device_bytes + (double)bytes > plan->memory_budget) return;
-  plan->lazy_room.base = (char*)plan_alloc(plan, bytes);
-  if (!plan->lazy_room.base) return (void)cudaGetLastError();
-  plan->lazy_room.size = bytes;
-  list_reserve(plan);
+  if (char* p = plan->own_room.take(bytes)) {
+    plan->lazy_room = TableRoom{p, bytes, 0};
+    plan->device_bytes += bytes;
+  } else {
+    plan->lazy_room.base = (char*)plan_alloc(plan, bytes);
+    if (!plan->lazy_room.base) return (void)cudaGetLastError();
+    plan->lazy_room.size = bytes;
+    list_reserve(plan);
+  }
   for (TableFill* f : {&plan->planes64_fill[0], &plan->planes32_fill[0]})  // a first apply's only event
     if (cudaEventCreateWithFlags(&f->ready, cudaEventDisableTiming) != cudaSuccess) (void)cudaGetLastError();
 }
