@@ -683,6 +683,14 @@ static int em_check(const pi_plan* plan) {
               "(qubit models with real one-body operators)");
 }
 
+// A copy on the plan's fill stream, waited for.  em_mu is held, so nothing here may wait for other work:
+// not for the plan's own stream, and not for the default stream, as cudaMemcpy would.
+static cudaError_t em_copy(pi_plan* plan, void* dst, const void* src, size_t bytes, cudaMemcpyKind kind) {
+  const cudaError_t e = cudaMemcpyAsync(dst, src, bytes, kind, plan->fill_stream);
+  const cudaError_t f = cudaStreamSynchronize(plan->fill_stream);
+  return e != cudaSuccess ? e : f;
+}
+
 // Builds (once per plan) the element-major tile list.  Caller holds plan->em_mu.
 static int em_tiles(pi_plan* plan) {
   if (!plan->em_tiles) {
@@ -694,7 +702,7 @@ static int em_tiles(pi_plan* plan) {
     }
     void* d = plan_alloc(plan, sizeof(DevTile) * tiles.size());
     if (!d) return fail(PI_ERR_OUT_OF_MEMORY, "element-major tile list");
-    cudaError_t e = cudaMemcpy(d, tiles.data(), sizeof(DevTile) * tiles.size(), cudaMemcpyHostToDevice);
+    cudaError_t e = em_copy(plan, d, tiles.data(), sizeof(DevTile) * tiles.size(), cudaMemcpyHostToDevice);
     if (e != cudaSuccess) return cuda_fail(e, "element-major tile list");
     plan->em_tiles = (const DevTile*)d;
     plan->em_ntiles = (int)tiles.size();
@@ -715,10 +723,10 @@ static int em_prepare(pi_plan* plan, int which, const float2** planes_out) {
     void* d = plan_alloc(plan, sizeof(float2) * (size_t)dp.dim * np);
     if (!d) return fail(PI_ERR_OUT_OF_MEMORY, "element-major coefficient planes");
     dim3 grid(64, (unsigned)dp.nsectors);
-    k_em_planes<float><<<grid, 256, 0, plan->stream>>>(dp.sectors, dp.canon, which ? dp.coef32z : dp.coef32x, np,
+    k_em_planes<float><<<grid, 256, 0, plan->fill_stream>>>(dp.sectors, dp.canon, which ? dp.coef32z : dp.coef32x, np,
                                                        (float2*)d);
     cudaError_t e = cudaGetLastError();
-    if (e == cudaSuccess) e = cudaStreamSynchronize(plan->stream);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(plan->fill_stream);
     if (e != cudaSuccess) return cuda_fail(e, "element-major coefficient planes");
     plan->em_planes32[which] = (const float2*)d;
   }
@@ -733,7 +741,7 @@ static int em_tma_tiles(pi_plan* plan, int ri, int gi, const TmTile** tiles_out,
   const DevicePlan& dp = plan->dev;
   if (!plan->em_tma_tiles[ri][gi]) {
     std::vector<DevSector> secs(dp.nsectors);
-    cudaError_t e = cudaMemcpy(secs.data(), dp.sectors, sizeof(DevSector) * secs.size(), cudaMemcpyDeviceToHost);
+    cudaError_t e = em_copy(plan, secs.data(), dp.sectors, sizeof(DevSector) * secs.size(), cudaMemcpyDeviceToHost);
     if (e != cudaSuccess) return cuda_fail(e, "element-major tile list");
     std::vector<TmTile> tiles;
     int loff = 0;
@@ -756,7 +764,7 @@ static int em_tma_tiles(pi_plan* plan, int ri, int gi, const TmTile** tiles_out,
     }
     void* d = plan_alloc(plan, sizeof(TmTile) * tiles.size());
     if (!d) return fail(PI_ERR_OUT_OF_MEMORY, "element-major tile list");
-    e = cudaMemcpy(d, tiles.data(), sizeof(TmTile) * tiles.size(), cudaMemcpyHostToDevice);
+    e = em_copy(plan, d, tiles.data(), sizeof(TmTile) * tiles.size(), cudaMemcpyHostToDevice);
     if (e != cudaSuccess) return cuda_fail(e, "element-major tile list");
     plan->em_tma_tiles[ri][gi] = d;
     plan->em_tma_ntiles[ri][gi] = (int)tiles.size();
@@ -782,12 +790,12 @@ static int em_prepare_split(pi_plan* plan, int which, pi_plan::EmSplit* out) {
     if (!ep) return fail(PI_ERR_OUT_OF_MEMORY, "element-major coefficient planes");
     float4 *lr = ep + entries, *rc = lr + lines, *sr = rc + lines, *sc = sr + lines * nf4;
     const float2* coef = which ? dp.coef32z : dp.coef32x;
-    k_em_split_planes<<<dim3(64, (unsigned)dp.nsectors), 256, 0, plan->stream>>>(dp.sectors, dp.canon, coef,
+    k_em_split_planes<<<dim3(64, (unsigned)dp.nsectors), 256, 0, plan->fill_stream>>>(dp.sectors, dp.canon, coef,
                                                                                  dp.line_off, ne, ep, lr, rc);
-    k_sep_planes<<<dim3(4, (unsigned)dp.nsectors), 128, 0, plan->stream>>>(dp.sectors, dp.canon, coef,
+    k_sep_planes<<<dim3(4, (unsigned)dp.nsectors), 128, 0, plan->fill_stream>>>(dp.sectors, dp.canon, coef,
                                                                            dp.line_off, nf4, sr, sc);
     cudaError_t e = cudaGetLastError();
-    if (e == cudaSuccess) e = cudaStreamSynchronize(plan->stream);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(plan->fill_stream);
     if (e != cudaSuccess) return cuda_fail(e, "element-major coefficient planes");
     sp.eplane = ep;
     sp.lrow = lr;

@@ -80,3 +80,48 @@ def test_first_applies_of_several_streams(torch_cuda):
                 picuda.apply_(y, compiled, x)
         torch.cuda.synchronize()
         assert all(torch.equal(y, ref) for y in ys)
+
+
+def test_first_element_major_apply_does_not_wait_for_a_running_solve(torch_cuda):
+    """The element-major tables are filled beside the plan's own stream as well, and FP64 applies do not
+    queue behind their lock."""
+    torch = torch_cuda
+    model = M.ensemble_c2(120)
+    n = len(model.basis)
+    X = torch.randn((n, 16), dtype=torch.complex64, device="cuda")
+    Y, ref = torch.zeros_like(X), torch.zeros_like(X)
+    rho = torch.from_numpy(picuda.computational_product_state(model.basis, 2).data).cuda()
+    warm = picuda.compile(model)  # loads the kernels
+    picuda.select_element_major_kernel(warm, 16, "tma", 32)
+    picuda.apply_element_major_(ref, warm, X)
+    dest = torch.empty_like(rho)
+    picuda.evolve_(dest, warm, rho, (0.0, 1e-3), steps=8)
+    torch.cuda.synchronize()
+    compiled = picuda.compile(model)
+    picuda.select_element_major_kernel(compiled, 16, "tma", 32)
+    span, started = {}, threading.Event()
+
+    def solve():
+        torch.cuda.set_device(0)
+        with torch.cuda.stream(torch.cuda.Stream()):
+            started.set()
+            span["begin"] = time.perf_counter()
+            picuda.evolve_(dest, compiled, rho, (0.0, 2.5), steps=16000)
+            span["end"] = time.perf_counter()
+
+    t = threading.Thread(target=solve)
+    t.start()
+    started.wait()
+    time.sleep(0.1)
+    with torch.cuda.stream(torch.cuda.Stream()):
+        t0 = time.perf_counter()
+        picuda.apply_element_major_(Y, compiled, X)
+        torch.cuda.current_stream().synchronize()
+        took = time.perf_counter() - t0
+        began_inside = "end" not in span
+    t.join()
+    torch.cuda.synchronize()
+    total = span["end"] - span["begin"]
+    assert began_inside and total > 0.3
+    assert took < 0.15 * total, (took, total)
+    assert torch.equal(Y, ref)
